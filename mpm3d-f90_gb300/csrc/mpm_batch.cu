@@ -4,8 +4,9 @@
 // A batch holds the scenes of one composition laid out back to back in device
 // memory. Changing the composition (mpm_batch_commit) builds a new layout:
 // resident scenes are moved on the device by a relocation kernel, new scenes
-// are uploaded, retired scenes are dropped. Every step sorts the particles of
-// all scenes by (scene, cell) and runs one launch per kernel for the batch.
+// are uploaded, retired scenes are dropped. A step runs one launch per kernel
+// for the batch; scenes whose particle order has become stale are re-sorted
+// by (scene, key) on the way.
 #include <cuda_runtime.h>
 
 
@@ -192,30 +193,28 @@ struct mpm_batch {
   bool inv_stale = false;  // steps ran since the inverse permutation was last built
   long long bytes = 0;
   int* d_target = nullptr;
-  // second stream: the energy / DT reduction of a step runs there while the
-  // next step's keys are sorted (the two touch disjoint arrays)
+  // second stream: the energy / DT reduction of a step runs there beside the
+  // next step's mass transfer (the two write disjoint arrays)
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int any_sgmp = 0, any_nonsgmp = 0, any_usf = 0, any_later = 0, any_musl = 0, any_jc = 0, any_dr = 0, any_uvfp = 0;
   int any_nonuvfp = 0;
   int any_prep = 0;  // scenes whose force input is not staged by their stress kernel (USL / MUSL, Johnson-Cook)
   unsigned stress_types = 0;  // stress instantiations to launch: bit MT per specialised type, bit 0 for the rest
-  cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // one step, per buffer parity and
-                                                                      // without / with the previous step's reduction
-  const double* set0_x = nullptr;                   // identifies particle buffer set 0
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step without / with the previous step's reduction
   int pblock = 256, nblock = 256;
   int scatter_blocks = 9728;  // scatter grid cap (64 blocks per SM; warps stride over the occupied cells)
-  int sort_blocks = 152;      // grid of the long-segment sort (one block per SM)
+  int sort_blocks = 152;      // grid cap of the re-sort (co-resident blocks, at most three per SM)
   int sms = 152;              // multiprocessors of the device
   int loop_min_steps = 0;     // steps a device loop takes before it honours an interrupt
   long long ntask = 0;        // particle tasks of the linear / GIMP / B-spline scenes (32 particles each)
   // device-resident run loop (mpm_batch_run_loop): its state, the host's
   // request flag (page-locked, mapped into the device's address space) and
-  // one loop graph per buffer parity
+  // the loop graph
   LoopCtl* ctl = nullptr;
   volatile int* loop_flag_h = nullptr;
   int* loop_flag_d = nullptr;
-  cudaGraphExec_t loop_graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t loop_graph = nullptr;
   Profiler prof;
   // particle value gather (curve output)
   GatherItem *g_items_h = nullptr, *g_items_d = nullptr;
@@ -349,7 +348,7 @@ long long scene_keys(const Geometry& g) { return (g.shape == 1 ? (long long)g.nn
 
 inline unsigned gridn(long long n, int blk) { return (unsigned)((n + blk - 1) / blk); }
 
-// inclusive scan in three passes over tiles (mpm_sort.cuh); tiles holds
+// inclusive scan in passes over tiles (mpm_sort.cuh); tiles holds
 // scan_tiles(src.n) values of the source's type
 template <class S>
 void scan_tiles_enqueue(const S& src, typename S::T* tiles, cudaStream_t st) {
@@ -364,66 +363,62 @@ void scan_tiles_enqueue(const S& src, typename S::T* tiles, cudaStream_t st) {
   }
 }
 
-// one step of every live scene (MPM3D.f90:69-118 for each scene)
-// The step in three parts. The front (sort keys, sort, per-key counts,
-// occupied keys) reads the positions and scene ids only; the back (begin,
-// permutation, transfers, stress, position) does the rest; the reduction
-// (calcEnergy, UpdateDT, damping) reads the final velocities, masses and
-// energies. The front does not depend on the begin kernel (which advances
-// the step count and time), so it runs first.
-int enqueue_front(mpm_batch* b) {
-  cudaStream_t st = b->stream;
-  BState& a = b->A;
-  const int pb = b->pblock;
-  prof_begin(K_LOCATE, st);
-  cudaMemsetAsync(a.seg, 0, sizeof(int) * (size_t)(a.NK + 1), st);
-  kb_keys<<<gridn(a.NP, pb), pb, 0, st>>>(a);
-  prof_end(K_LOCATE, st);
-  // counting sort by key (mpm_sort.cuh): segment ends and the occupied
-  // keys, placement, then the stable order inside each segment
-  prof_begin(K_SORT, st);
-  scan_tiles_enqueue(SegScan{a.seg, a.fill, a.NK}, a.tiles, st);  // (zeroes the fill counters; kb_keys the long-segment count)
-  ks_place<<<gridn(a.NP, 256), 256, 0, st>>>(a.key, a.seg, a.fill, a.perm, a.NP);
-  ks_segments<<<gridn(a.NK, 256), 256, 0, st>>>(a.seg, a.NK, a.perm, a.big, a.nbig);
-  ks_long_segments<<<b->sort_blocks, kSegThreads, 0, st>>>(a.seg, a.perm, a.big, a.nbig);
-  prof_end(K_SORT, st);
+// the re-sort of the scenes marked by the mass finalize: one cooperative
+// launch of at most three blocks per SM
+int enqueue_resort(mpm_batch* b) {
+  prof_begin(K_SORT, b->stream);
+  const long long want = gridn(std::max(b->A.NP, b->A.NK), kSortThreads);
+  const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(want, b->sort_blocks));
+  void* args[] = {&b->A, &b->B};
+  BCK(cudaLaunchCooperativeKernel((const void*)kb_resort, dim3(grid), dim3(kSortThreads), args, 0, b->stream));
+  prof_end(K_SORT, b->stream);
   return MPM_OK;
 }
 
-int enqueue_back(mpm_batch* b) {
-  cudaStream_t st = b->stream;
-  BState& a = b->A;
-  const int pb = b->pblock, nb = b->nblock;
-  prof_begin(K_BEGIN, st);
-  kb_begin<<<gridn(a.nscene, 128), 128, 0, st>>>(a, b->d_target);
-  prof_end(K_BEGIN, st);
-  prof_begin(K_PERMUTE, st);
-  kb_permute<<<gridn(a.NP, pb), pb, 0, st>>>(a, b->B);
-  prof_end(K_PERMUTE, st);
-  // swap the particle buffer sets (node and scene arrays are shared)
-  std::swap(b->A, b->B);
-  BState& s = b->A;
+// one step of every live scene (MPM3D.f90:69-118 for each scene) in two
+// parts. The first part (begin, mass and momentum transfer) reads positions
+// and the FP32 velocities and masses, none of which the previous step's
+// reduction (calcEnergy, UpdateDT) writes; the second needs that reduction's
+// DT.
+void enqueue_scatter(mpm_batch* b, int mode) {
+  constexpr int w0 = PartShape<0>::WARPS, w1 = PartShape<1>::WARPS, w2 = PartShape<2>::WARPS;
   auto pgrid = [&](int warps) {
     return (unsigned)std::max<long long>(1, std::min<long long>(b->scatter_blocks, (b->ntask + warps - 1) / warps));
   };
   // particle -> grid transfers: particle tasks of every scene
-  auto scatter = [&](int mode) {
-    constexpr int w0 = PartShape<0>::WARPS, w1 = PartShape<1>::WARPS, w2 = PartShape<2>::WARPS;
-    if (mode == 0) kb_part_scatter<0><<<pgrid(w0), 32 * w0, 0, st>>>(s);
-    else if (mode == 1) kb_part_scatter<1><<<pgrid(w1), 32 * w1, 0, st>>>(s);
-    else kb_part_scatter<2><<<pgrid(w2), 32 * w2, 0, st>>>(s);
-  };
+  cudaStream_t st = b->stream;
+  if (mode == 0) kb_part_scatter<0><<<pgrid(w0), 32 * w0, 0, st>>>(b->A);
+  else if (mode == 1) kb_part_scatter<1><<<pgrid(w1), 32 * w1, 0, st>>>(b->A);
+  else kb_part_scatter<2><<<pgrid(w2), 32 * w2, 0, st>>>(b->A);
+}
+
+int enqueue_front(mpm_batch* b) {
+  cudaStream_t st = b->stream;
+  BState& s = b->A;
+  const int nb = b->nblock;
+  prof_begin(K_BEGIN, st);
+  kb_begin<<<gridn(s.nscene, 128), 128, 0, st>>>(s, b->d_target);
+  prof_end(K_BEGIN, st);
   if (b->any_sgmp) {
     prof_begin(K_SG_CLEAR, st);
     kb_sg_clear<<<gridn(s.NC, nb), nb, 0, st>>>(s);
     prof_end(K_SG_CLEAR, st);
   }
   prof_begin(K_SCATTER_MASS, st);
-  scatter(0);
+  enqueue_scatter(b, 0);
   prof_end(K_SCATTER_MASS, st);
+  return MPM_OK;
+}
+
+int enqueue_back(mpm_batch* b) {
+  cudaStream_t st = b->stream;
+  BState& s = b->A;
+  const int pb = b->pblock, nb = b->nblock;
   prof_begin(K_P2G_MASS, st);
-  kb_p2g_mass<<<gridn(s.NN, nb), nb, 0, st>>>(s, 1, 1);
+  kb_p2g_mass<<<gridn(s.NN, nb) + 1, nb, 0, st>>>(s, 1, 1, b->d_target);  // (its last block starts the step)
   prof_end(K_P2G_MASS, st);
+  int r = enqueue_resort(b);
+  if (r) return r;
   auto stress = [&](int usf_pass) -> int {
     if (b->any_sgmp) {
       prof_begin(K_SG_GRADIENT, st);
@@ -461,7 +456,6 @@ int enqueue_back(mpm_batch* b) {
     }
     return MPM_OK;
   };
-  int r;
   if (b->any_usf && (r = stress(1))) return r;
   if (b->any_prep) {  // (USF scenes without Johnson-Cook tails are staged by their stress kernel)
     prof_begin(K_FORCE_PREP, st);
@@ -469,7 +463,7 @@ int enqueue_back(mpm_batch* b) {
     prof_end(K_FORCE_PREP, st);
   }
   prof_begin(K_SCATTER_FORCE, st);
-  scatter(2);
+  enqueue_scatter(b, 2);
   prof_end(K_SCATTER_FORCE, st);
   prof_begin(K_P2G_FORCE, st);
   kb_p2g_force<<<gridn(s.NN, nb), nb, 0, st>>>(s);
@@ -484,7 +478,7 @@ int enqueue_back(mpm_batch* b) {
   prof_end(K_POSITION, st);
   if (b->any_musl) {
     prof_begin(K_SCATTER_MOM, st);
-    scatter(1);
+    enqueue_scatter(b, 1);
     prof_end(K_SCATTER_MOM, st);
     prof_begin(K_P2G_MOM, st);
     kb_p2g_momentum<<<gridn(s.NN, nb), nb, 0, st>>>(s);
@@ -521,19 +515,22 @@ int enqueue_step(mpm_batch* b) {
   return r;
 }
 
-// one step whose front overlaps the previous step's reduction (lead), which
-// then runs on the side stream; without lead the step ends before its own
-// reduction, which the caller enqueues (the next step's lead, or the tail of
-// a run)
+// one step whose first part overlaps the previous step's reduction (lead),
+// which then runs on the side stream (in order before it where a scene has
+// dynamic relaxation, whose damping changes the velocities); without lead the
+// step ends before its own reduction, which the caller enqueues (the next
+// step's lead, or the tail of a run)
 int enqueue_step_overlapped(mpm_batch* b, bool lead) {
-  if (lead) {
+  const bool fork = lead && !b->any_dr;
+  if (fork) {
     BCK(cudaEventRecord(b->ev_fork, b->stream));
     BCK(cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-    if (int r = enqueue_reduce(b, b->side)) return r;
-    BCK(cudaEventRecord(b->ev_join, b->side));
   }
+  if (lead)
+    if (int r = enqueue_reduce(b, fork ? b->side : b->stream)) return r;
+  if (fork) BCK(cudaEventRecord(b->ev_join, b->side));
   int r = enqueue_front(b);
-  if (lead) BCK(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
+  if (fork) BCK(cudaStreamWaitEvent(b->stream, b->ev_join, 0));
   if (!r) r = enqueue_back(b);
   if (!r) {
     cudaError_t e = cudaGetLastError();
@@ -543,20 +540,16 @@ int enqueue_step_overlapped(mpm_batch* b, bool lead) {
 }
 
 void drop_graph(mpm_batch* b) {
-  for (auto& gp : b->graph)
-    for (auto& g : gp) {
-      if (g) cudaGraphExecDestroy(g);
-      g = nullptr;
-    }
-  for (auto& g : b->loop_graph) {
+  for (auto& g : b->graph) {
     if (g) cudaGraphExecDestroy(g);
     g = nullptr;
   }
+  if (b->loop_graph) cudaGraphExecDestroy(b->loop_graph);
+  b->loop_graph = nullptr;
 }
 
-// capture nsteps steps into an executable graph; the host-side buffer handles
-// end swapped nsteps times, as after running the steps eagerly. lead < 0:
-// whole steps in order; otherwise one overlapped step (with or without the
+// capture nsteps steps into an executable graph. lead < 0: whole steps in
+// order; otherwise one overlapped step (with or without the
 // previous step's reduction)
 int capture(mpm_batch* b, int nsteps, cudaGraphExec_t* out, int lead = -1) {
   cudaGraph_t g;
@@ -591,7 +584,8 @@ __device__ __forceinline__ void loop_decide(const BState& b, const int* target, 
   pending = __syncthreads_or(pending);
   if (threadIdx.x == 0) {
     const LoopCtl& c = *b.ctl;
-    const bool go = pending && c.finished == c.fin0 && (*flag == 0 || c.iters < c.min_iters) && c.iters < c.max_iters;
+    const bool go = pending && c.finished == c.fin0 && (*flag == 0 || c.iters < c.min_iters) && c.iters < c.max_iters &&
+                    b.gbar[1] == 0u;
     cudaGraphSetConditional(h, go ? 1u : 0u);
   }
 }
@@ -614,11 +608,9 @@ __global__ void kb_loop_test(BState b, const int* target, const volatile int* fl
   loop_decide(b, target, flag, h);
 }
 
-// The loop graph of the current buffer parity: a test kernel, then a WHILE
-// node whose body is two overlapped steps (each with the previous step's
-// reduction beside its sort) and the test again. Two steps per iteration
-// bring the particle buffer sets back to the parity the graph was built
-// for.
+// The loop graph: a test kernel, then a WHILE node whose body is two
+// overlapped steps (each with the previous step's reduction beside its mass
+// transfer) and the test again.
 int build_loop(mpm_batch* b, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   BCK(cudaGraphCreate(&g, 0));
@@ -665,18 +657,15 @@ int build_loop(mpm_batch* b, cudaGraphExec_t* out) {
   return r;
 }
 
-// one step replayed from the graph of the current buffer parity (captured on
-// first use); lead: with the previous step's reduction beside the sort
+// one step replayed from its graph (captured on first use); lead: with the
+// previous step's reduction beside the mass transfer
 int replay_step(mpm_batch* b, int lead) {
-  const int par = b->A.x == b->set0_x ? 0 : 1;
-  if (!b->graph[par][lead]) {
+  if (!b->graph[lead]) {
     cudaGraphExec_t ge = nullptr;
     if (int r = capture(b, 1, &ge, lead)) return r;
-    b->graph[par][lead] = ge;
-    std::swap(b->A, b->B);  // capture swapped the host handles; the launch below does the step
+    b->graph[lead] = ge;
   }
-  BCK(cudaGraphLaunch(b->graph[par][lead], b->stream));
-  std::swap(b->A, b->B);
+  BCK(cudaGraphLaunch(b->graph[lead], b->stream));
   return MPM_OK;
 }
 
@@ -697,7 +686,6 @@ int commit(mpm_batch* b) {
     b->bytes = 0;
     b->A = BState{};
     b->B = BState{};
-    b->set0_x = nullptr;
     b->dirty = false;
     return MPM_OK;
   }
@@ -809,6 +797,12 @@ int commit(mpm_batch* b) {
   shared.rscene = al.get<uint16_t>(NR);
   shared.scenes = al.get<Scene>((long long)b->order.size());
   shared.task0 = al.get<int>((long long)b->order.size() + 1);
+  shared.disorder = al.get<int>((long long)b->order.size());
+  shared.resort = al.get<int>((long long)b->order.size());
+  shared.shift = al.get<int>((long long)b->order.size());
+  shared.ract = al.get<int>((long long)b->order.size());
+  shared.any_resort = al.get<int>(1);
+  shared.gbar = al.get<unsigned>(2);
   shared.sst = al.get<SceneState>((long long)b->order.size());
   shared.mats = al.get<DevMaterial>(nmat);
   shared.fmats = al.get<DevMaterialF>(nmat);
@@ -850,7 +844,8 @@ int commit(mpm_batch* b) {
     s.cw = shared.cw; s.cdefp = shared.cdefp; s.cvx = shared.cvx; s.cax = shared.cax; s.cscene = shared.cscene;
     s.setter = shared.setter; s.setter_scan = shared.setter_scan; s.dep = shared.dep; s.jc_aux = shared.jc_aux;
     s.deferred = shared.deferred; s.red_part = shared.red_part; s.rscene = shared.rscene; s.scenes = shared.scenes;
-    s.task0 = shared.task0;
+    s.task0 = shared.task0; s.disorder = shared.disorder; s.resort = shared.resort; s.shift = shared.shift;
+    s.ract = shared.ract; s.any_resort = shared.any_resort; s.gbar = shared.gbar;
     s.sst = shared.sst; s.mats = shared.mats; s.fmats = shared.fmats; s.bodies = shared.bodies;
   };
   share(A);
@@ -884,6 +879,7 @@ int commit(mpm_batch* b) {
   std::vector<uint8_t> fix((size_t)NN), bd((size_t)NN);
   std::vector<int> target;
   std::vector<SceneState> sst;
+  std::vector<int> ract;
   std::vector<int> task0;  // first particle task of each scene (32 particles)
   long long ntask = 0;
   for (HostScene* h : b->order) {
@@ -940,8 +936,9 @@ int commit(mpm_batch* b) {
     }
     s0.fdt = (float)s0.dt;
     s0.ftime = (float)s0.time;
-    s0.active = h->resident ? 0 : 1;  // the initial energy pass below runs for new scenes only
+    s0.active = h->resident ? 0 : 1;  // the initial bounds and energy pass below run for new scenes only
     sst.push_back(s0);
+    ract.push_back(s0.active);
   }
   task0.push_back((int)ntask);
   b->ntask = ntask;
@@ -959,6 +956,9 @@ int commit(mpm_batch* b) {
   BCK(cudaMemcpyAsync(shared.rscene, rscene.data(), 2 * NR, cudaMemcpyHostToDevice, st));
   BCK(cudaMemcpyAsync(d_target, target.data(), sizeof(int) * target.size(), cudaMemcpyHostToDevice, st));
   BCK(cudaMemcpyAsync(shared.sst, sst.data(), sizeof(SceneState) * sst.size(), cudaMemcpyHostToDevice, st));
+  BCK(cudaMemsetAsync(shared.any_resort, 0, sizeof(int), st));
+  BCK(cudaMemsetAsync(shared.gbar, 0, 2 * sizeof(unsigned), st));
+  BCK(cudaMemcpyAsync(shared.ract, ract.data(), sizeof(int) * ract.size(), cudaMemcpyHostToDevice, st));
   BCK(cudaMemsetAsync(shared.mg, 0, sizeof(double) * NN, st));
   BCK(cudaMemsetAsync(shared.px, 0, sizeof(double) * 3 * NN, st));
   BCK(cudaMemsetAsync(shared.fx, 0, sizeof(double) * 3 * NN, st));
@@ -981,6 +981,7 @@ int commit(mpm_batch* b) {
   // download or probe after later steps)
   kb_inverse<<<gridn(NP, 256), 256, 0, st>>>(A);
   b->inv_stale = false;
+  kb_init_f32<<<gridn(NP, 256), 256, 0, st>>>(A, -1, 1);
   // calcEnergy of the new scenes (MPM3D.f90:42)
   kb_reduce_chunks<<<(unsigned)NR, 256, 0, st>>>(A, 1);
   BCK(cudaGetLastError());
@@ -993,7 +994,6 @@ int commit(mpm_batch* b) {
   A.ctl = B.ctl = b->ctl;
   b->A = A;
   b->B = B;
-  b->set0_x = A.x;
   b->d_target = d_target;
   for (HostScene* h : b->order) {
     if (!h->resident) h->release_inputs();  // the scene's inputs are on the device now
@@ -1030,8 +1030,10 @@ int mpm_batch_create(int device, mpm_batch** out) {
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) == cudaSuccess && sms > 0)
   {
     b->scatter_blocks = 64 * sms;
-    b->sort_blocks = sms;
     b->sms = sms;
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_resort, kSortThreads, 0) != cudaSuccess) per = 1;
+    b->sort_blocks = sms * std::max(1, std::min(per, 3));
   }
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1136,8 +1138,8 @@ int mpm_batch_run(mpm_batch* b, int nsteps, int use_graph) {
   b->inv_stale = true;
   BProfScope ps(b);
   if (!use_graph) {
-    // each step's reduction overlaps the next step's sort; the last one ends
-    // the run, so nothing is pending between calls
+    // each step's reduction overlaps the next step's mass transfer; the last
+    // one ends the run, so nothing is pending between calls
     for (int i = 0; i < nsteps; ++i)
       if ((r = enqueue_step_overlapped(b, i > 0))) return r;
     return enqueue_reduce(b, b->stream);
@@ -1154,10 +1156,9 @@ int mpm_batch_run(mpm_batch* b, int nsteps, int use_graph) {
     if (e != cudaSuccess) return berr(b, MPM_ERR_CUDA, "graph launch: %s", cudaGetErrorString(e));
     return MPM_OK;
   }
-  // one graph of one step per buffer parity (the step swaps the two particle
-  // buffer sets, so the graph captured from either set is replayed
-  // alternately), the steps after the first of the run with the previous
-  // step's reduction overlapping their sort; the run's last reduction ends it
+  // one graph of one step, the steps after the first of the run with the
+  // previous step's reduction overlapping their mass transfer; the run's last
+  // reduction ends it
   for (int i = 0; i < nsteps; ++i)
     if ((r = replay_step(b, i > 0 ? 1 : 0))) return r;
   return enqueue_reduce(b, b->stream);
@@ -1176,13 +1177,12 @@ int mpm_batch_run_loop(mpm_batch* b, int max_steps, int* steps) {
   // loop's iterations of two steps, then the last step's reduction
   kb_loop_arm<<<1, 1, 0, b->stream>>>(b->ctl, (max_steps - 1) / 2, b->loop_min_steps / 2);
   if ((r = replay_step(b, 0))) return r;
-  const int par = b->A.x == b->set0_x ? 0 : 1;
-  if (!b->loop_graph[par]) {
+  if (!b->loop_graph) {
     cudaGraphExec_t ge = nullptr;
     if ((r = build_loop(b, &ge))) return r;
-    b->loop_graph[par] = ge;
+    b->loop_graph = ge;
   }
-  BCK(cudaGraphLaunch(b->loop_graph[par], b->stream));
+  BCK(cudaGraphLaunch(b->loop_graph, b->stream));
   if ((r = enqueue_reduce(b, b->stream))) return r;
   LoopCtl c{};
   BCK(cudaMemcpyAsync(&c, b->ctl, sizeof c, cudaMemcpyDeviceToHost, b->stream));
@@ -1204,6 +1204,8 @@ int mpm_batch_sync(mpm_batch* b) {
   if (b->A.nscene == 0) return MPM_OK;
   std::vector<SceneState> s((size_t)b->A.nscene);
   BCK(cudaMemcpy(s.data(), b->A.sst, sizeof(SceneState) * s.size(), cudaMemcpyDeviceToHost));
+  for (auto& x : s)
+    if (x.status & ST_STALLED) return berr(b, MPM_ERR_TIMEOUT, "a re-sort's grid barrier ran out of time");
   for (auto& x : s)
     if (x.status & ST_NONFINITE) return berr(b, MPM_ERR_NONFINITE, "non-finite particle state");
   return MPM_OK;
@@ -1435,7 +1437,14 @@ int mpm_batch_scene_restore(mpm_batch* b, int id, const unsigned char* in, size_
   // positions and their copy agree at the end of every step
   for (int a = 0; a < 3; ++a)
     BCK(cudaMemcpy(s.xx + a * NP + p0, s.x + a * NP + p0, sizeof(double) * np, cudaMemcpyDeviceToDevice));
+  // (images of USF scenes written before the momentum bound was carried from
+  // step to step have none)
+  const bool bounds = st.qmax[Q_MOM_MUSL] == 0u;
+  if (bounds) st.active = 1;
   BCK(cudaMemcpy(s.sst + h->index, &st, sizeof st, cudaMemcpyHostToDevice));
+  kb_init_f32<<<gridn(NP, 256), 256, 0, b->stream>>>(s, h->index, bounds ? 1 : 0);
+  BCK(cudaGetLastError());
+  BCK(cudaStreamSynchronize(b->stream));
   h->st = st;
   b->inv_stale = true;
   return MPM_OK;
@@ -1651,6 +1660,7 @@ int batch_progress(mpm_batch* b, std::vector<BatchProgress>& out) {
   BCK(cudaMemcpy(s.data(), b->A.sst, sizeof(SceneState) * s.size(), cudaMemcpyDeviceToHost));
   for (HostScene* h : b->order) {
     const SceneState& t = s[h->index];
+    if (t.status & ST_STALLED) return berr(b, MPM_ERR_TIMEOUT, "a re-sort's grid barrier ran out of time");
     out.push_back(BatchProgress{h->id, t.istep, h->steps, h->np, t.status});
   }
   return MPM_OK;

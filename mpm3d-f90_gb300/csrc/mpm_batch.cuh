@@ -2,13 +2,14 @@
 // advanced together by one set of kernels indexed by per-scene offset tables.
 //
 // Layout (all scenes concatenated; scene s owns the ranges in its Scene entry):
-//   particles, kept physically sorted by (scene, cell) at the start of every
-//   step (stable sort of the previous order, then a permutation of every
-//   field), component-major over the total particle count NP:
+//   particles, kept physically sorted by (scene, key) -- near enough: a scene
+//   is re-sorted (stable sort, then a permutation of every field) on its first
+//   step and whenever its mass transfer meets too many particles out of order
+//   (step_tick) -- component-major over the total particle count NP:
 //     FP64: x[3], xx[3], v[3], fxp[3], mass, ie
 //     FP32: vol, evol (V / V0 - 1), sig_y, sm, seqv, sd[6], fp[9], epeff, celsius,
 //     dmg, lt, cp, q
-//     per step (written by the permutation): cell (scene-local cell, -1
+//     per step (written by the mass transfer): cell (scene-local cell, -1
 //     outside), off[3] (offset in the cell, in cells), SGMP dual cell, nearest
 //     node, xxn[3], xn[3]; body, scene, orig (scene-local input index)
 //   grid nodes concatenated: FP64 mg, px[3], fx[3]; FP32 float4 velocity and
@@ -89,22 +90,28 @@ struct BState {
   long long NP, NN, NK, NC, NR;
   int nscene;
   int any_uvfp, any_sgmp, any_jc;
-  // particles (A = current, B = permutation target)
+  // particles (A = the working set, B = the re-sort's permutation target)
   double *x, *xx, *v, *fxp, *mass, *ie;
   float *vol, *evol, *sig_y, *sm, *seqv, *sd, *fp, *epeff, *celsius, *dmg, *lt, *cp, *q;
   uint8_t* failure;
   uint16_t *body, *scene;
   int* orig;
   int* inv;  // position of a particle by scene p0 + deck index (rebuilt before downloads and probes)
-  // per-step derived (written by the permutation)
+  // per-step derived (written by the mass transfer; by the permutation for a re-sorted scene)
   int *cell, *dual, *inode;
   float *off, *xxn, *xn;
   float* fs;  // force staging [9][NP]: sigma*vol (xx, yy, zz, xy, yz, xz), fext (3)
-  float *m32, *v32;  // FP32 mass and velocity [3][NP] for the momentum transfers (permutation; position update)
+  float *m32, *v32;  // FP32 mass and velocity [3][NP] for the momentum transfers (kept by the position update)
   // sort (mpm_sort.cuh)
   unsigned* key;
   int *perm, *seg;
   int *fill, *tiles, *big, *nbig;  // per-key slots taken, scan tile totals, long segments
+  // re-sort control, per scene: particles out of order (counted by the mass
+  // transfer), re-sorted this step, number of a re-sorted scene's particle i =
+  // i - shift; ract: the scene takes the step whose reduction runs next
+  int *disorder, *resort, *shift, *ract;
+  int* any_resort;  // some scene is re-sorted this step
+  unsigned* gbar;   // grid barrier of the re-sort: arrivals, a wait that ran out (stays set)
   LoopCtl* ctl;  // run-loop state (one per batch, outside the layout arena)
   int* task0;  // first particle task (32 sorted particles) of each scene, nscene + 1 entries; SGMP scenes have none
   // grid

@@ -4,6 +4,7 @@
 
 #include "mpm_batch.cuh"
 #include "mpm_kernels.cuh"
+#include "mpm_sort.cuh"
 
 namespace mpm {
 namespace bm {
@@ -64,20 +65,31 @@ __device__ __forceinline__ void bsp1(int t, float off, float& w, float& d) {
 }
 
 
+// per-scene bound slots of the transfers (SceneState::qmax, float bits):
+// mass (set when a scene is laid out), momentum of the step's first transfer,
+// force, and momentum with the updated velocities (the MUSL transfer's bound
+// and the next step's Q_MOM)
+enum QSlot { Q_MASS = 0, Q_MOM = 1, Q_FORCE = 2, Q_MOM_MUSL = 3 };
+
 // ------------------------------------------------------------- begin step
+// A step starts in two kernels. kb_begin (which scenes take the step, the
+// transfers' bounds and counters) touches nothing that the previous step's
+// energy / DT reduction reads or writes, so the two may run side by side;
+// step_tick (step count, time, the re-sort decision) needs the reduction's DT
+// and the mass transfer's count of particles out of order, and runs as the
+// last block of the mass finalize.
 __global__ void kb_begin(BState b, const int* target) {
   int s = (int)btid();
+  if (s == 0) b.gbar[0] = 0u;  // the re-sort's barrier
   if (s >= b.nscene) return;
   SceneState& t = b.sst[s];
   t.active = t.istep < target[s] ? 1 : 0;
+  b.disorder[s] = 0;
   if (!t.active) return;
-  t.istep = t.istep + 1;
-  if (t.istep == target[s]) atomicAdd(&b.ctl->finished, 1);  // the scene's last step
-  t.time = t.time + t.dt;
-  t.ftime = (float)t.time;
-  t.ie = 0.0;
   t.active_nodes = 0;
-  for (int k = 0; k < 4; ++k) t.qmax[k] = 0u;
+  // the momentum bound taken with the last step's final velocities
+  t.qmax[Q_MOM] = t.qmax[Q_MOM_MUSL];
+  t.qmax[Q_FORCE] = t.qmax[Q_MOM_MUSL] = 0u;
 }
 
 // ---------------------------------------------- FP64 <-> FP32 off the FP64 pipe
@@ -247,80 +259,115 @@ __device__ __forceinline__ bool sg_locate_df(const Scene& sc, const double x[3],
   return true;
 }
 
-// ------------------------------------------------------------------ keys
-// Sort key of a particle: its scene's key base plus its cell (linear,
-// B-spline), its nearest node (GIMP) or its dual cell (SGMP); the scene's
-// last key collects the particles outside the grid. Sorting keeps the
-// particles of a key contiguous, which the transfers rely on for locality
-// (and the SGMP centre gathers for their particle ranges). A GIMP particle
-// reaches the nodes within 1.25 cells of it (the cpGIMP quarter rule of
-// FindInflNode), i.e. at most one node either side of its nearest node in
-// each direction: binned by nearest node, a key's particles reach a 3 x 3 x
-// 3 box of nodes instead of the 4 x 4 x 4 box of a cell's particles.
-__global__ void kb_keys(BState b) {
-  const long long i = btid();
-  if (i == 0) *b.nbig = 0;  // long-segment count of this step's sort
-  unsigned key = 0xffffffffu;
-  if (i < b.NP) {
-    const long long NP = b.NP;
-    const Scene& sc = b.scenes[b.scene[i]];
-    double x[3] = {b.x[i], b.x[NP + i], b.x[2 * NP + i]};
-    long long c = -1;
-    if (sc.shape == 3) {
-      int cc[3], nd[3];
-      float off[3];
-      if (!sg_locate_df(sc, x, cc, off, nd, c)) c = dual_cell(sc, x);
-    } else {
-      // The coordinate in cells is formed in FP32 from the positions
-      // truncated to FP32 by integer operations (GB300's FP64 pipe is
-      // narrow), so it can put a particle within a few FP32 roundings of
-      // the coordinate (about 1e-7 of it) on the other side of a face. The
-      // sort only groups particles: the transfers take every particle's cell
-      // and offsets from the permutation's exact routine (cell_of), so a
-      // particle that this rounding puts on the other side of a cell face
-      // (or of the grid's edge) is still transferred exactly, in a segment
-      // of its own.
-      int cc[3];
-      float u[3];
-      bool in = true;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        u[a] = (f32_trunc(x[a]) - sc.fspan0[a]) * sc.fidcell;
-        in = in && u[a] >= 0.f;
-        cc[a] = (int)u[a];
-      }
-      if (in && cc[0] < sc.NCx && cc[1] < sc.NCy && cc[2] < sc.NCz) {
-        if (sc.shape == 1) {  // nearest node: the cell's lower node, or the upper one from half a cell on
-#pragma unroll
-          for (int a = 0; a < 3; ++a) cc[a] += u[a] - (float)cc[a] >= 0.5f;
-          c = ((long long)cc[2] * sc.NGy + cc[1]) * sc.NGx + cc[0];
-        } else {
-          c = ((long long)cc[2] * sc.NCy + cc[1]) * sc.NCx + cc[0];
-        }
-      }
+// -------------------------------------------------------------- locate
+// The step's derived data of a particle at position x (ParticleInitial,
+// update_step.f90:408-453, in FP32 form): cell (-1 off the grid) and offset in
+// it; for SGMP also the dual cell, the nearest node and the coordinates about
+// both. cc, off and dual return what the transfers need.
+__device__ __forceinline__ bool locate_one(const BState& b, const Scene& sc, long long i, const double x[3], int cc[3],
+                                           float off[3], long long& dual) {
+  const long long NP = b.NP;
+  int nd[3];
+  dual = -1;
+  bool in;
+  if (sc.shape != 3) {
+    in = cell_of_df(sc, x, cc, off);
+  } else if (sg_locate_df(sc, x, cc, off, nd, dual)) {
+    in = true;
+  } else {
+    in = cell_of(sc, x, cc, off);
+    for (int a = 0; a < 3; ++a) {
+      const double u = (x[a] - sc.span0[a]) * sc.idcell;  // (as in cell_of)
+      nd[a] = cc[a] + (u - (double)cc[a] >= 0.5);
     }
-    key = (unsigned)(sc.k0 + (c >= 0 ? c : sc.nk - 1));
-    b.key[i] = key;
+    dual = dual_cell(sc, x);
   }
-  // per-key counts: the particles arrive sorted by the last step's keys, so
-  // a warp's lanes mostly share a few keys -- one atomic per key and warp
-  const unsigned grp = __match_any_sync(0xffffffffu, key);
-  if (key != 0xffffffffu && (threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&b.seg[key], __popc(grp));
+  for (int a = 0; a < 3; ++a) b.off[a * NP + i] = off[a];
+  b.cell[i] = in ? (cc[2] * sc.NCy + cc[1]) * sc.NCx + cc[0] : -1;
+  if (sc.shape == 3) {
+    // dual (cell-centre) grid: CenterInWhichCell (as the sort keys) and the
+    // nearest node with the particle's coordinates about it, both decided
+    // as in FP64 (sg_locate_df or the FP64 routines above: the node must
+    // stay the one above the dual cell, deciding on the FP32 offset would
+    // move particles within 3e-8 of the half onto the other node);
+    // XXN = 2 off - 2 (upper node) or 2 off in FP32
+    b.dual[i] = (int)dual;
+    bool nin = nd[0] >= 0 && nd[0] < sc.NGx && nd[1] >= 0 && nd[1] < sc.NGy && nd[2] >= 0 && nd[2] < sc.NGz;
+    int ln = nin ? (nd[2] * sc.NGy + nd[1]) * sc.NGx + nd[0] : -1;
+    b.inode[i] = ln;
+    int bd = ln >= 0 ? b.bd[sc.n0 + ln] : 0;
+    for (int a = 0; a < 3; ++a) {
+      float xxn = off[a] * 2.f - (nd[a] > cc[a] ? 2.f : 0.f);
+      if ((bd >> (2 * a)) & 3) xxn = xxn > 0.f ? 1.f : (xxn < 0.f ? -1.f : 0.f);
+      b.xxn[a * NP + i] = xxn;
+      b.xn[a * NP + i] = off[a] * 2.f - 1.f;
+    }
+  }
+  return in;
+}
+
+// sort key of a particle from its cell (linear, B-spline), its nearest node
+// (GIMP, the upper one from half a cell on) or its dual cell (SGMP), relative
+// to its scene's keys; -1 off the grid. A GIMP particle reaches the nodes
+// within 1.25 cells of it (the cpGIMP quarter rule of FindInflNode), i.e. at
+// most one node either side of its nearest node in each direction: binned by
+// nearest node, a key's particles reach a 3 x 3 x 3 box of nodes instead of
+// the 4 x 4 x 4 box of a cell's particles. The scatters' segments are runs of
+// equal keys of the same definition.
+__device__ __forceinline__ int gimp_key(const Scene& sc, int c[3], const float off[3]) {
+  for (int a = 0; a < 3; ++a) c[a] += off[a] >= 0.5f;
+  return (c[2] * sc.NGy + c[1]) * sc.NGx + c[0];
+}
+
+// ------------------------------------------------------------------ keys
+// Sort keys and per-key counts of the scenes that are re-sorted this step
+// (BState::resort), from the step's derived data; the scene's last key
+// collects the particles outside the grid. Scenes that keep their order get
+// no key and no count.
+__device__ __forceinline__ void sort_keys(BState& b) {
+  const long long NP = b.NP;
+  for (long long b0 = (long long)blockIdx.x * kSortThreads; b0 < NP; b0 += (long long)gridDim.x * kSortThreads) {
+    const long long i = b0 + threadIdx.x;
+    unsigned key = kNoKey;
+    if (i < NP) {
+      const int s = b.scene[i];
+      if (b.resort[s]) {
+        const Scene& sc = b.scenes[s];
+        int k = sc.shape == 3 ? b.dual[i] : b.cell[i];
+        if (sc.shape == 1 && k >= 0) {
+          int c[3];
+          c[2] = div_by(k, sc.mNCxy);
+          const int rem = k - c[2] * sc.NCxy;
+          c[1] = div_by(rem, sc.mNCx);
+          c[0] = rem - c[1] * sc.NCx;
+          const float off[3] = {b.off[i], b.off[NP + i], b.off[2 * NP + i]};
+          k = gimp_key(sc, c, off);
+        }
+        key = (unsigned)(sc.k0 + (k >= 0 ? k : sc.nk - 1));
+      }
+      b.key[i] = key;
+    }
+    // per-key counts: neighbours mostly share a key -- one atomic per key and
+    // warp
+    const unsigned grp = __match_any_sync(0xffffffffu, key);
+    if (key != kNoKey && (threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&b.seg[key], __popc(grp));
+  }
 }
 
 // ---------------------------------------------------- permutation + derived
-// dst[i] = src[perm[i]] for every persistent particle field, then the per-step
-// derived data of the particle at its new position (ParticleInitial,
-// update_step.f90:408-453, in FP32 form).
-// returns the particle's scene; mass and velocity for the transfer bounds
-__device__ __forceinline__ int permute_one(const BState& src, BState& dst, long long i, double& m_out,
-                                           double (&v_out)[3]) {
+// dst[i] = src[perm[i]] for every persistent particle field of the scenes
+// being re-sorted, then the step's derived data of the particle at its new
+// place; permute_back returns the fields to the set every other kernel
+// uses. The sort numbers the re-sorted scenes' particles without gaps, a
+// scene's particle i being number i - shift[scene].
+__device__ __forceinline__ void permute_one(const BState& src, BState& dst, long long i) {
+  const int s = src.scene[i];  // (a scene's particles stay in its range)
+  if (!src.resort[s]) return;
   // every value is loaded before the first store: the stores could alias the
   // loads as far as the compiler knows, so interleaving them would serialise
   // one memory round trip per field
   const long long NP = src.NP;
-  const long long j = src.perm[i];
-  const int s = src.scene[j];
+  const long long j = src.perm[i - src.shift[s]];
   const Scene& sc = src.scenes[s];
   // (the external forces move only in scenes that have some: elsewhere
   // they are zero and nothing reads them)
@@ -365,50 +412,65 @@ __device__ __forceinline__ int permute_one(const BState& src, BState& dst, long 
   dst.q[i] = q;
   dst.failure[i] = failure;
   dst.body[i] = body;
-  dst.scene[i] = (uint16_t)s;
   dst.orig[i] = orig;
   // derived
   int cc[3];
   float off[3];
-  int nd[3];
-  long long dualc = -1;
-  bool in;
-  if (sc.shape != 3) {
-    in = cell_of_df(sc, x, cc, off);
-  } else if (sg_locate_df(sc, x, cc, off, nd, dualc)) {
-    in = true;
-  } else {
-    in = cell_of(sc, x, cc, off);
-    for (int a = 0; a < 3; ++a) {
-      const double u = (x[a] - sc.span0[a]) * sc.idcell;  // (as in cell_of)
-      nd[a] = cc[a] + (u - (double)cc[a] >= 0.5);
-    }
-    dualc = dual_cell(sc, x);
+  long long dual;
+  locate_one(dst, sc, i, x, cc, off, dual);
+  dst.m32[i] = f32_rn(mass);
+  for (int a = 0; a < 3; ++a) dst.v32[a * NP + i] = f32_rn(v[a]);
+}
+
+// the re-sorted scenes' fields from the permutation's target set back to the
+// working set (a straight copy)
+__device__ __forceinline__ void permute_back(const BState& src, BState& dst, long long i) {
+  const long long NP = src.NP;
+  const int s = dst.scene[i];
+  if (!src.resort[s]) return;
+  const Scene& sc = src.scenes[s];
+  double x[3], v[3], f[3] = {0.0, 0.0, 0.0};
+  for (int a = 0; a < 3; ++a) {
+    x[a] = src.x[a * NP + i];
+    v[a] = src.v[a * NP + i];
+    if (sc.has_fxp) f[a] = src.fxp[a * NP + i];
   }
-  for (int a = 0; a < 3; ++a) dst.off[a * NP + i] = off[a];
-  dst.cell[i] = in ? (cc[2] * sc.NCy + cc[1]) * sc.NCx + cc[0] : -1;
-  if (sc.shape == 3) {
-    // dual (cell-centre) grid: CenterInWhichCell (as the sort keys) and the
-    // nearest node with the particle's coordinates about it, both decided
-    // as in FP64 (sg_locate_df or the FP64 routines above: the node must
-    // stay the one above the dual cell, deciding on the FP32 offset would
-    // move particles within 3e-8 of the half onto the other node);
-    // XXN = 2 off - 2 (upper node) or 2 off in FP32
-    dst.dual[i] = (int)dualc;
-    bool nin = nd[0] >= 0 && nd[0] < sc.NGx && nd[1] >= 0 && nd[1] < sc.NGy && nd[2] >= 0 && nd[2] < sc.NGz;
-    int ln = nin ? (nd[2] * sc.NGy + nd[1]) * sc.NGx + nd[0] : -1;
-    dst.inode[i] = ln;
-    int bd = ln >= 0 ? src.bd[sc.n0 + ln] : 0;
-    for (int a = 0; a < 3; ++a) {
-      float xxn = off[a] * 2.f - (nd[a] > cc[a] ? 2.f : 0.f);
-      if ((bd >> (2 * a)) & 3) xxn = xxn > 0.f ? 1.f : (xxn < 0.f ? -1.f : 0.f);
-      dst.xxn[a * NP + i] = xxn;
-      dst.xn[a * NP + i] = off[a] * 2.f - 1.f;
-    }
+  const double mass = src.mass[i], ie = src.ie[i];
+  const float vol = src.vol[i], evol = src.evol[i], sig_y = src.sig_y[i], sm = src.sm[i], seqv = src.seqv[i];
+  float sd[6];
+  for (int a = 0; a < 6; ++a) sd[a] = src.sd[a * NP + i];
+  const float epeff = src.epeff[i], celsius = src.celsius[i], dmg = src.dmg[i], lt = src.lt[i], cp = src.cp[i],
+              q = src.q[i];
+  const uint8_t failure = src.failure[i];
+  const uint16_t body = src.body[i];
+  const int orig = src.orig[i];
+  for (int a = 0; a < 3; ++a) {
+    dst.x[a * NP + i] = x[a];
+    dst.v[a * NP + i] = v[a];
+    if (sc.has_fxp) dst.fxp[a * NP + i] = f[a];
   }
-  m_out = mass;
-  for (int a = 0; a < 3; ++a) v_out[a] = v[a];
-  return s;
+  dst.mass[i] = mass;
+  dst.ie[i] = ie;
+  dst.vol[i] = vol;
+  dst.evol[i] = evol;
+  dst.sig_y[i] = sig_y;
+  dst.sm[i] = sm;
+  dst.seqv[i] = seqv;
+  for (int a = 0; a < 6; ++a) dst.sd[a * NP + i] = sd[a];
+  dst.epeff[i] = epeff;
+  dst.celsius[i] = celsius;
+  dst.dmg[i] = dmg;
+  dst.lt[i] = lt;
+  dst.cp[i] = cp;
+  dst.q[i] = q;
+  dst.failure[i] = failure;
+  dst.body[i] = body;
+  dst.orig[i] = orig;
+  if (src.any_uvfp) {
+    float fp[18];
+    for (int a = 0; a < 18; ++a) fp[a] = src.fp[a * NP + i];
+    for (int a = 0; a < 18; ++a) dst.fp[a * NP + i] = fp[a];
+  }
 }
 
 // ------------------------------------------- deterministic P2G scatter
@@ -426,9 +488,6 @@ __device__ __forceinline__ int permute_one(const BState& src, BState& dst, long 
 // is far below its FP32 rounding.
 // The bounds are taken by the kernels that run before each transfer
 // (permutation, force staging, position update).
-
-// per-scene bound slots (SceneState::qmax, float bits, reset every step)
-enum QSlot { Q_MASS = 0, Q_MOM = 1, Q_FORCE = 2, Q_MOM_MUSL = 3 };
 
 // Max of non-negative values v[k] over the block into sst[s].qmax[slot[k]],
 // per scene s (s < 0: no value). Every thread of the block must call it.
@@ -521,28 +580,60 @@ __device__ __forceinline__ int dim_nodes(int shape, float off, int& t0, float w[
   return 2 + (off < 0.25f) + (off > 0.75f);
 }
 
-// permutation kernel; it also takes the mass and momentum bounds of the
-// step's first particle -> node transfer
-__global__ void kb_permute(BState src, BState dst) {
-  const long long i = btid();
+// The re-sort of the scenes marked by step_tick, in one cooperative launch:
+// counting sort by key (mpm_sort.cuh), then every field permuted into the
+// second particle set and back. A step in which no scene is re-sorted -- most
+// of them -- pays one launch that returns at once: 1.6 us of the step, against
+// 10 us for an IF node around the phases as kernels of their own and 16 to 34
+// us for those kernels returning one by one (5.8 k to 1.2 M particles). The
+// barriers between the phases cost a re-sort about what launches would.
+__global__ void __launch_bounds__(kSortThreads, 3) kb_resort(BState a, BState o) {
+  if (!*a.any_resort) return;
+  __shared__ int sm[kSmemSeg];  // (the scan's tile, then the long segments)
+  __shared__ int thr[kSortThreads], wsum[32];
+  const long long g0 = (long long)blockIdx.x * kSortThreads + threadIdx.x, gs = (long long)gridDim.x * kSortThreads;
+  unsigned round = 0;
+  for (long long k = g0; k < a.NK; k += gs) a.seg[k] = 0;
+  if (g0 == 0) *a.nbig = 0;
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_keys(a);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_tile_totals(a.seg, a.NK, a.tiles, thr, wsum);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_tile_prefix(a.NK, a.tiles, thr, wsum);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_tile_scan(a.seg, a.fill, a.NK, a.tiles, sm, thr, wsum);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_place(a.key, a.seg, a.fill, a.perm, a.NP);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_segments(a.seg, a.NK, a.perm, a.big, a.nbig);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  sort_long(a.seg, a.perm, a.big, a.nbig, sm);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  for (long long i = g0; i < a.NP; i += gs) permute_one(a, o, i);
+  if (!grid_barrier(a.gbar, ++round)) return;
+  for (long long i = g0; i < a.NP; i += gs) permute_back(o, a, i);
+}
+
+// FP32 mass and velocity of the particles of a scene (-1: of every scene),
+// when a layout is new or a scene's state was restored (from then on the
+// position update keeps the velocity); bounds: also the mass and momentum
+// bounds of the first step, for the scenes marked active (new ones -- the
+// others carry the bounds of their last step)
+__global__ void kb_init_f32(BState b, int scene, int bounds) {
+  const long long i = btid(), NP = b.NP;
   int s = -1;
   float bm = 0.f, bv = 0.f;
-  if (i < src.NP) {
-    double m, v[3];
-    s = permute_one(src, dst, i, m, v);
-    // FP32 mass and velocity for the first transfer (the conversions run
-    // once per particle here, not in every transfer lane)
-    const float m32 = f32_rn(m), v32[3] = {f32_rn(v[0]), f32_rn(v[1]), f32_rn(v[2])};
-    dst.m32[i] = m32;
-    for (int a = 0; a < 3; ++a) dst.v32[a * dst.NP + i] = v32[a];
-    if (scene_live(dst, s)) {
-      bm = m32;
-      bv = bm * fmaxf(fabsf(v32[0]), fmaxf(fabsf(v32[1]), fabsf(v32[2]))) * 1.0001f;
-    } else {
-      s = -1;
-    }
+  if (i < NP && (scene < 0 || b.scene[i] == scene)) {
+    s = b.scene[i];
+    bm = f32_rn(b.mass[i]);
+    const float v[3] = {f32_rn(b.v[i]), f32_rn(b.v[NP + i]), f32_rn(b.v[2 * NP + i])};
+    b.m32[i] = bm;
+    for (int a = 0; a < 3; ++a) b.v32[a * NP + i] = v[a];
+    bv = bm * fmaxf(fabsf(v[0]), fmaxf(fabsf(v[1]), fabsf(v[2]))) * 1.0001f;
+    if (!bounds || !scene_live(b, s)) s = -1;
   }
-  block_scene_max<2>(dst, s, {Q_MASS, Q_MOM}, {bm, bv});
+  block_scene_max<2>(b, s, {Q_MASS, Q_MOM_MUSL}, {bm, bv});
 }
 
 // Corner k of the dual cell (dx, dy, dz) as a scene cell (its centre node),
@@ -606,37 +697,53 @@ __device__ __forceinline__ void part_tab(float off, float idc, float (&w)[3], fl
   }
 }
 
+// The mass transfer (mode 0) opens the step: it locates the particles and
+// stores the step's derived data, and returns how many of the task's
+// particles come after one with a larger key (0 otherwise).
+__device__ __forceinline__ int count_disorder(int key, int cnt) {
+  const int lane = threadIdx.x & 31;
+  const unsigned prev = (unsigned)__shfl_up_sync(0xffffffffu, key, 1);
+  return __popc(__ballot_sync(0xffffffffu, lane > 0 && lane < cnt && prev > (unsigned)key));
+}
+
 template <int MODE, int SH>
-__device__ __forceinline__ void part_scatter_task(BState& b, const Scene& sc, long long i0, int cnt, float sA,
-                                                  float sB, float* ws) {
+__device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, long long i0, int cnt, float sA,
+                                                 float sB, float* ws) {
   using PS = PartShape<MODE>;
   constexpr int NV = PS::NV, NX = PS::NX, NK = PS::NK, ST = PS::STRIDE;
   constexpr int nt = SH == 0 ? 2 : 3, tlo = SH == 0 ? 0 : -1, NS = nt * nt * nt;
   const int lane = threadIdx.x & 31;
   const long long NP = b.NP, i = i0 + lane;
-  const int cl = lane < cnt ? b.cell[i] : -1;
   int c[3] = {0, 0, 0};
   float off[3] = {0.f, 0.f, 0.f};
   int key = -1;
-  if (cl >= 0) {
-    c[2] = div_by(cl, sc.mNCxy);
-    const int rem = cl - c[2] * sc.NCxy;
-    c[1] = div_by(rem, sc.mNCx);
-    c[0] = rem - c[1] * sc.NCx;
+  if (MODE == 0) {
+    if (lane < cnt) {
+      const double x[3] = {b.x[i], b.x[NP + i], b.x[2 * NP + i]};
+      const bool in = cell_of_df(sc, x, c, off);
+      const int cl = (c[2] * sc.NCy + c[1]) * sc.NCx + c[0];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) off[a] = b.off[a * NP + i];
-    if (SH == 1) {
+      for (int a = 0; a < 3; ++a) b.off[a * NP + i] = off[a];
+      b.cell[i] = in ? cl : -1;
+      if (in) key = SH == 1 ? gimp_key(sc, c, off) : cl;
+    }
+  } else {
+    const int cl = lane < cnt ? b.cell[i] : -1;
+    if (cl >= 0) {
+      c[2] = div_by(cl, sc.mNCxy);
+      const int rem = cl - c[2] * sc.NCxy;
+      c[1] = div_by(rem, sc.mNCx);
+      c[0] = rem - c[1] * sc.NCx;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) c[a] += off[a] >= 0.5f;
-      key = (c[2] * sc.NGy + c[1]) * sc.NGx + c[0];
-    } else {
-      key = cl;
+      for (int a = 0; a < 3; ++a) off[a] = b.off[a * NP + i];
+      key = SH == 1 ? gimp_key(sc, c, off) : cl;
     }
   }
+  const int dis = MODE == 0 ? count_disorder(key, cnt) : 0;
   // segment ends: the last lane of every run of equal keys
   const int knext = __shfl_down_sync(0xffffffffu, key, 1);
   const unsigned lasts = __ballot_sync(0xffffffffu, key >= 0 && (lane == 31 || knext != key));
-  if (lasts == 0u) return;  // (uniform) nothing of this task on the grid
+  if (lasts == 0u) return dis;  // (uniform) nothing of this task on the grid
   // the segment's first box node (scene-local flat index) and whether the
   // whole box lies inside the grid
   const int nbase = ((c[2] + tlo) * sc.NGy + (c[1] + tlo)) * sc.NGx + (c[0] + tlo);
@@ -743,6 +850,7 @@ __device__ __forceinline__ void part_scatter_task(BState& b, const Scene& sc, lo
     }
   }
   __syncwarp();
+  return dis;
 }
 
 // The SGMP form of a particle task: the key is the particle's dual cell,
@@ -756,16 +864,29 @@ __device__ __forceinline__ void part_scatter_task(BState& b, const Scene& sc, lo
 // force (Cfext, Cfint); a lane takes the corner lane / 4 (mode 0) or lane / 3
 // (modes 1, 2: one channel, or three force channels g, g + 3, g + 6).
 template <int MODE>
-__device__ __forceinline__ void sg_part_task(BState& b, const Scene& sc, long long i0, int cnt, float sA, float sB,
+__device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long long i0, int cnt, float sA, float sB,
                                              float* ws) {
   constexpr int ST = PartShape<MODE>::STRIDE;
   constexpr int CH0 = MODE == 2 ? CQ_FE : (MODE == 1 ? CQ_P : CQ_M);  // first accumulator channel
   const int lane = threadIdx.x & 31;
   const long long NP = b.NP, i = i0 + lane;
-  const int d = lane < cnt ? b.dual[i] : -1;
+  int d = -1;
+  if (lane < cnt) {
+    if (MODE == 0) {
+      const double x[3] = {b.x[i], b.x[NP + i], b.x[2 * NP + i]};
+      int cc[3];
+      float off[3];
+      long long dual;
+      locate_one(b, sc, i, x, cc, off, dual);
+      d = (int)dual;
+    } else {
+      d = b.dual[i];
+    }
+  }
+  const int dis = MODE == 0 ? count_disorder(d, cnt) : 0;
   const int knext = __shfl_down_sync(0xffffffffu, d, 1);
   const unsigned lasts = __ballot_sync(0xffffffffu, d >= 0 && (lane == 31 || knext != d));
-  if (lasts == 0u) return;  // (uniform) nothing of this task on the dual grid
+  if (lasts == 0u) return dis;  // (uniform) nothing of this task on the dual grid
   // phase 1: rows 0..7 the corner weights (times the mass for modes 0, 1),
   // then the values (velocity, or the 9 force inputs)
   {
@@ -834,6 +955,7 @@ __device__ __forceinline__ void sg_part_task(BState& b, const Scene& sc, long lo
     }
   }
   __syncwarp();
+  return dis;
 }
 
 template <int MODE>
@@ -842,6 +964,7 @@ __global__ void __launch_bounds__(32 * PartShape<MODE>::WARPS, MODE == 2 ? 6 : 4
   __shared__ float wsp[PS::WARPS][PS::ROWS * PS::STRIDE];
   const int warp = threadIdx.x >> 5;
   const int nt = b.task0[b.nscene];
+  int ds = -1, dis = 0;  // scene of the warp's last task, its particles out of order so far
   for (int t = blockIdx.x * PS::WARPS + warp; t < nt; t += gridDim.x * PS::WARPS) {
     // the scene of the task: the last scene whose first task is at or before t
     int lo = 0, hi = b.nscene - 1;
@@ -859,13 +982,19 @@ __global__ void __launch_bounds__(32 * PartShape<MODE>::WARPS, MODE == 2 ? 6 : 4
     const float sA = q_scale(q_shift(sc, st.qmax[MODE == 0 ? Q_MASS : (MODE == 1 ? Q_MOM_MUSL : Q_FORCE)]));
     const float sB = MODE == 0 ? q_scale(q_shift(sc, st.qmax[Q_MOM])) : sA;
     float* ws = wsp[warp];
+    if (MODE == 0 && s != ds) {
+      if (dis && (threadIdx.x & 31) == 0) atomicAdd(&b.disorder[ds], dis);
+      ds = s;
+      dis = 0;
+    }
     switch (sc.shape) {
-      case 0: part_scatter_task<MODE, 0>(b, sc, sc.p0 + first, cnt, sA, sB, ws); break;
-      case 1: part_scatter_task<MODE, 1>(b, sc, sc.p0 + first, cnt, sA, sB, ws); break;
-      case 2: part_scatter_task<MODE, 2>(b, sc, sc.p0 + first, cnt, sA, sB, ws); break;
-      default: sg_part_task<MODE>(b, sc, sc.p0 + first, cnt, sA, sB, ws);
+      case 0: dis += part_scatter_task<MODE, 0>(b, sc, sc.p0 + first, cnt, sA, sB, ws); break;
+      case 1: dis += part_scatter_task<MODE, 1>(b, sc, sc.p0 + first, cnt, sA, sB, ws); break;
+      case 2: dis += part_scatter_task<MODE, 2>(b, sc, sc.p0 + first, cnt, sA, sB, ws); break;
+      default: dis += sg_part_task<MODE>(b, sc, sc.p0 + first, cnt, sA, sB, ws);
     }
   }
+  if (MODE == 0 && dis && (threadIdx.x & 31) == 0) atomicAdd(&b.disorder[ds], dis);
 }
 
 // Accumulated channels 0..nv-1 of node n in FP64 (the accumulators cleared
@@ -917,7 +1046,53 @@ __device__ __forceinline__ void node_finish(BState& b, const Scene& sc, long lon
   }
 }
 
-__global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf) {
+// Step count and time of the scenes taking the step, and which of them are
+// re-sorted before the step goes on: a scene on its first step, and one whose
+// mass transfer met more than kDisorder out-of-order particles per task of
+// 32. Every particle out of order splits a run of equal keys in two (one more
+// flush of a node box per transfer), so the order is renewed once that costs
+// about as much as a sort does; results depend on the order only through FP32
+// partial sums, and the decision only on the scene's own particles and order.
+// Also numbers the re-sorted scenes' particles for the sort (shift). One
+// block.
+constexpr float kDisorder = 0.5f;
+
+__device__ __forceinline__ void step_tick(BState& b, const int* target) {
+  __shared__ long long thr[512], wsum[32];
+  long long carry = 0;
+  int any = 0;
+  for (int s0 = 0; s0 < b.nscene; s0 += blockDim.x) {
+    const int s = s0 + threadIdx.x;
+    long long np = 0;
+    int rs = 0;
+    if (s < b.nscene) {
+      SceneState& t = b.sst[s];
+      b.ract[s] = t.active;
+      if (t.active) {
+        t.istep = t.istep + 1;
+        if (t.istep == target[s]) atomicAdd(&b.ctl->finished, 1);  // the scene's last step
+        t.time = t.time + t.dt;
+        t.ftime = (float)t.time;
+        const long long n = b.scenes[s].np;
+        rs = t.istep == 1 || (float)b.disorder[s] > kDisorder * (float)((n + 31) / 32);
+        if (rs) np = n;
+      }
+      b.resort[s] = rs;
+    }
+    const long long before = block_scan<long long, ScanSum>(np, thr, wsum);
+    const long long total = thr[blockDim.x - 1];
+    if (rs) b.shift[s] = b.scenes[s].p0 - (carry + before);
+    carry += total;
+    any = __syncthreads_or(any || rs);
+  }
+  if (threadIdx.x == 0) *b.any_resort = any;
+}
+
+__global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target) {
+  if (blockIdx.x == gridDim.x - 1) {  // the last block starts the step instead of finishing nodes
+    step_tick(b, target);
+    return;
+  }
   long long n = btid();
   bool act = false;
   int s = -1;
@@ -1630,11 +1805,10 @@ __device__ __forceinline__ float position_one(BState& b, long long i) {
     const double vn = st.istep == 1 ? vv + f64_of(acc[a]) * dt * 0.5 : vv + f64_of(acc[a]) * dt;
     b.v[a * NP + i] = vn;
     pv[a] = f32_rn(vn);
-    b.v32[a * NP + i] = pv[a];  // for GridMomentumMUSL's transfer
+    b.v32[a * NP + i] = pv[a];  // for the momentum transfers of this step (MUSL) and the next
     if (sc.usf) b.x[a * NP + i] = xx;
   }
-  if (!sc.musl) return -1.f;
-  // bound of GridMomentumMUSL's contributions with the updated velocity
+  // bound of those transfers' contributions
   const float m = b.m32[i];
   return m * fmaxf(fabsf(pv[0]), fmaxf(fabsf(pv[1]), fabsf(pv[2]))) * 1.0001f;
 }
@@ -1726,6 +1900,7 @@ __device__ __forceinline__ void reduce_scene_finish(BState& b, int s, int mode, 
   }
   if (threadIdx.x != 0) return;
   SceneState& st = b.sst[s];
+  if (b.gbar[1]) st.status |= (unsigned)ST_STALLED;  // a re-sort gave up
   if (mode & 1) {
     st.ke_prev = st.ke;
     st.ke = sh[0][0];
@@ -1761,7 +1936,7 @@ __global__ void __launch_bounds__(256) kb_reduce_chunks(BState b, int mode) {
   __shared__ int last;
   const long long r = blockIdx.x;
   const int s = b.rscene[r];
-  if (!scene_live(b, s)) return;  // (uniform: every block of the scene returns)
+  if (!b.ract[s]) return;  // (uniform: every block of the scene returns)
   const Scene& sc = b.scenes[s];
   const long long NP = b.NP;
   double acc[6] = {0, 0, 0, 0, 0, 0};
@@ -1801,19 +1976,20 @@ __global__ void kb_dr_damping(BState b) {
   if (i >= b.NP) return;
   const int s = b.scene[i];
   const Scene& sc = b.scenes[s];
-  if (!sc.drdamp || !scene_live(b, s)) return;
+  if (!sc.drdamp || !b.ract[s]) return;
   const SceneState& st = b.sst[s];
   if (!(st.ke - st.ke_prev <= 0.0)) return;
   const long long NP = b.NP;
-  b.v[i] = 0;
-  b.v[NP + i] = 0;
-  b.v[2 * NP + i] = 0;
+  for (int a = 0; a < 3; ++a) {
+    b.v[a * NP + i] = 0;
+    b.v32[a * NP + i] = 0.f;
+  }
 }
 
 __global__ void kb_dr_finish(BState b) {
   int s = (int)btid();
   if (s >= b.nscene) return;
-  if (!b.scenes[s].drdamp || !scene_live(b, s)) return;
+  if (!b.scenes[s].drdamp || !b.ract[s]) return;
   SceneState& st = b.sst[s];
   if (st.ke - st.ke_prev <= 0.0) st.ke = 0;
 }

@@ -1,10 +1,11 @@
-// mpm_sort.cuh -- the batched engine's per-step counting sort of particles by
-// sort key, and the tile scans it uses.
+// mpm_sort.cuh -- the batched engine's counting sort of particles by sort
+// key, and the tile scans it uses. It runs on the scenes whose order has
+// become stale (step_tick); the others have no key (kNoKey) and no count.
 //
-// The particles arrive in the last step's key order and move less than a
-// cell per step (the CFL bound), so a key's particles are nearly contiguous
-// already and a key holds a handful of particles (about 8 at 8 particles
-// per cell). The sort is a counting sort: per-key counts (taken by kb_keys),
+// The particles arrive in the last sort's key order with a few per cent moved
+// to a neighbouring key, so a key's particles are nearly contiguous already
+// and a key holds a handful of particles (about 8 at 8 particles per cell).
+// The sort is a counting sort: per-key counts (taken by kb_keys),
 // an inclusive scan of the counts into segment ends, placement of every
 // particle into its key's segment through a per-key fill counter (one
 // atomic per key and warp), then the order inside each segment restored to
@@ -171,76 +172,147 @@ struct IntScan {
   __device__ __forceinline__ void store(long long g, int v, int) const { out[g] = v; }
 };
 
-// the per-key counts scanned in place into segment ends, the keys' fill
-// counters zeroed on the way (the placement's slots start at zero)
-struct SegScan {
-  using T = int;
-  using Op = ScanSum;
-  int* seg;
-  int* fill;
-  long long n;
-  __device__ __forceinline__ int load(long long g) const { return seg[g]; }
-  __device__ __forceinline__ void store(long long g, int v, int) const {
-    seg[g] = v;
-    fill[g] = 0;
+// ------------------------------------------------------------ grid barrier
+// Barrier over the blocks of one cooperative launch. bar[0] counts arrivals
+// (zero when the launch starts, never reset inside it), so round r is complete
+// at r * gridDim.x arrivals; bar[1] is set when a wait runs out, after which
+// every block leaves its launch at its next barrier. Returns false then.
+constexpr int kBarrierSpins = 1 << 22;  // about a second of polling
+
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&bar[0], 1u);
+    const unsigned want = round * gridDim.x;
+    volatile unsigned* v = bar;
+    int spins = 0;
+    while (v[0] < want && v[1] == 0u && ++spins < kBarrierSpins) __nanosleep(100);
+    if (v[0] < want) atomicExch(&bar[1], 1u);
+    ok = v[1] == 0u;
+    __threadfence();
   }
-};
+  __syncthreads();
+  const bool r = ok != 0;
+  __syncthreads();  // ok is written again by the next barrier
+  return r;
+}
 
 // ---------------------------------------------------------- counting sort
+// The phases of the sort as device functions over the whole grid of one
+// cooperative kernel (kb_resort), a grid barrier between them.
 constexpr int kRegSeg = 32;         // segments up to this length are ordered by one thread
-constexpr int kSegThreads = 256;    // threads of the long-segment blocks
+constexpr int kSortThreads = 256;   // threads of a block
 constexpr int kSmemSeg = 8192;      // long segments up to this length are ordered in shared memory
 
-// perm[seg start + slot] = i for every particle i, the slot taken from the
-// key's fill counter (one atomic per key and warp; lanes of a warp with the
-// same key take consecutive slots in lane order)
-__global__ void ks_place(const unsigned* key, const int* seg, int* fill, int* perm, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned k = i < n ? key[i] : 0xffffffffu;
-  const unsigned grp = __match_any_sync(0xffffffffu, k);
-  if (i >= n) return;
-  const int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
-  const int rank = __popc(grp & ((1u << lane) - 1u));
-  int base = 0;
-  if (lane == leader) base = atomicAdd(&fill[k], __popc(grp));
-  base = __shfl_sync(grp, base, leader);
-  const int start = k == 0 ? 0 : seg[k - 1];
-  perm[start + base + rank] = (int)i;
+constexpr unsigned kNoKey = 0xffffffffu;  // a particle that is not sorted
+
+// seg (per-key counts) into inclusive segment ends in three phases over tiles
+// of kScanTile keys, fill zeroed on the way; tile = kScanTile ints and thr,
+// wsum of block_scan in shared memory
+__device__ __forceinline__ void sort_tile_totals(const int* seg, long long nk, int* tiles, int* thr, int* wsum) {
+  const long long nt = (nk + kScanTile - 1) / kScanTile;
+  for (long long t = blockIdx.x; t < nt; t += gridDim.x) {
+    const long long base = t * kScanTile;
+    int v = 0;
+    for (int e = threadIdx.x; e < kScanTile; e += kSortThreads)
+      if (base + e < nk) v += seg[base + e];
+    block_scan<int, ScanSum>(v, thr, wsum);
+    if (threadIdx.x == 0) tiles[t] = thr[kSortThreads - 1];
+    __syncthreads();
+  }
+}
+
+// exclusive prefixes of the tile totals, by the first block
+__device__ __forceinline__ void sort_tile_prefix(long long nk, int* tiles, int* thr, int* wsum) {
+  if (blockIdx.x != 0) return;
+  const long long nt = (nk + kScanTile - 1) / kScanTile;
+  int carry = 0;
+  for (long long b0 = 0; b0 < nt; b0 += kSortThreads) {
+    const long long t = b0 + threadIdx.x;
+    const int ex = block_scan<int, ScanSum>(t < nt ? tiles[t] : 0, thr, wsum);
+    const int total = thr[kSortThreads - 1];
+    if (t < nt) tiles[t] = carry + ex;
+    carry += total;
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ void sort_tile_scan(int* seg, int* fill, long long nk, const int* tiles, int* tile, int* thr,
+                                               int* wsum) {
+  const long long nt = (nk + kScanTile - 1) / kScanTile;
+  for (long long t = blockIdx.x; t < nt; t += gridDim.x) {
+    const long long base = t * kScanTile;
+    for (int e = threadIdx.x; e < kScanTile; e += kSortThreads) tile[e] = base + e < nk ? seg[base + e] : 0;
+    __syncthreads();
+    int r[kScanItems], v = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) r[k] = v += tile[threadIdx.x * kScanItems + k];
+    const int pre = tiles[t] + block_scan<int, ScanSum>(v, thr, wsum);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) tile[threadIdx.x * kScanItems + k] = pre + r[k];
+    __syncthreads();
+    for (int e = threadIdx.x; e < kScanTile; e += kSortThreads)
+      if (base + e < nk) {
+        seg[base + e] = tile[e];
+        fill[base + e] = 0;  // the placement's slots start at zero
+      }
+    __syncthreads();
+  }
+}
+
+// perm[seg start + slot] = i for every particle i with a key, the slot taken
+// from the key's fill counter (one atomic per key and warp; lanes of a warp
+// with the same key take consecutive slots in lane order)
+__device__ __forceinline__ void sort_place(const unsigned* key, const int* seg, int* fill, int* perm, long long n) {
+  const int lane = threadIdx.x & 31;
+  for (long long b0 = (long long)blockIdx.x * kSortThreads; b0 < n; b0 += (long long)gridDim.x * kSortThreads) {
+    const long long i = b0 + threadIdx.x;
+    const unsigned k = i < n ? key[i] : kNoKey;
+    const unsigned grp = __match_any_sync(0xffffffffu, k);
+    const int leader = __ffs(grp) - 1, rank = __popc(grp & ((1u << lane) - 1u));
+    int base = 0;
+    if (lane == leader && k != kNoKey) base = atomicAdd(&fill[k], __popc(grp));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (k != kNoKey) perm[(k == 0 ? 0 : seg[k - 1]) + base + rank] = (int)i;
+  }
 }
 
 // Ascending order of perm inside each key's segment: segments of up to
 // kRegSeg particles by one thread (insertion sort, skipped when already in
-// order -- the common case), longer ones listed in big for ks_long_segments.
-__global__ void ks_segments(const int* seg, long long nk, int* perm, int* big, int* nbig) {
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nk) return;
-  const int a = k == 0 ? 0 : seg[k - 1], e = seg[k];
-  const int n = e - a;
-  if (n <= 1) return;
-  if (n > kRegSeg) {
-    big[atomicAdd(nbig, 1)] = (int)k;
-    return;
-  }
-  int* p = perm + a;
-  bool sorted = true;
-  int prev = p[0];
-  for (int j = 1; j < n; ++j) {
-    const int c = p[j];
-    sorted = sorted && prev < c;
-    prev = c;
-  }
-  if (sorted) return;
-  int v[kRegSeg];
-  for (int j = 0; j < n; ++j) {
-    const int c = p[j];
-    int m = j;
-    while (m > 0 && v[m - 1] > c) {
-      v[m] = v[m - 1];
-      --m;
+// order -- the common case), longer ones listed in big for sort_long.
+__device__ __forceinline__ void sort_segments(const int* seg, long long nk, int* perm, int* big, int* nbig) {
+  for (long long k = (long long)blockIdx.x * kSortThreads + threadIdx.x; k < nk;
+       k += (long long)gridDim.x * kSortThreads) {
+    const int a = k == 0 ? 0 : seg[k - 1], e = seg[k];
+    const int n = e - a;
+    if (n <= 1) continue;
+    if (n > kRegSeg) {
+      big[atomicAdd(nbig, 1)] = (int)k;
+      continue;
     }
-    v[m] = c;
+    int* p = perm + a;
+    bool sorted = true;
+    int prev = p[0];
+    for (int j = 1; j < n; ++j) {
+      const int c = p[j];
+      sorted = sorted && prev < c;
+      prev = c;
+    }
+    if (sorted) continue;
+    int v[kRegSeg];
+    for (int j = 0; j < n; ++j) {
+      const int c = p[j];
+      int m = j;
+      while (m > 0 && v[m - 1] > c) {
+        v[m] = v[m - 1];
+        --m;
+      }
+      v[m] = c;
+    }
+    for (int j = 0; j < n; ++j) p[j] = v[j];
   }
-  for (int j = 0; j < n; ++j) p[j] = v[j];
 }
 
 // ascending sort of d[0, n) (distinct values) by one block: a bitonic
@@ -277,10 +349,9 @@ __device__ __forceinline__ void block_bitonic(int* d, int n) {
 }
 
 // the long segments: one block per segment (grid-stride over the list), in
-// shared memory up to kSmemSeg particles, in place in global memory beyond
-__global__ void __launch_bounds__(kSegThreads) ks_long_segments(const int* seg, int* perm, const int* big,
-                                                                const int* nbig) {
-  __shared__ int sm[kSmemSeg];
+// shared memory (sm, kSmemSeg ints) up to kSmemSeg particles, in place in
+// global memory beyond
+__device__ __forceinline__ void sort_long(const int* seg, int* perm, const int* big, const int* nbig, int* sm) {
   const int nb = *nbig;
   for (int b = blockIdx.x; b < nb; b += gridDim.x) {
     const int k = big[b];
