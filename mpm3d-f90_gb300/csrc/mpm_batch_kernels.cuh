@@ -1055,7 +1055,7 @@ __device__ __forceinline__ void node_finish(BState& b, const Scene& sc, long lon
 // partial sums, and the decision only on the scene's own particles and order.
 // Also numbers the re-sorted scenes' particles for the sort (shift). One
 // block.
-constexpr float kDisorder = 0.5f;
+constexpr float kDisorder = 1.f;
 
 __device__ __forceinline__ void step_tick(BState& b, const int* target) {
   __shared__ long long thr[512], wsum[32];

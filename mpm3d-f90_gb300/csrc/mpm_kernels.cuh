@@ -3,10 +3,11 @@
 // form; mpm_gpu.cu sequences them (MPM3D.f90:69-118).
 //
 // Determinism: no kernel accumulates floating-point values with atomics.
-//   * particle -> node transfers run one thread per node over that node's
-//     slice of the node-sorted pair list, which holds the node's
-//     (particle, slot) contributions in the reference order (particle index,
-//     then slot), so every node sum is the reference's sequential sum;
+//   * particle -> node transfers walk each node's slice of the node-sorted
+//     pair list, which holds the node's (particle, slot) contributions in the
+//     reference order (particle index, then slot): the contributions are
+//     formed in parallel and added in that order (pair_walk), so every node
+//     sum is the reference's sequential sum;
 //   * node -> particle transfers run one thread per particle over its slots
 //     in the reference slot order;
 //   * reductions use a fixed block tree and a fixed final order.
@@ -300,35 +301,121 @@ __device__ __forceinline__ void count_active(bool active, unsigned long long* ou
   if ((threadIdx.x & 31) == 0 && b) atomicAdd(out, (unsigned long long)__popc(b));
 }
 
+// ------------------------------------------------------------- pair walk
+// Sums over the pair slices of kWalkNodes consecutive nodes (or SGMP cells) by
+// one block: in rounds of kWalkPairs pairs per node, eight threads per node
+// form the pairs' addends (every gather and product of the round in flight
+// at once) into shared memory, and then one warp per channel, lane = node,
+// adds them in pair order -- the reference's sequential sum, each addend
+// rounded as it would be there. A thread per node did both alone, one pair's
+// gathers after the other's sum: the walk waited on memory with a fraction of
+// the chip's threads (nodes are an eighth of the particles, and only the ones
+// with pairs work). Bound now by the FP64 pipe and the gathers. One node per
+// lane keeps the adds at full warps, which cost the FP64 pipe the same as one
+// lane would. Measured on a GB300 (force transfer with the momentum
+// integration): see the figures at k_p2g_force.
+//
+// NV addends per pair, NC channels: channel c adds NA[c] of them, starting
+// at c * 2 for the TWO first channels and one each after those.
+// prod(p, idx, v) forms a pair's addends from the particle and the index in
+// the shape cache; fin(n, acc) gets a node's sums.
+constexpr int kWalkNodes = 32;
+constexpr int kWalkPairs = 16;   // pairs per node and round
+constexpr int kWalkPitch = 36;   // nodes' row pitch (the four nodes x eight pairs a warp writes fall on distinct banks)
+static_assert(kBlock == 8 * kWalkNodes, "eight threads per node");
+
+template <int NV, int NC, int TWO, class Prod, class Fin>
+__device__ __forceinline__ void pair_walk(const int* seg, const unsigned* val, long long np, long long nn, Prod prod,
+                                          Fin fin) {
+  static_assert(NV == NC + TWO, "addends");
+  constexpr int NW = kBlock / 32, PER = (NC + NW - 1) / NW;  // channels a warp sums
+  __shared__ double buf[NV][kWalkPairs][kWalkPitch];
+  __shared__ int s_end[kWalkNodes + 1];
+  __shared__ int s_rounds;
+  const long long n0 = (long long)blockIdx.x * kWalkNodes;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (warp == 0) {
+    const long long n = n0 + lane;
+    const int e = seg[n < nn ? n : nn - 1];
+    const int first = n0 == 0 ? 0 : seg[n0 - 1];
+    s_end[lane + 1] = e;
+    if (lane == 0) s_end[0] = first;
+    int len = __shfl_up_sync(0xffffffffu, e, 1);
+    len = e - (lane == 0 ? first : len);
+    const int longest = __reduce_max_sync(0xffffffffu, len);
+    if (lane == 0) s_rounds = (longest + kWalkPairs - 1) / kWalkPairs;
+  }
+  __syncthreads();
+  const int rounds = s_rounds;
+  const int g = t >> 3, q = t & 7;
+  const int ja = s_end[g] + q, je = s_end[g + 1];       // the thread's pairs: ja, ja + 8, ja + 16, ...
+  const int len = s_end[lane + 1] - s_end[lane];        // pairs of the lane's node (summing warps)
+  double acc[PER];
+#pragma unroll
+  for (int e = 0; e < PER; ++e) acc[e] = 0.0;
+  for (int r = 0; r < rounds; ++r) {
+#pragma unroll
+    for (int u = 0; u < kWalkPairs / 8; ++u) {
+      const int j = ja + r * kWalkPairs + 8 * u;
+      if (j < je) {
+        const unsigned pv = val[j];
+        const long long p = (long long)(pv >> 5);
+        double v[NV];
+        prod(p, (long long)(pv & 31u) * np + p, v);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) buf[k][q + 8 * u][g] = v[k];
+      }
+    }
+    __syncthreads();
+    const int cnt = min(len - r * kWalkPairs, kWalkPairs);
+#pragma unroll
+    for (int e = 0; e < PER; ++e) {
+      const int c = warp + e * NW;
+      if (c < TWO) {
+#pragma unroll 8
+        for (int k = 0; k < cnt; ++k) acc[e] = acc[e] + buf[2 * c][k][lane] + buf[2 * c + 1][k][lane];
+      } else if (c < NC) {
+#pragma unroll 8
+        for (int k = 0; k < cnt; ++k) acc[e] = acc[e] + buf[c + TWO][k][lane];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int e = 0; e < PER; ++e)
+    if (warp + e * NW < NC) buf[warp + e * NW][0][lane] = acc[e];
+  __syncthreads();
+  if (warp == 0) {
+    double a[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) a[c] = buf[c][0][lane];
+    fin(n0 + lane, n0 + lane < nn, a);
+  }
+}
+
 // --------------------------------------------------- P2G: mass, momentum
 // GridMomentumInitial (update_step.f90:288-406), non-SGMP.
 template <class P>
 __global__ void k_p2g_mass(St<P> s, Geometry g, int bc, int vel) {
-  const long long n = gtid();
-  const long long nn = g.nnt;  // every grid component
-  bool act = false;
-  if (n < nn) {
-    const long long np = g.np;
-    double m = 0.0, px = 0.0, py = 0.0, pz = 0.0;
-    const int j0 = n == 0 ? 0 : s.seg[n - 1], j1 = s.seg[n];
-    for (int j = j0; j < j1; ++j) {
-      long long p, idx;
-      decode_pair(s.val_sorted[j], np, &p, &idx);
-      double shm = (double)s.shp[idx] * s.mass[p];
-      m = m + shm;
-      px = px + s.vxp[p] * shm;
-      py = py + s.vxp[np + p] * shm;
-      pz = pz + s.vxp[2 * np + p] * shm;
-    }
-    s.mg[n] = m;
-    s.px[n] = px;
-    s.px[nn + n] = py;
-    s.px[2LL * nn + n] = pz;
-    act = m > 0.0;
-    if (bc) node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
-    if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
-  }
-  count_active(act, &s.sc->active_nodes);
+  const long long nn = g.nnt, np = g.np;  // nn: every grid component
+  pair_walk<4, 4, 0>(
+      s.seg, s.val_sorted, np, nn,
+      [&](long long p, long long idx, double* v) {
+        const double shm = (double)s.shp[idx] * s.mass[p];
+        v[0] = shm;
+        v[1] = s.vxp[p] * shm;
+        v[2] = s.vxp[np + p] * shm;
+        v[3] = s.vxp[2 * np + p] * shm;
+      },
+      [&](long long n, bool in, const double* a) {
+        if (in) {
+          s.mg[n] = a[0];
+          for (int c = 0; c < 3; ++c) s.px[c * nn + n] = a[1 + c];
+          if (bc) node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
+          if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+        }
+        count_active(in && a[0] > 0.0, &s.sc->active_nodes);
+      });
 }
 
 // seg holds per-node counts after k_locate; turn them into exclusive ends
@@ -910,54 +997,41 @@ __device__ __forceinline__ void node_integrate(St<P>& s, const Geometry& g, long
   node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
 }
 
-template <class P>
+// CONTACT: also the mass gradient of the node, the contact normal
+// (update_step.f90:977-982)
+template <class P, bool CONTACT>
 __global__ void k_p2g_force(St<P> s, Geometry g, int integ) {
-  using R = typename P::R;
-  const long long n = gtid();
-  const long long nn = g.nnt;  // every grid component
-  if (n >= nn) return;
-  const long long np = g.np;
-  double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-  double nd0 = 0.0, nd1 = 0.0, nd2 = 0.0;  // contact normal: mass gradient (update_step.f90:977-982)
-  const int j0 = n == 0 ? 0 : s.seg[n - 1], j1 = s.seg[n];
-  for (int j = j0; j < j1; ++j) {
-    long long p, idx;
-    decode_pair(s.val_sorted[j], np, &p, &idx);
-    R sk = s.shp[idx], dx = s.dndx[idx], dy = s.dndy[idx], dz = s.dndz[idx];
-    if (g.contact) {
-      const double mp = s.mass[p];
-      nd0 = nd0 + (double)dx * mp;
-      nd1 = nd1 + (double)dy * mp;
-      nd2 = nd2 + (double)dz * mp;
-    }
-    R sxx = (R)s.sdiag[p], syy = (R)s.sdiag[np + p], szz = (R)s.sdiag[2 * np + p];
-    R sxy = (R)s.sd[3 * np + p], syz = (R)s.sd[4 * np + p], sxz = (R)s.sd[5 * np + p];
-    R vol = (R)s.vol[p];
-    R fi0 = -(sxx * dx + sxy * dy + sxz * dz) * vol;
-    R fi1 = -(sxy * dx + syy * dy + syz * dz) * vol;
-    R fi2 = -(sxz * dx + syz * dy + szz * dz) * vol;
-    if constexpr (P::kExact) {
-      f0 = f0 + fi0 + s.fext[p] * sk;
-      f1 = f1 + fi1 + s.fext[np + p] * sk;
-      f2 = f2 + fi2 + s.fext[2 * np + p] * sk;
-    } else {
-      f0 = f0 + (double)(fi0 + (R)s.fext[p] * sk);
-      f1 = f1 + (double)(fi1 + (R)s.fext[np + p] * sk);
-      f2 = f2 + (double)(fi2 + (R)s.fext[2 * np + p] * sk);
-    }
-  }
-  s.fx[n] = f0;
-  s.fx[nn + n] = f1;
-  s.fx[2LL * nn + n] = f2;
-  if (g.contact) {
-    s.ndir[n] = nd0;
-    s.ndir[nn + n] = nd1;
-    s.ndir[2LL * nn + n] = nd2;
-  }
-  if (integ) {
-    double fxn[3] = {f0, f1, f2};
-    node_integrate<P>(s, g, n, fxn);
-  }
+  const long long nn = g.nnt, np = g.np;  // nn: every grid component
+  pair_walk<CONTACT ? 9 : 6, CONTACT ? 6 : 3, 3>(
+      s.seg, s.val_sorted, np, nn,
+      [&](long long p, long long idx, double* v) {
+        const double sk = s.shp[idx], dx = s.dndx[idx], dy = s.dndy[idx], dz = s.dndz[idx];
+        const double sxx = s.sdiag[p], syy = s.sdiag[np + p], szz = s.sdiag[2 * np + p];
+        const double sxy = s.sd[3 * np + p], syz = s.sd[4 * np + p], sxz = s.sd[5 * np + p];
+        const double vol = s.vol[p];
+        v[0] = -(sxx * dx + sxy * dy + sxz * dz) * vol;
+        v[1] = s.fext[p] * sk;
+        v[2] = -(sxy * dx + syy * dy + syz * dz) * vol;
+        v[3] = s.fext[np + p] * sk;
+        v[4] = -(sxz * dx + syz * dy + szz * dz) * vol;
+        v[5] = s.fext[2 * np + p] * sk;
+        if (CONTACT) {
+          const double mp = s.mass[p];
+          v[6] = dx * mp;
+          v[7] = dy * mp;
+          v[8] = dz * mp;
+        }
+      },
+      [&](long long n, bool in, const double* a) {
+        if (!in) return;
+        for (int c = 0; c < 3; ++c) s.fx[c * nn + n] = a[c];
+        if (CONTACT)
+          for (int c = 0; c < 3; ++c) s.ndir[c * nn + n] = a[3 + c];
+        if (integ) {
+          double fxn[3] = {a[0], a[1], a[2]};
+          node_integrate<P>(s, g, n, fxn);
+        }
+      });
 }
 
 template <class P>
@@ -1164,25 +1238,19 @@ __global__ void k_position(St<P> s, Geometry g) {
 // GridMomentumMUSL (update_step.f90:1668-1793), non-SGMP.
 template <class P>
 __global__ void k_p2g_momentum(St<P> s, Geometry g, int vel) {
-  const long long n = gtid();
-  const long long nn = g.nnt;  // every grid component
-  if (n >= nn) return;
-  const long long np = g.np;
-  double px = 0.0, py = 0.0, pz = 0.0;
-  const int j0 = n == 0 ? 0 : s.seg[n - 1], j1 = s.seg[n];
-  for (int j = j0; j < j1; ++j) {
-    long long p, idx;
-    decode_pair(s.val_sorted[j], np, &p, &idx);
-    double shm = (double)s.shp[idx] * s.mass[p];
-    px = px + s.vxp[p] * shm;
-    py = py + s.vxp[np + p] * shm;
-    pz = pz + s.vxp[2 * np + p] * shm;
-  }
-  s.px[n] = px;
-  s.px[nn + n] = py;
-  s.px[2LL * nn + n] = pz;
-  node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
-  if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+  const long long nn = g.nnt, np = g.np;  // nn: every grid component
+  pair_walk<3, 3, 0>(
+      s.seg, s.val_sorted, np, nn,
+      [&](long long p, long long idx, double* v) {
+        const double shm = (double)s.shp[idx] * s.mass[p];
+        for (int c = 0; c < 3; ++c) v[c] = s.vxp[c * np + p] * shm;
+      },
+      [&](long long n, bool in, const double* a) {
+        if (!in) return;
+        for (int c = 0; c < 3; ++c) s.px[c * nn + n] = a[c];
+        node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
+        if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+      });
 }
 
 // ================================================================ SGMP
@@ -1214,25 +1282,19 @@ __device__ __forceinline__ void for_adjacent_cells(const Geometry& g, long long 
 // GridMomentumInitial, SGMP branch: particles -> cells
 template <class P>
 __global__ void k_sg_cell_mass(St<P> s, Geometry g) {
-  const long long c = gtid();
-  const int nc = g.ncell;
-  if (c >= nc) return;
-  const long long np = g.np;
-  double m = 0.0, px = 0.0, py = 0.0, pz = 0.0;
-  const int j0 = c == 0 ? 0 : s.seg[c - 1], j1 = s.seg[c];
-  for (int j = j0; j < j1; ++j) {
-    long long p, idx;
-    decode_pair(s.val_sorted[j], np, &p, &idx);
-    double shm = (double)s.shp[idx] * s.mass[p];
-    m = m + shm;
-    px = px + s.vxp[p] * shm;
-    py = py + s.vxp[np + p] * shm;
-    pz = pz + s.vxp[2 * np + p] * shm;
-  }
-  s.cmg[c] = m;
-  s.cpx[c] = px;
-  s.cpx[nc + c] = py;
-  s.cpx[2LL * nc + c] = pz;
+  const long long np = g.np, nc = g.ncell;
+  pair_walk<4, 4, 0>(
+      s.seg, s.val_sorted, np, nc,
+      [&](long long p, long long idx, double* v) {
+        const double shm = (double)s.shp[idx] * s.mass[p];
+        v[0] = shm;
+        for (int c = 0; c < 3; ++c) v[1 + c] = s.vxp[c * np + p] * shm;
+      },
+      [&](long long c, bool in, const double* a) {
+        if (!in) return;
+        s.cmg[c] = a[0];
+        for (int k = 0; k < 3; ++k) s.cpx[k * nc + c] = a[1 + k];
+      });
 }
 
 // ... cells -> nodes (mass and momentum, only cells above the cut-off)
@@ -1304,28 +1366,20 @@ __global__ void k_sg_cell_gradient(St<P> s, Geometry g) {
 // GridMomentumUpdate, SGMP branch: particles -> cells
 template <class P>
 __global__ void k_sg_cell_force(St<P> s, Geometry g) {
-  using R = typename P::R;
-  const long long c = gtid();
-  const int nc = g.ncell;
-  if (c >= nc) return;
-  const long long np = g.np;
-  double fe[3] = {0, 0, 0}, fi[6] = {0, 0, 0, 0, 0, 0};
-  const int j0 = c == 0 ? 0 : s.seg[c - 1], j1 = s.seg[c];
-  for (int j = j0; j < j1; ++j) {
-    long long p, idx;
-    decode_pair(s.val_sorted[j], np, &p, &idx);
-    double sk = (double)s.shp[idx];
-    double vol = (double)s.vol[p];
-    for (int d = 0; d < 3; ++d) fe[d] = fe[d] + s.fext[d * np + p] * sk;
-    fi[0] = fi[0] + sk * s.sdiag[p] * vol;
-    fi[1] = fi[1] + sk * s.sdiag[np + p] * vol;
-    fi[2] = fi[2] + sk * s.sdiag[2 * np + p] * vol;
-    fi[3] = fi[3] + sk * (double)s.sd[3 * np + p] * vol;
-    fi[4] = fi[4] + sk * (double)s.sd[4 * np + p] * vol;
-    fi[5] = fi[5] + sk * (double)s.sd[5 * np + p] * vol;
-  }
-  for (int d = 0; d < 3; ++d) s.cfext[(long long)d * nc + c] = fe[d];
-  for (int d = 0; d < 6; ++d) s.cfint[(long long)d * nc + c] = fi[d];
+  const long long np = g.np, nc = g.ncell;
+  pair_walk<9, 9, 0>(
+      s.seg, s.val_sorted, np, nc,
+      [&](long long p, long long idx, double* v) {
+        const double sk = s.shp[idx], vol = s.vol[p];
+        for (int d = 0; d < 3; ++d) v[d] = s.fext[d * np + p] * sk;
+        for (int d = 0; d < 3; ++d) v[3 + d] = sk * s.sdiag[d * np + p] * vol;
+        for (int d = 3; d < 6; ++d) v[3 + d] = sk * s.sd[d * np + p] * vol;
+      },
+      [&](long long c, bool in, const double* a) {
+        if (!in) return;
+        for (int d = 0; d < 3; ++d) s.cfext[d * nc + c] = a[d];
+        for (int d = 0; d < 6; ++d) s.cfint[d * nc + c] = a[3 + d];
+      });
 }
 
 // ... cells -> nodes (every cell, no cut-off), then optionally integrate
@@ -1415,23 +1469,17 @@ __global__ void k_sg_cell_velocity(St<P> s, Geometry g) {
 // GridMomentumMUSL, SGMP branch
 template <class P>
 __global__ void k_sg_cell_momentum(St<P> s, Geometry g) {
-  const long long c = gtid();
-  const int nc = g.ncell;
-  if (c >= nc) return;
-  const long long np = g.np;
-  double px = 0.0, py = 0.0, pz = 0.0;
-  const int j0 = c == 0 ? 0 : s.seg[c - 1], j1 = s.seg[c];
-  for (int j = j0; j < j1; ++j) {
-    long long p, idx;
-    decode_pair(s.val_sorted[j], np, &p, &idx);
-    double shm = (double)s.shp[idx] * s.mass[p];
-    px = px + s.vxp[p] * shm;
-    py = py + s.vxp[np + p] * shm;
-    pz = pz + s.vxp[2 * np + p] * shm;
-  }
-  s.cpx[c] = px;
-  s.cpx[nc + c] = py;
-  s.cpx[2LL * nc + c] = pz;
+  const long long np = g.np, nc = g.ncell;
+  pair_walk<3, 3, 0>(
+      s.seg, s.val_sorted, np, nc,
+      [&](long long p, long long idx, double* v) {
+        const double shm = (double)s.shp[idx] * s.mass[p];
+        for (int c = 0; c < 3; ++c) v[c] = s.vxp[c * np + p] * shm;
+      },
+      [&](long long c, bool in, const double* a) {
+        if (!in) return;
+        for (int k = 0; k < 3; ++k) s.cpx[k * nc + c] = a[k];
+      });
 }
 
 template <class P>

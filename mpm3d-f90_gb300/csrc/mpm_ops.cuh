@@ -7,6 +7,8 @@
 namespace mpm {
 
 inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
+// blocks of a pair_walk kernel over n nodes or cells
+inline unsigned walk_grid(long long n) { return (unsigned)((n + kWalkNodes - 1) / kWalkNodes); }
 
 template <class P>
 struct Ops {
@@ -26,10 +28,10 @@ struct Ops {
   static void p2g_mass(void* st, const Geometry& g, int bc, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      k_sg_cell_mass<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_mass<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
       k_sg_node_mass<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, bc, vel);
     } else {
-      k_p2g_mass<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g, bc, vel);
+      k_p2g_mass<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, bc, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
@@ -63,10 +65,11 @@ struct Ops {
   static void p2g_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
-      k_sg_cell_force<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_force<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
       k_sg_node_force<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, integ);
     } else {
-      k_p2g_force<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
+      if (g.contact) k_p2g_force<P, true><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
+      else k_p2g_force<P, false><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
     }
     prof_end(K_P2G_FORCE, s);
   }
@@ -84,10 +87,10 @@ struct Ops {
   static void p2g_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MOM, s);
     if (g.shape == 3) {
-      k_sg_cell_momentum<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
       k_sg_node_momentum<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, vel);
     } else {
-      k_p2g_momentum<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
+      k_p2g_momentum<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
     }
     prof_end(K_P2G_MOM, s);
   }
@@ -114,10 +117,10 @@ struct Ops {
   static void tl_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      k_sg_cell_momentum<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
       k_tl_sg_node_momentum<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, vel);
     } else {
-      k_p2g_momentum<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
+      k_p2g_momentum<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
