@@ -531,6 +531,9 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
   c->red_blocks = (int)std::min<long long>(1024, (np + kBlock - 1) / kBlock);
   const size_t B = c->ops->bulk_size, Rz = c->ops->real_size;
   DevState<double, double>& s = c->st;
+  s.mat_type = c->mats[0].mat_type;
+  for (const DevMaterial& m : c->mats)
+    if (m.mat_type != s.mat_type) s.mat_type = 0;
   // particle arrays
 #define AL(ptr, T, n) \
   if ((r = dalloc(c, (T**)&(ptr), (n)))) goto fail;
@@ -554,6 +557,7 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
     AL(s.key_sorted, unsigned, c->npairs); AL(s.val_sorted, unsigned, c->npairs);
     AL(s.seg, int, (long long)c->nkeys + 1);
     AL(s.mg, double, nnt); AL(s.px, double, 3 * nnt); AL(s.fx, double, 3 * nnt); AL(s.vg, double, 3 * nnt);
+    AL(s.rm, double, 2 * nnt);
     AL(s.fix, uint8_t, nn); AL(s.bd, uint8_t, nn);
     if (g.contact) { AL(s.ndir, double, 3 * nnt); AL(s.cforce, double, 3 * nn); }
     if (g.tlmpm) {
@@ -636,6 +640,7 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
     CKF(cudaMemsetAsync(s.px, 0, sizeof(double) * 3 * nnt, c->stream));
     CKF(cudaMemsetAsync(s.fx, 0, sizeof(double) * 3 * nnt, c->stream));
     CKF(cudaMemsetAsync(s.vg, 0, sizeof(double) * 3 * nnt, c->stream));
+    CKF(cudaMemsetAsync(s.rm, 0, sizeof(double) * 2 * nnt, c->stream));
     if (s.ndir) CKF(cudaMemsetAsync(s.ndir, 0, sizeof(double) * 3 * nnt, c->stream));
     if (s.cforce) CKF(cudaMemsetAsync(s.cforce, 0, sizeof(double) * 3 * nn, c->stream));
     CKF(cudaMemsetAsync(s.red_count, 0, sizeof(unsigned), c->stream));

@@ -17,7 +17,7 @@
 //     the reference's summation order (ascending particle, then slot);
 //     seg[n] = end of node n's slice (inclusive prefix sum of the counts).
 //   grid, FP64, flat reference node order: mg[Nn], px[3][Nn], fx[3][Nn],
-//     vg[3][Nn] (= px/mg), uint8 fix[Nn] (bit c = DOF c fixed), uint8 bd[Nn];
+//     vg[3][Nn] (= px/mg), rm[2][Nn] (= 1/mg), uint8 fix[Nn] (bit c = DOF c fixed), uint8 bd[Nn];
 //     with several grid components (contact) the value arrays hold ncomp
 //     grids back to back (Nn = ncomp * nodes), a particle reaching its body's
 //     component through the node index of its shape cache
@@ -148,6 +148,7 @@ struct DevState {
   int* seg;
   // grid
   double *mg, *px, *fx, *vg;
+  double* rm;  // [2][Nn] reciprocal of the node's mass as a two-part sum (nodes above the cut-off)
   uint8_t *fix, *bd;
   // SGMP centre grid
   double *cmg, *cpx, *cfext, *cfint, *co, *cw, *cdefp, *cvx, *cax;
@@ -170,6 +171,7 @@ struct DevState {
   DevMaterial* mats;
   DevBody* bodies;
   DevScalars* sc;
+  int mat_type;  // the type of every material of the deck, 0 if they differ
 };
 
 // One launch table per arithmetic form; each form is compiled in its own

@@ -288,11 +288,58 @@ __device__ __forceinline__ void node_bc(const uint8_t fix, double* px, double* f
     }
 }
 
-__device__ __forceinline__ void node_vel(const double* mg, const double* px, double* vg, long long n, long long nn,
-                                         double cutoff) {
-  double m = mg[n];
-  if (m > cutoff)
-    for (int c = 0; c < 3; ++c) vg[(long long)c * nn + n] = px[(long long)c * nn + n] / m;
+// Division by a node's mass. The node and particle kernels divide by each
+// node's mass tens of times a step (the position update alone three times per
+// particle and slot), and an FP64 division costs GB300's narrow FP64 pipe
+// about ten instructions. With the mass known in advance four suffice:
+// its reciprocal is kept as yh + yl (yh = 1/m rounded, yl = (1 - m yh) yh),
+// q0 = x yh + x yl is within one ulp of x / m, r = x - q0 m is exact (fused
+// multiply-add), and q0 + r yh is then x / m correctly rounded -- Markstein's
+// theorem (IBM J. Res. Dev. 34, 1990) with the two-part reciprocal of
+// Brisebarre, Muller and Raina (IEEE Trans. Comput. 53, 2004); so the result
+// is the division's, bit for bit (tests/test_fp64_division.py). Operands near
+// the ends of the exponent range take the division itself: yh = 0 marks such
+// a mass, and x is checked by its exponent. The sign of a zero quotient may
+// differ, which no sum it is added to shows (the sums start at +0).
+struct Recip {
+  double yh, yl;
+};
+__device__ __forceinline__ Recip recip_of(double m) {
+  const unsigned e = ((unsigned)__double2hiint(m) >> 20) & 0x7ffu;
+  Recip r = {0.0, 0.0};
+  if (e - 623u <= 800u) {  // 2^-400 .. 2^400
+    r.yh = 1.0 / m;
+    r.yl = __fma_rn(-r.yh, m, 1.0) * r.yh;
+  }
+  return r;
+}
+// (a call: inlined, the division would be executed for every lane and selected)
+static __device__ __noinline__ double div_plain(double x, double m) { return x / m; }
+
+__device__ __forceinline__ double div_known(double x, double m, const Recip& y) {
+  const double q0 = __fma_rn(x, y.yh, x * y.yl);
+  double q = __fma_rn(__fma_rn(-q0, m, x), y.yh, q0);
+  const int hi = __double2hiint(x) & 0x7fffffff;
+  const unsigned e = (unsigned)hi >> 20;
+  if ((e - 523u > 1000u || __double2hiint(y.yh) == 0) && (hi | __double2loint(x)) != 0) q = div_plain(x, m);
+  return q;
+}
+
+// node velocity; the mass's reciprocal is stored with the mass
+__device__ __forceinline__ void node_vel(const double* mg, const double* rm, const double* px, double* vg, long long n,
+                                         long long nn, double cutoff) {
+  const double m = mg[n];
+  if (m > cutoff) {
+    const Recip y = {rm[n], rm[nn + n]};
+    for (int c = 0; c < 3; ++c) vg[(long long)c * nn + n] = div_known(px[(long long)c * nn + n], m, y);
+  }
+}
+__device__ __forceinline__ void store_recip(double* rm, long long n, long long nn, double m, double cutoff) {
+  if (m > cutoff) {
+    const Recip y = recip_of(m);
+    rm[n] = y.yh;
+    rm[nn + n] = y.yl;
+  }
 }
 
 // count of nodes with mass (for the algorithmic-bytes figure)
@@ -410,9 +457,10 @@ __global__ void k_p2g_mass(St<P> s, Geometry g, int bc, int vel) {
       [&](long long n, bool in, const double* a) {
         if (in) {
           s.mg[n] = a[0];
+          store_recip(s.rm, n, nn, a[0], g.cutoff);
           for (int c = 0; c < 3; ++c) s.px[c * nn + n] = a[1 + c];
           if (bc) node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
-          if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+          if (vel) node_vel(s.mg, s.rm, s.px, s.vg, n, nn, g.cutoff);
         }
         count_active(in && a[0] > 0.0, &s.sc->active_nodes);
       });
@@ -425,7 +473,7 @@ template <class P>
 __global__ void k_node_velocity(St<P> s, Geometry g) {
   const long long n = gtid();
   if (n >= g.nnt) return;
-  node_vel(s.mg, s.px, s.vg, n, g.nnt, g.cutoff);
+  node_vel(s.mg, s.rm, s.px, s.vg, n, g.nnt, g.cutoff);
 }
 
 template <class P>
@@ -765,8 +813,15 @@ __device__ __forceinline__ void constitution(PState<typename P::R>& ps, const Ma
   ps.failure = failure;
 }
 
-template <class P>
-__global__ void k_stress(St<P> s, Geometry g) {
+// MT: the material type of every particle (0: read per particle), UV: the deck
+// tracks the deformation gradient. An instantiation per common type keeps the
+// other models' registers out (the general kernel's 164 leave one 256-thread
+// block per SM), and without UV the gather drops the gradient's six sums
+// beyond the strain rate's (the diagonal ones are the same).
+constexpr bool stress_has(int mt) { return mt == 1 || mt == 7 || mt == 9 || mt == 10 || mt == 11; }
+
+template <class P, int MT, int UV>
+__global__ void __launch_bounds__(kBlock, MT == 0 ? 1 : 2) k_stress(St<P> s, Geometry g) {
   using R = typename P::R;
   using B = typename P::B;
   const long long p = gtid();
@@ -787,33 +842,54 @@ __global__ void k_stress(St<P> s, Geometry g) {
       R sk = s.shp[k * np + p];
       for (int i = 0; i < 6; ++i) de[i] = de[i] + (R)s.co[i * nc + c] * sk;
       for (int i = 0; i < 3; ++i) vort[i] = vort[i] + (R)s.cw[i * nc + c] * sk;
-      for (int i = 0; i < 3; ++i)
+      for (int i = 0; UV && i < 3; ++i)
         for (int j = 0; j < 3; ++j) deFp[i][j] = deFp[i][j] + sk * (R)s.cdefp[(i * 3 + j) * nc + c];
     }
   } else {
     if (s.icell[p] < 0) return;
-    for (int k = 0; k < g.K; ++k) {
-      int n = s.snode[k * np + p];
-      if (n < 0) continue;
-      if (!(s.mg[n] > g.cutoff)) continue;
-      R v[3] = {(R)s.vg[n], (R)s.vg[nn + n], (R)s.vg[2LL * nn + n]};
-      const long long idx = k * np + p;
-      R dx = s.dndx[idx], dy = s.dndy[idx], dz = s.dndz[idx];
-      de[0] = de[0] + dx * v[0];
-      de[1] = de[1] + dy * v[1];
-      de[2] = de[2] + dz * v[2];
-      de[3] = de[3] + (dy * v[2] + dz * v[1]);
-      de[4] = de[4] + (dz * v[0] + dx * v[2]);
-      de[5] = de[5] + (dx * v[1] + dy * v[0]);
-      vort[0] = vort[0] + (dy * v[2] - dz * v[1]);
-      vort[1] = vort[1] + (dz * v[0] - dx * v[2]);
-      vort[2] = vort[2] + (dx * v[1] - dy * v[0]);
-      for (int i = 0; i < 3; ++i) {
-        deFp[i][0] = deFp[i][0] + dx * v[i];
-        deFp[i][1] = deFp[i][1] + dy * v[i];
-        deFp[i][2] = deFp[i][2] + dz * v[i];
+    constexpr int U = 3;  // slots whose gathers are in flight together
+    for (int k0 = 0; k0 < g.K; k0 += U) {
+      int n[U];
+      double m[U], v[U][3], dn[U][3];
+#pragma unroll
+      for (int u = 0; u < U; ++u) n[u] = k0 + u < g.K ? s.snode[(k0 + u) * np + p] : -1;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        m[u] = 0.0;
+        if (n[u] < 0) continue;
+        const long long idx = (k0 + u) * np + p;
+        m[u] = s.mg[n[u]];
+        for (int c = 0; c < 3; ++c) v[u][c] = s.vg[(long long)c * nn + n[u]];
+        dn[u][0] = s.dndx[idx];
+        dn[u][1] = s.dndy[idx];
+        dn[u][2] = s.dndz[idx];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (n[u] < 0 || !(m[u] > g.cutoff)) continue;
+        const double* w = v[u];
+        const double dx = dn[u][0], dy = dn[u][1], dz = dn[u][2];
+        const double xv = dx * w[1], xw = dx * w[2], yu = dy * w[0], yw = dy * w[2], zu = dz * w[0], zv = dz * w[1];
+        de[0] = de[0] + dx * w[0];
+        de[1] = de[1] + dy * w[1];
+        de[2] = de[2] + dz * w[2];
+        de[3] = de[3] + (yw + zv);
+        de[4] = de[4] + (zu + xw);
+        de[5] = de[5] + (xv + yu);
+        vort[0] = vort[0] + (yw - zv);
+        vort[1] = vort[1] + (zu - xw);
+        vort[2] = vort[2] + (xv - yu);
+        if (UV) {
+          deFp[0][1] = deFp[0][1] + yu;
+          deFp[0][2] = deFp[0][2] + zu;
+          deFp[1][0] = deFp[1][0] + xv;
+          deFp[1][2] = deFp[1][2] + zv;
+          deFp[2][0] = deFp[2][0] + xw;
+          deFp[2][1] = deFp[2][1] + yw;
+        }
       }
     }
+    for (int i = 0; i < 3; ++i) deFp[i][i] = de[i];
   }
   const DevScalars& sc = *s.sc;
   const R DT = (R)sc.dt;
@@ -822,7 +898,7 @@ __global__ void k_stress(St<P> s, Geometry g) {
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) deFp[i][j] = deFp[i][j] * DT;
   R Fpn[3][3];
-  if (g.uvfp) {
+  if (UV) {
     R F0[3][3];
     for (int i = 0; i < 9; ++i) F0[i / 3][i % 3] = (R)s.fp[i * np + p];
     for (int i = 0; i < 3; ++i)
@@ -851,7 +927,7 @@ __global__ void k_stress(St<P> s, Geometry g) {
   ps.evol = (R)0;
   const DevMaterial& mt = s.mats[s.bodies[s.body[p]].mat];
   CResult<R> res;
-  constitution<P>(ps, mt, de, vort, deFp, Fpn, g.uvfp != 0, DT, s.sc->time, (R)g.dcell, (R)g.bq1, (R)g.bq2, res);
+  constitution<P, MT>(ps, mt, de, vort, deFp, Fpn, UV != 0, DT, s.sc->time, (R)g.dcell, (R)g.bq1, (R)g.bq2, res);
   if (res.negative_volume) atomicOr(&s.sc->status, (unsigned)ST_NEGATIVE_VOLUME);
   if (!res.eos_ok) atomicOr(&s.sc->status, (unsigned)ST_BAD_EOS);
   if (res.defer && res.tail == 7) {
@@ -994,7 +1070,7 @@ __device__ __forceinline__ void node_integrate(St<P>& s, const Geometry& g, long
     s.px[(long long)c * nn + n] = pxc;
   }
   node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
-  node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+  node_vel(s.mg, s.rm, s.px, s.vg, n, nn, g.cutoff);
 }
 
 // CONTACT: also the mass gradient of the node, the contact normal
@@ -1115,8 +1191,8 @@ __global__ void k_contact(St<P> s, Geometry g) {
       s.px[c * nt + n] = p1[c] - cforce[c] * dt;
       s.px[c * nt + n2] = p2[c] + cforce[c] * dt;
     }
-    node_vel(s.mg, s.px, s.vg, n, nt, g.cutoff);
-    node_vel(s.mg, s.px, s.vg, n2, nt, g.cutoff);
+    node_vel(s.mg, s.rm, s.px, s.vg, n, nt, g.cutoff);
+    node_vel(s.mg, s.rm, s.px, s.vg, n2, nt, g.cutoff);
   }
   for (int c = 0; c < 3; ++c) s.cforce[c * nn + n] = cforce[c];
 }
@@ -1187,36 +1263,33 @@ __global__ void k_position(St<P> s, Geometry g) {
     }
   } else {
     if (s.icell[p] < 0) return;
-    if constexpr (P::kExact) {
-      for (int k = 0; k < g.K; ++k) {
-        int n = s.snode[k * np + p];
-        if (n < 0) continue;
-        double m = s.mg[n];
-        if (!(m > g.cutoff)) continue;
-        double sk = s.shp[k * np + p];
+    // (the gathers of a few slots in flight before the first one's sums)
+    constexpr int U = 3;
+    for (int k0 = 0; k0 < g.K; k0 += U) {
+      int n[U];
+      double m[U], sk[U], v[U][3], f[U][3];
+      Recip y[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) n[u] = k0 + u < g.K ? s.snode[(k0 + u) * np + p] : -1;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        m[u] = 0.0;
+        if (n[u] < 0) continue;
+        m[u] = s.mg[n[u]];
+        sk[u] = s.shp[(k0 + u) * np + p];
+        y[u] = Recip{s.rm[n[u]], s.rm[nn + n[u]]};
         for (int d = 0; d < 3; ++d) {
-          vx[d] = vx[d] + sk * s.vg[(long long)d * nn + n];
-          ax[d] = ax[d] + sk * s.fx[(long long)d * nn + n] / m;
+          v[u][d] = s.vg[(long long)d * nn + n[u]];
+          f[u][d] = s.fx[(long long)d * nn + n[u]];
         }
       }
-    } else {
-      // mixed form: FP32 interpolation of the node velocity / acceleration
-      float v32[3] = {0, 0, 0}, a32[3] = {0, 0, 0};
-      for (int k = 0; k < g.K; ++k) {
-        int n = s.snode[k * np + p];
-        if (n < 0) continue;
-        double m = s.mg[n];
-        if (!(m > g.cutoff)) continue;
-        float sk = (float)s.shp[k * np + p];
-        float im = (float)(1.0 / m);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (n[u] < 0 || !(m[u] > g.cutoff)) continue;
         for (int d = 0; d < 3; ++d) {
-          v32[d] = v32[d] + sk * (float)s.vg[(long long)d * nn + n];
-          a32[d] = a32[d] + sk * (float)s.fx[(long long)d * nn + n] * im;
+          vx[d] = vx[d] + sk[u] * v[u][d];
+          ax[d] = ax[d] + div_known(sk[u] * f[u][d], m[u], y[u]);
         }
-      }
-      for (int d = 0; d < 3; ++d) {
-        vx[d] = v32[d];
-        ax[d] = a32[d];
       }
     }
   }
@@ -1249,7 +1322,7 @@ __global__ void k_p2g_momentum(St<P> s, Geometry g, int vel) {
         if (!in) return;
         for (int c = 0; c < 3; ++c) s.px[c * nn + n] = a[c];
         node_bc(s.fix[n % g.nn], s.px, s.fx, n, nn);
-        if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+        if (vel) node_vel(s.mg, s.rm, s.px, s.vg, n, nn, g.cutoff);
       });
 }
 
@@ -1315,12 +1388,13 @@ __global__ void k_sg_node_mass(St<P> s, Geometry g, int bc, int vel) {
       pz = pz + 0.125 * s.cpx[2 * nc + c];
     });
     s.mg[n] = m;
+    store_recip(s.rm, n, nn, m, g.cutoff);
     s.px[n] = px;
     s.px[nn + n] = py;
     s.px[2LL * nn + n] = pz;
     act = m > 0.0;
     if (bc) node_bc(s.fix[n], s.px, s.fx, (int)n, nn);
-    if (vel) node_vel(s.mg, s.px, s.vg, (int)n, nn, g.cutoff);
+    if (vel) node_vel(s.mg, s.rm, s.px, s.vg, (int)n, nn, g.cutoff);
   }
   count_active(act, &s.sc->active_nodes);
 }
@@ -1432,9 +1506,10 @@ __global__ void k_sg_cell_velocity(St<P> s, Geometry g) {
       int n = n1 + kCorner[j][0] + kCorner[j][1] * g.NGx + kCorner[j][2] * g.NGxy;
       double m = s.mg[n];
       if (!(m > g.cutoff)) continue;
+      const Recip y = {s.rm[n], s.rm[(long long)nn + n]};
       for (int d = 0; d < 3; ++d) {
-        v[d] = v[d] + 0.125 * s.px[(long long)d * nn + n] / m;
-        a[d] = a[d] + 0.125 * s.fx[(long long)d * nn + n] / m;
+        v[d] = v[d] + div_known(0.125 * s.px[(long long)d * nn + n], m, y);
+        a[d] = a[d] + div_known(0.125 * s.fx[(long long)d * nn + n], m, y);
       }
     }
   } else {
@@ -1454,9 +1529,10 @@ __global__ void k_sg_cell_velocity(St<P> s, Geometry g) {
       double w = sx * sy * sz * 0.125;
       double m = s.mg[n];
       if (!(m > g.cutoff)) continue;
+      const Recip y = {s.rm[n], s.rm[(long long)nn + n]};
       for (int d = 0; d < 3; ++d) {
-        v[d] = v[d] + w * s.px[(long long)d * nn + n] / m;
-        a[d] = a[d] + w * s.fx[(long long)d * nn + n] / m;
+        v[d] = v[d] + div_known(w * s.px[(long long)d * nn + n], m, y);
+        a[d] = a[d] + div_known(w * s.fx[(long long)d * nn + n], m, y);
       }
     }
   }
@@ -1498,7 +1574,7 @@ __global__ void k_sg_node_momentum(St<P> s, Geometry g, int vel) {
   s.px[nn + n] = py;
   s.px[2LL * nn + n] = pz;
   node_bc(s.fix[n], s.px, s.fx, (int)n, nn);
-  if (vel) node_vel(s.mg, s.px, s.vg, (int)n, nn, g.cutoff);
+  if (vel) node_vel(s.mg, s.rm, s.px, s.vg, (int)n, nn, g.cutoff);
 }
 
 // ================================================================= TLMPM
@@ -1560,7 +1636,7 @@ __global__ void k_tl_sg_node_momentum(St<P> s, Geometry g, int vel) {
   s.px[nn + n] = py;
   s.px[2LL * nn + n] = pz;
   node_bc(s.fix[n], s.px, s.fx, n, nn);
-  if (vel) node_vel(s.mg, s.px, s.vg, n, nn, g.cutoff);
+  if (vel) node_vel(s.mg, s.rm, s.px, s.vg, n, nn, g.cutoff);
 }
 
 // TLParticleStressUpdate + TLConstitution / M3DM11 (update_step.f90:649-828,

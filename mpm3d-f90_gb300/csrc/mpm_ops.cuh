@@ -6,7 +6,18 @@
 
 namespace mpm {
 
-inline unsigned grid_for(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
+// Launch shape of the one-thread-per-item kernels: blocks of 256, halved down
+// to one warp while there would be fewer than two blocks per SM. These kernels
+// are bound by the FP64 pipe of the SMs they run on (2 lanes per SM and clock),
+// so a small scene has to reach every SM: 5.8 k particles in blocks of 256
+// keep 23 of 152 SMs busy.
+struct Shape {
+  unsigned grid, block;
+  explicit Shape(long long n) : block(kBlock) {
+    while (block > 32 && (n + block - 1) / block < 304) block >>= 1;
+    grid = (unsigned)((n + block - 1) / block);
+  }
+};
 // blocks of a pair_walk kernel over n nodes or cells
 inline unsigned walk_grid(long long n) { return (unsigned)((n + kWalkNodes - 1) / kWalkNodes); }
 
@@ -21,7 +32,7 @@ struct Ops {
   }
   static void locate(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_LOCATE, s);
-    k_locate<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g, g.shape == 3 ? g.ncell : (int)g.nnt);
+    k_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g, g.shape == 3 ? g.ncell : (int)g.nnt);
     prof_end(K_LOCATE, s);
   }
   static void node_offsets(void*, const Geometry&, long long, cudaStream_t) {}
@@ -29,7 +40,7 @@ struct Ops {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
       k_sg_cell_mass<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
-      k_sg_node_mass<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, bc, vel);
+      k_sg_node_mass<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, bc, vel);
     } else {
       k_p2g_mass<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, bc, vel);
     }
@@ -37,36 +48,50 @@ struct Ops {
   }
   static void node_velocity(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_NODE_VEL, s);
-    k_node_velocity<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g);
+    k_node_velocity<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
     prof_end(K_NODE_VEL, s);
   }
   static void apply_bc(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_BC, s);
-    k_apply_bc<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g);
+    k_apply_bc<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
     prof_end(K_BC, s);
+  }
+  // the stress update's instantiation for the deck's one material type
+  template <int UV>
+  static void stress_of(void* st, const Geometry& g, cudaStream_t s) {
+    const Shape h(g.np);
+    switch (stress_has(S(st).mat_type) ? S(st).mat_type : 0) {
+      case 1: k_stress<P, 1, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 7: k_stress<P, 7, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 9: k_stress<P, 9, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 10: k_stress<P, 10, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 11: k_stress<P, 11, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      default: k_stress<P, 0, UV><<<h.grid, h.block, 0, s>>>(S(st), g);
+    }
   }
   static void stress(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_STRESS, s);
-    if (g.shape == 3) k_sg_cell_gradient<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
-    k_stress<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    if (g.shape == 3) k_sg_cell_gradient<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+    if (g.uvfp) stress_of<1>(st, g, s);
+    else stress_of<0>(st, g, s);
     prof_end(K_STRESS, s);
   }
   static void depeff_apply(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_DEPEFF, s);
-    k_depeff_apply<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    k_depeff_apply<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     k_depeff_carry<P><<<1, 1, 0, s>>>(S(st), g);
     prof_end(K_DEPEFF, s);
   }
   static void force_prep(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_FORCE_PREP, s);
-    k_force_prep<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    k_force_prep<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     prof_end(K_FORCE_PREP, s);
   }
   static void p2g_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
       k_sg_cell_force<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
-      k_sg_node_force<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, integ);
+      k_sg_node_force<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, integ);
     } else {
       if (g.contact) k_p2g_force<P, true><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
       else k_p2g_force<P, false><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
@@ -75,20 +100,20 @@ struct Ops {
   }
   static void integrate(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_INTEGRATE, s);
-    k_integrate<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g);
+    k_integrate<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
     prof_end(K_INTEGRATE, s);
   }
   static void position(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_POSITION, s);
-    if (g.shape == 3) k_sg_cell_velocity<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
-    k_position<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    if (g.shape == 3) k_sg_cell_velocity<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+    k_position<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     prof_end(K_POSITION, s);
   }
   static void p2g_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MOM, s);
     if (g.shape == 3) {
       k_sg_cell_momentum<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
-      k_sg_node_momentum<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, vel);
+      k_sg_node_momentum<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, vel);
     } else {
       k_p2g_momentum<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
     }
@@ -101,24 +126,24 @@ struct Ops {
   }
   static void dr_damping(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_DR, s);
-    k_dr_damping<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    k_dr_damping<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     k_dr_finish<<<1, 1, 0, s>>>(S(st).sc);
     prof_end(K_DR, s);
   }
 
   static void fixed_locate(void* st, const Geometry& g, int with_comp, cudaStream_t s) {
     prof_begin(K_LOCATE, s);
-    k_fixed_locate<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g, g.shape == 3 ? g.ncell : (int)g.nnt, with_comp);
+    k_fixed_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g, g.shape == 3 ? g.ncell : (int)g.nnt, with_comp);
     prof_end(K_LOCATE, s);
   }
   static void tl_initial(void* st, const Geometry& g, cudaStream_t s) {
-    k_tl_initial<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    k_tl_initial<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
   }
   static void tl_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
       k_sg_cell_momentum<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
-      k_tl_sg_node_momentum<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, vel);
+      k_tl_sg_node_momentum<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, vel);
     } else {
       k_p2g_momentum<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
     }
@@ -126,36 +151,36 @@ struct Ops {
   }
   static void tl_stress(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_STRESS, s);
-    if (g.shape == 3) k_sg_cell_gradient<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
-    k_tl_stress<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    if (g.shape == 3) k_sg_cell_gradient<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+    k_tl_stress<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     prof_end(K_STRESS, s);
   }
   static void tl_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
-      k_tl_sg_cell_force<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
-      k_tl_sg_node_force<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g, integ);
+      k_tl_sg_cell_force<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+      k_tl_sg_node_force<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, integ);
     } else {
-      k_tl_p2g_force<P><<<grid_for(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
+      k_tl_p2g_force<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g, integ);
     }
     prof_end(K_P2G_FORCE, s);
   }
   static void smooth(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_SMOOTH, s);
     if (g.shape == 3) {
-      k_smooth_cell<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
-      k_smooth_sg_node<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g);
-      k_smooth_sg_back<P><<<grid_for(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_smooth_cell<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+      k_smooth_sg_node<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
+      k_smooth_sg_back<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
     } else {
-      k_smooth_node<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g);
+      k_smooth_node<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
     }
-    k_smooth_g2p<P><<<grid_for(g.np), kBlock, 0, s>>>(S(st), g);
+    k_smooth_g2p<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     prof_end(K_SMOOTH, s);
   }
 
   static void contact(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_CONTACT, s);
-    k_contact<P><<<grid_for(g.nn), kBlock, 0, s>>>(S(st), g);
+    k_contact<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
     k_contact_sum<P><<<1, kBlock, 0, s>>>(S(st), g);
     prof_end(K_CONTACT, s);
   }
