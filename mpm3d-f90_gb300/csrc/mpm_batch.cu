@@ -354,12 +354,12 @@ template <class S>
 void scan_tiles_enqueue(const S& src, typename S::T* tiles, cudaStream_t st) {
   const long long nt = scan_tiles(src.n);
   if (nt <= 0) return;
-  ks_tile_total<S><<<(unsigned)nt, kScanThreads, 0, st>>>(src, tiles);
+  launch_chained(ks_tile_total<S>, (unsigned)nt, kScanThreads, st, src, tiles);
   if (nt <= kFusedTiles) {
-    ks_tile_scan<S, true><<<(unsigned)nt, kScanThreads, 0, st>>>(src, tiles);
+    launch_chained(ks_tile_scan<S, true>, (unsigned)nt, kScanThreads, st, src, tiles);
   } else {
-    ks_tile_prefix<typename S::T, typename S::Op><<<1, kScanThreads, 0, st>>>(tiles, nt);
-    ks_tile_scan<S, false><<<(unsigned)nt, kScanThreads, 0, st>>>(src, tiles);
+    launch_chained(ks_tile_prefix<typename S::T, typename S::Op>, 1, kScanThreads, st, tiles, nt);
+    launch_chained(ks_tile_scan<S, false>, (unsigned)nt, kScanThreads, st, src, tiles);
   }
 }
 
@@ -387,9 +387,9 @@ void enqueue_scatter(mpm_batch* b, int mode) {
   };
   // particle -> grid transfers: particle tasks of every scene
   cudaStream_t st = b->stream;
-  if (mode == 0) kb_part_scatter<0><<<pgrid(w0), 32 * w0, 0, st>>>(b->A);
-  else if (mode == 1) kb_part_scatter<1><<<pgrid(w1), 32 * w1, 0, st>>>(b->A);
-  else kb_part_scatter<2><<<pgrid(w2), 32 * w2, 0, st>>>(b->A);
+  if (mode == 0) launch_chained(kb_part_scatter<0>, pgrid(w0), 32 * w0, st, b->A);
+  else if (mode == 1) launch_chained(kb_part_scatter<1>, pgrid(w1), 32 * w1, st, b->A);
+  else launch_chained(kb_part_scatter<2>, pgrid(w2), 32 * w2, st, b->A);
 }
 
 int enqueue_front(mpm_batch* b) {
@@ -397,11 +397,11 @@ int enqueue_front(mpm_batch* b) {
   BState& s = b->A;
   const int nb = b->nblock;
   prof_begin(K_BEGIN, st);
-  kb_begin<<<gridn(s.nscene, 128), 128, 0, st>>>(s, b->d_target);
+  launch_chained(kb_begin, gridn(s.nscene, 128), 128, st, s, b->d_target);
   prof_end(K_BEGIN, st);
   if (b->any_sgmp) {
     prof_begin(K_SG_CLEAR, st);
-    kb_sg_clear<<<gridn(s.NC, nb), nb, 0, st>>>(s);
+    launch_chained(kb_sg_clear, gridn(s.NC, nb), nb, st, s);
     prof_end(K_SG_CLEAR, st);
   }
   prof_begin(K_SCATTER_MASS, st);
@@ -415,14 +415,14 @@ int enqueue_back(mpm_batch* b) {
   BState& s = b->A;
   const int pb = b->pblock, nb = b->nblock;
   prof_begin(K_P2G_MASS, st);
-  kb_p2g_mass<<<gridn(s.NN, nb) + 1, nb, 0, st>>>(s, 1, 1, b->d_target);  // (its last block starts the step)
+  launch_chained(kb_p2g_mass, gridn(s.NN, nb) + 1, nb, st, s, 1, 1, b->d_target);  // (its last block starts the step)
   prof_end(K_P2G_MASS, st);
   int r = enqueue_resort(b);
   if (r) return r;
   auto stress = [&](int usf_pass) -> int {
     if (b->any_sgmp) {
       prof_begin(K_SG_GRADIENT, st);
-      kb_sg_centre_gradient<<<gridn(s.NC, nb), nb, 0, st>>>(s, usf_pass);
+      launch_chained(kb_sg_centre_gradient, gridn(s.NC, nb), nb, st, s, usf_pass);
       prof_end(K_SG_GRADIENT, st);
     }
     prof_begin(K_STRESS, st);
@@ -431,7 +431,7 @@ int enqueue_back(mpm_batch* b) {
     // (and per volume update: by Fp or not)
     const unsigned ty = b->stress_types;
     const int f = __builtin_popcount(ty) > 1, uvf = b->any_uvfp && b->any_nonuvfp;
-    auto launch = [&](auto kern) { kern<<<gridn(s.NP, pb), pb, 0, st>>>(s, usf_pass, f, uvf); };
+    auto launch = [&](auto kern) { launch_chained(kern, gridn(s.NP, pb), pb, st, s, usf_pass, f, uvf); };
     if (b->any_nonuvfp) {
       if (ty & (1u << 1)) launch(kb_stress<1, 0>);
       if (ty & (1u << 9)) launch(kb_stress<9, 0>);
@@ -450,8 +450,8 @@ int enqueue_back(mpm_batch* b) {
     if (b->any_jc) {
       prof_begin(K_DEPEFF, st);
       scan_tiles_enqueue(IntScan<ScanMax>{s.setter, s.setter_scan, s.NP}, s.tiles, st);
-      kb_depeff_apply<<<gridn(s.NP, pb), pb, 0, st>>>(s, usf_pass);
-      kb_depeff_carry<<<gridn(s.nscene, 128), 128, 0, st>>>(s, usf_pass);
+      launch_chained(kb_depeff_apply, gridn(s.NP, pb), pb, st, s, usf_pass);
+      launch_chained(kb_depeff_carry, gridn(s.nscene, 128), 128, st, s, usf_pass);
       prof_end(K_DEPEFF, st);
     }
     return MPM_OK;
@@ -459,29 +459,29 @@ int enqueue_back(mpm_batch* b) {
   if (b->any_usf && (r = stress(1))) return r;
   if (b->any_prep) {  // (USF scenes without Johnson-Cook tails are staged by their stress kernel)
     prof_begin(K_FORCE_PREP, st);
-    kb_force_prep<<<gridn(s.NP, pb), pb, 0, st>>>(s);
+    launch_chained(kb_force_prep, gridn(s.NP, pb), pb, st, s);
     prof_end(K_FORCE_PREP, st);
   }
   prof_begin(K_SCATTER_FORCE, st);
   enqueue_scatter(b, 2);
   prof_end(K_SCATTER_FORCE, st);
   prof_begin(K_P2G_FORCE, st);
-  kb_p2g_force<<<gridn(s.NN, nb), nb, 0, st>>>(s);
+  launch_chained(kb_p2g_force, gridn(s.NN, nb), nb, st, s);
   prof_end(K_P2G_FORCE, st);
   if (b->any_sgmp) {
     prof_begin(K_SG_VELOCITY, st);
-    kb_sg_centre_velocity<<<gridn(s.NC, nb), nb, 0, st>>>(s);
+    launch_chained(kb_sg_centre_velocity, gridn(s.NC, nb), nb, st, s);
     prof_end(K_SG_VELOCITY, st);
   }
   prof_begin(K_POSITION, st);
-  kb_position<<<gridn(s.NP, pb), pb, 0, st>>>(s);
+  launch_chained(kb_position, gridn(s.NP, pb), pb, st, s);
   prof_end(K_POSITION, st);
   if (b->any_musl) {
     prof_begin(K_SCATTER_MOM, st);
     enqueue_scatter(b, 1);
     prof_end(K_SCATTER_MOM, st);
     prof_begin(K_P2G_MOM, st);
-    kb_p2g_momentum<<<gridn(s.NN, nb), nb, 0, st>>>(s);
+    launch_chained(kb_p2g_momentum, gridn(s.NN, nb), nb, st, s);
     prof_end(K_P2G_MOM, st);
   }
   if (b->any_later && (r = stress(0))) return r;
@@ -494,12 +494,12 @@ int enqueue_reduce(mpm_batch* b, cudaStream_t st) {
   BState& s = b->A;
   const int pb = b->pblock;
   prof_begin(K_REDUCE, st);
-  kb_reduce_chunks<<<(unsigned)s.NR, 256, 0, st>>>(s, 3);
+  launch_chained(kb_reduce_chunks, (unsigned)s.NR, 256, st, s, 3);
   prof_end(K_REDUCE, st);
   if (b->any_dr) {
     prof_begin(K_DR, st);
-    kb_dr_damping<<<gridn(s.NP, pb), pb, 0, st>>>(s);
-    kb_dr_finish<<<gridn(s.nscene, 128), 128, 0, st>>>(s);
+    launch_chained(kb_dr_damping, gridn(s.NP, pb), pb, st, s);
+    launch_chained(kb_dr_finish, gridn(s.nscene, 128), 128, st, s);
     prof_end(K_DR, st);
   }
   cudaError_t e = cudaGetLastError();
@@ -603,6 +603,7 @@ __global__ void kb_loop_start(BState b, const int* target, const volatile int* f
 }
 
 __global__ void kb_loop_test(BState b, const int* target, const volatile int* flag, cudaGraphConditionalHandle h) {
+  chain_entry();
   if (threadIdx.x == 0) b.ctl->iters = b.ctl->iters + 1;
   __syncthreads();
   loop_decide(b, target, flag, h);
@@ -645,7 +646,7 @@ int build_loop(mpm_batch* b, cudaGraphExec_t* out) {
   }
   r = enqueue_step_overlapped(b, true);
   if (!r) r = enqueue_step_overlapped(b, true);
-  if (!r) kb_loop_test<<<1, 256, 0, b->stream>>>(b->A, tgt, flag, h);
+  if (!r) launch_chained(kb_loop_test, 1, 256, b->stream, b->A, tgt, flag, h);
   cudaGraph_t body = nullptr;
   e = cudaStreamEndCapture(b->stream, &body);
   if (!r && e != cudaSuccess) r = berr(b, MPM_ERR_CUDA, "loop body capture: %s", cudaGetErrorString(e));
@@ -718,7 +719,7 @@ int commit(mpm_batch* b) {
     h->k0 = NK;
     h->c0 = NC;
     h->r0 = NR;
-    h->nr = (h->np + kChunk - 1) / kChunk;
+    h->nr = (h->np + reduce_chunk(h->np) - 1) / reduce_chunk(h->np);
     if (h->nr == 0) h->nr = 1;
     h->mat0 = nmat;
     h->body0 = nbody;
@@ -903,6 +904,8 @@ int commit(mpm_batch* b) {
     sc.fdcell = (float)g.dcell; sc.fidcell = (float)g.iDCell; sc.fbq1 = (float)g.bq1; sc.fbq2 = (float)g.bq2;
     sc.fdamp = (float)g.damp_factor; sc.fiJacobi4 = (float)g.iJacobi4; sc.fnp = (float)h->np;
     sc.has_fxp = h->any_fxp;
+    sc.chunk = reduce_chunk(h->np);
+    sc.wave = wave_speed(h->su.mats);
     for (int k = 0; k < 3; ++k) {
       sc.fspan0[k] = (float)g.span0[k];
       sc.fspan0_lo[k] = (float)(g.span0[k] - (double)sc.fspan0[k]);

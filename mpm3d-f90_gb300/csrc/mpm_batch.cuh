@@ -63,6 +63,8 @@ struct Scene {
   // n * m for 0 <= n < 2^32, m = floor(2^64 / d) + 1 (0 for d = 1), see div_by
   unsigned long long mNGx, mNGxy, mNCx, mNCxy, mCNCx, mCNCxy;
   int has_fxp;  // some particle of the scene carries an external force
+  int chunk;    // particles per reduction chunk
+  double wave;  // largest wave speed of the scene's materials (UpdateDT), < 0: none counts
 };
 
 struct SceneState {
@@ -138,7 +140,15 @@ struct BState {
   DevBody* bodies;   // gravp; mat = global material index
 };
 
-constexpr int kChunk = 2048;  // particles per reduction chunk
+// Particles per chunk of the energy reduction (one 256-thread block each). The
+// reduction is FP64 arithmetic on a pipe of two lanes per SM: 2048 particles
+// keep one SM's busy for about 10 us, which a small scene's step waits for
+// (it is over before the mass transfer beside it only from some 50 k particles
+// on); shorter chunks spend more on the blocks' summation trees, which a batch
+// of many scenes feels (512 for every scene up to 78 k: twelve served scenes
+// 334 -> 338 us per step; 2048 for every scene: 5.8 k particles 76 -> 82). A
+// function of the scene alone, so that its sums do not depend on the batch.
+inline int reduce_chunk(long long np) { return np <= 16384 ? 512 : (np <= 304 * 1024 ? 1024 : 2048); }
 
 // detonation points of a scene (the lighting time of explosive particles)
 struct DetoPoints {

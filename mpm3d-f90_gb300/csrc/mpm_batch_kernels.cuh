@@ -79,6 +79,7 @@ enum QSlot { Q_MASS = 0, Q_MOM = 1, Q_FORCE = 2, Q_MOM_MUSL = 3 };
 // and the mass transfer's count of particles out of order, and runs as the
 // last block of the mass finalize.
 __global__ void kb_begin(BState b, const int* target) {
+  chain_entry();
   int s = (int)btid();
   if (s == 0) b.gbar[0] = 0u;  // the re-sort's barrier
   if (s >= b.nscene) return;
@@ -588,6 +589,7 @@ __device__ __forceinline__ int dim_nodes(int shape, float off, int& t0, float w[
 // us for those kernels returning one by one (5.8 k to 1.2 M particles). The
 // barriers between the phases cost a re-sort about what launches would.
 __global__ void __launch_bounds__(kSortThreads, 3) kb_resort(BState a, BState o) {
+  chain_entry();
   if (!*a.any_resort) return;
   __shared__ int sm[kSmemSeg];  // (the scan's tile, then the long segments)
   __shared__ int thr[kSortThreads], wsum[32];
@@ -960,6 +962,7 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
 
 template <int MODE>
 __global__ void __launch_bounds__(32 * PartShape<MODE>::WARPS, MODE == 2 ? 6 : 4) kb_part_scatter(BState b) {
+  chain_entry();
   using PS = PartShape<MODE>;
   __shared__ float wsp[PS::WARPS][PS::ROWS * PS::STRIDE];
   const int warp = threadIdx.x >> 5;
@@ -1089,6 +1092,7 @@ __device__ __forceinline__ void step_tick(BState& b, const int* target) {
 }
 
 __global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target) {
+  chain_entry();
   if (blockIdx.x == gridDim.x - 1) {  // the last block starts the step instead of finishing nodes
     step_tick(b, target);
     return;
@@ -1402,6 +1406,7 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
 template <int MT, int UV>
 __global__ void __launch_bounds__(512, MT == 10 ? 3 : (MT ? 2 : 1))
     kb_stress(BState b, int usf_pass, int filter, int uvf) {
+  chain_entry();
   const long long i = btid();
   float bound = -1.f;
   if (i < b.NP) bound = stress_one<MT, UV>(b, i, usf_pass, filter, uvf);
@@ -1411,6 +1416,7 @@ __global__ void __launch_bounds__(512, MT == 10 ? 3 : (MT ? 2 : 1))
 // Johnson-Cook tails waiting for the depeff carried from the previous particle
 // in the reference order (scene-local input order)
 __global__ void kb_depeff_apply(BState b, int usf_pass) {
+  chain_entry();
   using P = PMixed;
   using R = float;
   long long i = btid();
@@ -1469,6 +1475,7 @@ __global__ void kb_depeff_apply(BState b, int usf_pass) {
 }
 
 __global__ void kb_depeff_carry(BState b, int usf_pass) {
+  chain_entry();
   int s = (int)btid();
   if (s >= b.nscene) return;
   const Scene& sc = b.scenes[s];
@@ -1530,6 +1537,7 @@ __device__ __forceinline__ float force_prep_one(BState& b, long long i) {
 }
 
 __global__ void kb_force_prep(BState b) {
+  chain_entry();
   const long long i = btid();
   float bound = -1.f;
   if (i < b.NP) bound = force_prep_one(b, i);
@@ -1561,6 +1569,7 @@ __device__ __forceinline__ void node_integrate(BState& b, const Scene& sc, long 
 }
 
 __global__ void kb_p2g_force(BState b) {
+  chain_entry();
   long long n = btid();
   if (n >= b.NN) return;
   const int s = b.node_scene[n];
@@ -1610,6 +1619,7 @@ __global__ void kb_p2g_force(BState b) {
 
 // SGMP: strain rate / spin at the centre nodes from the 8 cell nodes
 __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
+  chain_entry();
   long long c = btid();
   if (c >= b.NC) return;
   int s = b.cscene[c];
@@ -1654,6 +1664,7 @@ __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
 // SGMP: centre-node velocity / acceleration (BoundaryAuxiliaryNodeUpdate on
 // the fixed / symmetric faces)
 __global__ void kb_sg_centre_velocity(BState b) {
+  chain_entry();
   long long c = btid();
   if (c >= b.NC) return;
   int s = b.cscene[c];
@@ -1703,6 +1714,7 @@ __global__ void kb_sg_centre_velocity(BState b) {
 // SGMP: clears the mass and momentum sums of the live scenes' centre nodes
 // before the step's first transfer (they stay readable between steps)
 __global__ void kb_sg_clear(BState b) {
+  chain_entry();
   const long long c = btid();
   if (c >= b.NC) return;
   if (!scene_live(b, b.cscene[c])) return;
@@ -1817,6 +1829,7 @@ __device__ __forceinline__ float position_one(BState& b, long long i) {
 // gathers' latency better than fewer blocks with more registers; a pblock of
 // 512 still launches)
 __global__ void __launch_bounds__(512, 3) kb_position(BState b) {
+  chain_entry();
   const long long i = btid();
   float bound = -1.f;
   if (i < b.NP) bound = position_one(b, i);
@@ -1825,6 +1838,7 @@ __global__ void __launch_bounds__(512, 3) kb_position(BState b) {
 
 // GridMomentumMUSL: momentum re-map with the new particle velocities
 __global__ void kb_p2g_momentum(BState b) {
+  chain_entry();
   long long n = btid();
   if (n >= b.NN) return;
   const int s = b.node_scene[n];
@@ -1874,7 +1888,7 @@ __global__ void kb_p2g_momentum(BState b) {
 }
 
 // ------------------------------------------------------------ reductions
-// calcEnergy + UpdateDT per scene: a block per chunk of kChunk particles of
+// calcEnergy + UpdateDT per scene: a block per chunk (Scene::chunk particles) of
 // one scene (chunks are fixed relative to the scene start, so the sums of a
 // scene do not depend on the other scenes of the batch), then a block per
 // scene combining its chunks in order.
@@ -1911,27 +1925,21 @@ __device__ __forceinline__ void reduce_scene_finish(BState& b, int s, int mode, 
   }
   st.max_vp = sh[5][0];
   if (mode & 2) {
+    // the least time over the materials is the fastest one's (both roundings
+    // are monotonic)
     double dt = (double)1e6f;
-    for (int m = sc.mat0; m < sc.mat0 + sc.nmat; ++m) {
-      const DevMaterial& mt = b.mats[m];
-      if (mt.mat_type == 12) continue;
-      double E = mt.young, nu = mt.poisson, ro = mt.density;
-      double vv = sqrt(E * (1 - nu) / (1 + nu) / (1 - 2 * nu) / ro);
-      vv = fmax(vv, mt.D);
-      vv = fmax(vv, mt.wavespd);
-      vv = vv + sh[5][0];
-      dt = fmin(dt, sc.dcell / vv);
-    }
+    if (sc.wave >= 0.0) dt = fmin(dt, sc.dcell / (sc.wave + sh[5][0]));
     st.dt = dt * sc.dtscale;
     st.fdt = (float)st.dt;
   }
 }
 
-// calcEnergy / UpdateDT: one block per chunk of kChunk particles of a live
+// calcEnergy / UpdateDT: one block per chunk of particles of a live
 // scene sums the chunk in FP64 (the energy balance stays in FP64) and writes
 // its partial sums; the scene's last chunk block to finish (a per-scene
 // counter, reset by that block) forms the scene totals.
 __global__ void __launch_bounds__(256) kb_reduce_chunks(BState b, int mode) {
+  chain_entry();
   __shared__ double sh[6][256];
   __shared__ int last;
   const long long r = blockIdx.x;
@@ -1940,8 +1948,8 @@ __global__ void __launch_bounds__(256) kb_reduce_chunks(BState b, int mode) {
   const Scene& sc = b.scenes[s];
   const long long NP = b.NP;
   double acc[6] = {0, 0, 0, 0, 0, 0};
-  const long long p_begin = sc.p0 + (r - sc.r0) * kChunk;
-  const long long p_end = min(p_begin + kChunk, sc.p0 + sc.np);
+  const long long p_begin = sc.p0 + (r - sc.r0) * sc.chunk;
+  const long long p_end = min(p_begin + sc.chunk, sc.p0 + sc.np);
   for (long long i = p_begin + threadIdx.x; i < p_end; i += blockDim.x) {
     const double v0 = b.v[i], v1 = b.v[NP + i], v2 = b.v[2 * NP + i], m = b.mass[i];
     acc[0] += (v0 * v0 + v1 * v1 + v2 * v2) * m * 0.5;
@@ -1972,6 +1980,7 @@ __global__ void __launch_bounds__(256) kb_reduce_chunks(BState b, int mode) {
 }
 
 __global__ void kb_dr_damping(BState b) {
+  chain_entry();
   long long i = btid();
   if (i >= b.NP) return;
   const int s = b.scene[i];
@@ -1987,6 +1996,7 @@ __global__ void kb_dr_damping(BState b) {
 }
 
 __global__ void kb_dr_finish(BState b) {
+  chain_entry();
   int s = (int)btid();
   if (s >= b.nscene) return;
   if (!b.scenes[s].drdamp || !b.ract[s]) return;

@@ -214,6 +214,31 @@ struct StepOps {
 extern const StepOps kOpsStrict;   // MPM_FP64_STRICT
 extern const StepOps kOpsNative;   // MPM_FP64_NATIVE
 
+// Programmatic dependent launch. A kernel launched with launch_chained may be
+// brought up as its predecessor's last blocks exit; chain_entry, first thing in
+// the kernel, waits until the predecessor's grid has completed with its writes
+// visible (a no-op in a kernel launched plainly), so order is as without it and
+// only launch latency overlaps: 0.4 us per kernel, 79 -> 74.5 us per step of a
+// 5.8 k-particle scene. No kernel signals its successor earlier: blocks brought
+// up beside a predecessor that still runs are spread over the SMs it has
+// left, unevenly, and the 94 k-particle beam went from 112 to 131 us per step.
+__device__ __forceinline__ void chain_entry() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
 // Kernel launch bookkeeping for per-kernel event timing.
 void prof_begin(int kernel_id, cudaStream_t s);
 void prof_end(int kernel_id, cudaStream_t s);

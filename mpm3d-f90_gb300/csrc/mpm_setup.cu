@@ -211,6 +211,17 @@ int scene_setup(const mpm_deck* d, SceneSetup& out, bool particle_fields) {
   return MPM_OK;
 }
 
+double wave_speed(const std::vector<DevMaterial>& mats) {
+  double c = -1.0;
+  for (const auto& m : mats) {
+    if (m.mat_type == 12) continue;
+    const double E = m.young, nu = m.poisson, ro = m.density;
+    const double v = std::sqrt(E * (1 - nu) / (1 + nu) / (1 - 2 * nu) / ro);
+    c = std::fmax(c, std::fmax(std::fmax(v, m.D), m.wavespd));  // (a NaN does not count)
+  }
+  return c;
+}
+
 double set_dt(const std::vector<DevMaterial>& mats, double dcell, double dtscale) {
   double dt = (double)1.0e6f;
   for (const auto& m : mats) {

@@ -24,5 +24,7 @@ struct SceneSetup {
 int scene_setup(const mpm_deck* d, SceneSetup& out, bool particle_fields = true);
 // SetDT: the first time step of a material set.
 double set_dt(const std::vector<DevMaterial>& mats, double dcell, double dtscale);
+// largest wave speed of the materials that limit the step (-1: none does)
+double wave_speed(const std::vector<DevMaterial>& mats);
 
 }  // namespace mpm

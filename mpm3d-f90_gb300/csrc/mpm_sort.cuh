@@ -91,6 +91,7 @@ __device__ __forceinline__ void load_tile(const S& src, long long t, typename S:
 
 template <class S>
 __global__ void __launch_bounds__(kScanThreads) ks_tile_total(S src, typename S::T* tiles) {
+  chain_entry();
   using T = typename S::T;
   using Op = typename S::Op;
   __shared__ T tile[kScanTile];
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(kScanThreads) ks_tile_total(S src, typename S:
 // kScanThreads threads
 template <class T, class Op>
 __global__ void __launch_bounds__(kScanThreads) ks_tile_prefix(T* tiles, long long nt) {
+  chain_entry();
   __shared__ T thr[kScanThreads], wsum[32];
   T carry = Op::template id<T>();
   for (long long b0 = 0; b0 < nt; b0 += kScanThreads) {
@@ -126,6 +128,7 @@ __global__ void __launch_bounds__(kScanThreads) ks_tile_prefix(T* tiles, long lo
 constexpr long long kFusedTiles = 4096;
 template <class S, bool FUSED>
 __global__ void __launch_bounds__(kScanThreads) ks_tile_scan(S src, const typename S::T* tiles) {
+  chain_entry();
   using T = typename S::T;
   using Op = typename S::Op;
   __shared__ T tile[kScanTile];
