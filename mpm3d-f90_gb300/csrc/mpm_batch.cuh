@@ -22,7 +22,7 @@
 //     (kept for SGMP scenes). Linear / B-spline: one key per cell; GIMP:
 //     one key per node (the particle's nearest node); SGMP: one key per dual
 //     cell.
-//   P2G accumulators: acc[4][NN] 64-bit fixed point (see the scatter kernels).
+//   P2G accumulators: acc[NN][4] 64-bit fixed point (see the scatter kernels).
 //
 // Transfers particle -> grid are scatters of FP32 per-cell partial sums
 // (one warp per occupied cell, or dual cell for SGMP), summed exactly in
@@ -119,7 +119,7 @@ struct BState {
   // grid
   double *mg, *px, *fx;
   float4 *nvel, *nacc;             // FP32 px / mg and fx / mg for the gathers (zero at or below the cut-off)
-  unsigned long long* acc;         // [4][NN] fixed-point P2G sums, zero between transfers
+  unsigned long long* acc;         // [NN][4] fixed-point P2G sums, zero between transfers
   uint8_t *fix, *bd;
   uint16_t* node_scene;
   // SGMP centre grid

@@ -660,11 +660,24 @@ __device__ __forceinline__ long long sg_corner_cell(const Scene& sc, int dx, int
 //   f_x = Dx (-s_xx Wy Wz) + Wx (b_x Wy Wz - s_xy Dy Wz - s_xz Wy Dz).
 // Two phases through the warp's shared workspace:
 //   1. lane = particle: its x factors (W, and D for the force) per x offset
-//      and its (y, z) factors per channel, one column per lane;
-//   2. lane = box slot: the walk along the task's particles in storage order
-//      (FP32 sums of x factor times (y, z) factor, every channel at once),
-//      flushed at every segment end -- quantised and added to the node's
-//      64-bit accumulators with one integer atomic per channel.
+//      and its (y, z) factors per channel;
+//   2. lane = (y, z) row of the box and channel: the walk along the task's
+//      particles in storage order (FP32 sums of x factor times (y, z) factor for
+//      the row's three nodes). The sums of a node are quantised and added to its
+//      64-bit accumulator with one integer atomic when the walk leaves the node:
+//      a segment whose box lies one node further along x -- the usual next key
+//      -- leaves one node of the row, any other box all three.
+// Bound by instruction issue and the shared-memory / L1 data pipe (76 and 60 % of
+// their slots for the mass transfer, 62 and 60 % for the force, on the 1.2
+// M-particle slope; L2 atomics 20 %). A lane per node and all its channels read
+// 5 (mass and momentum), 8 (force) and 4 (MUSL) shared words per particle and
+// flushed every node at every segment end; a lane per row and channel reads its
+// own factors and the x factors that all lanes share (a broadcast): 4, 4 and 2,
+// the force's as pairs for paired multiply-adds (two per instruction), and
+// flushes under half as often. A node's accumulators are adjacent
+// (acc[node][4], one 32-byte sector), which a row's lanes hit together. Force
+// 93 -> 79, mass 84 -> 78 us (1.2 M particles, GIMP); 309 -> 250, 282 -> 250,
+// MUSL 229 -> 181 us (4.1 M); 120 -> 109, 107 -> 105, 87 -> 77 us (2 M, B-spline).
 // The task boundaries are fixed by the scene's own sorted order (32 t from
 // the scene's first particle), so a scene's sums are the same alone or in a
 // batch. Phase 2's walk and its segment ends are the same for every lane
@@ -672,13 +685,28 @@ __device__ __forceinline__ long long sg_corner_cell(const Scene& sc, int dx, int
 // there.
 template <int MODE>
 struct PartShape {
-  static constexpr int NV = MODE == 0 ? 4 : 3;          // channels
-  static constexpr int NX = MODE == 2 ? 6 : 3;          // x-factor rows (W, and D, per x offset)
-  static constexpr int NK = MODE == 2 ? 2 : 1;          // (y, z) factors per channel and (ty, tz)
-  static constexpr int ROWS = NX + 9 * NV * NK;         // workspace rows (one column per lane)
-  static constexpr int STRIDE = 33;                     // row stride: conflict-free in both phases
+  static constexpr int PF = MODE == 2 ? 6 : 3;          // (y, z) factors per particle and (ty, tz)
+  // floats per (ty, tz) row of 32 particles: the rows' factors of one particle
+  // and the particles' of one row both fall on distinct banks
+  static constexpr int PITCH = 32 * PF + PF;
+  static constexpr int XF = MODE == 2 ? 8 : 4;          // x factors per particle: W, or (D, W), per offset
+  static constexpr int XAT = (9 * PITCH + 3) / 4 * 4;   // the x factors' place in the workspace
+  static constexpr int STRIDE = 33;                     // row stride of the mass factors and of the SGMP form
+  static constexpr int MAT = XAT + 32 * XF;             // the mass factors' place (mode 0)
+  static constexpr int WS = MAT + (MODE == 0 ? 9 * STRIDE + 3 : 0);  // workspace floats of a warp (a multiple of 4)
   static constexpr int WARPS = MODE == 2 ? 4 : 8;       // warps (tasks) per block (static shared memory)
 };
+
+// acc + a * b on both halves of a pair (one instruction)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 acc) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(acc.x), "f"(acc.y));
+  return d;
+}
 
 // 1-D weight w[t] and derivative d[t] (per unit length) of node offset t
 // from the key's base (linear: 0..1 from the cell; B-spline: -1..1 from the
@@ -712,8 +740,8 @@ template <int MODE, int SH>
 __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, long long i0, int cnt, float sA,
                                                  float sB, float* ws) {
   using PS = PartShape<MODE>;
-  constexpr int NV = PS::NV, NX = PS::NX, NK = PS::NK, ST = PS::STRIDE;
-  constexpr int nt = SH == 0 ? 2 : 3, tlo = SH == 0 ? 0 : -1, NS = nt * nt * nt;
+  constexpr int PF = PS::PF, PITCH = PS::PITCH, XF = PS::XF;
+  constexpr int nt = SH == 0 ? 2 : 3, tlo = SH == 0 ? 0 : -1, NL = 3 * nt * nt;
   const int lane = threadIdx.x & 31;
   const long long NP = b.NP, i = i0 + lane;
   int c[3] = {0, 0, 0};
@@ -775,82 +803,122 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
 #pragma unroll
       for (int a = 0; a < 3; ++a) part_tab<SH>(off[a], idc, w[a], d[a]);
     }
-    float* col = ws + lane;
-#pragma unroll
-    for (int t = 0; t < nt; ++t) {
-      col[t * ST] = w[0][t];
-      if (MODE == 2) col[(3 + t) * ST] = d[0][t];
+    float* xf = ws + PS::XAT + lane * XF;
+    if (MODE != 2) {
+      *reinterpret_cast<float4*>(xf) = make_float4(w[0][0], w[0][1], w[0][2], 0.f);
+    } else {
+      *reinterpret_cast<float4*>(xf) = make_float4(d[0][0], w[0][0], d[0][1], w[0][1]);
+      if (nt == 3) *reinterpret_cast<float2*>(xf + 4) = make_float2(d[0][2], w[0][2]);
     }
+    float* col = ws + lane * PF;
 #pragma unroll
     for (int tz = 0; tz < nt; ++tz)
 #pragma unroll
       for (int ty = 0; ty < nt; ++ty) {
-        const int yz = tz * nt + ty;
+        float* f = col + (tz * nt + ty) * PITCH;
         const float A = w[1][ty] * w[2][tz];
         if (MODE == 2) {
           const float B = d[1][ty] * w[2][tz], C = w[1][ty] * d[2][tz];
-          // per channel: o0 (times D) and o1 (times W)
-          col[(NX + 0 * 9 + yz) * ST] = -pv[0] * A;
-          col[(NX + 1 * 9 + yz) * ST] = pv[6] * A - pv[3] * B - pv[5] * C;
-          col[(NX + 2 * 9 + yz) * ST] = -pv[3] * A;
-          col[(NX + 3 * 9 + yz) * ST] = pv[7] * A - pv[1] * B - pv[4] * C;
-          col[(NX + 4 * 9 + yz) * ST] = -pv[5] * A;
-          col[(NX + 5 * 9 + yz) * ST] = pv[8] * A - pv[4] * B - pv[2] * C;
+          // per channel: the factor of D and the factor of W
+          float2* f2 = reinterpret_cast<float2*>(f);
+          f2[0] = make_float2(-pv[0] * A, pv[6] * A - pv[3] * B - pv[5] * C);
+          f2[1] = make_float2(-pv[3] * A, pv[7] * A - pv[1] * B - pv[4] * C);
+          f2[2] = make_float2(-pv[5] * A, pv[8] * A - pv[4] * B - pv[2] * C);
         } else {
           const float M = pv[0] * A;
-          if (MODE == 0) col[(NX + yz) * ST] = M;
+          if (MODE == 0) ws[PS::MAT + (tz * nt + ty) * PS::STRIDE + lane] = M;
 #pragma unroll
-          for (int a = 0; a < 3; ++a) col[(NX + (MODE == 0 ? 1 + a : a) * 9 + yz) * ST] = M * pv[1 + a];
+          for (int a = 0; a < 3; ++a) f[a] = M * pv[1 + a];
         }
       }
   }
   __syncwarp();
-  // phase 2: lane = box slot (sx, sy, sz), the walk along the particles
-  const int sz = lane / (nt * nt), sy = (lane / nt) % nt, sx = lane % nt;
-  const int yz = lane < NS ? sz * nt + sy : 0;
-  const int soff = (sz * sc.NGy + sy) * sc.NGx + sx;
-  const float* xw = ws + (lane < NS ? sx : 0) * ST;
-  const float* xd = ws + (lane < NS ? 3 + sx : 0) * ST;
-  const float* fr = ws + (NX + yz) * ST;
+  // phase 2: lane = (y, z) row of the box and channel, the walk along the
+  // particles
+  const int yz = lane < NL ? lane / 3 : 0, ch = lane % 3;
+  const int sz = yz / nt, sy = yz % nt;
+  const int soff = (sz * sc.NGy + sy) * sc.NGx;
+  const float* xr = ws + PS::XAT;
+  const float* fr = ws + yz * PITCH + (MODE == 2 ? 2 * ch : ch);
+  const float* mr = ws + (MODE == 0 ? PS::MAT + yz * PS::STRIDE : 0);
   // segment by segment: the segment ends come from a warp vote, so the walk
-  // and its flushes are the same for every lane
+  // and its flushes are the same for every lane. acc[a] is the lane's channel
+  // at node a of its row's window; a segment whose box lies one node further
+  // along x slides the window (its first node is flushed, the other two go
+  // on), any other box flushes it
+  unsigned long long* an = nullptr;  // the window's first node, and its x
+  int wb = -2, wx = 0;
+  bool row_in = false;
+  float acc[3] = {0.f, 0.f, 0.f}, mass = 0.f;  // (mode 0: mass = node ch of the window)
+  auto flush = [&](int a) {
+    const long long q = quant(acc[a], MODE == 0 ? sB : sA);
+    if (q && row_in && wx + a >= 0 && wx + a < sc.NGx)
+      atomicAdd(an + 4 * a + (MODE == 0 ? 1 + ch : ch), (unsigned long long)q);
+  };
+  auto flush_mass = [&](bool mine) {
+    const long long q = quant(mass, sA);
+    if (q && mine && row_in && wx + ch >= 0 && wx + ch < sc.NGx) atomicAdd(an + 4 * ch, (unsigned long long)q);
+  };
   unsigned rem = lasts;
   int j = 0;
   while (rem) {
     const int e = __ffs(rem) - 1;  // the segment's last lane
     rem &= rem - 1;
-    float acc[NV];
+    const int nb = __shfl_sync(0xffffffffu, nbase, e), jx = __shfl_sync(0xffffffffu, c[0], e) + tlo;
+    if (nb == wb + 1 && jx == wx + 1) {
+      flush(0);
+      if (MODE == 0) {
+        flush_mass(ch == 0);
+        mass = __shfl_down_sync(0xffffffffu, mass, 1);
+        if (ch == nt - 1) mass = 0.f;
+      }
+      acc[0] = acc[1];
+      acc[1] = nt == 3 ? acc[2] : 0.f;
+      acc[2] = 0.f;
+      an += 4;
+    } else {
+      if (an) {
 #pragma unroll
-    for (int v = 0; v < NV; ++v) acc[v] = 0.f;
+        for (int a = 0; a < nt; ++a) flush(a);
+        if (MODE == 0) flush_mass(ch < nt);
+      }
+      row_in = lane < NL;
+      if (!__shfl_sync(0xffffffffu, (int)inner, e)) {  // (uniform) a box at the grid's edge
+        const int jy = __shfl_sync(0xffffffffu, c[1], e) + tlo + sy, jz = __shfl_sync(0xffffffffu, c[2], e) + tlo + sz;
+        row_in = row_in && jy >= 0 && jy < sc.NGy && jz >= 0 && jz < sc.NGz;
+      }
+      acc[0] = acc[1] = acc[2] = mass = 0.f;
+      an = b.acc + 4 * (sc.n0 + nb + soff);
+    }
+    wb = nb;
+    wx = jx;
+    if (MODE != 2) {
 #pragma unroll 4
-    for (; j <= e; ++j) {
-      const float x = xw[j];
-      if (MODE == 2) {
-        const float dx = xd[j];
-#pragma unroll
-        for (int v = 0; v < 3; ++v) acc[v] += dx * fr[(2 * v) * 9 * ST + j] + x * fr[(2 * v + 1) * 9 * ST + j];
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v] += x * fr[v * 9 * ST + j];
+      for (; j <= e; ++j) {
+        const float4 x = *reinterpret_cast<const float4*>(xr + j * XF);
+        const float f = fr[j * PF];
+        acc[0] += x.x * f;
+        acc[1] += x.y * f;
+        if (nt == 3) acc[2] += x.z * f;
+        if (MODE == 0) mass += xr[j * XF + ch] * mr[j];
       }
-    }
-    // flush the segment's sums into the nodes
-    const int nb = __shfl_sync(0xffffffffu, nbase, e);
-    bool ok = lane < NS;
-    if (!__shfl_sync(0xffffffffu, (int)inner, e)) {  // (uniform) a box at the grid's edge
-      const int jx = __shfl_sync(0xffffffffu, c[0], e) + tlo + sx, jy = __shfl_sync(0xffffffffu, c[1], e) + tlo + sy,
-                jz = __shfl_sync(0xffffffffu, c[2], e) + tlo + sz;
-      ok = ok && jx >= 0 && jx < sc.NGx && jy >= 0 && jy < sc.NGy && jz >= 0 && jz < sc.NGz;
-    }
-    if (ok) {
-      const long long n = sc.n0 + nb + soff;
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        const long long q = quant(acc[v], MODE == 0 && v > 0 ? sB : sA);
-        if (q) atomicAdd(&b.acc[v * b.NN + n], (unsigned long long)q);
+    } else {
+      float2 s[3] = {{acc[0], 0.f}, {acc[1], 0.f}, {acc[2], 0.f}};
+#pragma unroll 4
+      for (; j <= e; ++j) {
+        const float4 x = *reinterpret_cast<const float4*>(xr + j * XF);
+        const float2 f = *reinterpret_cast<const float2*>(fr + j * PF);
+        s[0] = fma2(make_float2(x.x, x.y), f, s[0]);
+        s[1] = fma2(make_float2(x.z, x.w), f, s[1]);
+        if (nt == 3) s[2] = fma2(*reinterpret_cast<const float2*>(xr + j * XF + 4), f, s[2]);
       }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) acc[a] = s[a].x + s[a].y;
     }
   }
+#pragma unroll
+  for (int a = 0; a < nt; ++a) flush(a);
+  if (MODE == 0) flush_mass(ch < nt);
   __syncwarp();
   return dis;
 }
@@ -964,7 +1032,7 @@ template <int MODE>
 __global__ void __launch_bounds__(32 * PartShape<MODE>::WARPS, MODE == 2 ? 6 : 4) kb_part_scatter(BState b) {
   chain_entry();
   using PS = PartShape<MODE>;
-  __shared__ float wsp[PS::WARPS][PS::ROWS * PS::STRIDE];
+  __shared__ __align__(16) float wsp[PS::WARPS][PS::WS];
   const int warp = threadIdx.x >> 5;
   const int nt = b.task0[b.nscene];
   int ds = -1, dis = 0;  // scene of the warp's last task, its particles out of order so far
@@ -1010,17 +1078,13 @@ __global__ void __launch_bounds__(32 * PartShape<MODE>::WARPS, MODE == 2 ? 6 : 4
 // integrates every node, so its momentum is F * DT) carries a mass of -0 as
 // the mark that its fields are not zero, and the next transfer clears them.
 __device__ __forceinline__ bool take_acc(BState& b, long long n, int nv, const double* unit, double* out) {
-  unsigned long long q[4];
-  unsigned long long any = 0ull;
-  for (int v = 0; v < nv; ++v) {
-    q[v] = b.acc[v * b.NN + n];
-    any |= q[v];
-  }
+  ulonglong2* qa = reinterpret_cast<ulonglong2*>(b.acc + 4 * n);
+  const ulonglong2 lo = qa[0], hi = qa[1];
+  const unsigned long long q[4] = {lo.x, lo.y, hi.x, hi.y};
+  const unsigned long long any = lo.x | lo.y | hi.x | hi.y;  // (a channel past nv is zero)
   if (any == 0ull && __double_as_longlong(b.mg[n]) == 0ll) return false;
-  for (int v = 0; v < nv; ++v) {
-    out[v] = (double)(long long)q[v] * unit[v];
-    if (q[v]) b.acc[v * b.NN + n] = 0ull;
-  }
+  for (int v = 0; v < nv; ++v) out[v] = (double)(long long)q[v] * unit[v];
+  if (any) qa[0] = qa[1] = make_ulonglong2(0ull, 0ull);
   return true;
 }
 
