@@ -290,7 +290,7 @@ long long scene_bytes(long long np, long long nn, long long ncell, bool sgmp, bo
   if (jc) per_p += 4 * 2 + 8 * 6 + 1;
   long long per_n = 8 * 13 + 4 + 8 * 4;
   long long per_k = 4 * 2;                                                // segment ends, fill counters
-  long long per_c = sgmp ? 8 * 39 + 2 : 0;
+  long long per_c = sgmp ? 8 * 13 + 16 * 5 + 1 + 2 : 0;  // sums, gradient + velocity + acceleration, mark, scene
   return np * per_p + nn * per_n + (std::max(nn, ncell) + 1) * per_k + ncell * per_c + 4096;
 }
 
@@ -415,7 +415,9 @@ int enqueue_back(mpm_batch* b) {
   BState& s = b->A;
   const int pb = b->pblock, nb = b->nblock;
   prof_begin(K_P2G_MASS, st);
-  launch_chained(kb_p2g_mass, gridn(s.NN, nb) + 1, nb, st, s, 1, 1, b->d_target);  // (its last block starts the step)
+  // (the last block of the first one starts the step)
+  if (b->any_nonsgmp) launch_chained(kb_p2g_mass<false>, gridn(s.NN, nb) + 1, nb, st, s, 1, 1, b->d_target, 1);
+  if (b->any_sgmp) launch_chained(kb_p2g_mass<true>, gridn(s.NN, nb) + 1, nb, st, s, 1, 1, b->d_target, !b->any_nonsgmp);
   prof_end(K_P2G_MASS, st);
   int r = enqueue_resort(b);
   if (r) return r;
@@ -466,7 +468,8 @@ int enqueue_back(mpm_batch* b) {
   enqueue_scatter(b, 2);
   prof_end(K_SCATTER_FORCE, st);
   prof_begin(K_P2G_FORCE, st);
-  launch_chained(kb_p2g_force, gridn(s.NN, nb), nb, st, s);
+  if (b->any_nonsgmp) launch_chained(kb_p2g_force<false>, gridn(s.NN, nb), nb, st, s);
+  if (b->any_sgmp) launch_chained(kb_p2g_force<true>, gridn(s.NN, nb), nb, st, s);
   prof_end(K_P2G_FORCE, st);
   if (b->any_sgmp) {
     prof_begin(K_SG_VELOCITY, st);
@@ -481,7 +484,8 @@ int enqueue_back(mpm_batch* b) {
     enqueue_scatter(b, 1);
     prof_end(K_SCATTER_MOM, st);
     prof_begin(K_P2G_MOM, st);
-    launch_chained(kb_p2g_momentum, gridn(s.NN, nb), nb, st, s);
+    if (b->any_nonsgmp) launch_chained(kb_p2g_momentum<false>, gridn(s.NN, nb), nb, st, s);
+    if (b->any_sgmp) launch_chained(kb_p2g_momentum<true>, gridn(s.NN, nb), nb, st, s);
     prof_end(K_P2G_MOM, st);
   }
   if (b->any_later && (r = stress(0))) return r;
@@ -781,11 +785,10 @@ int commit(mpm_batch* b) {
   shared.bd = al.get<uint8_t>(NN);
   shared.node_scene = al.get<uint16_t>(NN);
   shared.cacc = al.get<unsigned long long>(CQ_N * NC);
-  shared.co = al.get<float>(6 * NC);
-  shared.cw = al.get<float>(3 * NC);
-  shared.cdefp = al.get<float>(9 * NC);
-  shared.cvx = al.get<float>(3 * NC);
-  shared.cax = al.get<float>(3 * NC);
+  shared.cact = al.get<uint8_t>(NC);
+  shared.cgrad = al.get<float4>(3 * NC);
+  shared.cvel = al.get<float4>(NC);
+  shared.cacl = al.get<float4>(NC);
   shared.cscene = al.get<uint16_t>(NC);
   if (b->any_jc) {
     shared.setter = al.get<int>(NP);
@@ -841,8 +844,8 @@ int commit(mpm_batch* b) {
     s.perm = shared.perm; s.seg = shared.seg; s.inv = shared.inv;
     s.fill = shared.fill; s.tiles = shared.tiles; s.big = shared.big; s.nbig = shared.nbig; s.mg = shared.mg; s.px = shared.px; s.fx = shared.fx;
     s.nvel = shared.nvel; s.nacc = shared.nacc; s.acc = shared.acc; s.fix = shared.fix; s.bd = shared.bd; s.node_scene = shared.node_scene;
-    s.cacc = shared.cacc; s.co = shared.co;
-    s.cw = shared.cw; s.cdefp = shared.cdefp; s.cvx = shared.cvx; s.cax = shared.cax; s.cscene = shared.cscene;
+    s.cacc = shared.cacc; s.cact = shared.cact; s.cgrad = shared.cgrad;
+    s.cvel = shared.cvel; s.cacl = shared.cacl; s.cscene = shared.cscene;
     s.setter = shared.setter; s.setter_scan = shared.setter_scan; s.dep = shared.dep; s.jc_aux = shared.jc_aux;
     s.deferred = shared.deferred; s.red_part = shared.red_part; s.rscene = shared.rscene; s.scenes = shared.scenes;
     s.task0 = shared.task0; s.disorder = shared.disorder; s.resort = shared.resort; s.shift = shared.shift;
@@ -968,7 +971,13 @@ int commit(mpm_batch* b) {
   BCK(cudaMemsetAsync(shared.nvel, 0, sizeof(float4) * NN, st));
   BCK(cudaMemsetAsync(shared.nacc, 0, sizeof(float4) * NN, st));
   BCK(cudaMemsetAsync(shared.acc, 0, sizeof(unsigned long long) * 4 * NN, st));
-  if (NC) BCK(cudaMemsetAsync(shared.cacc, 0, sizeof(unsigned long long) * CQ_N * NC, st));
+  if (NC) {
+    BCK(cudaMemsetAsync(shared.cacc, 0, sizeof(unsigned long long) * CQ_N * NC, st));
+    BCK(cudaMemsetAsync(shared.cact, 0, NC, st));
+    BCK(cudaMemsetAsync(shared.cgrad, 0, sizeof(float4) * 3 * NC, st));
+    BCK(cudaMemsetAsync(shared.cvel, 0, sizeof(float4) * NC, st));
+    BCK(cudaMemsetAsync(shared.cacl, 0, sizeof(float4) * NC, st));
+  }
   // every depeff setter entry is -1 or its own index (the max-scan relies on
   // it); only Johnson-Cook scenes rewrite theirs each step
   if (b->any_jc) {

@@ -16,7 +16,7 @@
 //     acceleration (for the particle gathers); fix, bd, node scene
 //   SGMP centre nodes (one per cell) concatenated: 64-bit fixed-point
 //     accumulators cacc[13] (mass, momentum[3], external force[3], internal
-//     force[6]); FP32 co[6], cw[3], cdefp[9], cvx[3], cax[3]
+//     force[6]); FP32 velocity gradient, velocity, acceleration
 //   sort keys: scene s owns keys [k0, k0 + nk), the last one collects the
 //     particles outside its grid; seg[k] = end of key k's particle range
 //     (kept for SGMP scenes). Linear / B-spline: one key per cell; GIMP:
@@ -123,8 +123,10 @@ struct BState {
   uint8_t *fix, *bd;
   uint16_t* node_scene;
   // SGMP centre grid
-  unsigned long long* cacc;            // [CQ_N][NC] fixed-point particle -> centre sums (channels below)
-  float *co, *cw, *cdefp, *cvx, *cax;  // derived from node velocities / accelerations (FP32)
+  unsigned long long* cacc;  // [CQ_N][NC] fixed-point particle -> centre sums (channels below)
+  uint8_t* cact;             // the cell is a corner of a dual cell with particles this step
+  float4* cgrad;             // [3][NC] velocity gradient, row a: dv_a / dx, dy, dz (FP32)
+  float4 *cvel, *cacl;       // velocity and acceleration (FP32)
   uint16_t* cscene;
   // Johnson-Cook depeff carry (indexed by scene particle range + orig)
   int *setter, *setter_scan;

@@ -929,13 +929,16 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
 // 8 corner weights -- times the mass for the momentum transfers -- and the
 // transferred values; phase 2 (lane = corner and channel) walks the task's
 // particles and flushes each segment's sums, quantised, into the centre
-// nodes' 64-bit accumulators. Channels: mode 0 mass and momentum (CenterNode
-// Mg, PXg), 1 momentum with the updated velocities, 2 external then internal
-// force (Cfext, Cfint); a lane takes the corner lane / 4 (mode 0) or lane / 3
-// (modes 1, 2: one channel, or three force channels g, g + 3, g + 6).
+// nodes' 64-bit accumulators. A segment whose dual
+// cell lies one further along x shares four corners with the one before: its
+// lanes take those sums over and only the four corners left behind are flushed.
+// Channels: mode 0 mass and momentum (CenterNode Mg, PXg), 1 momentum with the
+// updated velocities, 2 external then internal force (Cfext, Cfint); a lane
+// takes the corner lane / 4 (mode 0) or lane / 3 (modes 1, 2: one channel, or
+// three force channels g, g + 3, g + 6), corners numbered x + 2 y + 4 z.
 template <int MODE>
 __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long long i0, int cnt, float sA, float sB,
-                                             float* ws) {
+                                            float* ws) {
   constexpr int ST = PartShape<MODE>::STRIDE;
   constexpr int CH0 = MODE == 2 ? CQ_FE : (MODE == 1 ? CQ_P : CQ_M);  // first accumulator channel
   const int lane = threadIdx.x & 31;
@@ -957,6 +960,11 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
   const int knext = __shfl_down_sync(0xffffffffu, d, 1);
   const unsigned lasts = __ballot_sync(0xffffffffu, d >= 0 && (lane == 31 || knext != d));
   if (lasts == 0u) return dis;  // (uniform) nothing of this task on the dual grid
+  int c1 = -1;  // first corner of the dual cell (sg_corner_cell)
+  if (d >= 0) {
+    const int dz = div_by(d, sc.mCNCxy), rm = d - dz * sc.CNCxy, dy = div_by(rm, sc.mCNCx), dx = rm - dy * sc.CNCx;
+    c1 = (dz * sc.NCy + dy) * sc.NCx + dx;
+  }
   // phase 1: rows 0..7 the corner weights (times the mass for modes 0, 1),
   // then the values (velocity, or the 9 force inputs)
   {
@@ -971,7 +979,7 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
     for (int k = 0; k < 8; ++k) {
       float w = 0.125f;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) w *= kCorner[k][a] ? 1.f + xx[a] : 1.f - xx[a];
+      for (int a = 0; a < 3; ++a) w *= (k >> a & 1) ? 1.f + xx[a] : 1.f - xx[a];
       col[k * ST] = d < 0 ? 0.f : (MODE == 2 ? w : w * m);
     }
     if (MODE == 2) {
@@ -986,18 +994,49 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
   // phase 2
   constexpr int NPER = MODE == 0 ? 4 : 3;  // lanes per corner
   const int k = lane / NPER, g = lane - k * NPER;
-  const bool active = k < 8;
+  const bool active = k < 8, left = (k & 1) == 0;
   const float* wr = ws + (active ? k : 0) * ST;
   const float* vr = ws + (8 + (MODE == 0 ? (g > 0 ? g - 1 : 0) : g)) * ST;
   constexpr int NA = MODE == 2 ? 3 : 1;  // accumulators per lane
+  const int koff = (k & 1) + (k >> 1 & 1) * sc.NCx + (k >> 2 & 1) * sc.NCxy;
+  const int ncell = sc.NCxy * sc.NCz;
+  float acc[NA];
+#pragma unroll
+  for (int a = 0; a < NA; ++a) acc[a] = 0.f;
+  int wc = -2;  // first corner of the window
+  auto flush = [&](bool mine) {
+    const int cid = wc + koff;  // (corners past the last cell are dropped)
+    if (!mine || !active || cid >= ncell) return;
+    unsigned long long* ca = b.cacc + (CH0 + g) * b.NC + sc.c0 + cid;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      const long long q = quant(acc[a], MODE == 0 && g != 0 ? sB : sA);
+      if (q) atomicAdd(ca + 3 * a * b.NC, (unsigned long long)q);
+    }
+    // every corner of a dual cell with particles takes part in the step,
+    // whether or not a sum reached it (the auxiliary weights near a fixed
+    // face differ from these)
+    if (MODE == 0 && g == 0) b.cact[sc.c0 + cid] = 1;
+  };
   unsigned rem = lasts;
   int j = 0;
   while (rem) {  // segment by segment (uniform: the segment ends come from a warp vote)
     const int e = __ffs(rem) - 1;
     rem &= rem - 1;
-    float acc[NA];
+    const int cj = __shfl_sync(0xffffffffu, c1, e);
+    if (cj == wc + 1) {
+      flush(left);
 #pragma unroll
-    for (int a = 0; a < NA; ++a) acc[a] = 0.f;
+      for (int a = 0; a < NA; ++a) {
+        const float r = __shfl_down_sync(0xffffffffu, acc[a], NPER);
+        acc[a] = left ? r : 0.f;
+      }
+    } else {
+      if (wc >= 0) flush(true);
+#pragma unroll
+      for (int a = 0; a < NA; ++a) acc[a] = 0.f;
+    }
+    wc = cj;
 #pragma unroll 4
     for (; j <= e; ++j) {
       const float w = wr[j];
@@ -1010,20 +1049,8 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
         acc[0] += w * vr[j];
       }
     }
-    const int dj = __shfl_sync(0xffffffffu, d, e);  // flush into the centre nodes
-    if (active) {
-      const int dz = div_by(dj, sc.mCNCxy), rm = dj - dz * sc.CNCxy, dy = div_by(rm, sc.mCNCx), dx = rm - dy * sc.CNCx;
-      const long long cid = sg_corner_cell(sc, dx, dy, dz, k);
-      if (cid >= 0) {
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          const int ch = MODE == 2 ? g + 3 * a : g;
-          const long long q = quant(acc[a], MODE == 0 && ch != 0 ? sB : sA);
-          if (q) atomicAdd(&b.cacc[(long long)(CH0 + ch) * b.NC + sc.c0 + cid], (unsigned long long)q);
-        }
-      }
-    }
   }
+  flush(true);
   __syncwarp();
   return dis;
 }
@@ -1155,9 +1182,30 @@ __device__ __forceinline__ void step_tick(BState& b, const int* target) {
   if (threadIdx.x == 0) *b.any_resort = any;
 }
 
-__global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target) {
+// the cells next to grid node j that take part in the step (bit dx + 2 dy + 4 dz
+// for the cell j - 1 + (dx, dy, dz)), and the flat index of such a cell
+__device__ __forceinline__ long long sg_near_cell(const Scene& sc, const int j[3], int k) {
+  const int cx = j[0] - 1 + (k & 1), cy = j[1] - 1 + (k >> 1 & 1), cz = j[2] - 1 + (k >> 2);
+  return sc.c0 + (cz * sc.NCy + cy) * sc.NCx + cx;
+}
+__device__ __forceinline__ unsigned sg_active_cells(const BState& b, const Scene& sc, const int j[3]) {
+  unsigned m = 0u;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int cx = j[0] - 1 + (k & 1), cy = j[1] - 1 + (k >> 1 & 1), cz = j[2] - 1 + (k >> 2);
+    if (cx >= 0 && cx < sc.NCx && cy >= 0 && cy < sc.NCy && cz >= 0 && cz < sc.NCz)
+      m |= (unsigned)b.cact[sg_near_cell(sc, j, k)] << k;
+  }
+  return m;
+}
+
+// SG: the nodes of the SGMP scenes (an instantiation of its own: the 8 cells' loads
+// in flight take registers that the others would pay for); tick: the last
+// block starts the step
+template <bool SG>
+__global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target, int tick) {
   chain_entry();
-  if (blockIdx.x == gridDim.x - 1) {  // the last block starts the step instead of finishing nodes
+  if (tick && blockIdx.x == gridDim.x - 1) {  // the last block starts the step instead of finishing nodes
     step_tick(b, target);
     return;
   }
@@ -1166,40 +1214,44 @@ __global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target
   int s = -1;
   if (n < b.NN) {
     s = b.node_scene[n];
-    if (scene_live(b, s)) {
+    if (scene_live(b, s) && (b.scenes[s].shape == 3) == SG) {
       const Scene& sc = b.scenes[s];
       const long long NN = b.NN;
       double M = 0, P0 = 0, P1 = 0, P2 = 0;
       bool live = true;
-      int j[3];
-      node_xyz(sc, n - sc.n0, j[0], j[1], j[2]);
-      if (sc.shape == 3) {
+      if (SG) {
+        int j[3];
+        node_xyz(sc, n - sc.n0, j[0], j[1], j[2]);
         // centre nodes -> node (GridMomentumInitial of SGMP): 1/8 of the
         // adjacent cells' mass and momentum, cells at or below the cut-off
         // mass left out; the cells' fixed-point sums are added exactly
+        const unsigned near = sg_active_cells(b, sc, j);
+        live = near || __double_as_longlong(b.mg[n]) != 0ll;  // (else idle, as in take_acc)
         const SceneState& st = b.sst[s];
         const int shm = q_shift(sc, st.qmax[Q_MASS]);
         const double um = q_unit(shm), up = q_unit(q_shift(sc, st.qmax[Q_MOM]));
         // cm = q * um > cutoff  <=>  q > floor(cutoff / um) (um a power of two)
         const double thr = ldexp(sc.cutoff, shm);
         const long long qcut = thr >= 9.0e18 ? LLONG_MAX : (long long)floor(thr);
-        const unsigned long long* ca = b.cacc;
-        const long long NC = b.NC;
         long long QM = 0, Q0 = 0, Q1 = 0, Q2 = 0;
-        for (int cz = j[2] - 1; cz <= j[2]; ++cz) {
-          if (cz < 0 || cz >= sc.NCz) continue;
-          for (int cy = j[1] - 1; cy <= j[1]; ++cy) {
-            if (cy < 0 || cy >= sc.NCy) continue;
-            for (int cx = j[0] - 1; cx <= j[0]; ++cx) {
-              if (cx < 0 || cx >= sc.NCx) continue;
-              const long long c = sc.c0 + (cz * sc.NCy + cy) * sc.NCx + cx;
-              const long long qm = (long long)ca[CQ_M * NC + c];
-              if (qm <= qcut) continue;
-              QM += qm;
-              Q0 += (long long)ca[CQ_P * NC + c];
-              Q1 += (long long)ca[(CQ_P + 1) * NC + c];
-              Q2 += (long long)ca[(CQ_P + 2) * NC + c];
-            }
+        const long long* ca = reinterpret_cast<const long long*>(b.cacc);
+#pragma unroll
+        for (int k0 = 0; k0 < 8; k0 += 4) {  // (four cells' loads in flight at a time)
+          long long q[4][4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const bool on = near >> (k0 + k) & 1u;
+            const long long c = sg_near_cell(sc, j, k0 + k);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) q[k][a] = on ? ca[(CQ_M + a) * b.NC + c] : 0;
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (q[k][0] <= qcut) continue;
+            QM += q[k][0];
+            Q0 += q[k][1];
+            Q1 += q[k][2];
+            Q2 += q[k][3];
           }
         }
         M = 0.125 * ((double)QM * um);
@@ -1224,7 +1276,7 @@ __global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target
         b.px[2 * NN + n] = P2;
         act = M > 0.0;
         node_finish(b, sc, n, bc_usf && sc.usf, vel_usf && sc.usf);
-        if (!(M != 0.0) && sc.shape != 3) {
+        if (!(M != 0.0)) {
           // the node goes idle: clear the rest of its fields once (the idle
           // test of the later transfers skips it from now on)
           for (int a = 0; a < 3; ++a) b.fx[a * NN + n] = 0.0;
@@ -1312,10 +1364,12 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
       const long long c = sc.c0 + cid;
       float w = 0.125f;
       for (int a = 0; a < 3; ++a) w *= oc[a] ? 1.f + xx[a] : 1.f - xx[a];
-      const long long NC = b.NC;
-      for (int a = 0; a < 6; ++a) de[a] += b.co[a * NC + c] * w;
-      for (int a = 0; a < 3; ++a) vort[a] += b.cw[a * NC + c] * w;
-      for (int a = 0; a < 9; ++a) deFp[a / 3][a % 3] += w * b.cdefp[a * NC + c];
+      for (int a = 0; a < 3; ++a) {
+        const float4 r = b.cgrad[a * b.NC + c];
+        deFp[a][0] += w * r.x;
+        deFp[a][1] += w * r.y;
+        deFp[a][2] += w * r.z;
+      }
     }
   } else {
     const int cl = b.cell[i];
@@ -1367,16 +1421,16 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
     const float idc = sc.fidcell;
     for (int a = 0; a < 3; ++a)
       for (int k = 0; k < 3; ++k) deFp[a][k] = L[a][k] * idc;
-    de[0] = deFp[0][0];
-    de[1] = deFp[1][1];
-    de[2] = deFp[2][2];
-    de[3] = deFp[2][1] + deFp[1][2];
-    de[4] = deFp[0][2] + deFp[2][0];
-    de[5] = deFp[1][0] + deFp[0][1];
-    vort[0] = deFp[2][1] - deFp[1][2];
-    vort[1] = deFp[0][2] - deFp[2][0];
-    vort[2] = deFp[1][0] - deFp[0][1];
   }
+  de[0] = deFp[0][0];
+  de[1] = deFp[1][1];
+  de[2] = deFp[2][2];
+  de[3] = deFp[2][1] + deFp[1][2];
+  de[4] = deFp[0][2] + deFp[2][0];
+  de[5] = deFp[1][0] + deFp[0][1];
+  vort[0] = deFp[2][1] - deFp[1][2];
+  vort[1] = deFp[0][2] - deFp[2][0];
+  vort[2] = deFp[1][0] - deFp[0][1];
   const SceneState& st = b.sst[s];
   const R DT = st.fdt;
   for (int a = 0; a < 6; ++a) de[a] *= DT;
@@ -1621,7 +1675,7 @@ __device__ __forceinline__ void node_integrate(BState& b, const Scene& sc, long 
   }
   node_finish(b, sc, n, 1, 1);
   const double m = b.mg[n];
-  if (m == 0.0 && sc.shape != 3) b.mg[n] = -0.0;  // fields not zero at a massless node (take_acc)
+  if (m == 0.0) b.mg[n] = -0.0;  // fields not zero at a massless node (take_acc)
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   if (m > sc.cutoff) {
     const float m32 = (float)m;
@@ -1632,43 +1686,51 @@ __device__ __forceinline__ void node_integrate(BState& b, const Scene& sc, long 
   b.nacc[n] = acc;
 }
 
-__global__ void kb_p2g_force(BState b) {
+// (the SGMP form keeps two cells' nine loads in flight at 64 registers)
+template <bool SG>
+__global__ void __launch_bounds__(512, SG ? 2 : 1) kb_p2g_force(BState b) {
   chain_entry();
   long long n = btid();
   if (n >= b.NN) return;
   const int s = b.node_scene[n];
   if (!scene_live(b, s)) return;
   const Scene& sc = b.scenes[s];
-  int j[3];
-  node_xyz(sc, n - sc.n0, j[0], j[1], j[2]);
+  if ((sc.shape == 3) != SG) return;
   double F[3] = {0, 0, 0};
-  if (sc.shape == 3) {
+  if (SG) {
+    int j[3];
+    node_xyz(sc, n - sc.n0, j[0], j[1], j[2]);
     // centre nodes -> node (GridMomentumUpdate of SGMP): 1/8 of the cells'
     // external force minus Cfint . dN, dN = +-1 / (4 Jacobi) per direction
     // by the node's side of the cell; the cells' fixed-point sums are
     // combined exactly, then scaled once
-    const long long NC = b.NC;
-    const unsigned long long* ca = b.cacc;
+    const unsigned near = sg_active_cells(b, sc, j);
+    if (!near && __double_as_longlong(b.mg[n]) == 0ll) return;  // idle node (as in take_acc)
     long long E[3] = {0, 0, 0}, T[3] = {0, 0, 0};
-    for (int cz = j[2] - 1; cz <= j[2]; ++cz) {
-      if (cz < 0 || cz >= sc.NCz) continue;
-      for (int cy = j[1] - 1; cy <= j[1]; ++cy) {
-        if (cy < 0 || cy >= sc.NCy) continue;
-        for (int cx = j[0] - 1; cx <= j[0]; ++cx) {
-          if (cx < 0 || cx >= sc.NCx) continue;
-          const long long c = sc.c0 + (cz * sc.NCy + cy) * sc.NCx + cx;
-          long long I[6];
-          for (int a = 0; a < 3; ++a) E[a] += (long long)ca[(CQ_FE + a) * NC + c];
-          for (int a = 0; a < 6; ++a) I[a] = (long long)ca[(CQ_FI + a) * NC + c];
-          // signed by the node's side: +dN at the upper corner of the cell
-          const bool ux = j[0] != cx, uy = j[1] != cy, uz = j[2] != cz;
-          const long long xx = ux ? I[0] : -I[0], xy_x = ux ? I[3] : -I[3], xz_x = ux ? I[5] : -I[5];
-          const long long xy_y = uy ? I[3] : -I[3], yy = uy ? I[1] : -I[1], yz_y = uy ? I[4] : -I[4];
-          const long long xz_z = uz ? I[5] : -I[5], yz_z = uz ? I[4] : -I[4], zz = uz ? I[2] : -I[2];
-          T[0] += xx + xy_y + xz_z;
-          T[1] += xy_x + yy + yz_z;
-          T[2] += xz_x + yz_y + zz;
-        }
+    const long long* ca = reinterpret_cast<const long long*>(b.cacc) + CQ_FE * b.NC;
+#pragma unroll
+    for (int k0 = 0; k0 < 8; k0 += 2) {  // (two cells' loads in flight at a time)
+      long long q[2][9];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const bool on = near >> (k0 + u) & 1u;
+        const long long c = sg_near_cell(sc, j, k0 + u);
+#pragma unroll
+        for (int a = 0; a < 9; ++a) q[u][a] = on ? ca[a * b.NC + c] : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int k = k0 + u;
+        const long long* I = q[u] + 3;
+        for (int a = 0; a < 3; ++a) E[a] += q[u][a];
+        // signed by the node's side: +dN at the upper corner of the cell
+        const bool ux = !(k & 1), uy = !(k & 2), uz = !(k & 4);
+        const long long xx = ux ? I[0] : -I[0], xy_x = ux ? I[3] : -I[3], xz_x = ux ? I[5] : -I[5];
+        const long long xy_y = uy ? I[3] : -I[3], yy = uy ? I[1] : -I[1], yz_y = uy ? I[4] : -I[4];
+        const long long xz_z = uz ? I[5] : -I[5], yz_z = uz ? I[4] : -I[4], zz = uz ? I[2] : -I[2];
+        T[0] += xx + xy_y + xz_z;
+        T[1] += xy_x + yy + yz_z;
+        T[2] += xz_x + yz_y + zz;
       }
     }
     const double u = q_unit(q_shift(sc, b.sst[s].qmax[Q_FORCE]));
@@ -1681,7 +1743,8 @@ __global__ void kb_p2g_force(BState b) {
   node_integrate(b, sc, n, F);
 }
 
-// SGMP: strain rate / spin at the centre nodes from the 8 cell nodes
+// SGMP: velocity gradient at the centre nodes from the 8 cell nodes (the strain
+// rate and spin of the particles are its symmetric and antisymmetric parts)
 __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
   chain_entry();
   long long c = btid();
@@ -1689,7 +1752,7 @@ __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
   int s = b.cscene[c];
   if (!scene_live(b, s)) return;
   const Scene& sc = b.scenes[s];
-  if (sc.usf != usf_pass) return;
+  if (sc.usf != usf_pass || !b.cact[c]) return;
   const long long NC = b.NC;
   long long lc = c - sc.c0;
   int q[3];
@@ -1697,7 +1760,7 @@ __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
   int rem = (int)(lc - (long long)q[2] * sc.NCxy);
   q[1] = div_by(rem, sc.mNCx);
   q[0] = rem - q[1] * sc.NCx;
-  float co[6] = {0, 0, 0, 0, 0, 0}, cw[3] = {0, 0, 0}, cf[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  float cf[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   const float j4 = sc.fiJacobi4;
   for (int k = 0; k < 8; ++k) {
     long long n = sc.n0 + ((long long)(q[2] + kCorner[k][2]) * sc.NGy + q[1] + kCorner[k][1]) * sc.NGx + q[0] +
@@ -1705,24 +1768,13 @@ __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
     const float4 v4 = b.nvel[n];  // zero below the cut-off mass
     const float v[3] = {v4.x, v4.y, v4.z};
     const float dx = kSN[0][k] * j4, dy = kSN[1][k] * j4, dz = kSN[2][k] * j4;
-    co[0] += dx * v[0];
-    co[1] += dy * v[1];
-    co[2] += dz * v[2];
-    co[3] += dz * v[1] + dy * v[2];
-    co[4] += dz * v[0] + dx * v[2];
-    co[5] += dy * v[0] + dx * v[1];
-    cw[0] += dy * v[2] - dz * v[1];
-    cw[1] += dz * v[0] - dx * v[2];
-    cw[2] += dx * v[1] - dy * v[0];
     for (int a = 0; a < 3; ++a) {
-      cf[a * 3 + 0] += dx * v[a];
-      cf[a * 3 + 1] += dy * v[a];
-      cf[a * 3 + 2] += dz * v[a];
+      cf[a][0] += dx * v[a];
+      cf[a][1] += dy * v[a];
+      cf[a][2] += dz * v[a];
     }
   }
-  for (int a = 0; a < 6; ++a) b.co[a * NC + c] = co[a];
-  for (int a = 0; a < 3; ++a) b.cw[a * NC + c] = cw[a];
-  for (int a = 0; a < 9; ++a) b.cdefp[a * NC + c] = cf[a];
+  for (int a = 0; a < 3; ++a) b.cgrad[a * NC + c] = make_float4(cf[a][0], cf[a][1], cf[a][2], 0.f);
 }
 
 // SGMP: centre-node velocity / acceleration (BoundaryAuxiliaryNodeUpdate on
@@ -1733,6 +1785,7 @@ __global__ void kb_sg_centre_velocity(BState b) {
   if (c >= b.NC) return;
   int s = b.cscene[c];
   if (!scene_live(b, s)) return;
+  if (!b.cact[c]) return;
   const Scene& sc = b.scenes[s];
   long long lc = c - sc.c0;
   int q[3];
@@ -1741,7 +1794,6 @@ __global__ void kb_sg_centre_velocity(BState b) {
   q[1] = div_by(rem, sc.mNCx);
   q[0] = rem - q[1] * sc.NCx;
   const int NCd[3] = {sc.NCx, sc.NCy, sc.NCz};
-  const long long NC = b.NC;
   bool boundary = false;
   for (int a = 0; a < 3; ++a)
     if (NCd[a] > 1 && ((q[a] == 0 && sc.fixs[2 * a] != 0) || (q[a] == NCd[a] - 1 && sc.fixs[2 * a + 1] != 0)))
@@ -1766,22 +1818,24 @@ __global__ void kb_sg_centre_velocity(BState b) {
     acc[1] += w * an.y;
     acc[2] += w * an.z;
   }
-  for (int a = 0; a < 3; ++a) {
-    b.cvx[a * NC + c] = v[a];
-    b.cax[a * NC + c] = acc[a];
-  }
+  b.cvel[c] = make_float4(v[0], v[1], v[2], 0.f);
+  b.cacl[c] = make_float4(acc[0], acc[1], acc[2], 0.f);
   // the force sums are consumed (and so are the momentum sums when the
   // MUSL transfer refills them): cleared for the next scatter
-  for (int a = sc.musl ? CQ_P : CQ_FE; a < CQ_N; ++a) b.cacc[a * NC + c] = 0ull;
+  for (int a = sc.musl ? CQ_P : CQ_FE; a < CQ_N; ++a) b.cacc[a * b.NC + c] = 0ull;
 }
 
 // SGMP: clears the mass and momentum sums of the live scenes' centre nodes
-// before the step's first transfer (they stay readable between steps)
+// before the step's first transfer (they stay readable between steps) and the
+// marks of the cells that took part in the last step. Only marked cells are
+// touched here, by the node kernels and by the centre kernels: a beam's grid
+// is five sixths empty.
 __global__ void kb_sg_clear(BState b) {
   chain_entry();
   const long long c = btid();
   if (c >= b.NC) return;
-  if (!scene_live(b, b.cscene[c])) return;
+  if (!scene_live(b, b.cscene[c]) || !b.cact[c]) return;
+  b.cact[c] = 0;
   for (int a = CQ_M; a < CQ_FE; ++a) b.cacc[a * b.NC + c] = 0ull;
 }
 
@@ -1817,18 +1871,19 @@ __device__ __forceinline__ float position_one(BState& b, long long i) {
     }
     if (bd == 0)
       for (int a = 0; a < 3; ++a) xx[a] = b.xxn[a * NP + i];
-    const long long NC = b.NC;
     for (int k = 0; k < 8; ++k) {
       int oc[3] = {kCorner[k][0], kCorner[k][1], kCorner[k][2]};
       const long long cid = sg_corner_cell(sc, dx, dy, dz, k);
       if (cid < 0) continue;
-      const long long c = sc.c0 + cid;
+      const float4 cv = b.cvel[sc.c0 + cid], ca = b.cacl[sc.c0 + cid];
       float w = 0.125f;
       for (int a = 0; a < 3; ++a) w *= oc[a] ? 1.f + xx[a] : 1.f - xx[a];
-      for (int a = 0; a < 3; ++a) {
-        v[a] += w * b.cvx[a * NC + c];
-        acc[a] += w * b.cax[a * NC + c];
-      }
+      v[0] += w * cv.x;
+      v[1] += w * cv.y;
+      v[2] += w * cv.z;
+      acc[0] += w * ca.x;
+      acc[1] += w * ca.y;
+      acc[2] += w * ca.z;
     }
   } else {
     const int cl = b.cell[i];
@@ -1901,6 +1956,7 @@ __global__ void __launch_bounds__(512, 3) kb_position(BState b) {
 }
 
 // GridMomentumMUSL: momentum re-map with the new particle velocities
+template <bool SG>
 __global__ void kb_p2g_momentum(BState b) {
   chain_entry();
   long long n = btid();
@@ -1908,27 +1964,31 @@ __global__ void kb_p2g_momentum(BState b) {
   const int s = b.node_scene[n];
   if (!scene_live(b, s)) return;
   const Scene& sc = b.scenes[s];
-  if (!sc.musl) return;
+  if (!sc.musl || (sc.shape == 3) != SG) return;
   const long long NN = b.NN;
-  int j[3];
-  node_xyz(sc, n - sc.n0, j[0], j[1], j[2]);
   double P0 = 0, P1 = 0, P2 = 0;
-  if (sc.shape == 3) {
+  if (SG) {
+    int j[3];
+    node_xyz(sc, n - sc.n0, j[0], j[1], j[2]);
     // centre nodes -> node (GridMomentumMUSL of SGMP), exact sums of the
     // cells' fixed-point momenta
-    const long long NC = b.NC;
-    const unsigned long long* ca = b.cacc;
+    const unsigned near = sg_active_cells(b, sc, j);
+    if (!near && __double_as_longlong(b.mg[n]) == 0ll) return;  // idle node (as in take_acc)
     long long Q[3] = {0, 0, 0};
-    for (int cz = j[2] - 1; cz <= j[2]; ++cz) {
-      if (cz < 0 || cz >= sc.NCz) continue;
-      for (int cy = j[1] - 1; cy <= j[1]; ++cy) {
-        if (cy < 0 || cy >= sc.NCy) continue;
-        for (int cx = j[0] - 1; cx <= j[0]; ++cx) {
-          if (cx < 0 || cx >= sc.NCx) continue;
-          const long long c = sc.c0 + (cz * sc.NCy + cy) * sc.NCx + cx;
-          for (int a = 0; a < 3; ++a) Q[a] += (long long)ca[(CQ_P + a) * NC + c];
-        }
+    const long long* ca = reinterpret_cast<const long long*>(b.cacc) + CQ_P * b.NC;
+#pragma unroll
+    for (int k0 = 0; k0 < 8; k0 += 4) {  // (four cells' loads in flight at a time)
+      long long q[4][3];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool on = near >> (k0 + k) & 1u;
+        const long long c = sg_near_cell(sc, j, k0 + k);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) q[k][a] = on ? ca[a * b.NC + c] : 0;
       }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        for (int a = 0; a < 3; ++a) Q[a] += q[k][a];
     }
     const double u = q_unit(q_shift(sc, b.sst[s].qmax[Q_MOM_MUSL]));
     P0 = 0.125 * ((double)Q[0] * u);
@@ -1946,7 +2006,7 @@ __global__ void kb_p2g_momentum(BState b) {
   b.px[n] = P0;
   b.px[NN + n] = P1;
   b.px[2 * NN + n] = P2;
-  if (sc.shape != 3 && b.mg[n] == 0.0 && (P0 != 0.0 || P1 != 0.0 || P2 != 0.0))
+  if (b.mg[n] == 0.0 && (P0 != 0.0 || P1 != 0.0 || P2 != 0.0))
     b.mg[n] = -0.0;  // momentum at a massless node (take_acc)
   node_finish(b, sc, n, 1, !sc.usf);
 }
@@ -2303,7 +2363,7 @@ __global__ void kb_centre_field(BState b, int scene, int comp, double* dst) {
   const SceneState& st = b.sst[scene];
   const int q = comp < 0 ? Q_MASS : (sc.musl ? Q_MOM_MUSL : Q_MOM);
   const int ch = comp < 0 ? CQ_M : CQ_P + comp;
-  dst[k] = (double)(long long)b.cacc[(long long)ch * b.NC + sc.c0 + k] * q_unit(q_shift(sc, st.qmax[q]));
+  dst[k] = (double)(long long)b.cacc[ch * b.NC + sc.c0 + k] * q_unit(q_shift(sc, st.qmax[q]));
 }
 
 }  // namespace bm
