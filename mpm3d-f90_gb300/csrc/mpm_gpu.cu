@@ -8,9 +8,6 @@
 // mpm_run replays it from a captured CUDA graph.
 #include <cuda_runtime.h>
 
-#include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
-
 #include <algorithm>
 #include <cstdarg>
 #include <cmath>
@@ -23,6 +20,8 @@
 
 #include "mpm3d_gpu.h"
 #include "mpm_gpu_internal.cuh"
+#include "mpm_ops.cuh"
+#include "mpm_pairs.cuh"
 #include "mpm_batch_host.h"
 #include "mpm_setup.h"
 
@@ -31,10 +30,6 @@ using namespace mpm;
 namespace {
 
 thread_local std::string g_lib_error;
-
-struct MaxOp {
-  __host__ __device__ int operator()(int a, int b) const { return a > b ? a : b; }
-};
 
 }  // namespace
 
@@ -57,10 +52,7 @@ struct mpm_ctx {
   long long bytes = 0;
   int nkeys = 0;
   long long npairs = 0;
-  int key_bits = 1;
   int red_blocks = 1;
-  void* cub_tmp = nullptr;
-  size_t cub_tmp_bytes = 0;
   cudaGraphExec_t graph_exec = nullptr;
   int graph_steps = 0;
   bool graph_prof = false;
@@ -289,27 +281,41 @@ int upload_as(mpm_ctx* c, void* dst, const double* src, long long n, size_t elem
 }
 
 // ------------------------------------------------------------ sorting
+template <class Src>
+void scan_tiles(const Src& src, typename Src::T* tiles, cudaStream_t st) {
+  const unsigned nt = (unsigned)bm::scan_tiles(src.n);
+  bm::ks_tile_total<Src><<<nt, bm::kScanThreads, 0, st>>>(src, tiles);
+  if (nt <= bm::kFusedTiles) {
+    bm::ks_tile_scan<Src, true><<<nt, bm::kScanThreads, 0, st>>>(src, tiles);
+  } else {
+    bm::ks_tile_prefix<typename Src::T, typename Src::Op><<<1, bm::kScanThreads, 0, st>>>(tiles, nt);
+    bm::ks_tile_scan<Src, false><<<nt, bm::kScanThreads, 0, st>>>(src, tiles);
+  }
+}
+
+// the node-sorted pair list from the slots' nodes and the per-node counts
 int sort_pairs(mpm_ctx* c) {
   DevState<double, double>& s = c->st;
-  prof_begin(K_SORT, c->stream);
-  size_t tmp = c->cub_tmp_bytes;
-  cudaError_t e = cub::DeviceRadixSort::SortPairs(c->cub_tmp, tmp, s.key, s.key_sorted, s.val, s.val_sorted,
-                                                  (int)c->npairs, 0, c->key_bits, c->stream);
-  if (e != cudaSuccess) return cuda_err(c, e, "radix sort");
-  // per-node pair counts -> inclusive prefix sums (segment ends)
-  tmp = c->cub_tmp_bytes;
-  e = cub::DeviceScan::InclusiveSum(c->cub_tmp, tmp, s.seg, s.seg, c->nkeys, c->stream);
-  if (e != cudaSuccess) return cuda_err(c, e, "segment scan");
-  prof_end(K_SORT, c->stream);
+  cudaStream_t st = c->stream;
+  const long long np = c->g.np;
+  prof_begin(K_SORT, st);
+  scan_tiles(PairScan{s.seg, s.fill, c->nkeys}, s.tiles, st);
+  k_pair_place<<<dim3((unsigned)((np + 255) / 256), (unsigned)c->g.K), 256, 0, st>>>(s.snode, s.seg, s.fill,
+                                                                                    s.val_sorted, np, s.nbig);
+  k_pair_order<<<(unsigned)(((long long)c->nkeys * 32 + 127) / 128), 128, 0, st>>>(s.seg, c->nkeys, s.val_sorted, s.big,
+                                                                                 s.nbig);
+  k_pair_long<<<76, bm::kSortThreads, 0, st>>>(s.seg, s.val_sorted, s.big, s.nbig);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_err(c, e, "pair sort");
+  prof_end(K_SORT, st);
   return MPM_OK;
 }
 
 int depeff_pass(mpm_ctx* c) {
   if (!c->g.has_jc) return MPM_OK;
   DevState<double, double>& s = c->st;
-  size_t tmp = c->cub_tmp_bytes;
-  cudaError_t e = cub::DeviceScan::InclusiveScan(c->cub_tmp, tmp, s.setter, s.setter_scan, MaxOp(),
-                                                 (int)c->g.np, c->stream);
+  scan_tiles(bm::IntScan<bm::ScanMax>{s.setter, s.setter_scan, c->g.np}, s.tiles, c->stream);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "depeff scan");
   c->ops->depeff_apply(&c->st, c->g, c->stream);
   return MPM_OK;
@@ -519,15 +525,13 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
   c->nkeys = g.shape == 3 ? (int)nc : (int)nnt;  // pair keys: (component, node) or centre node
   c->npairs = np * K;
   if (c->npairs >= (1LL << 31) || np >= (1LL << 27) || nnt >= (1LL << 31)) {
-    // pair values hold particle * 32 + slot in 32 bits, segment ends and the
-    // sort's item count are 32-bit ints
+    // pair values hold particle * 32 + slot in 32 bits, segment ends are
+    // 32-bit ints
     set_err(c, MPM_ERR_UNSUPPORTED, "FP64 forms: %lld particles x %d slots exceed the 32-bit pair indices", np, K);
     g_lib_error = c->err;
     free_ctx(c);
     return MPM_ERR_UNSUPPORTED;
   }
-  c->key_bits = 1;
-  while ((1LL << c->key_bits) <= (long long)c->nkeys) c->key_bits++;
   c->red_blocks = (int)std::min<long long>(1024, (np + kBlock - 1) / kBlock);
   const size_t B = c->ops->bulk_size, Rz = c->ops->real_size;
   DevState<double, double>& s = c->st;
@@ -553,9 +557,10 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
     AL(s.snode, int, (long long)K * np);
     ALR(s.shp, (long long)K * np);
     if (g.shape != 3) { ALR(s.dndx, (long long)K * np); ALR(s.dndy, (long long)K * np); ALR(s.dndz, (long long)K * np); }
-    AL(s.key, unsigned, c->npairs); AL(s.val, unsigned, c->npairs);
-    AL(s.key_sorted, unsigned, c->npairs); AL(s.val_sorted, unsigned, c->npairs);
-    AL(s.seg, int, (long long)c->nkeys + 1);
+    AL(s.val_sorted, unsigned, c->npairs);
+    AL(s.seg, int, (long long)c->nkeys + 1); AL(s.fill, int, c->nkeys);
+    AL(s.tiles, int, std::max(bm::scan_tiles(c->nkeys), bm::scan_tiles(np)) + 1);
+    AL(s.big, int, c->npairs / (kWarpPairs + 1) + 1); AL(s.nbig, int, 1);
     AL(s.mg, double, nnt); AL(s.px, double, 3 * nnt); AL(s.fx, double, 3 * nnt); AL(s.vg, double, 3 * nnt);
     AL(s.rm, double, 2 * nnt);
     AL(s.fix, uint8_t, nn); AL(s.bd, uint8_t, nn);
@@ -584,16 +589,6 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
 #undef AL
 #undef ALB
 #undef ALR
-  {
-    // CUB temporary storage: the largest of the three primitives
-    size_t t1 = 0, t2 = 0, t3 = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, t1, s.key, s.key_sorted, s.val, s.val_sorted, (int)c->npairs, 0,
-                                    c->key_bits, c->stream);
-    cub::DeviceScan::InclusiveSum(nullptr, t2, s.seg, s.seg, c->nkeys, c->stream);
-    if (g.has_jc) cub::DeviceScan::InclusiveScan(nullptr, t3, s.setter, s.setter_scan, MaxOp(), (int)np, c->stream);
-    c->cub_tmp_bytes = std::max(t1, std::max(t2, t3));
-    if ((r = dalloc(c, (char**)&c->cub_tmp, (long long)c->cub_tmp_bytes))) goto fail;
-  }
   // uploads
   {
 #define UPB(dst, src, n) \

@@ -12,8 +12,8 @@
 //   particle pass of the step; type R = double / float):
 //     node[K][Np] int32 (0-based node, -1 = not an influence node),
 //     shp / dndx / dndy / dndz [K][Np]
-//   node-sorted pair list: key[K*Np] = node, val[K*Np] = (p << 5) | slot,
-//     stably radix-sorted by node so that each node's contributions appear in
+//   node-sorted pair list: val_sorted = (p << 5) | slot, grouped by node and
+//     ascending in each group, so that each node's contributions appear in
 //     the reference's summation order (ascending particle, then slot);
 //     seg[n] = end of node n's slice (inclusive prefix sum of the counts).
 //   grid, FP64, flat reference node order: mg[Nn], px[3][Nn], fx[3][Nn],
@@ -144,8 +144,8 @@ struct DevState {
   int* snode;
   R *shp, *dndx, *dndy, *dndz;
   // pairs
-  unsigned *key, *val, *key_sorted, *val_sorted;
-  int* seg;
+  unsigned* val_sorted;  // node-sorted pairs (mpm_pairs.cuh)
+  int *seg, *fill, *tiles, *big, *nbig;  // segment ends, places taken, scan tile totals, long segments
   // grid
   double *mg, *px, *fx, *vg;
   double* rm;  // [2][Nn] reciprocal of the node's mass as a two-part sum (nodes above the cut-off)

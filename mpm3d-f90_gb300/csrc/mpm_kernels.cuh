@@ -196,21 +196,15 @@ __device__ __forceinline__ int slot_shapes(St<P>& s, const Geometry& g, long lon
   return nvalid;
 }
 
-// pair keys of particle p's slots (node-sorted list; pair j = p*K + k keeps
-// (particle, slot) order for the stable sort; invalid slots get the
-// sentinel key nkeys) and the per-node pair counts; cbase = the first node
-// of the particle's grid component
+// the nodes of particle p's slots and the per-node pair counts; cbase = the
+// first node of the particle's grid component
 template <class P>
 __device__ __forceinline__ void write_pairs(St<P>& s, const Geometry& g, long long p, int nvalid,
-                                            const int slot_node[27], int nkeys, int cbase) {
+                                            const int slot_node[27], int cbase) {
   const long long np = g.np;
-  const int K = g.K;
-  for (int k = 0; k < K; ++k) {
+  for (int k = 0; k < g.K; ++k) {
     int nd = k < nvalid && slot_node[k] >= 0 ? cbase + slot_node[k] : -1;
     s.snode[k * np + p] = nd;
-    long long j = p * K + k;
-    s.key[j] = nd >= 0 ? (unsigned)nd : (unsigned)nkeys;
-    s.val[j] = ((unsigned)p << 5) | (unsigned)k;
     if (nd >= 0) atomicAdd(&s.seg[nd], 1);  // per-node pair count (integer, deterministic)
   }
 }
@@ -218,11 +212,10 @@ __device__ __forceinline__ void write_pairs(St<P>& s, const Geometry& g, long lo
 // ----------------------------------------------------------------- locate
 // ParticleInitial (update_step.f90:408-453) plus the shape functions of the
 // step (NShape / FindInflNode+NShape_GIMP / BFindInflNode+NShape_Bspline /
-// SGNShape), cached per (slot, particle), and the pair keys of the
-// node-sorted list. Pair j = p*K + k keeps (particle, slot) order for the
-// stable sort; invalid slots get the sentinel key nkeys.
+// SGNShape), cached per (slot, particle), with the nodes of the slots and the
+// pair counts of the node-sorted list (mpm_pairs.cuh).
 template <class P>
-__global__ void k_locate(St<P> s, Geometry g, int nkeys) {
+__global__ void k_locate(St<P> s, Geometry g) {
   using B = typename P::B;
   const long long p = gtid();
   if (p >= g.np) return;
@@ -269,7 +262,7 @@ __global__ void k_locate(St<P> s, Geometry g, int nkeys) {
   }
   int slot_node[27];
   const int nvalid = slot_shapes<P>(s, g, p, x, icell, xn, cc, xxn, slot_node);
-  write_pairs<P>(s, g, p, nvalid, slot_node, nkeys, g.shape == 3 ? 0 : s.bodies[s.body[p]].comp * g.nn);
+  write_pairs<P>(s, g, p, nvalid, slot_node, g.shape == 3 ? 0 : s.bodies[s.body[p]].comp * g.nn);
 }
 
 __device__ __forceinline__ void decode_pair(unsigned v, long long np, long long* p, long long* idx) {
@@ -359,8 +352,9 @@ __device__ __forceinline__ void count_active(bool active, unsigned long long* ou
 // the chip's threads (nodes are an eighth of the particles, and only the ones
 // with pairs work). Bound now by the FP64 pipe and the gathers. One node per
 // lane keeps the adds at full warps, which cost the FP64 pipe the same as one
-// lane would. Measured on a GB300 (force transfer with the momentum
-// integration): see the figures at k_p2g_force.
+// lane would. Force transfer with the momentum integration on a GB300,
+// before and after: dam break 31 k particles 508 -> 133 us, slope 159 k
+// 426 -> 246, Taylor bar 17 k 102 -> 46, Cook 5.8 k 72 -> 26.
 //
 // NV addends per pair, NC channels: channel c adds NA[c] of them, starting
 // at c * 2 for the TWO first channels and one each after those.
@@ -1860,7 +1854,7 @@ __global__ void k_tl_sg_node_force(St<P> s, Geometry g, int integ) {
 // TLMPM): GIMP / B-spline weights at the current position, linear ones at
 // XN, SGMP ones at XXN; with_comp: keys in the particle's grid component
 template <class P>
-__global__ void k_fixed_locate(St<P> s, Geometry g, int nkeys, int with_comp) {
+__global__ void k_fixed_locate(St<P> s, Geometry g, int with_comp) {
   const long long p = gtid();
   if (p >= g.np) return;
   const long long np = g.np;
@@ -1875,7 +1869,7 @@ __global__ void k_fixed_locate(St<P> s, Geometry g, int nkeys, int with_comp) {
   int slot_node[27];
   const int nvalid = slot_shapes<P>(s, g, p, x, g.shape == 3 ? 0 : icell, xn, cc, xxn, slot_node);
   const int cbase = with_comp && g.shape != 3 ? s.bodies[s.body[p]].comp * g.nn : 0;  // smoothing: component 1
-  write_pairs<P>(s, g, p, nvalid, slot_node, nkeys, cbase);
+  write_pairs<P>(s, g, p, nvalid, slot_node, cbase);
 }
 
 // pressure * volume and volume of one (node or centre node) slice of pairs,

@@ -32,7 +32,7 @@ struct Ops {
   }
   static void locate(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_LOCATE, s);
-    k_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g, g.shape == 3 ? g.ncell : (int)g.nnt);
+    k_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     prof_end(K_LOCATE, s);
   }
   static void node_offsets(void*, const Geometry&, long long, cudaStream_t) {}
@@ -133,7 +133,7 @@ struct Ops {
 
   static void fixed_locate(void* st, const Geometry& g, int with_comp, cudaStream_t s) {
     prof_begin(K_LOCATE, s);
-    k_fixed_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g, g.shape == 3 ? g.ncell : (int)g.nnt, with_comp);
+    k_fixed_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g, with_comp);
     prof_end(K_LOCATE, s);
   }
   static void tl_initial(void* st, const Geometry& g, cudaStream_t s) {

@@ -1,0 +1,114 @@
+// mpm_pairs.cuh -- the node-sorted pair list of the FP64 forms: for every node
+// (SGMP: centre node) its (particle, slot) pairs in ascending order, which is
+// the reference's summation order.
+//
+// The locate kernel counts the pairs per node; here the counts are scanned into
+// segment ends (mpm_sort.cuh), every pair takes a place in its node's segment
+// through a per-node fill counter, and each segment is put in ascending order of
+// (particle << 5 | slot) by one warp (a bitonic network over its registers up to
+// 256 pairs), one block beyond. The result is what a stable radix sort of all
+// pairs by node gives, whatever order the placement's atomics ran in. A radix
+// sort moved 27 slots per particle (unused ones under a sentinel) five times
+// through memory; this moves each used pair once. One step's pairs, before and
+// after, GB300: slope 159 k particles 115 -> 58 us, dam break 31 k
+// 50 -> 31, Taylor bar 17 k 39 -> 20, Cook 5.8 k 40 -> 20.
+#pragma once
+
+#include "mpm_kernels.cuh"
+#include "mpm_sort.cuh"
+
+namespace mpm {
+
+// per-node counts scanned in place into segment ends, the fill counters zeroed
+// on the way
+struct PairScan {
+  using T = int;
+  using Op = bm::ScanSum;
+  int* seg;
+  int* fill;
+  long long n;
+  __device__ __forceinline__ int load(long long g) const { return seg[g]; }
+  __device__ __forceinline__ void store(long long g, int v, int) const {
+    seg[g] = v;
+    fill[g] = 0;
+  }
+};
+
+constexpr int kWarpPairs = 256;  // longest segment a warp orders
+
+// a place in its node's segment for each pair (thread = particle, blockIdx.y =
+// slot: every pair's atomic in flight at once). Neighbouring particles often
+// share a slot's node: one atomic per node and warp.
+__global__ void k_pair_place(const int* snode, const int* seg, int* fill, unsigned* val, long long np, int* nbig) {
+  const long long p = gtid();
+  const int k = blockIdx.y, lane = threadIdx.x & 31;
+  if (p == 0 && k == 0) *nbig = 0;
+  const int nd = p < np ? snode[k * np + p] : -1;
+  const unsigned grp = __match_any_sync(0xffffffffu, nd);
+  const int leader = __ffs(grp) - 1, rank = __popc(grp & ((1u << lane) - 1u));
+  int base = 0;
+  if (lane == leader && nd >= 0) base = atomicAdd(&fill[nd], __popc(grp));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (nd >= 0) val[(nd == 0 ? 0 : seg[nd - 1]) + base + rank] = ((unsigned)p << 5) | (unsigned)k;
+}
+
+// ascending order of n <= 32 R values at v by one warp, lane l holding the
+// elements l, l + 32, ...: a bitonic network, comparators at distances below
+// 32 across lanes, the others within a lane's registers
+template <int R>
+__device__ __forceinline__ void warp_order(unsigned* v, int n) {
+  const int lane = threadIdx.x & 31;
+  unsigned x[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) x[r] = r * 32 + lane < n ? v[r * 32 + lane] : 0xffffffffu;
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+    for (int s = k >> 1; s > 0; s >>= 1) {
+      if (s >= 32) {
+        const int d = s >> 5;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (r & d) continue;
+          const bool up = ((r * 32 + lane) & k) == 0;
+          const unsigned a = x[r], b = x[r | d];
+          x[r] = up ? min(a, b) : max(a, b);
+          x[r | d] = up ? max(a, b) : min(a, b);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const bool up = ((r * 32 + lane) & k) == 0, low = (lane & s) == 0;
+          const unsigned o = __shfl_xor_sync(0xffffffffu, x[r], s);
+          x[r] = up == low ? min(x[r], o) : max(x[r], o);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r * 32 + lane < n) v[r * 32 + lane] = x[r];
+}
+
+// each node's segment in ascending order, one warp per node; segments longer
+// than kWarpPairs are listed for k_pair_long
+__global__ void k_pair_order(const int* seg, long long nk, unsigned* val, int* big, int* nbig) {
+  const long long k = gtid() >> 5;
+  if (k >= nk) return;
+  const int a = k == 0 ? 0 : seg[k - 1], n = seg[k] - a;
+  unsigned* v = val + a;
+  if (n <= 1) return;
+  if (n <= 32) warp_order<1>(v, n);
+  else if (n <= 64) warp_order<2>(v, n);
+  else if (n <= 128) warp_order<4>(v, n);
+  else if (n <= kWarpPairs) warp_order<8>(v, n);
+  else if ((threadIdx.x & 31) == 0) big[atomicAdd(nbig, 1)] = (int)k;
+}
+
+__global__ void __launch_bounds__(bm::kSortThreads) k_pair_long(const int* seg, unsigned* val, const int* big,
+                                                                const int* nbig) {
+  __shared__ unsigned sm[bm::kSmemSeg];
+  bm::sort_long(seg, val, big, nbig, sm);
+}
+
+}  // namespace mpm

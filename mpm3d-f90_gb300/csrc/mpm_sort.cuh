@@ -323,7 +323,8 @@ __device__ __forceinline__ void sort_segments(const int* seg, long long nk, int*
 // value first (the first merge step of each stage compares mirrored
 // partners), so the virtual elements past n (taken as +infinity) never move
 // and are never touched
-__device__ __forceinline__ void block_bitonic(int* d, int n) {
+template <class T>
+__device__ __forceinline__ void block_bitonic(T* d, int n) {
   int N = 1;
   while (N < n) N <<= 1;
   for (int k = 2; k <= N; k <<= 1) {
@@ -339,7 +340,7 @@ __device__ __forceinline__ void block_bitonic(int* d, int n) {
           j = i + s;
         }
         if (j < n) {
-          const int x = d[i], y = d[j];
+          const T x = d[i], y = d[j];
           if (x > y) {
             d[i] = y;
             d[j] = x;
@@ -352,14 +353,15 @@ __device__ __forceinline__ void block_bitonic(int* d, int n) {
 }
 
 // the long segments: one block per segment (grid-stride over the list), in
-// shared memory (sm, kSmemSeg ints) up to kSmemSeg particles, in place in
+// shared memory (sm, kSmemSeg values) up to kSmemSeg values, in place in
 // global memory beyond
-__device__ __forceinline__ void sort_long(const int* seg, int* perm, const int* big, const int* nbig, int* sm) {
+template <class T>
+__device__ __forceinline__ void sort_long(const int* seg, T* perm, const int* big, const int* nbig, T* sm) {
   const int nb = *nbig;
   for (int b = blockIdx.x; b < nb; b += gridDim.x) {
     const int k = big[b];
     const int a = k == 0 ? 0 : seg[k - 1], n = seg[k] - a;
-    int* p = perm + a;
+    T* p = perm + a;
     if (n <= kSmemSeg) {
       for (int j = threadIdx.x; j < n; j += blockDim.x) sm[j] = p[j];
       __syncthreads();
