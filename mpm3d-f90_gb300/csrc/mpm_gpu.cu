@@ -299,12 +299,14 @@ int sort_pairs(mpm_ctx* c) {
   cudaStream_t st = c->stream;
   const long long np = c->g.np;
   prof_begin(K_SORT, st);
-  scan_tiles(PairScan{s.seg, s.fill, c->nkeys}, s.tiles, st);
-  k_pair_place<<<dim3((unsigned)((np + 255) / 256), (unsigned)c->g.K), 256, 0, st>>>(s.snode, s.seg, s.fill,
-                                                                                    s.val_sorted, np, s.nbig);
+  scan_tiles(PairScan{s.seg, s.fill, s.wcnt, c->nkeys}, s.tiles, st);
+  const dim3 rows((unsigned)((np + 255) / 256), (unsigned)c->g.K + 1);
+  k_pair_place<<<rows, 256, 0, st>>>(s.snode, s.seg, s.fill, s.val_sorted, np, c->g.K, c->nkeys, s.wcnt, s.nbig);
   k_pair_order<<<(unsigned)(((long long)c->nkeys * 32 + 127) / 128), 128, 0, st>>>(s.seg, c->nkeys, s.val_sorted, s.big,
                                                                                  s.nbig);
-  k_pair_long<<<76, bm::kSortThreads, 0, st>>>(s.seg, s.val_sorted, s.big, s.nbig);
+  const unsigned tiles = (unsigned)((c->nkeys + bm::kSortThreads - 1) / bm::kSortThreads);
+  k_pair_long<<<std::min(std::max(tiles, 76u), 608u), bm::kSortThreads, 0, st>>>(s.seg, s.val_sorted, s.big, s.nbig,
+                                                                                c->nkeys, s.wcnt, s.walk);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "pair sort");
   prof_end(K_SORT, st);
@@ -560,6 +562,7 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
     AL(s.val_sorted, unsigned, c->npairs);
     AL(s.seg, int, (long long)c->nkeys + 1); AL(s.fill, int, c->nkeys);
     AL(s.tiles, int, std::max(bm::scan_tiles(c->nkeys), bm::scan_tiles(np)) + 1);
+    AL(s.walk, int, c->nkeys); AL(s.wcnt, int, 2 * kWalkClasses);
     AL(s.big, int, c->npairs / (kWarpPairs + 1) + 1); AL(s.nbig, int, 1);
     AL(s.mg, double, nnt); AL(s.px, double, 3 * nnt); AL(s.fx, double, 3 * nnt); AL(s.vg, double, 3 * nnt);
     AL(s.rm, double, 2 * nnt);

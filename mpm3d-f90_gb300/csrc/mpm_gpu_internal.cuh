@@ -146,6 +146,7 @@ struct DevState {
   // pairs
   unsigned* val_sorted;  // node-sorted pairs (mpm_pairs.cuh)
   int *seg, *fill, *tiles, *big, *nbig;  // segment ends, places taken, scan tile totals, long segments
+  int *walk, *wcnt;  // order the transfers take the nodes in, its class counters
   // grid
   double *mg, *px, *fx, *vg;
   double* rm;  // [2][Nn] reciprocal of the node's mass as a two-part sum (nodes above the cut-off)

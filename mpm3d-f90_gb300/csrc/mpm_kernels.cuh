@@ -342,95 +342,130 @@ __device__ __forceinline__ void count_active(bool active, unsigned long long* ou
 }
 
 // ------------------------------------------------------------- pair walk
-// Sums over the pair slices of kWalkNodes consecutive nodes (or SGMP cells) by
-// one block: in rounds of kWalkPairs pairs per node, eight threads per node
-// form the pairs' addends (every gather and product of the round in flight
-// at once) into shared memory, and then one warp per channel, lane = node,
-// adds them in pair order -- the reference's sequential sum, each addend
-// rounded as it would be there. A thread per node did both alone, one pair's
-// gathers after the other's sum: the walk waited on memory with a fraction of
-// the chip's threads (nodes are an eighth of the particles, and only the ones
-// with pairs work). Bound now by the FP64 pipe and the gathers. One node per
-// lane keeps the adds at full warps, which cost the FP64 pipe the same as one
-// lane would. Force transfer with the momentum integration on a GB300,
-// before and after: dam break 31 k particles 508 -> 133 us, slope 159 k
-// 426 -> 246, Taylor bar 17 k 102 -> 46, Cook 5.8 k 72 -> 26.
+// Sums over the pair slices of kWalkNodes nodes (or SGMP cells) by one block,
+// in rounds of PAIRS pairs per node: PAIRS threads per node form one pair's
+// addends each, in parallel, into shared memory, and then one thread per node
+// and channel adds them in pair order -- the reference's sequential sum, each
+// addend rounded as it would be there. The values of the next round are
+// fetched before a round is summed. (A thread per node did all of it alone,
+// one pair's gathers after the other's sum, with a fraction of the chip's
+// threads: nodes are an eighth of the particles, and only those with pairs
+// work.)
 //
-// NV addends per pair, NC channels: channel c adds NA[c] of them, starting
-// at c * 2 for the TWO first channels and one each after those.
-// prod(p, idx, v) forms a pair's addends from the particle and the index in
-// the shape cache; fin(n, acc) gets a node's sums.
-constexpr int kWalkNodes = 32;
-constexpr int kWalkPairs = 16;   // pairs per node and round
-constexpr int kWalkPitch = 36;   // nodes' row pitch (the four nodes x eight pairs a warp writes fall on distinct banks)
-static_assert(kBlock == 8 * kWalkNodes, "eight threads per node");
+// The nodes are taken in the order of walk, which groups slices of about the
+// same length and puts the longest first (mpm_pairs.cuh): the lanes of a
+// summing warp work as long as the longest of its nodes, and in the grid's
+// order they added 0.6 of that time on a slope. Bound now by the FP64 pipe
+// (the force transfer of the slope executes 27 FP64 instructions a pair, 114
+// of its 165 us), or, where the longest slices make the time of a small scene
+// (dam break, 216 pairs a node), by the latency of their rounds.
+//
+// Eight nodes per block: finer blocks even out the SMs' shares (the dam break
+// of 31 k particles has 5600 nodes: as 32 nodes per block, 177 blocks for 152
+// SMs, its force transfer takes 114 us, by 16 95, by 8 85), while the adds of
+// fewer nodes fill less of a warp, which costs the FP64 pipe the same (by 4:
+// slope 165 -> 214). PAIRS is 8 for the transfers with many products a pair
+// (16: slope 179 us for 165, dam 83 for 85) and 16 for the ones with few,
+// where the rounds' latency counts (dam 35 -> 31, slope 58.6 -> 57).
+//
+// Force transfer with the momentum integration, GB300, from the thread per
+// node to the grid's order to now: dam break 31 k particles 508 -> 133 -> 85
+// us, slope 159 k 426 -> 246 -> 165, Taylor bar 17 k 102 -> 46 -> 28, Cook
+// 5.8 k 72 -> 26 -> 22.
+//
+// NV addends per pair, NC channels: channel c adds two of them, 2 c and
+// 2 c + 1, for the TWO first channels and one, c + TWO, after those.
+// load(p, idx, raw) fetches the NR values a pair's addends are formed of, for
+// the particle and the index in the shape cache, form(raw, v) forms them;
+// fin(n, in, acc) gets a node's sums (in: there is a node).
+constexpr int kWalkNodes = 8;
+constexpr int kWalkFew = 16;   // PAIRS of the transfers with few products a pair
+constexpr int kWalkMany = 8;   // ... with many
 
-template <int NV, int NC, int TWO, class Prod, class Fin>
-__device__ __forceinline__ void pair_walk(const int* seg, const unsigned* val, long long np, long long nn, Prod prod,
-                                          Fin fin) {
+template <int PAIRS, int NR, int NV, int NC, int TWO, class Load, class Form, class Fin>
+__device__ __forceinline__ void pair_walk(const int* walk, const int* seg, const unsigned* val, long long np,
+                                          long long nn, Load load, Form form, Fin fin) {
   static_assert(NV == NC + TWO, "addends");
-  constexpr int NW = kBlock / 32, PER = (NC + NW - 1) / NW;  // channels a warp sums
-  __shared__ double buf[NV][kWalkPairs][kWalkPitch];
-  __shared__ int s_end[kWalkNodes + 1];
+  // (row pitch: the nodes and pairs of a half-warp fall on distinct banks)
+  constexpr int PITCH = kWalkNodes + (PAIRS > 8 ? 1 : 2);
+  constexpr int PER = (NC + PAIRS - 1) / PAIRS;  // channels a thread sums
+  __shared__ double buf[2][NV][PAIRS][PITCH];
+  __shared__ int s_beg[kWalkNodes], s_end[kWalkNodes];
   __shared__ int s_rounds;
-  const long long n0 = (long long)blockIdx.x * kWalkNodes;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  if (warp == 0) {
-    const long long n = n0 + lane;
-    const int e = seg[n < nn ? n : nn - 1];
-    const int first = n0 == 0 ? 0 : seg[n0 - 1];
-    s_end[lane + 1] = e;
-    if (lane == 0) s_end[0] = first;
-    int len = __shfl_up_sync(0xffffffffu, e, 1);
-    len = e - (lane == 0 ? first : len);
-    const int longest = __reduce_max_sync(0xffffffffu, len);
-    if (lane == 0) s_rounds = (longest + kWalkPairs - 1) / kWalkPairs;
+  const int t = threadIdx.x;
+  int node = -1;  // of the thread (the first kWalkNodes)
+  if (t < 32) {
+    const long long w = (long long)blockIdx.x * kWalkNodes + t;
+    int a = 0, e = 0;
+    if (t < kWalkNodes && w < nn) {
+      node = walk[w];
+      a = node == 0 ? 0 : seg[node - 1];
+      e = seg[node];
+    }
+    if (t < kWalkNodes) {
+      s_beg[t] = a;
+      s_end[t] = e;
+    }
+    const int longest = __reduce_max_sync(0xffffffffu, e - a);
+    if (t == 0) s_rounds = (longest + PAIRS - 1) / PAIRS;
   }
   __syncthreads();
   const int rounds = s_rounds;
-  const int g = t >> 3, q = t & 7;
-  const int ja = s_end[g] + q, je = s_end[g + 1];       // the thread's pairs: ja, ja + 8, ja + 16, ...
-  const int len = s_end[lane + 1] - s_end[lane];        // pairs of the lane's node (summing warps)
+  const int g = t / PAIRS, q = t % PAIRS;
+  int j = s_beg[g] + q;                  // the thread's pairs: j, j + PAIRS, ...
+  const int je = s_end[g];
+  const int sn = t % kWalkNodes, sc = t / kWalkNodes;  // the node and first channel the thread sums
+  const int len = s_end[sn] - s_beg[sn];
   double acc[PER];
 #pragma unroll
   for (int e = 0; e < PER; ++e) acc[e] = 0.0;
-  for (int r = 0; r < rounds; ++r) {
-#pragma unroll
-    for (int u = 0; u < kWalkPairs / 8; ++u) {
-      const int j = ja + r * kWalkPairs + 8 * u;
-      if (j < je) {
-        const unsigned pv = val[j];
-        const long long p = (long long)(pv >> 5);
-        double v[NV];
-        prod(p, (long long)(pv & 31u) * np + p, v);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) buf[k][q + 8 * u][g] = v[k];
-      }
+  double raw[NR];
+  auto fetch = [&] {
+    if (j < je) {
+      const unsigned pv = val[j];
+      const long long p = (long long)(pv >> 5);
+      load(p, (long long)(pv & 31u) * np + p, raw);
     }
+  };
+  fetch();
+  for (int r = 0; r < rounds; ++r) {
+    double(*b)[PAIRS][PITCH] = buf[r & 1];
+    if (j < je) {
+      double v[NV];
+      form(raw, v);
+#pragma unroll
+      for (int k = 0; k < NV; ++k) b[k][q][g] = v[k];
+    }
+    j += PAIRS;
+    fetch();
+    // (one barrier a round: this half of buf is written again after the next
+    // one, which the summing warps reach when they are done with it)
     __syncthreads();
-    const int cnt = min(len - r * kWalkPairs, kWalkPairs);
+    const int cnt = min(len - r * PAIRS, PAIRS);
 #pragma unroll
     for (int e = 0; e < PER; ++e) {
-      const int c = warp + e * NW;
+      const int c = sc + e * PAIRS;
       if (c < TWO) {
-#pragma unroll 8
-        for (int k = 0; k < cnt; ++k) acc[e] = acc[e] + buf[2 * c][k][lane] + buf[2 * c + 1][k][lane];
+#pragma unroll
+        for (int k = 0; k < PAIRS; ++k)
+          if (k < cnt) acc[e] = acc[e] + b[2 * c][k][sn] + b[2 * c + 1][k][sn];
       } else if (c < NC) {
-#pragma unroll 8
-        for (int k = 0; k < cnt; ++k) acc[e] = acc[e] + buf[c + TWO][k][lane];
+#pragma unroll
+        for (int k = 0; k < PAIRS; ++k)
+          if (k < cnt) acc[e] = acc[e] + b[c + TWO][k][sn];
       }
     }
-    __syncthreads();
   }
+  __syncthreads();
 #pragma unroll
   for (int e = 0; e < PER; ++e)
-    if (warp + e * NW < NC) buf[warp + e * NW][0][lane] = acc[e];
+    if (sc + e * PAIRS < NC) buf[0][sc + e * PAIRS][0][sn] = acc[e];
   __syncthreads();
-  if (warp == 0) {
+  if (t < 32) {
     double a[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) a[c] = buf[c][0][lane];
-    fin(n0 + lane, n0 + lane < nn, a);
+    for (int c = 0; c < NC; ++c) a[c] = buf[0][c][0][sn];
+    fin(node, node >= 0, a);
   }
 }
 
@@ -439,14 +474,16 @@ __device__ __forceinline__ void pair_walk(const int* seg, const unsigned* val, l
 template <class P>
 __global__ void k_p2g_mass(St<P> s, Geometry g, int bc, int vel) {
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
-  pair_walk<4, 4, 0>(
-      s.seg, s.val_sorted, np, nn,
-      [&](long long p, long long idx, double* v) {
-        const double shm = (double)s.shp[idx] * s.mass[p];
-        v[0] = shm;
-        v[1] = s.vxp[p] * shm;
-        v[2] = s.vxp[np + p] * shm;
-        v[3] = s.vxp[2 * np + p] * shm;
+  pair_walk<kWalkFew, 5, 4, 4, 0>(
+      s.walk, s.seg, s.val_sorted, np, nn,
+      [&](long long p, long long idx, double* r) {
+        r[0] = (double)s.shp[idx];
+        r[1] = s.mass[p];
+        for (int c = 0; c < 3; ++c) r[2 + c] = s.vxp[c * np + p];
+      },
+      [&](const double* r, double* v) {
+        v[0] = r[0] * r[1];
+        for (int c = 0; c < 3; ++c) v[1 + c] = r[2 + c] * v[0];
       },
       [&](long long n, bool in, const double* a) {
         if (in) {
@@ -1072,24 +1109,32 @@ __device__ __forceinline__ void node_integrate(St<P>& s, const Geometry& g, long
 template <class P, bool CONTACT>
 __global__ void k_p2g_force(St<P> s, Geometry g, int integ) {
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
-  pair_walk<CONTACT ? 9 : 6, CONTACT ? 6 : 3, 3>(
-      s.seg, s.val_sorted, np, nn,
-      [&](long long p, long long idx, double* v) {
-        const double sk = s.shp[idx], dx = s.dndx[idx], dy = s.dndy[idx], dz = s.dndz[idx];
-        const double sxx = s.sdiag[p], syy = s.sdiag[np + p], szz = s.sdiag[2 * np + p];
-        const double sxy = s.sd[3 * np + p], syz = s.sd[4 * np + p], sxz = s.sd[5 * np + p];
-        const double vol = s.vol[p];
+  pair_walk<kWalkMany, CONTACT ? 15 : 14, CONTACT ? 9 : 6, CONTACT ? 6 : 3, 3>(
+      s.walk, s.seg, s.val_sorted, np, nn,
+      [&](long long p, long long idx, double* r) {
+        r[0] = s.shp[idx];
+        r[1] = s.dndx[idx];
+        r[2] = s.dndy[idx];
+        r[3] = s.dndz[idx];
+        for (int d = 0; d < 3; ++d) r[4 + d] = s.sdiag[d * np + p];
+        for (int d = 0; d < 3; ++d) r[7 + d] = s.sd[(3 + d) * np + p];
+        r[10] = s.vol[p];
+        for (int d = 0; d < 3; ++d) r[11 + d] = s.fext[d * np + p];
+        if (CONTACT) r[14] = s.mass[p];
+      },
+      [&](const double* r, double* v) {
+        const double sk = r[0], dx = r[1], dy = r[2], dz = r[3];
+        const double sxx = r[4], syy = r[5], szz = r[6], sxy = r[7], syz = r[8], sxz = r[9], vol = r[10];
         v[0] = -(sxx * dx + sxy * dy + sxz * dz) * vol;
-        v[1] = s.fext[p] * sk;
+        v[1] = r[11] * sk;
         v[2] = -(sxy * dx + syy * dy + syz * dz) * vol;
-        v[3] = s.fext[np + p] * sk;
+        v[3] = r[12] * sk;
         v[4] = -(sxz * dx + syz * dy + szz * dz) * vol;
-        v[5] = s.fext[2 * np + p] * sk;
+        v[5] = r[13] * sk;
         if (CONTACT) {
-          const double mp = s.mass[p];
-          v[6] = dx * mp;
-          v[7] = dy * mp;
-          v[8] = dz * mp;
+          v[6] = dx * r[14];
+          v[7] = dy * r[14];
+          v[8] = dz * r[14];
         }
       },
       [&](long long n, bool in, const double* a) {
@@ -1306,11 +1351,16 @@ __global__ void k_position(St<P> s, Geometry g) {
 template <class P>
 __global__ void k_p2g_momentum(St<P> s, Geometry g, int vel) {
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
-  pair_walk<3, 3, 0>(
-      s.seg, s.val_sorted, np, nn,
-      [&](long long p, long long idx, double* v) {
-        const double shm = (double)s.shp[idx] * s.mass[p];
-        for (int c = 0; c < 3; ++c) v[c] = s.vxp[c * np + p] * shm;
+  pair_walk<kWalkFew, 5, 3, 3, 0>(
+      s.walk, s.seg, s.val_sorted, np, nn,
+      [&](long long p, long long idx, double* r) {
+        r[0] = (double)s.shp[idx];
+        r[1] = s.mass[p];
+        for (int c = 0; c < 3; ++c) r[2 + c] = s.vxp[c * np + p];
+      },
+      [&](const double* r, double* v) {
+        const double shm = r[0] * r[1];
+        for (int c = 0; c < 3; ++c) v[c] = r[2 + c] * shm;
       },
       [&](long long n, bool in, const double* a) {
         if (!in) return;
@@ -1350,12 +1400,16 @@ __device__ __forceinline__ void for_adjacent_cells(const Geometry& g, long long 
 template <class P>
 __global__ void k_sg_cell_mass(St<P> s, Geometry g) {
   const long long np = g.np, nc = g.ncell;
-  pair_walk<4, 4, 0>(
-      s.seg, s.val_sorted, np, nc,
-      [&](long long p, long long idx, double* v) {
-        const double shm = (double)s.shp[idx] * s.mass[p];
-        v[0] = shm;
-        for (int c = 0; c < 3; ++c) v[1 + c] = s.vxp[c * np + p] * shm;
+  pair_walk<kWalkFew, 5, 4, 4, 0>(
+      s.walk, s.seg, s.val_sorted, np, nc,
+      [&](long long p, long long idx, double* r) {
+        r[0] = (double)s.shp[idx];
+        r[1] = s.mass[p];
+        for (int c = 0; c < 3; ++c) r[2 + c] = s.vxp[c * np + p];
+      },
+      [&](const double* r, double* v) {
+        v[0] = r[0] * r[1];
+        for (int c = 0; c < 3; ++c) v[1 + c] = r[2 + c] * v[0];
       },
       [&](long long c, bool in, const double* a) {
         if (!in) return;
@@ -1435,13 +1489,18 @@ __global__ void k_sg_cell_gradient(St<P> s, Geometry g) {
 template <class P>
 __global__ void k_sg_cell_force(St<P> s, Geometry g) {
   const long long np = g.np, nc = g.ncell;
-  pair_walk<9, 9, 0>(
-      s.seg, s.val_sorted, np, nc,
-      [&](long long p, long long idx, double* v) {
-        const double sk = s.shp[idx], vol = s.vol[p];
-        for (int d = 0; d < 3; ++d) v[d] = s.fext[d * np + p] * sk;
-        for (int d = 0; d < 3; ++d) v[3 + d] = sk * s.sdiag[d * np + p] * vol;
-        for (int d = 3; d < 6; ++d) v[3 + d] = sk * s.sd[d * np + p] * vol;
+  pair_walk<kWalkMany, 11, 9, 9, 0>(
+      s.walk, s.seg, s.val_sorted, np, nc,
+      [&](long long p, long long idx, double* r) {
+        r[0] = s.shp[idx];
+        r[1] = s.vol[p];
+        for (int d = 0; d < 3; ++d) r[2 + d] = s.fext[d * np + p];
+        for (int d = 0; d < 3; ++d) r[5 + d] = s.sdiag[d * np + p];
+        for (int d = 3; d < 6; ++d) r[5 + d] = s.sd[d * np + p];
+      },
+      [&](const double* r, double* v) {
+        for (int d = 0; d < 3; ++d) v[d] = r[2 + d] * r[0];
+        for (int d = 3; d < 9; ++d) v[d] = r[0] * r[2 + d] * r[1];
       },
       [&](long long c, bool in, const double* a) {
         if (!in) return;
@@ -1540,11 +1599,16 @@ __global__ void k_sg_cell_velocity(St<P> s, Geometry g) {
 template <class P>
 __global__ void k_sg_cell_momentum(St<P> s, Geometry g) {
   const long long np = g.np, nc = g.ncell;
-  pair_walk<3, 3, 0>(
-      s.seg, s.val_sorted, np, nc,
-      [&](long long p, long long idx, double* v) {
-        const double shm = (double)s.shp[idx] * s.mass[p];
-        for (int c = 0; c < 3; ++c) v[c] = s.vxp[c * np + p] * shm;
+  pair_walk<kWalkFew, 5, 3, 3, 0>(
+      s.walk, s.seg, s.val_sorted, np, nc,
+      [&](long long p, long long idx, double* r) {
+        r[0] = (double)s.shp[idx];
+        r[1] = s.mass[p];
+        for (int c = 0; c < 3; ++c) r[2 + c] = s.vxp[c * np + p];
+      },
+      [&](const double* r, double* v) {
+        const double shm = r[0] * r[1];
+        for (int c = 0; c < 3; ++c) v[c] = r[2 + c] * shm;
       },
       [&](long long c, bool in, const double* a) {
         if (!in) return;
@@ -1872,43 +1936,42 @@ __global__ void k_fixed_locate(St<P> s, Geometry g, int with_comp) {
   write_pairs<P>(s, g, p, nvalid, slot_node, cbase);
 }
 
-// pressure * volume and volume of one (node or centre node) slice of pairs,
-// in particle order; returns false for an empty slice
-template <class P>
-__device__ __forceinline__ bool smooth_sums(const St<P>& s, const Geometry& g, int j0, int j1, double& gp, double& gv) {
-  const long long np = g.np;
-  gp = 0.0;
-  gv = 0.0;
-  for (int j = j0; j < j1; ++j) {
-    long long p, idx;
-    decode_pair(s.val_sorted[j], np, &p, &idx);
-    const double shp = (double)s.shp[idx], sm = (double)s.sm[p];
-    const double vol = g.tlmpm ? (double)s.vol0[p] : (double)s.vol[p];  // TLSmoothStressbyGrid: VOL0
-    gp = gp + shp * (-1 * sm) * vol;
-    gv = gv + shp * vol;
-  }
-  return j1 > j0;
+// pressure * volume and volume of every (node's or centre node's) slice of
+// pairs, in particle order
+template <class P, class Fin>
+__device__ __forceinline__ void smooth_sums(const St<P>& s, const Geometry& g, long long nn, Fin fin) {
+  pair_walk<kWalkFew, 3, 2, 2, 0>(
+      s.walk, s.seg, s.val_sorted, g.np, nn,
+      [&](long long p, long long idx, double* r) {
+        r[0] = (double)s.shp[idx];
+        r[1] = (double)s.sm[p];
+        r[2] = g.tlmpm ? (double)s.vol0[p] : (double)s.vol[p];  // TLSmoothStressbyGrid: VOL0
+      },
+      [&](const double* r, double* v) {
+        v[0] = r[0] * (-1 * r[1]) * r[2];
+        v[1] = r[0] * r[2];
+      },
+      fin);
 }
 
-// particles -> nodes, Gpre / GV_all on the mapped nodes
+// particles -> nodes, Gpre / GV_all on the mapped nodes (component 1)
 template <class P>
 __global__ void k_smooth_node(St<P> s, Geometry g) {
-  const long long n = gtid();
-  if (n >= g.nn) return;
-  double gp, gv;
-  const bool mapped = smooth_sums<P>(s, g, n == 0 ? 0 : s.seg[n - 1], s.seg[n], gp, gv);
-  s.gpre[n] = mapped ? gp / gv : gp;
+  smooth_sums<P>(s, g, g.nnt, [&](long long n, bool in, const double* a) {
+    if (!in || n >= g.nn) return;
+    const bool mapped = s.seg[n] > (n == 0 ? 0 : s.seg[n - 1]);
+    s.gpre[n] = mapped ? a[0] / a[1] : a[0];
+  });
 }
 
 // SGMP: particles -> centre nodes
 template <class P>
 __global__ void k_smooth_cell(St<P> s, Geometry g) {
-  const long long c = gtid();
-  if (c >= g.ncell) return;
-  double gp, gv;
-  smooth_sums<P>(s, g, c == 0 ? 0 : s.seg[c - 1], s.seg[c], gp, gv);
-  s.cgpre[c] = gp;
-  s.cgvall[c] = gv;
+  smooth_sums<P>(s, g, g.ncell, [&](long long c, bool in, const double* a) {
+    if (!in) return;
+    s.cgpre[c] = a[0];
+    s.cgvall[c] = a[1];
+  });
 }
 
 // SGMP: centre nodes -> nodes (1/8 of every adjacent cell; every node is

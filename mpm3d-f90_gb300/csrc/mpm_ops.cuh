@@ -39,10 +39,10 @@ struct Ops {
   static void p2g_mass(void* st, const Geometry& g, int bc, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      k_sg_cell_mass<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_mass<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
       k_sg_node_mass<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, bc, vel);
     } else {
-      k_p2g_mass<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, bc, vel);
+      k_p2g_mass<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g, bc, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
@@ -90,11 +90,11 @@ struct Ops {
   static void p2g_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
-      k_sg_cell_force<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_force<P><<<walk_grid(g.ncell), kWalkNodes * kWalkMany, 0, s>>>(S(st), g);
       k_sg_node_force<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, integ);
     } else {
-      if (g.contact) k_p2g_force<P, true><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
-      else k_p2g_force<P, false><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, integ);
+      if (g.contact) k_p2g_force<P, true><<<walk_grid(g.nnt), kWalkNodes * kWalkMany, 0, s>>>(S(st), g, integ);
+      else k_p2g_force<P, false><<<walk_grid(g.nnt), kWalkNodes * kWalkMany, 0, s>>>(S(st), g, integ);
     }
     prof_end(K_P2G_FORCE, s);
   }
@@ -112,10 +112,10 @@ struct Ops {
   static void p2g_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MOM, s);
     if (g.shape == 3) {
-      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
       k_sg_node_momentum<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, vel);
     } else {
-      k_p2g_momentum<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
+      k_p2g_momentum<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g, vel);
     }
     prof_end(K_P2G_MOM, s);
   }
@@ -142,10 +142,10 @@ struct Ops {
   static void tl_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kBlock, 0, s>>>(S(st), g);
+      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
       k_tl_sg_node_momentum<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, vel);
     } else {
-      k_p2g_momentum<P><<<walk_grid(g.nnt), kBlock, 0, s>>>(S(st), g, vel);
+      k_p2g_momentum<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
@@ -168,11 +168,11 @@ struct Ops {
   static void smooth(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_SMOOTH, s);
     if (g.shape == 3) {
-      k_smooth_cell<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+      k_smooth_cell<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
       k_smooth_sg_node<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
       k_smooth_sg_back<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
     } else {
-      k_smooth_node<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
+      k_smooth_node<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
     }
     k_smooth_g2p<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
     prof_end(K_SMOOTH, s);

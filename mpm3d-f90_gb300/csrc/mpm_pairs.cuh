@@ -11,7 +11,8 @@
 // sort moved 27 slots per particle (unused ones under a sentinel) five times
 // through memory; this moves each used pair once. One step's pairs, before and
 // after, GB300: slope 159 k particles 115 -> 58 us, dam break 31 k
-// 50 -> 31, Taylor bar 17 k 39 -> 20, Cook 5.8 k 40 -> 20.
+// 50 -> 31, Taylor bar 17 k 39 -> 20, Cook 5.8 k 40 -> 20. The order in which
+// the transfers take the nodes is made beside it (1.5 us of each).
 #pragma once
 
 #include "mpm_kernels.cuh"
@@ -19,18 +20,30 @@
 
 namespace mpm {
 
-// per-node counts scanned in place into segment ends, the fill counters zeroed
-// on the way
+// The order the transfers take the nodes in (pair_walk): by classes of the
+// number of eights of pairs in a segment, longest first, empty segments
+// last, about the grid's order within a class. The order has no bearing on
+// results.
+constexpr int kWalkClasses = 32;
+__device__ __forceinline__ int walk_class(int n) {
+  return kWalkClasses - 1 - min((n + 7) / 8, kWalkClasses - 1);
+}
+
+// per-node counts scanned in place into segment ends, the fill counters and
+// the class counters (nodes of each class, then nodes placed) zeroed on the way
 struct PairScan {
   using T = int;
   using Op = bm::ScanSum;
   int* seg;
   int* fill;
+  int* wcnt;
   long long n;
   __device__ __forceinline__ int load(long long g) const { return seg[g]; }
   __device__ __forceinline__ void store(long long g, int v, int) const {
     seg[g] = v;
     fill[g] = 0;
+    if (g == 0)
+      for (int c = 0; c < 2 * kWalkClasses; ++c) wcnt[c] = 0;
   }
 };
 
@@ -38,11 +51,27 @@ constexpr int kWarpPairs = 256;  // longest segment a warp orders
 
 // a place in its node's segment for each pair (thread = particle, blockIdx.y =
 // slot: every pair's atomic in flight at once). Neighbouring particles often
-// share a slot's node: one atomic per node and warp.
-__global__ void k_pair_place(const int* snode, const int* seg, int* fill, unsigned* val, long long np, int* nbig) {
+// share a slot's node: one atomic per node and warp. The blocks of one more row
+// count the nodes of each class.
+__global__ void __launch_bounds__(256) k_pair_place(const int* snode, const int* seg, int* fill, unsigned* val,
+                                                    long long np, int K, long long nk, int* wcnt, int* nbig) {
   const long long p = gtid();
   const int k = blockIdx.y, lane = threadIdx.x & 31;
   if (p == 0 && k == 0) *nbig = 0;
+  if (k == K) {
+    __shared__ int hist[kWalkClasses];
+    if (threadIdx.x < kWalkClasses) hist[threadIdx.x] = 0;
+    __syncthreads();
+    for (long long n0 = (long long)blockIdx.x * 256; n0 < nk; n0 += (long long)gridDim.x * 256) {
+      const long long n = n0 + threadIdx.x;
+      const int c = n < nk ? walk_class(seg[n] - (n == 0 ? 0 : seg[n - 1])) : -1;
+      const unsigned grp = __match_any_sync(0xffffffffu, c);
+      if (c >= 0 && lane == __ffs(grp) - 1) atomicAdd(&hist[c], __popc(grp));
+    }
+    __syncthreads();
+    if (threadIdx.x < kWalkClasses && hist[threadIdx.x]) atomicAdd(&wcnt[threadIdx.x], hist[threadIdx.x]);
+    return;
+  }
   const int nd = p < np ? snode[k * np + p] : -1;
   const unsigned grp = __match_any_sync(0xffffffffu, nd);
   const int leader = __ffs(grp) - 1, rank = __popc(grp & ((1u << lane) - 1u));
@@ -105,10 +134,48 @@ __global__ void k_pair_order(const int* seg, long long nk, unsigned* val, int* b
   else if ((threadIdx.x & 31) == 0) big[atomicAdd(nbig, 1)] = (int)k;
 }
 
+// the segments listed in big in ascending order, and the nodes into walk
 __global__ void __launch_bounds__(bm::kSortThreads) k_pair_long(const int* seg, unsigned* val, const int* big,
-                                                                const int* nbig) {
+                                                                const int* nbig, long long nk, int* wcnt, int* walk) {
   __shared__ unsigned sm[bm::kSmemSeg];
   bm::sort_long(seg, val, big, nbig, sm);
+
+  constexpr int NW = bm::kSortThreads / 32;
+  static_assert(kWalkClasses == 32, "a lane per class");
+  __shared__ int cnt[NW][kWalkClasses], base[kWalkClasses];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int start = 0;  // of the lane's class (first warp)
+  if (warp == 0) {
+    const int own = wcnt[lane];
+    start = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, start, o);
+      if (lane >= o) start += u;
+    }
+    start -= own;
+  }
+  for (long long n0 = (long long)blockIdx.x * bm::kSortThreads; n0 < nk; n0 += (long long)gridDim.x * bm::kSortThreads) {
+    const long long n = n0 + threadIdx.x;
+    const int c = n < nk ? walk_class(seg[n] - (n == 0 ? 0 : seg[n - 1])) : -1;
+    const unsigned grp = __match_any_sync(0xffffffffu, c);
+    cnt[warp][lane] = 0;
+    __syncwarp();
+    if (c >= 0 && lane == __ffs(grp) - 1) cnt[warp][c] = __popc(grp);
+    __syncthreads();
+    if (warp == 0) {  // lane = class: the warps' offsets, and the tile's place in the class
+      int tot = 0;
+      for (int q = 0; q < NW; ++q) {
+        const int v = cnt[q][lane];
+        cnt[q][lane] = tot;
+        tot += v;
+      }
+      base[lane] = start + (tot ? atomicAdd(&wcnt[kWalkClasses + lane], tot) : 0);
+    }
+    __syncthreads();
+    if (c >= 0) walk[base[c] + cnt[warp][c] + __popc(grp & ((1u << lane) - 1u))] = (int)n;
+    __syncthreads();
+  }
 }
 
 }  // namespace mpm
