@@ -293,6 +293,10 @@ void scan_tiles(const Src& src, typename Src::T* tiles, cudaStream_t st) {
   }
 }
 
+// the per-node counts, and behind them the lengths of the slot lists: zeroed
+// together before the particles are located
+size_t seg_words(const mpm_ctx* c) { return (size_t)c->nkeys + 4; }
+
 // the node-sorted pair list from the slots' nodes and the per-node counts
 int sort_pairs(mpm_ctx* c) {
   DevState<double, double>& s = c->st;
@@ -324,7 +328,7 @@ int depeff_pass(mpm_ctx* c) {
 }
 
 int build_pairs(mpm_ctx* c) {
-  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * ((size_t)c->nkeys + 1), c->stream);
+  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
   c->ops->locate(&c->st, c->g, c->stream);
   return sort_pairs(c);
@@ -333,7 +337,7 @@ int build_pairs(mpm_ctx* c) {
 // SmoothStressbyGrid: shapes and pairs of the step's cells, then the maps
 int smooth_pass(mpm_ctx* c) {
   if (!c->st.spre) return set_err(c, MPM_ERR_ARG, "stress smoothing is off for this deck (no 'smoo')");
-  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * ((size_t)c->nkeys + 1), c->stream);
+  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), c->stream);
   if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
   c->ops->fixed_locate(&c->st, c->g, 0, c->stream);
   int r = sort_pairs(c);
@@ -355,7 +359,7 @@ int enqueue_step_tl(mpm_ctx* c) {
   cudaStream_t s = c->stream;
   int r;
   o->begin_step(st, g, s);
-  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * ((size_t)c->nkeys + 1), s);
+  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), s);
   if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
   o->fixed_locate(st, g, 1, s);
   if ((r = sort_pairs(c))) return r;
@@ -560,7 +564,10 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
     ALR(s.shp, (long long)K * np);
     if (g.shape != 3) { ALR(s.dndx, (long long)K * np); ALR(s.dndy, (long long)K * np); ALR(s.dndz, (long long)K * np); }
     AL(s.val_sorted, unsigned, c->npairs);
-    AL(s.seg, int, (long long)c->nkeys + 1); AL(s.fill, int, c->nkeys);
+    AL(s.seg, int, seg_words(c)); AL(s.fill, int, c->nkeys);
+    s.slot_cnt = s.seg + c->nkeys;
+    if (g.shape == 1) AL(s.slot_list, int, 4 * np);
+    AL(s.axis, double, g.NGx + g.NGy + g.NGz + 12);
     AL(s.tiles, int, std::max(bm::scan_tiles(c->nkeys), bm::scan_tiles(np)) + 1);
     AL(s.walk, int, c->nkeys); AL(s.wcnt, int, 2 * kWalkClasses);
     AL(s.big, int, c->npairs / (kWarpPairs + 1) + 1); AL(s.nbig, int, 1);
@@ -598,6 +605,16 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
   if ((r = upload_as<double>(c, (dst), (src), (n), B))) goto fail;
 #define CKF(call)                                              \
   if ((e = (call)) != cudaSuccess) { r = cuda_err(c, e, #call); goto fail; }
+    // node coordinates as node_coord rounds them, and the cell size's reciprocal
+    std::vector<double> axis;
+    for (int a = 0; a < 3; ++a)
+      for (int i = -1; i < (a == 0 ? g.NGx : (a == 1 ? g.NGy : g.NGz)) + 3; ++i) axis.push_back((double)i * g.dcell + g.span0[a]);
+    CKF(cudaMemcpyAsync(s.axis, axis.data(), sizeof(double) * axis.size(), cudaMemcpyHostToDevice, c->stream));
+    s.rdcell[0] = s.rdcell[1] = 0.0;
+    if (std::fabs(std::ilogb(g.dcell)) <= 400) {
+      s.rdcell[0] = 1.0 / g.dcell;
+      s.rdcell[1] = std::fma(-s.rdcell[0], g.dcell, 1.0) * s.rdcell[0];
+    }
     CKF(cudaMemcpyAsync(s.xp, d->xp, sizeof(double) * 3 * np, cudaMemcpyHostToDevice, c->stream));
     // XX (the position at t + DT) is written by ParticlePositionUpdate for
     // the particles inside the grid only (update_step.f90:1477, 1515); the
@@ -659,7 +676,7 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
       CKF(cudaMemsetAsync(s.pk, 0, sizeof(double) * 9 * np, c->stream));
       CKF(cudaMemcpyAsync(s.vol0, s.vol, sizeof(double) * np, cudaMemcpyDeviceToDevice, c->stream));
       c->ops->tl_initial(&c->st, g, c->stream);
-      CKF(cudaMemsetAsync(s.seg, 0, sizeof(int) * ((size_t)c->nkeys + 1), c->stream));
+      CKF(cudaMemsetAsync(s.seg, 0, sizeof(int) * seg_words(c), c->stream));
       c->ops->fixed_locate(&c->st, g, 1, c->stream);
       if ((r = sort_pairs(c))) goto fail;
       c->ops->p2g_mass(&c->st, g, 0, 0, c->stream);
@@ -697,7 +714,7 @@ int mpm_step_phase(mpm_ctx* c, int phase) {
     case MPM_PHASE_BEGIN_STEP: o->begin_step(st, g, s); break;
     case MPM_PHASE_GRID_MOMENTUM_INITIAL:
       if (g.tlmpm) {  // TLGridMomentumInitial: momentum with the cells of the initial positions
-        cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * ((size_t)c->nkeys + 1), s);
+        cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), s);
         if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
         o->fixed_locate(st, g, 1, s);
         if ((r = sort_pairs(c))) return r;

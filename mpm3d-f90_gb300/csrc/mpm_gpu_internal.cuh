@@ -143,6 +143,11 @@ struct DevState {
   // shape cache
   int* snode;
   R *shp, *dndx, *dndy, *dndz;
+  // particles by their number of cpGIMP slots (k_gimp_slots): four lists [4][Np]
+  // and their lengths (behind seg); null for the other shapes and TLMPM
+  int *slot_list, *slot_cnt;
+  double* axis;      // node coordinates of the three axes (axis_coord)
+  double rdcell[2];  // reciprocal of the cell size as a two-part sum
   // pairs
   unsigned* val_sorted;  // node-sorted pairs (mpm_pairs.cuh)
   int *seg, *fill, *tiles, *big, *nbig;  // segment ends, places taken, scan tile totals, long segments

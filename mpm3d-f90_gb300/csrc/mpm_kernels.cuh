@@ -53,234 +53,6 @@ __device__ __forceinline__ void gimp_1d(R rr, R& sh, R& dn) {
   }
 }
 
-// Influence slots of particle p (node or, for SGMP, centre-node index per
-// slot, -1 when invalid) and their shape functions, written to the shape
-// cache; returns the number of slots used. x = the position the GIMP and
-// B-spline weights are taken at, icell / xn = the particle's cell and its
-// natural coordinates (linear), cc / xxn = its dual cell and coordinates
-// (SGMP). ParticleInitial passes the state at the start of the step;
-// SmoothStressbyGrid passes the current position with the step's cells.
-template <class P>
-__device__ __forceinline__ int slot_shapes(St<P>& s, const Geometry& g, long long p, const double x[3], int icell,
-                                           const double xn[3], int cc, const double xxn[3], int slot_node[27]) {
-  using R = typename P::R;
-  const long long np = g.np;
-  int nvalid = 0;
-  if (g.shape == 3) {
-    if (cc > 0) {
-      int c = cc - 1;
-      int cz = c / g.CNCxy, rem = c - cz * g.CNCxy, cy = rem / g.CNCx, cx = rem - cy * g.CNCx;
-      int c1 = cz * g.NCxy + cy * g.NCx + cx;  // CenterCellNode(:,1), 0-based cell
-      for (int k = 0; k < 8; ++k) {
-        int cid = c1 + kCorner[k][0] + kCorner[k][1] * g.NCx + kCorner[k][2] * g.NCxy;
-        bool ok = cid >= 0 && cid < g.ncell;
-        slot_node[k] = ok ? cid : -1;
-        R sx = (R)kSN[0][k] * (R)xxn[0] + (R)1.0;
-        R sy = (R)kSN[1][k] * (R)xxn[1] + (R)1.0;
-        R sz = (R)kSN[2][k] * (R)xxn[2] + (R)1.0;
-        s.shp[k * np + p] = sx * sy * sz * (R)0.125;
-      }
-      nvalid = 8;
-    }
-  } else if (icell > 0) {
-    const int n1 = cell_node1(g, icell);
-    if (g.shape == 0) {  // linear hexahedron, NShape
-      for (int k = 0; k < 8; ++k) {
-        slot_node[k] = n1 + kCorner[k][0] + kCorner[k][1] * g.NGx + kCorner[k][2] * g.NGxy;
-        R sx = (R)kSN[0][k] * (R)xn[0] + (R)1.0;
-        R sy = (R)kSN[1][k] * (R)xn[1] + (R)1.0;
-        R sz = (R)kSN[2][k] * (R)xn[2] + (R)1.0;
-        const R j4 = (R)g.iJacobi4;
-        s.shp[k * np + p] = sx * sy * sz * (R)0.125;
-        s.dndx[k * np + p] = (R)kSN[0][k] * sy * sz * j4;
-        s.dndy[k * np + p] = (R)kSN[1][k] * sx * sz * j4;
-        s.dndz[k * np + p] = (R)kSN[2][k] * sx * sy * j4;
-      }
-      nvalid = 8;
-    } else if (g.shape == 1) {  // cpGIMP
-      int i1[3];
-      {
-        int iz = n1 / g.NGxy, rem = n1 - iz * g.NGxy, iy = rem / g.NGx;
-        i1[0] = rem - iy * g.NGx;
-        i1[1] = iy;
-        i1[2] = iz;
-      }
-      double rel[3];
-      for (int d = 0; d < 3; ++d) rel[d] = (x[d] - node_coord(g, n1, d)) * g.iDCell;
-      int q[3];
-      for (int d = 0; d < 3; ++d) q[d] = rel[d] < 0.25 ? 0 : (rel[d] > 0.75 ? 2 : 1);
-      const GimpCase& gc = kGimp[q[2] * 9 + q[1] * 3 + q[0]];
-      nvalid = gc.n;
-      const R idc = (R)g.iDCell;
-      // 1-D shape values for the four node offsets -1..2 of each direction
-      // (NShape_GIMP, Grid.f90:577-591): every slot whose node is not a
-      // wrapped flat index uses these, so each r is computed once
-      R sh1[3][4], dn1[3][4];
-      for (int d = 0; d < 3; ++d)
-        for (int o = 0; o < 4; ++o) {
-          R rr;
-          if constexpr (P::kExact)
-            rr = (x[d] - ((double)(i1[d] + o - 1) * g.dcell + g.span0[d])) * g.iDCell;
-          else
-            rr = (R)rel[d] - (R)(o - 1);
-          gimp_1d<R>(rr, sh1[d][o], dn1[d][o]);
-        }
-      const int NGd[3] = {g.NGx, g.NGy, g.NGz};
-      for (int k = 0; k < gc.n; ++k) {
-        int off = gc.off[k];
-        int od[3] = {(off & 3), ((off >> 2) & 3), (off >> 4)};  // offset + 1
-        int nd = n1 + (od[0] - 1) + (od[1] - 1) * g.NGx + (od[2] - 1) * g.NGxy;  // flat arithmetic
-        bool ok = nd >= 0 && nd < g.nn;
-        slot_node[k] = ok ? nd : -1;
-        if (!ok) continue;
-        R sh[3], dn[3];
-        bool wrapped = false;
-        for (int d = 0; d < 2; ++d) {
-          int id = i1[d] + od[d] - 1;
-          if (id < 0 || id >= NGd[d]) wrapped = true;
-        }
-        if (!wrapped) {
-          for (int d = 0; d < 3; ++d) {
-            sh[d] = sh1[d][od[d]];
-            dn[d] = dn1[d][od[d]];
-          }
-        } else {  // the +-1 / +-NGx offset crossed a grid row: the node lies elsewhere
-          int iz = nd / g.NGxy, rem = nd - iz * g.NGxy, iy = rem / g.NGx, ix = rem - iy * g.NGx;
-          for (int d = 0; d < 3; ++d) {
-            R rr;
-            if constexpr (P::kExact) {
-              rr = (x[d] - node_coord(g, nd, d)) * g.iDCell;
-            } else {
-              int id = d == 0 ? ix : (d == 1 ? iy : iz);
-              rr = (R)rel[d] - (R)(id - i1[d]);
-            }
-            gimp_1d<R>(rr, sh[d], dn[d]);
-          }
-        }
-        s.shp[k * np + p] = sh[0] * sh[1] * sh[2];
-        s.dndx[k * np + p] = dn[0] * sh[1] * sh[2] * idc;
-        s.dndy[k * np + p] = sh[0] * dn[1] * sh[2] * idc;
-        s.dndz[k * np + p] = sh[0] * sh[1] * dn[2] * idc;
-      }
-    } else {  // quadratic B-spline
-      R sh[3][3], dn[3][3];
-      const R c02 = f32<R>(0.2f), c04 = f32<R>(0.4f), idc = (R)g.iDCell;
-      for (int d = 0; d < 3; ++d) {
-        R r;
-        if constexpr (P::kExact)
-          r = (x[d] - node_coord(g, n1, d)) * g.iDCell * (double)0.2f + (double)0.4f;
-        else
-          r = (R)((x[d] - node_coord(g, n1, d)) * g.iDCell) * c02 + c04;
-        R a = (R)3 - (R)5 * r;
-        R b = (R)5 * r - (R)2;
-        sh[0][d] = (R)0.5 * (a * a);
-        sh[1][d] = -((R)25 * (r * r)) + (R)25 * r - (R)5.5;
-        sh[2][d] = (R)0.5 * (b * b);
-        dn[0][d] = ((R)5 * r - (R)3) * (R)5 * c02 * idc;
-        dn[1][d] = (-((R)50 * r) + (R)25) * c02 * idc;
-        dn[2][d] = ((R)5 * r - (R)2) * (R)5 * c02 * idc;
-      }
-      for (int k = 0; k < 27; ++k) {
-        int a = kBsp[k][0], b = kBsp[k][1], c = kBsp[k][2];
-        int nd = n1 + (a - 1) + (b - 1) * g.NGx + (c - 1) * g.NGxy;
-        bool ok = nd >= 0 && nd < g.nn;
-        slot_node[k] = ok ? nd : -1;
-        s.shp[k * np + p] = sh[a][0] * sh[b][1] * sh[c][2];
-        s.dndx[k * np + p] = dn[a][0] * sh[b][1] * sh[c][2];
-        s.dndy[k * np + p] = sh[a][0] * dn[b][1] * sh[c][2];
-        s.dndz[k * np + p] = sh[a][0] * sh[b][1] * dn[c][2];
-      }
-      nvalid = 27;
-    }
-  }
-  return nvalid;
-}
-
-// the nodes of particle p's slots and the per-node pair counts; cbase = the
-// first node of the particle's grid component
-template <class P>
-__device__ __forceinline__ void write_pairs(St<P>& s, const Geometry& g, long long p, int nvalid,
-                                            const int slot_node[27], int cbase) {
-  const long long np = g.np;
-  for (int k = 0; k < g.K; ++k) {
-    int nd = k < nvalid && slot_node[k] >= 0 ? cbase + slot_node[k] : -1;
-    s.snode[k * np + p] = nd;
-    if (nd >= 0) atomicAdd(&s.seg[nd], 1);  // per-node pair count (integer, deterministic)
-  }
-}
-
-// ----------------------------------------------------------------- locate
-// ParticleInitial (update_step.f90:408-453) plus the shape functions of the
-// step (NShape / FindInflNode+NShape_GIMP / BFindInflNode+NShape_Bspline /
-// SGNShape), cached per (slot, particle), with the nodes of the slots and the
-// pair counts of the node-sorted list (mpm_pairs.cuh).
-template <class P>
-__global__ void k_locate(St<P> s, Geometry g) {
-  using B = typename P::B;
-  const long long p = gtid();
-  if (p >= g.np) return;
-  const long long np = g.np;
-  double x[3] = {s.xp[p], s.xp[np + p], s.xp[2 * np + p]};
-  int icell = in_which_cell(g, x);
-  s.icell[p] = icell;
-  double xn[3] = {0, 0, 0};
-  if (icell > 0) {
-    int n1 = cell_node1(g, icell);
-    for (int d = 0; d < 3; ++d) {
-      double cxg = node_coord(g, n1, d) + g.dcell / 2.0;  // Cxg, Grid.f90:380
-      xn[d] = (x[d] - cxg) * g.iJacobi;
-      s.xn[d * np + p] = (B)xn[d];
-    }
-  } else {
-    atomicOr(&s.sc->status, (unsigned)ST_OUT_OF_GRID);
-  }
-  int cc = 0;
-  double xxn[3] = {0, 0, 0};
-  if (g.shape == 3) {  // SGMP: the dual (cell-centre) grid
-    cc = center_in_which_cell(g, x);
-    s.centericell[p] = cc;
-    int ix = (int)((x[0] - g.span0[0]) / g.dcell + 0.5) + 1;
-    int iy = (int)((x[1] - g.span0[1]) / g.dcell + 0.5) + 1;
-    int iz = (int)((x[2] - g.span0[2]) / g.dcell + 0.5) + 1;
-    long long inode = (long long)(iz - 1) * g.NGxy + (long long)(iy - 1) * g.NGx + ix;
-    s.inode[p] = (int)inode;
-    if (inode >= 1 && inode <= g.nn) {
-      int bd = s.bd[inode - 1];
-      for (int d = 0; d < 3; ++d) {
-        double xg = node_coord(g, (int)inode - 1, d);
-        xxn[d] = (x[d] - xg) * g.iJacobi;
-        int bt = (bd >> (2 * d)) & 3;
-        if (bt != 0) {
-          if (xxn[d] > 0) xxn[d] = 1;
-          else if (xxn[d] < 0) xxn[d] = -1;
-        }
-        s.xxn[d * np + p] = (B)xxn[d];
-      }
-    } else {
-      for (int d = 0; d < 3; ++d) xxn[d] = (double)s.xxn[d * np + p];
-    }
-  }
-  int slot_node[27];
-  const int nvalid = slot_shapes<P>(s, g, p, x, icell, xn, cc, xxn, slot_node);
-  write_pairs<P>(s, g, p, nvalid, slot_node, g.shape == 3 ? 0 : s.bodies[s.body[p]].comp * g.nn);
-}
-
-__device__ __forceinline__ void decode_pair(unsigned v, long long np, long long* p, long long* idx) {
-  long long pp = (long long)(v >> 5);
-  int k = (int)(v & 31u);
-  *p = pp;
-  *idx = (long long)k * np + pp;
-}
-
-// ----------------------------------------------------- node-level helpers
-__device__ __forceinline__ void node_bc(const uint8_t fix, double* px, double* fx, long long n, long long nn) {
-  for (int c = 0; c < 3; ++c)
-    if (fix & (1 << c)) {
-      px[(long long)c * nn + n] = 0.0;
-      fx[(long long)c * nn + n] = 0.0;
-    }
-}
-
 // Division by a node's mass. The node and particle kernels divide by each
 // node's mass tens of times a step (the position update alone three times per
 // particle and slot), and an FP64 division costs GB300's narrow FP64 pipe
@@ -316,6 +88,349 @@ __device__ __forceinline__ double div_known(double x, double m, const Recip& y) 
   const unsigned e = (unsigned)hi >> 20;
   if ((e - 523u > 1000u || __double2hiint(y.yh) == 0) && (hi | __double2loint(x)) != 0) q = div_plain(x, m);
   return q;
+}
+
+// The same in FP64 with fewer instructions, each result the one above's: the
+// comparisons are integer ones (the bounds have no low words), the scalings by
+// powers of two are folded into exact fused multiply-adds (7 - 16 a^2 over 8 =
+// 0.875 - 2 a^2 and (5 - 4 a) / 4 = 1.25 - a, rounded alike), and the pieces
+// share theirs: four FP64 instructions for fifteen.
+__device__ __forceinline__ void gimp_1d_f64(double rr, double& sh, double& dn) {
+  const int hi = __double2hiint(rr) & 0x7fffffff;
+  const double a = fabs(rr);
+  const bool in = hi < 0x3fd00000, mid = hi < 0x3fe80000, out = hi >= 0x3ff40000;  // < 1/4, < 3/4, not < 5/4
+  const double t = (mid ? 1.0 : 1.25) - a;
+  const double m = in ? a : t, sq = m * m;
+  sh = in ? __fma_rn(-2.0, sq, 0.875) : (mid ? t : sq);
+  dn = __fma_rn(in ? -4.0 : 2.0, rr, in ? -0.0 : -copysign(2.5, rr));
+  if (mid && !in) dn = -copysign(1.0, rr);
+  if (out) sh = dn = 0.0;
+}
+
+// ------------------------------------------------------------------ slots
+// A particle's influence slots (node or, for SGMP, centre-node index per slot,
+// -1 when invalid) and their shape functions, written to the shape cache, with
+// the pair counts of the node-sorted list (mpm_pairs.cuh). cbase: the first
+// node of the particle's grid component.
+template <class P>
+__device__ __forceinline__ void put_slot(St<P>& s, long long np, long long p, int k, int nd) {
+  s.snode[k * np + p] = nd;
+  if (nd >= 0) atomicAdd(&s.seg[nd], 1);  // per-node pair count (integer, deterministic)
+}
+
+// node coordinate i of axis d (i from -1 to two beyond the last), as node_coord
+// computes it: the FP64 pipe that the conversion and the product would take
+// bounds the kernels that ask
+template <class P>
+__device__ __forceinline__ double axis_coord(const St<P>& s, const Geometry& g, int d, int i) {
+  return s.axis[(d > 0 ? g.NGx + 4 : 0) + (d > 1 ? g.NGy + 4 : 0) + 1 + i];
+}
+
+__device__ __forceinline__ void cell_coords(const Geometry& g, int icell, int i1[3]) {
+  const int c = icell - 1;
+  i1[2] = c / g.NCxy;
+  const int rem = c - i1[2] * g.NCxy;
+  i1[1] = rem / g.NCx;
+  i1[0] = rem - i1[1] * g.NCx;
+}
+
+// Slots of every shape but cpGIMP. x = the position the B-spline weights are
+// taken at, icell / xn = the particle's cell and its natural coordinates
+// (linear), cc / xxn = its dual cell and coordinates (SGMP).
+// ParticleInitial passes the state at the start of the step;
+// SmoothStressbyGrid the current position with the step's cells. Fully
+// unrolled, so that the slots share their products.
+template <class P, int SH>
+__device__ __forceinline__ void write_slots(St<P>& s, const Geometry& g, long long p, const double x[3], int icell,
+                                            const double xn[3], int cc, const double xxn[3], int cbase) {
+  using R = typename P::R;
+  const long long np = g.np;
+  constexpr int NS = SH == 2 ? 27 : 8;
+  if (SH == 3 ? cc <= 0 : icell <= 0) {
+#pragma unroll 1
+    for (int k = 0; k < NS; ++k) s.snode[k * np + p] = -1;
+    return;
+  }
+  if constexpr (SH == 2) {  // quadratic B-spline
+    int i1[3];
+    cell_coords(g, icell, i1);
+    const int n1 = i1[2] * g.NGxy + i1[1] * g.NGx + i1[0];
+    R sh[3][3], dn[3][3];
+    const R c02 = f32<R>(0.2f), c04 = f32<R>(0.4f), idc = (R)g.iDCell;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const R r = (x[d] - axis_coord<P>(s, g, d, i1[d])) * g.iDCell * (double)0.2f + (double)0.4f;
+      R a = (R)3 - (R)5 * r;
+      R b = (R)5 * r - (R)2;
+      sh[0][d] = (R)0.5 * (a * a);
+      sh[1][d] = -((R)25 * (r * r)) + (R)25 * r - (R)5.5;
+      sh[2][d] = (R)0.5 * (b * b);
+      dn[0][d] = ((R)5 * r - (R)3) * (R)5 * c02 * idc;
+      dn[1][d] = (-((R)50 * r) + (R)25) * c02 * idc;
+      dn[2][d] = ((R)5 * r - (R)2) * (R)5 * c02 * idc;
+    }
+    constexpr unsigned char kB[27][3] = MPM_BSP_SLOTS;
+#pragma unroll
+    for (int k = 0; k < 27; ++k) {
+      const int a = kB[k][0], b = kB[k][1], c = kB[k][2];
+      const int nd = n1 + (a - 1) + (b - 1) * g.NGx + (c - 1) * g.NGxy;
+      put_slot<P>(s, np, p, k, nd >= 0 && nd < g.nn ? cbase + nd : -1);
+      s.shp[k * np + p] = sh[a][0] * sh[b][1] * sh[c][2];
+      s.dndx[k * np + p] = dn[a][0] * sh[b][1] * sh[c][2];
+      s.dndy[k * np + p] = sh[a][0] * dn[b][1] * sh[c][2];
+      s.dndz[k * np + p] = sh[a][0] * sh[b][1] * dn[c][2];
+    }
+  } else {
+    constexpr unsigned char kC[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
+                                        {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};  // kCorner
+    R w[3][2];  // 1 -+ the natural coordinate
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const R v = (R)(SH == 3 ? xxn[d] : xn[d]);
+      w[d][0] = (R)1.0 - v;
+      w[d][1] = (R)1.0 + v;
+    }
+    int first, stepy, stepz;
+    if constexpr (SH == 3) {  // the dual cell's centre nodes, as cells
+      const int c = cc - 1;
+      const int cz = c / g.CNCxy, rem = c - cz * g.CNCxy, cy = rem / g.CNCx, cx = rem - cy * g.CNCx;
+      first = cz * g.NCxy + cy * g.NCx + cx;  // CenterCellNode(:,1), 0-based cell
+      stepy = g.NCx;
+      stepz = g.NCxy;
+    } else {
+      first = cell_node1(g, icell) + cbase;
+      stepy = g.NGx;
+      stepz = g.NGxy;
+    }
+    const R j4 = (R)g.iJacobi4;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int a = kC[k][0], b = kC[k][1], c = kC[k][2];
+      int nd = first + a + b * stepy + c * stepz;
+      if (SH == 3 && (nd < 0 || nd >= g.ncell)) nd = -1;
+      put_slot<P>(s, np, p, k, nd);
+      s.shp[k * np + p] = w[0][a] * w[1][b] * w[2][c] * (R)0.125;
+      if (SH == 0) {  // linear hexahedron, NShape
+        const R gx = w[1][b] * w[2][c] * j4, gy = w[0][a] * w[2][c] * j4, gz = w[0][a] * w[1][b] * j4;
+        s.dndx[k * np + p] = a ? gx : -gx;
+        s.dndy[k * np + p] = b ? gy : -gy;
+        s.dndz[k * np + p] = c ? gz : -gz;
+      }
+    }
+  }
+}
+
+// --------------------------------------------------------- cpGIMP slots
+// A particle has 27, 18, 12 or 8 cpGIMP slots, for each axis three where it
+// lies within a quarter of a cell of a node plane and two elsewhere. The
+// passes over a particle's slots are FP64 work that a warp executes as often
+// as its longest lane asks (26.9 of 27 times on average in a loosened soil,
+// whose particles have 15.6), so they take the particles by the number of
+// slots: slot_list holds them in four lists, longest first, slot_cnt their
+// lengths. A list keeps about the particles' order, so that a warp's accesses
+// stay within a few hundred particles; the order has no bearing on results.
+// Slope of 159 k particles, GB300: stress update 320 -> 235 us, position update
+// 269 -> 147, shape functions 318 -> 159 (with gimp_1d_f64 and the weights in
+// shared memory instead of a local array).
+template <class P>
+__device__ __forceinline__ void list_particle(St<P>& s, long long np, long long p, bool in, int c) {
+  const unsigned grp = __match_any_sync(0xffffffffu, in ? c : -1);
+  const int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
+  int base = 0;
+  if (in && lane == leader) base = atomicAdd(&s.slot_cnt[c], __popc(grp));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (in) s.slot_list[c * np + base + __popc(grp & ((1u << lane) - 1u))] = (int)p;
+}
+
+// the t-th particle to process and its number of slots at most; -1 past the last
+template <class P>
+__device__ __forceinline__ long long take_particle(const St<P>& s, const Geometry& g, long long t, int& K) {
+  const long long np = g.np;
+  K = g.K;
+  if (t >= np) return -1;
+  if (!s.slot_list) return t;
+  const int n0 = s.slot_cnt[0], n1 = n0 + s.slot_cnt[1], n2 = n1 + s.slot_cnt[2], n3 = n2 + s.slot_cnt[3];
+  if (t >= n3) return -1;
+  const int c = t < n0 ? 0 : (t < n1 ? 1 : (t < n2 ? 2 : 3));
+  K = c == 0 ? 27 : (c == 1 ? 18 : (c == 2 ? 12 : 8));
+  return s.slot_list[c * np + t - (c == 0 ? 0 : (c == 1 ? n0 : (c == 2 ? n1 : n2)))];
+}
+
+// which of the three parts of its cell a particle lies in, per axis
+__device__ __forceinline__ int gimp_part(double rel) { return rel < 0.25 ? 0 : (rel > 0.75 ? 2 : 1); }
+
+// list of a particle with these parts (0: 27 slots)
+__device__ __forceinline__ int gimp_list(const int q[3]) { return (q[0] == 1) + (q[1] == 1) + (q[2] == 1); }
+
+// LISTED: the particles in the order of the lists, which k_locate filled;
+// otherwise (the current positions with the step's cells) in their own order,
+// filling the lists. with_comp: keys in the particle's grid component.
+// The 1-D weights of the node offsets -1..2 of each axis (NShape_GIMP,
+// Grid.f90:577-591) are taken once per particle, into shared memory, where the
+// slots pick theirs; a slot whose offset crossed the end of a grid row lies
+// elsewhere and takes its own.
+constexpr int kGimpBlock = 128;
+template <class P, bool LISTED>
+__global__ void __launch_bounds__(kGimpBlock) k_gimp_slots(St<P> s, Geometry g, int with_comp) {
+  extern __shared__ double wt[];  // [24][blockDim.x]: weights (axis, offset), then derivatives
+  __shared__ unsigned char tab[27 * sizeof(GimpCase)];
+  for (int i = threadIdx.x; i < (int)sizeof tab; i += blockDim.x) tab[i] = reinterpret_cast<const unsigned char*>(kGimp)[i];
+  __syncthreads();
+  const long long np = g.np;
+  const int nt = blockDim.x, t = threadIdx.x;
+  int K = g.K;
+  long long p = gtid();
+  if (LISTED) {
+    p = take_particle<P>(s, g, p, K);
+    if (p < 0) return;
+  }
+  const bool in = p < np;
+  const int icell = in ? s.icell[p] : 0;
+  int q[3] = {1, 1, 1}, i1[3] = {0, 0, 0};
+  double x[3];
+  if (icell > 0) {
+    cell_coords(g, icell, i1);
+    for (int d = 0; d < 3; ++d) {
+      x[d] = s.xp[d * np + p];
+      const double c0 = axis_coord<P>(s, g, d, i1[d]);
+      const double r0 = (x[d] - c0) * g.iDCell;
+      q[d] = gimp_part(r0);
+      // offsets 0 and 1, and the one beyond on the particle's side
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const int o = e == 0 ? 1 : (e == 1 ? 2 : (q[d] == 0 ? 0 : 3));
+        const double rr = e == 0 ? r0 : (x[d] - axis_coord<P>(s, g, d, i1[d] + o - 1)) * g.iDCell;
+        double sh, dn;
+        gimp_1d_f64(rr, sh, dn);
+        wt[(d * 4 + o) * nt + t] = sh;
+        wt[(12 + d * 4 + o) * nt + t] = dn;
+      }
+    }
+  }
+  if (!LISTED) {
+    list_particle<P>(s, np, p, in, gimp_list(q));
+    if (!in) return;
+  }
+  int n = 0;
+  if (icell > 0) {
+    const unsigned char* gc = tab + (q[2] * 9 + q[1] * 3 + q[0]) * sizeof(GimpCase);
+    n = gc[0];
+    const int n1 = i1[2] * g.NGxy + i1[1] * g.NGx + i1[0];
+    const int cbase = with_comp ? s.bodies[s.body[p]].comp * g.nn : 0;
+    const double idc = g.iDCell;
+    for (int k = 0; k < n; ++k) {
+      const int off = gc[1 + k];
+      const int o0 = off & 3, o1 = (off >> 2) & 3, o2 = off >> 4;                    // offset + 1
+      const int nd = n1 + (o0 - 1) + (o1 - 1) * g.NGx + (o2 - 1) * g.NGxy;           // flat arithmetic
+      const bool ok = nd >= 0 && nd < g.nn;
+      put_slot<P>(s, np, p, k, ok ? cbase + nd : -1);
+      if (!ok) continue;
+      double sh[3], dn[3];
+      const int ix = i1[0] + o0 - 1, iy = i1[1] + o1 - 1;
+      if ((unsigned)ix < (unsigned)g.NGx && (unsigned)iy < (unsigned)g.NGy) {
+        const int o[3] = {o0, o1, o2};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          sh[d] = wt[(d * 4 + o[d]) * nt + t];
+          dn[d] = wt[(12 + d * 4 + o[d]) * nt + t];
+        }
+      } else {
+        for (int d = 0; d < 3; ++d) gimp_1d_f64((x[d] - node_coord(g, nd, d)) * g.iDCell, sh[d], dn[d]);
+      }
+      const double xy = sh[0] * sh[1];
+      s.shp[k * np + p] = xy * sh[2];
+      s.dndx[k * np + p] = dn[0] * sh[1] * sh[2] * idc;
+      s.dndy[k * np + p] = sh[0] * dn[1] * sh[2] * idc;
+      s.dndz[k * np + p] = xy * dn[2] * idc;
+    }
+  }
+  for (int k = n; k < g.K; ++k) s.snode[k * np + p] = -1;
+}
+
+// ----------------------------------------------------------------- locate
+// ParticleInitial (update_step.f90:408-453) plus the shape functions of the
+// step (NShape / BFindInflNode+NShape_Bspline / SGNShape; those of
+// FindInflNode+NShape_GIMP: k_gimp_slots, in the order listed here)
+template <class P, int SH>
+__global__ void k_locate(St<P> s, Geometry g) {
+  using B = typename P::B;
+  const long long p = gtid();
+  const long long np = g.np;
+  int q[3] = {1, 1, 1};
+  if (p < np) {
+    const double x[3] = {s.xp[p], s.xp[np + p], s.xp[2 * np + p]};
+    // InWhichCell, Grid.f90:123-155
+    const Recip rc = {s.rdcell[0], s.rdcell[1]};
+    int icell = -1, i[3];
+    bool in = true;
+    double r[3];  // cells from the grid's corner
+    for (int d = 0; d < 3; ++d) {
+      in = in && !(x[d] < g.span0[d] || x[d] > g.span1[d]);
+      r[d] = div_known(x[d] - g.span0[d], g.dcell, rc);
+      i[d] = (int)r[d];
+    }
+    if (in) {
+      const long long c = (long long)i[2] * g.NCxy + (long long)i[1] * g.NCx + i[0] + 1;
+      if (c > 0 && c <= g.ncell) icell = (int)c;
+    }
+    s.icell[p] = icell;
+    double xn[3] = {0, 0, 0};
+    if (icell > 0) {
+      int i1[3];
+      cell_coords(g, icell, i1);
+      for (int d = 0; d < 3; ++d) {
+        const double c0 = axis_coord<P>(s, g, d, i1[d]);
+        const double cxg = c0 + g.dcell / 2.0;  // Cxg, Grid.f90:380
+        xn[d] = (x[d] - cxg) * g.iJacobi;
+        s.xn[d * np + p] = (B)xn[d];
+        if (SH == 1) q[d] = gimp_part((x[d] - c0) * g.iDCell);
+      }
+    } else {
+      atomicOr(&s.sc->status, (unsigned)ST_OUT_OF_GRID);
+    }
+    int cc = 0;
+    double xxn[3] = {0, 0, 0};
+    if (SH == 3) {  // SGMP: the dual (cell-centre) grid
+      cc = center_in_which_cell(g, x);
+      s.centericell[p] = cc;
+      const int ix = (int)(r[0] + 0.5) + 1, iy = (int)(r[1] + 0.5) + 1, iz = (int)(r[2] + 0.5) + 1;
+      const long long inode = (long long)(iz - 1) * g.NGxy + (long long)(iy - 1) * g.NGx + ix;
+      s.inode[p] = (int)inode;
+      if (inode >= 1 && inode <= g.nn) {
+        const int bd = s.bd[inode - 1];
+        for (int d = 0; d < 3; ++d) {
+          const double xg = node_coord(g, (int)inode - 1, d);
+          xxn[d] = (x[d] - xg) * g.iJacobi;
+          const int bt = (bd >> (2 * d)) & 3;
+          if (bt != 0) {
+            if (xxn[d] > 0) xxn[d] = 1;
+            else if (xxn[d] < 0) xxn[d] = -1;
+          }
+          s.xxn[d * np + p] = (B)xxn[d];
+        }
+      } else {
+        for (int d = 0; d < 3; ++d) xxn[d] = (double)s.xxn[d * np + p];
+      }
+    }
+    if (SH != 1) write_slots<P, SH>(s, g, p, x, icell, xn, cc, xxn, SH == 3 ? 0 : s.bodies[s.body[p]].comp * g.nn);
+  }
+  if (SH == 1) list_particle<P>(s, np, p, p < np, gimp_list(q));
+}
+
+__device__ __forceinline__ void decode_pair(unsigned v, long long np, long long* p, long long* idx) {
+  long long pp = (long long)(v >> 5);
+  int k = (int)(v & 31u);
+  *p = pp;
+  *idx = (long long)k * np + pp;
+}
+
+// ----------------------------------------------------- node-level helpers
+__device__ __forceinline__ void node_bc(const uint8_t fix, double* px, double* fx, long long n, long long nn) {
+  for (int c = 0; c < 3; ++c)
+    if (fix & (1 << c)) {
+      px[(long long)c * nn + n] = 0.0;
+      fx[(long long)c * nn + n] = 0.0;
+    }
 }
 
 // node velocity; the mass's reciprocal is stored with the mass
@@ -855,8 +970,9 @@ template <class P, int MT, int UV>
 __global__ void __launch_bounds__(kBlock, MT == 0 ? 1 : 2) k_stress(St<P> s, Geometry g) {
   using R = typename P::R;
   using B = typename P::B;
-  const long long p = gtid();
-  if (p >= g.np) return;
+  int K;
+  const long long p = take_particle<P>(s, g, gtid(), K);
+  if (p < 0) return;
   const long long np = g.np;
   const long long nn = g.nnt;  // node arrays of every grid component
   if (g.has_jc) {
@@ -879,11 +995,11 @@ __global__ void __launch_bounds__(kBlock, MT == 0 ? 1 : 2) k_stress(St<P> s, Geo
   } else {
     if (s.icell[p] < 0) return;
     constexpr int U = 3;  // slots whose gathers are in flight together
-    for (int k0 = 0; k0 < g.K; k0 += U) {
+    for (int k0 = 0; k0 < K; k0 += U) {
       int n[U];
       double m[U], v[U][3], dn[U][3];
 #pragma unroll
-      for (int u = 0; u < U; ++u) n[u] = k0 + u < g.K ? s.snode[(k0 + u) * np + p] : -1;
+      for (int u = 0; u < U; ++u) n[u] = k0 + u < K ? s.snode[(k0 + u) * np + p] : -1;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         m[u] = 0.0;
@@ -1261,8 +1377,9 @@ __global__ void k_contact_sum(St<P> s, Geometry g) {
 template <class P>
 __global__ void k_position(St<P> s, Geometry g) {
   using R = typename P::R;
-  const long long p = gtid();
-  if (p >= g.np) return;
+  int K;
+  const long long p = take_particle<P>(s, g, gtid(), K);
+  if (p < 0) return;
   const long long np = g.np;
   const long long nn = g.nnt;  // node arrays of every grid component
   const DevScalars& sc = *s.sc;
@@ -1304,12 +1421,12 @@ __global__ void k_position(St<P> s, Geometry g) {
     if (s.icell[p] < 0) return;
     // (the gathers of a few slots in flight before the first one's sums)
     constexpr int U = 3;
-    for (int k0 = 0; k0 < g.K; k0 += U) {
+    for (int k0 = 0; k0 < K; k0 += U) {
       int n[U];
       double m[U], sk[U], v[U][3], f[U][3];
       Recip y[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) n[u] = k0 + u < g.K ? s.snode[(k0 + u) * np + p] : -1;
+      for (int u = 0; u < U; ++u) n[u] = k0 + u < K ? s.snode[(k0 + u) * np + p] : -1;
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         m[u] = 0.0;
@@ -1917,23 +2034,19 @@ __global__ void k_tl_sg_node_force(St<P> s, Geometry g, int integ) {
 // the start of the step for the smoothing, those of the start of the run for
 // TLMPM): GIMP / B-spline weights at the current position, linear ones at
 // XN, SGMP ones at XXN; with_comp: keys in the particle's grid component
-template <class P>
+template <class P, int SH>
 __global__ void k_fixed_locate(St<P> s, Geometry g, int with_comp) {
   const long long p = gtid();
   if (p >= g.np) return;
   const long long np = g.np;
   const double x[3] = {s.xp[p], s.xp[np + p], s.xp[2 * np + p]};
-  const int icell = s.icell[p];
   double xn[3] = {0, 0, 0}, xxn[3] = {0, 0, 0};
   for (int d = 0; d < 3; ++d) {
     xn[d] = (double)s.xn[d * np + p];
-    if (g.shape == 3) xxn[d] = (double)s.xxn[d * np + p];
+    if (SH == 3) xxn[d] = (double)s.xxn[d * np + p];
   }
-  const int cc = g.shape == 3 ? s.centericell[p] : 0;
-  int slot_node[27];
-  const int nvalid = slot_shapes<P>(s, g, p, x, g.shape == 3 ? 0 : icell, xn, cc, xxn, slot_node);
-  const int cbase = with_comp && g.shape != 3 ? s.bodies[s.body[p]].comp * g.nn : 0;  // smoothing: component 1
-  write_pairs<P>(s, g, p, nvalid, slot_node, cbase);
+  const int cbase = with_comp && SH != 3 ? s.bodies[s.body[p]].comp * g.nn : 0;  // smoothing: component 1
+  write_slots<P, SH>(s, g, p, x, s.icell[p], xn, SH == 3 ? s.centericell[p] : 0, xxn, cbase);
 }
 
 // pressure * volume and volume of every (node's or centre node's) slice of

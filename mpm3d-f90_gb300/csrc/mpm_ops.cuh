@@ -30,9 +30,25 @@ struct Ops {
     k_begin_step<<<1, 1, 0, s>>>(S(st).sc);
     prof_end(K_BEGIN, s);
   }
+  template <bool LISTED>
+  static void gimp_slots(void* st, const Geometry& g, int with_comp, cudaStream_t s) {
+    const Shape h(g.np);
+    const unsigned block = h.block < kGimpBlock ? h.block : kGimpBlock;
+    k_gimp_slots<P, LISTED><<<(unsigned)((g.np + block - 1) / block), block, 24 * sizeof(double) * block, s>>>(
+        S(st), g, with_comp);
+  }
   static void locate(void* st, const Geometry& g, cudaStream_t s) {
+    const Shape h(g.np);
     prof_begin(K_LOCATE, s);
-    k_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
+    switch (g.shape) {
+      case 0: k_locate<P, 0><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 1:
+        k_locate<P, 1><<<h.grid, h.block, 0, s>>>(S(st), g);
+        gimp_slots<true>(st, g, 1, s);
+        break;
+      case 2: k_locate<P, 2><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      default: k_locate<P, 3><<<h.grid, h.block, 0, s>>>(S(st), g);
+    }
     prof_end(K_LOCATE, s);
   }
   static void node_offsets(void*, const Geometry&, long long, cudaStream_t) {}
@@ -133,7 +149,13 @@ struct Ops {
 
   static void fixed_locate(void* st, const Geometry& g, int with_comp, cudaStream_t s) {
     prof_begin(K_LOCATE, s);
-    k_fixed_locate<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g, with_comp);
+    const Shape h(g.np);
+    switch (g.shape) {
+      case 0: k_fixed_locate<P, 0><<<h.grid, h.block, 0, s>>>(S(st), g, with_comp); break;
+      case 1: gimp_slots<false>(st, g, with_comp, s); break;
+      case 2: k_fixed_locate<P, 2><<<h.grid, h.block, 0, s>>>(S(st), g, with_comp); break;
+      default: k_fixed_locate<P, 3><<<h.grid, h.block, 0, s>>>(S(st), g, with_comp);
+    }
     prof_end(K_LOCATE, s);
   }
   static void tl_initial(void* st, const Geometry& g, cudaStream_t s) {

@@ -110,7 +110,7 @@ struct GimpCase {
   unsigned char n;
   unsigned char off[27];
 };
-__constant__ const GimpCase kGimp[27] = {
+__device__ const GimpCase kGimp[27] = {
     {27, {21, 22, 26, 25, 37, 38, 42, 41, 5, 6, 10, 9, 1, 2, 17, 18, 33, 34, 20, 24, 36, 40, 4, 8, 0, 16, 32}},
     {18, {21, 22, 26, 25, 37, 38, 42, 41, 5, 6, 10, 9, 1, 2, 17, 18, 33, 34}},
     {27, {21, 22, 26, 25, 37, 38, 42, 41, 5, 6, 10, 9, 1, 2, 17, 18, 33, 34, 23, 27, 39, 43, 7, 11, 3, 19, 35}},
@@ -143,10 +143,11 @@ __constant__ const GimpCase kGimp[27] = {
 // Quadratic B-spline: 27 slots in BFindInflNode order (Grid.f90:852-895);
 // per slot the 1-D piece used in x, y, z (0 lower node, 1 own, 2 upper),
 // which is also the node offset + 1 (NShape_Bspline, Grid.f90:932-1048).
-__constant__ const unsigned char kBsp[27][3] = {
-    {1, 1, 1}, {2, 1, 1}, {2, 2, 1}, {1, 2, 1}, {1, 1, 2}, {2, 1, 2}, {2, 2, 2}, {1, 2, 2}, {1, 1, 0},
-    {2, 1, 0}, {2, 2, 0}, {1, 2, 0}, {1, 0, 0}, {2, 0, 0}, {1, 0, 1}, {2, 0, 1}, {1, 0, 2}, {2, 0, 2},
-    {0, 1, 1}, {0, 2, 1}, {0, 1, 2}, {0, 2, 2}, {0, 1, 0}, {0, 2, 0}, {0, 0, 0}, {0, 0, 1}, {0, 0, 2}};
+#define MPM_BSP_SLOTS \
+  { \
+  {1, 1, 1}, {2, 1, 1}, {2, 2, 1}, {1, 2, 1}, {1, 1, 2}, {2, 1, 2}, {2, 2, 2}, {1, 2, 2}, {1, 1, 0}, \
+  {2, 1, 0}, {2, 2, 0}, {1, 2, 0}, {1, 0, 0}, {2, 0, 0}, {1, 0, 1}, {2, 0, 1}, {1, 0, 2}, {2, 0, 2}, \
+  {0, 1, 1}, {0, 2, 1}, {0, 1, 2}, {0, 2, 2}, {0, 1, 0}, {0, 2, 0}, {0, 0, 0}, {0, 0, 1}, {0, 0, 2}}
 
 // Flat node id (0-based) of the corner-1 node of a 1-based cell id.
 __device__ __forceinline__ int cell_node1(const Geometry& g, int icell) {
