@@ -230,7 +230,7 @@ __device__ __forceinline__ void write_slots(St<P>& s, const Geometry& g, long lo
 // lengths. A list keeps about the particles' order, so that a warp's accesses
 // stay within a few hundred particles; the order has no bearing on results.
 // Slope of 159 k particles, GB300: stress update 320 -> 235 us, position update
-// 269 -> 147, shape functions 318 -> 159 (with gimp_1d_f64 and the weights in
+// 269 -> 146, shape functions 318 -> 129 (with gimp_1d_f64 and the weights in
 // shared memory instead of a local array).
 template <class P>
 __device__ __forceinline__ void list_particle(St<P>& s, long long np, long long p, bool in, int c) {
@@ -269,48 +269,55 @@ __device__ __forceinline__ int gimp_list(const int q[3]) { return (q[0] == 1) + 
 // Grid.f90:577-591) are taken once per particle, into shared memory, where the
 // slots pick theirs; a slot whose offset crossed the end of a grid row lies
 // elsewhere and takes its own.
-constexpr int kGimpBlock = 128;
+// A block takes 32 particles: its first three warps an axis each for the
+// weights, then every warp a quarter of the slots. (One thread per particle
+// had its 27 slots' FP64 instructions in series, 64 cycles each of a warp's
+// share of the pipe; a small scene has not the warps to fill it: with it Cook
+// 5.8 k particles took 31 us for 18, slope 159 k 159 for 129.)
+constexpr int kGimpWarps = 4;
 template <class P, bool LISTED>
-__global__ void __launch_bounds__(kGimpBlock) k_gimp_slots(St<P> s, Geometry g, int with_comp) {
-  extern __shared__ double wt[];  // [24][blockDim.x]: weights (axis, offset), then derivatives
-  __shared__ unsigned char tab[27 * sizeof(GimpCase)];
-  for (int i = threadIdx.x; i < (int)sizeof tab; i += blockDim.x) tab[i] = reinterpret_cast<const unsigned char*>(kGimp)[i];
-  __syncthreads();
+__global__ void __launch_bounds__(32 * kGimpWarps) k_gimp_slots(St<P> s, Geometry g, int with_comp) {
+  __shared__ double wt[24][32];  // weights (axis, offset), then derivatives
+  __shared__ signed char part[3][32];
+  __shared__ __align__(4) unsigned char tab[27 * sizeof(GimpCase)];
+  for (int i = threadIdx.x; i < (int)(sizeof tab / 4); i += blockDim.x)
+    reinterpret_cast<int*>(tab)[i] = reinterpret_cast<const int*>(kGimp)[i];
   const long long np = g.np;
-  const int nt = blockDim.x, t = threadIdx.x;
-  int K = g.K;
-  long long p = gtid();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  long long p = (long long)blockIdx.x * 32 + lane;
   if (LISTED) {
+    int K;
     p = take_particle<P>(s, g, p, K);
-    if (p < 0) return;
+  } else if (p >= np) {
+    p = -1;
   }
-  const bool in = p < np;
-  const int icell = in ? s.icell[p] : 0;
-  int q[3] = {1, 1, 1}, i1[3] = {0, 0, 0};
-  double x[3];
-  if (icell > 0) {
-    cell_coords(g, icell, i1);
-    for (int d = 0; d < 3; ++d) {
-      x[d] = s.xp[d * np + p];
-      const double c0 = axis_coord<P>(s, g, d, i1[d]);
-      const double r0 = (x[d] - c0) * g.iDCell;
-      q[d] = gimp_part(r0);
+  const int icell = p >= 0 ? s.icell[p] : 0;
+  int i1[3] = {0, 0, 0};
+  if (icell > 0) cell_coords(g, icell, i1);
+  if (warp < 3) {
+    const int d = warp;
+    int q = 1;
+    if (icell > 0) {
+      const int i = d == 0 ? i1[0] : (d == 1 ? i1[1] : i1[2]);
+      const double x = s.xp[d * np + p], r0 = (x - axis_coord<P>(s, g, d, i)) * g.iDCell;
+      q = gimp_part(r0);
       // offsets 0 and 1, and the one beyond on the particle's side
 #pragma unroll
       for (int e = 0; e < 3; ++e) {
-        const int o = e == 0 ? 1 : (e == 1 ? 2 : (q[d] == 0 ? 0 : 3));
-        const double rr = e == 0 ? r0 : (x[d] - axis_coord<P>(s, g, d, i1[d] + o - 1)) * g.iDCell;
+        const int o = e == 0 ? 1 : (e == 1 ? 2 : (q == 0 ? 0 : 3));
+        const double rr = e == 0 ? r0 : (x - axis_coord<P>(s, g, d, i + o - 1)) * g.iDCell;
         double sh, dn;
         gimp_1d_f64(rr, sh, dn);
-        wt[(d * 4 + o) * nt + t] = sh;
-        wt[(12 + d * 4 + o) * nt + t] = dn;
+        wt[d * 4 + o][lane] = sh;
+        wt[12 + d * 4 + o][lane] = dn;
       }
     }
+    part[d][lane] = (signed char)q;
   }
-  if (!LISTED) {
-    list_particle<P>(s, np, p, in, gimp_list(q));
-    if (!in) return;
-  }
+  __syncthreads();
+  const int q[3] = {part[0][lane], part[1][lane], part[2][lane]};
+  if (!LISTED && warp == 0) list_particle<P>(s, np, p, p >= 0, gimp_list(q));
+  if (p < 0) return;
   int n = 0;
   if (icell > 0) {
     const unsigned char* gc = tab + (q[2] * 9 + q[1] * 3 + q[0]) * sizeof(GimpCase);
@@ -318,7 +325,7 @@ __global__ void __launch_bounds__(kGimpBlock) k_gimp_slots(St<P> s, Geometry g, 
     const int n1 = i1[2] * g.NGxy + i1[1] * g.NGx + i1[0];
     const int cbase = with_comp ? s.bodies[s.body[p]].comp * g.nn : 0;
     const double idc = g.iDCell;
-    for (int k = 0; k < n; ++k) {
+    for (int k = warp; k < n; k += kGimpWarps) {
       const int off = gc[1 + k];
       const int o0 = off & 3, o1 = (off >> 2) & 3, o2 = off >> 4;                    // offset + 1
       const int nd = n1 + (o0 - 1) + (o1 - 1) * g.NGx + (o2 - 1) * g.NGxy;           // flat arithmetic
@@ -331,11 +338,11 @@ __global__ void __launch_bounds__(kGimpBlock) k_gimp_slots(St<P> s, Geometry g, 
         const int o[3] = {o0, o1, o2};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          sh[d] = wt[(d * 4 + o[d]) * nt + t];
-          dn[d] = wt[(12 + d * 4 + o[d]) * nt + t];
+          sh[d] = wt[d * 4 + o[d]][lane];
+          dn[d] = wt[12 + d * 4 + o[d]][lane];
         }
       } else {
-        for (int d = 0; d < 3; ++d) gimp_1d_f64((x[d] - node_coord(g, nd, d)) * g.iDCell, sh[d], dn[d]);
+        for (int d = 0; d < 3; ++d) gimp_1d_f64((s.xp[d * np + p] - node_coord(g, nd, d)) * g.iDCell, sh[d], dn[d]);
       }
       const double xy = sh[0] * sh[1];
       s.shp[k * np + p] = xy * sh[2];
@@ -344,7 +351,7 @@ __global__ void __launch_bounds__(kGimpBlock) k_gimp_slots(St<P> s, Geometry g, 
       s.dndz[k * np + p] = xy * dn[2] * idc;
     }
   }
-  for (int k = n; k < g.K; ++k) s.snode[k * np + p] = -1;
+  for (int k = n + warp; k < g.K; k += kGimpWarps) s.snode[k * np + p] = -1;
 }
 
 // ----------------------------------------------------------------- locate
@@ -964,24 +971,20 @@ __device__ __forceinline__ void constitution(PState<typename P::R>& ps, const Ma
 // other models' registers out (the general kernel's 164 leave one 256-thread
 // block per SM), and without UV the gather drops the gradient's six sums
 // beyond the strain rate's (the diagonal ones are the same).
+constexpr int kAxesBlock = 96;
 constexpr bool stress_has(int mt) { return mt == 1 || mt == 7 || mt == 9 || mt == 10 || mt == 11; }
 
-template <class P, int MT, int UV>
-__global__ void __launch_bounds__(kBlock, MT == 0 ? 1 : 2) k_stress(St<P> s, Geometry g) {
+// Velocity gradient sums of particle p over its K slots: strain rate, spin and
+// (UV) the gradient. False outside the grid.
+template <class P, int UV>
+__device__ __forceinline__ bool gather_gradient(const St<P>& s, const Geometry& g, long long p, int K,
+                                                typename P::R (&de)[6], typename P::R (&vort)[3],
+                                                typename P::R (&deFp)[3][3]) {
   using R = typename P::R;
-  using B = typename P::B;
-  int K;
-  const long long p = take_particle<P>(s, g, gtid(), K);
-  if (p < 0) return;
   const long long np = g.np;
   const long long nn = g.nnt;  // node arrays of every grid component
-  if (g.has_jc) {
-    s.setter[p] = -1;
-    s.deferred[p] = 0;
-  }
-  R de[6] = {0, 0, 0, 0, 0, 0}, vort[3] = {0, 0, 0}, deFp[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   if (g.shape == 3) {
-    if (s.centericell[p] < 0) return;
+    if (s.centericell[p] < 0) return false;
     const long long nc = g.ncell;
     for (int k = 0; k < 8; ++k) {
       int c = s.snode[k * np + p];
@@ -993,7 +996,7 @@ __global__ void __launch_bounds__(kBlock, MT == 0 ? 1 : 2) k_stress(St<P> s, Geo
         for (int j = 0; j < 3; ++j) deFp[i][j] = deFp[i][j] + sk * (R)s.cdefp[(i * 3 + j) * nc + c];
     }
   } else {
-    if (s.icell[p] < 0) return;
+    if (s.icell[p] < 0) return false;
     constexpr int U = 3;  // slots whose gathers are in flight together
     for (int k0 = 0; k0 < K; k0 += U) {
       int n[U];
@@ -1038,11 +1041,123 @@ __global__ void __launch_bounds__(kBlock, MT == 0 ? 1 : 2) k_stress(St<P> s, Geo
     }
     for (int i = 0; i < 3; ++i) deFp[i][i] = de[i];
   }
+  return true;
+}
+
+// The sums of one axis e (0..2): de[e], de[3 + e], vort[e] and (UV) the
+// gradient's two components across it.
+template <class P, int UV>
+__device__ __forceinline__ void gather_axis(const St<P>& s, const Geometry& g, long long p, int K, int e,
+                                            typename P::R (&acc)[5]) {
+  using R = typename P::R;
+  const long long np = g.np;
+  const long long nn = g.nnt;
+  const int a = e == 2 ? 0 : e + 1, b = e == 0 ? 2 : e - 1;  // the axes after e
+  if (g.shape == 3) {
+    const long long nc = g.ncell;
+    for (int k = 0; k < 8; ++k) {
+      int c = s.snode[k * np + p];
+      if (c < 0) continue;
+      R sk = s.shp[k * np + p];
+      acc[0] = acc[0] + (R)s.co[e * nc + c] * sk;
+      acc[1] = acc[1] + (R)s.co[(3 + e) * nc + c] * sk;
+      acc[2] = acc[2] + (R)s.cw[e * nc + c] * sk;
+      if (UV) {
+        acc[3] = acc[3] + sk * (R)s.cdefp[(b * 3 + a) * nc + c];
+        acc[4] = acc[4] + sk * (R)s.cdefp[(a * 3 + b) * nc + c];
+      }
+    }
+  } else {
+    const double *ve = s.vg + e * nn, *va = s.vg + a * nn, *vb = s.vg + b * nn;
+    const R *de = e == 0 ? s.dndx : (e == 1 ? s.dndy : s.dndz), *da = a == 0 ? s.dndx : (a == 1 ? s.dndy : s.dndz),
+            *db = b == 0 ? s.dndx : (b == 1 ? s.dndy : s.dndz);
+    constexpr int U = 3;  // slots whose gathers are in flight together
+    for (int k0 = 0; k0 < K; k0 += U) {
+      int n[U];
+      double m[U], v[U][3], dn[U][3];
+#pragma unroll
+      for (int u = 0; u < U; ++u) n[u] = k0 + u < K ? s.snode[(k0 + u) * np + p] : -1;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        m[u] = 0.0;
+        if (n[u] < 0) continue;
+        const long long idx = (k0 + u) * np + p;
+        m[u] = s.mg[n[u]];
+        v[u][0] = ve[n[u]];
+        v[u][1] = va[n[u]];
+        v[u][2] = vb[n[u]];
+        dn[u][0] = de[idx];
+        dn[u][1] = da[idx];
+        dn[u][2] = db[idx];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (n[u] < 0 || !(m[u] > g.cutoff)) continue;
+        const double ab = dn[u][1] * v[u][2], ba = dn[u][2] * v[u][1];
+        acc[0] = acc[0] + dn[u][0] * v[u][0];
+        acc[1] = acc[1] + (ab + ba);
+        acc[2] = acc[2] + (ab - ba);
+        if (UV) {
+          acc[3] = acc[3] + ab;
+          acc[4] = acc[4] + ba;
+        }
+      }
+    }
+  }
+}
+
+// AXES: a block takes 32 particles with a warp per axis for the gather, and one
+// of the warps goes on alone. The gather is half of the work and a thread's
+// FP64 instructions are in series on a pipe that gives a warp one in 64 cycles,
+// so a scene with fewer warps of particles than the chip has schedulers (608)
+// is done sooner: Cook 5.8 k particles 48 -> 38 us, Taylor bar 17 k 44 both
+// ways; beyond, the blocks' waves cost more than that (dam break 31 k 61 -> 74).
+template <class P, int MT, int UV, bool AXES>
+__global__ void __launch_bounds__(AXES ? kAxesBlock : kBlock, AXES || MT == 0 ? 1 : 2) k_stress(St<P> s, Geometry g) {
+  using R = typename P::R;
+  using B = typename P::B;
+  int K;
+  const int lane = threadIdx.x & 31;
+  const long long p = take_particle<P>(s, g, AXES ? (long long)blockIdx.x * 32 + lane : gtid(), K);
+  const long long np = g.np;
+  if (!AXES && p < 0) return;
+  const int e = threadIdx.x >> 5;
+  const bool own = !AXES || e == (int)(blockIdx.x % 3);  // the thread updates the stress
+  if (p >= 0 && g.has_jc && own) {
+    s.setter[p] = -1;
+    s.deferred[p] = 0;
+  }
+  R de[6] = {0, 0, 0, 0, 0, 0}, vort[3] = {0, 0, 0}, deFp[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+  if constexpr (AXES) {
+    constexpr int NS = UV ? 5 : 3;
+    __shared__ double sums[3][NS][32];
+    const bool in = p >= 0 && (g.shape == 3 ? s.centericell[p] : s.icell[p]) >= 0;
+    R acc[5] = {0, 0, 0, 0, 0};
+    if (in) gather_axis<P, UV>(s, g, p, K, e, acc);
+#pragma unroll
+    for (int q = 0; q < NS; ++q) sums[e][q][lane] = acc[q];
+    __syncthreads();
+    if (!own || !in) return;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      de[i] = sums[i][0][lane];
+      de[3 + i] = sums[i][1][lane];
+      vort[i] = sums[i][2][lane];
+      if (UV) {
+        const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+        deFp[i2][i1] = sums[i][3][lane];
+        deFp[i1][i2] = sums[i][4][lane];
+      }
+      deFp[i][i] = de[i];
+    }
+  } else {
+    if (!gather_gradient<P, UV>(s, g, p, K, de, vort, deFp)) return;
+  }
   const DevScalars& sc = *s.sc;
   const R DT = (R)sc.dt;
   for (int i = 0; i < 6; ++i) de[i] = de[i] * DT;
   for (int i = 0; i < 3; ++i) vort[i] = vort[i] * DT / (R)2.0;
-  for (int i = 0; i < 3; ++i)
+  for (int i = 0; UV && i < 3; ++i)
     for (int j = 0; j < 3; ++j) deFp[i][j] = deFp[i][j] * DT;
   R Fpn[3][3];
   if (UV) {
@@ -1374,16 +1489,22 @@ __global__ void k_contact_sum(St<P> s, Geometry g) {
 
 // ------------------------------------------------------ position update
 // ParticlePositionUpdate (update_step.f90:1378-1526), non-SGMP and SGMP.
+// Thread = particle and axis (blockIdx.y): the axes are independent, and one
+// thread's FP64 instructions are in series on a pipe that gives a warp one in
+// 64 cycles, so a small scene wants three times the warps. GB300: Cook 5.8 k
+// particles 40 -> 24 us, dam break 31 k 60 -> 52, Taylor bar 17 k 17.5 -> 15.5,
+// slope 159 k 147 -> 146.
 template <class P>
 __global__ void k_position(St<P> s, Geometry g) {
   using R = typename P::R;
   int K;
   const long long p = take_particle<P>(s, g, gtid(), K);
   if (p < 0) return;
+  const int d = blockIdx.y;
   const long long np = g.np;
   const long long nn = g.nnt;  // node arrays of every grid component
   const DevScalars& sc = *s.sc;
-  double vx[3] = {0, 0, 0}, ax[3] = {0, 0, 0};
+  double vx = 0.0, ax = 0.0;
   if (g.shape == 3) {
     if (s.centericell[p] < 0) return;
     const long long nc = g.ncell;
@@ -1394,12 +1515,12 @@ __global__ void k_position(St<P> s, Geometry g) {
       for (int k = 0; k < 8; ++k) w[k] = s.shp[k * np + p];
     } else {  // AuxiliaryGridSHP, Grid.f90:193-220
       R xinb[3];
-      for (int d = 0; d < 3; ++d) {
-        R xnd = (R)s.xn[d * np + p];
-        if ((bd >> (2 * d)) & 3)
-          xinb[d] = xnd < (R)0 ? (R)1 + (R)2 * xnd : (R)2 * xnd - (R)1;
+      for (int e = 0; e < 3; ++e) {
+        R xnd = (R)s.xn[e * np + p];
+        if ((bd >> (2 * e)) & 3)
+          xinb[e] = xnd < (R)0 ? (R)1 + (R)2 * xnd : (R)2 * xnd - (R)1;
         else
-          xinb[d] = (R)s.xxn[d * np + p];
+          xinb[e] = (R)s.xxn[e * np + p];
       }
       for (int k = 0; k < 8; ++k) {
         R sx = (R)kSN[0][k] * xinb[0] + (R)1.0;
@@ -1408,22 +1529,22 @@ __global__ void k_position(St<P> s, Geometry g) {
         w[k] = sx * sy * sz * (R)0.125;
       }
     }
+    const double *cv = s.cvx + d * nc, *ca = s.cax + d * nc;
     for (int k = 0; k < 8; ++k) {
       int c = s.snode[k * np + p];
       if (c < 0) continue;
       double sk = (double)w[k];
-      for (int d = 0; d < 3; ++d) {
-        vx[d] = vx[d] + sk * s.cvx[d * nc + c];
-        ax[d] = ax[d] + sk * s.cax[d * nc + c];
-      }
+      vx = vx + sk * cv[c];
+      ax = ax + sk * ca[c];
     }
   } else {
     if (s.icell[p] < 0) return;
+    const double *vg = s.vg + d * nn, *fx = s.fx + d * nn;
     // (the gathers of a few slots in flight before the first one's sums)
     constexpr int U = 3;
     for (int k0 = 0; k0 < K; k0 += U) {
       int n[U];
-      double m[U], sk[U], v[U][3], f[U][3];
+      double m[U], sk[U], v[U], f[U];
       Recip y[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) n[u] = k0 + u < K ? s.snode[(k0 + u) * np + p] : -1;
@@ -1434,33 +1555,27 @@ __global__ void k_position(St<P> s, Geometry g) {
         m[u] = s.mg[n[u]];
         sk[u] = s.shp[(k0 + u) * np + p];
         y[u] = Recip{s.rm[n[u]], s.rm[nn + n[u]]};
-        for (int d = 0; d < 3; ++d) {
-          v[u][d] = s.vg[(long long)d * nn + n[u]];
-          f[u][d] = s.fx[(long long)d * nn + n[u]];
-        }
+        v[u] = vg[n[u]];
+        f[u] = fx[n[u]];
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (n[u] < 0 || !(m[u] > g.cutoff)) continue;
-        for (int d = 0; d < 3; ++d) {
-          vx[d] = vx[d] + sk[u] * v[u][d];
-          ax[d] = ax[d] + div_known(sk[u] * f[u][d], m[u], y[u]);
-        }
+        vx = vx + sk[u] * v[u];
+        ax = ax + div_known(sk[u] * f[u], m[u], y[u]);
       }
     }
   }
   const double dt = sc.dt;
-  for (int d = 0; d < 3; ++d) {
-    double xx = s.xp[d * np + p] + vx[d] * dt;
-    s.xx[d * np + p] = xx;
-    double v = s.vxp[d * np + p];
-    if (sc.istep == 1)
-      v = v + ax[d] * dt * 0.5;
-    else
-      v = v + ax[d] * dt;
-    s.vxp[d * np + p] = v;
-    if (g.usf) s.xp[d * np + p] = xx;
-  }
+  const double xx = s.xp[d * np + p] + vx * dt;
+  s.xx[d * np + p] = xx;
+  double v = s.vxp[d * np + p];
+  if (sc.istep == 1)
+    v = v + ax * dt * 0.5;
+  else
+    v = v + ax * dt;
+  s.vxp[d * np + p] = v;
+  if (g.usf) s.xp[d * np + p] = xx;
 }
 
 // ------------------------------------------------------ MUSL momentum

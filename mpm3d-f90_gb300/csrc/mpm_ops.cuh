@@ -32,10 +32,7 @@ struct Ops {
   }
   template <bool LISTED>
   static void gimp_slots(void* st, const Geometry& g, int with_comp, cudaStream_t s) {
-    const Shape h(g.np);
-    const unsigned block = h.block < kGimpBlock ? h.block : kGimpBlock;
-    k_gimp_slots<P, LISTED><<<(unsigned)((g.np + block - 1) / block), block, 24 * sizeof(double) * block, s>>>(
-        S(st), g, with_comp);
+    k_gimp_slots<P, LISTED><<<(unsigned)((g.np + 31) / 32), 32 * kGimpWarps, 0, s>>>(S(st), g, with_comp);
   }
   static void locate(void* st, const Geometry& g, cudaStream_t s) {
     const Shape h(g.np);
@@ -72,17 +69,24 @@ struct Ops {
     k_apply_bc<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
     prof_end(K_BC, s);
   }
-  // the stress update's instantiation for the deck's one material type
+  // the stress update's instantiation for the deck's one material type; scenes
+  // with fewer than a warp of particles per scheduler share a particle's gather
+  // among three warps (k_stress; registers do not matter there)
+  static constexpr long long kAxesMost = 304 * 32;
   template <int UV>
   static void stress_of(void* st, const Geometry& g, cudaStream_t s) {
     const Shape h(g.np);
+    if (g.np <= kAxesMost) {
+      k_stress<P, 0, UV, true><<<(unsigned)((g.np + 31) / 32), kAxesBlock, 0, s>>>(S(st), g);
+      return;
+    }
     switch (stress_has(S(st).mat_type) ? S(st).mat_type : 0) {
-      case 1: k_stress<P, 1, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 7: k_stress<P, 7, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 9: k_stress<P, 9, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 10: k_stress<P, 10, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 11: k_stress<P, 11, UV><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      default: k_stress<P, 0, UV><<<h.grid, h.block, 0, s>>>(S(st), g);
+      case 1: k_stress<P, 1, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 7: k_stress<P, 7, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 9: k_stress<P, 9, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 10: k_stress<P, 10, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 11: k_stress<P, 11, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      default: k_stress<P, 0, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g);
     }
   }
   static void stress(void* st, const Geometry& g, cudaStream_t s) {
@@ -122,7 +126,8 @@ struct Ops {
   static void position(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_POSITION, s);
     if (g.shape == 3) k_sg_cell_velocity<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
-    k_position<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
+    const Shape h(g.np);
+    k_position<P><<<dim3(h.grid, 3), h.block, 0, s>>>(S(st), g);
     prof_end(K_POSITION, s);
   }
   static void p2g_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {

@@ -106,7 +106,7 @@ __constant__ const unsigned char kCorner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0
 // count and, per slot, the node offset from the cell's first corner packed as
 // (dx+1) + 4(dy+1) + 16(dz+1). Slot order is that of FindInflNode
 // (Grid.f90:602-849); the same table drives every particle pass.
-struct GimpCase {
+struct alignas(4) GimpCase {  // (copied as words)
   unsigned char n;
   unsigned char off[27];
 };
