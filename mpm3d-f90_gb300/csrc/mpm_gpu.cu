@@ -284,18 +284,24 @@ int upload_as(mpm_ctx* c, void* dst, const double* src, long long n, size_t elem
 template <class Src>
 void scan_tiles(const Src& src, typename Src::T* tiles, cudaStream_t st) {
   const unsigned nt = (unsigned)bm::scan_tiles(src.n);
-  bm::ks_tile_total<Src><<<nt, bm::kScanThreads, 0, st>>>(src, tiles);
+  launch_chained(bm::ks_tile_total<Src>, nt, bm::kScanThreads, st, src, tiles);
   if (nt <= bm::kFusedTiles) {
-    bm::ks_tile_scan<Src, true><<<nt, bm::kScanThreads, 0, st>>>(src, tiles);
+    launch_chained(bm::ks_tile_scan<Src, true>, nt, bm::kScanThreads, st, src, tiles);
   } else {
-    bm::ks_tile_prefix<typename Src::T, typename Src::Op><<<1, bm::kScanThreads, 0, st>>>(tiles, nt);
-    bm::ks_tile_scan<Src, false><<<nt, bm::kScanThreads, 0, st>>>(src, tiles);
+    launch_chained(bm::ks_tile_prefix<typename Src::T, typename Src::Op>, 1, bm::kScanThreads, st, tiles, nt);
+    launch_chained(bm::ks_tile_scan<Src, false>, nt, bm::kScanThreads, st, src, tiles);
   }
 }
 
 // the per-node counts, and behind them the lengths of the slot lists: zeroed
 // together before the particles are located
 size_t seg_words(const mpm_ctx* c) { return (size_t)c->nkeys + 4; }
+
+// (by a kernel: a memset would break the chain of launches)
+cudaError_t zero_counts(mpm_ctx* c) {
+  const long long n = (long long)seg_words(c);
+  return launch_chained(k_zero_words, (unsigned)std::min<long long>((n + 255) / 256, 608), 256, c->stream, c->st.seg, n);
+}
 
 // the node-sorted pair list from the slots' nodes and the per-node counts
 int sort_pairs(mpm_ctx* c) {
@@ -305,12 +311,13 @@ int sort_pairs(mpm_ctx* c) {
   prof_begin(K_SORT, st);
   scan_tiles(PairScan{s.seg, s.fill, s.wcnt, c->nkeys}, s.tiles, st);
   const dim3 rows((unsigned)((np + 255) / 256), (unsigned)c->g.K + 1);
-  k_pair_place<<<rows, 256, 0, st>>>(s.snode, s.seg, s.fill, s.val_sorted, np, c->g.K, c->nkeys, s.wcnt, s.nbig);
-  k_pair_order<<<(unsigned)(((long long)c->nkeys * 32 + 127) / 128), 128, 0, st>>>(s.seg, c->nkeys, s.val_sorted, s.big,
-                                                                                 s.nbig);
+  launch_chained(k_pair_place, rows, 256, st, s.snode, s.seg, s.fill, s.val_sorted, np, c->g.K, (long long)c->nkeys,
+                 s.wcnt, s.nbig);
+  launch_chained(k_pair_order, (unsigned)(((long long)c->nkeys * 32 + 127) / 128), 128, st, s.seg, (long long)c->nkeys,
+                 s.val_sorted, s.big, s.nbig);
   const unsigned tiles = (unsigned)((c->nkeys + bm::kSortThreads - 1) / bm::kSortThreads);
-  k_pair_long<<<std::min(std::max(tiles, 76u), 608u), bm::kSortThreads, 0, st>>>(s.seg, s.val_sorted, s.big, s.nbig,
-                                                                                c->nkeys, s.wcnt, s.walk);
+  launch_chained(k_pair_long, std::min(std::max(tiles, 76u), 608u), bm::kSortThreads, st, s.seg, s.val_sorted, s.big,
+                 s.nbig, (long long)c->nkeys, s.wcnt, s.walk);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "pair sort");
   prof_end(K_SORT, st);
@@ -328,7 +335,7 @@ int depeff_pass(mpm_ctx* c) {
 }
 
 int build_pairs(mpm_ctx* c) {
-  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), c->stream);
+  cudaError_t e = zero_counts(c);
   if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
   c->ops->locate(&c->st, c->g, c->stream);
   return sort_pairs(c);
@@ -337,7 +344,7 @@ int build_pairs(mpm_ctx* c) {
 // SmoothStressbyGrid: shapes and pairs of the step's cells, then the maps
 int smooth_pass(mpm_ctx* c) {
   if (!c->st.spre) return set_err(c, MPM_ERR_ARG, "stress smoothing is off for this deck (no 'smoo')");
-  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), c->stream);
+  cudaError_t e = zero_counts(c);
   if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
   c->ops->fixed_locate(&c->st, c->g, 0, c->stream);
   int r = sort_pairs(c);
@@ -359,7 +366,7 @@ int enqueue_step_tl(mpm_ctx* c) {
   cudaStream_t s = c->stream;
   int r;
   o->begin_step(st, g, s);
-  cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), s);
+  cudaError_t e = zero_counts(c);
   if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
   o->fixed_locate(st, g, 1, s);
   if ((r = sort_pairs(c))) return r;
@@ -610,6 +617,7 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
     for (int a = 0; a < 3; ++a)
       for (int i = -1; i < (a == 0 ? g.NGx : (a == 1 ? g.NGy : g.NGz)) + 3; ++i) axis.push_back((double)i * g.dcell + g.span0[a]);
     CKF(cudaMemcpyAsync(s.axis, axis.data(), sizeof(double) * axis.size(), cudaMemcpyHostToDevice, c->stream));
+    s.wave = wave_speed(c->mats);
     s.rdcell[0] = s.rdcell[1] = 0.0;
     if (std::fabs(std::ilogb(g.dcell)) <= 400) {
       s.rdcell[0] = 1.0 / g.dcell;
@@ -676,7 +684,7 @@ int mpm_create(const mpm_deck* d, int precision, int device, mpm_ctx** out) {
       CKF(cudaMemsetAsync(s.pk, 0, sizeof(double) * 9 * np, c->stream));
       CKF(cudaMemcpyAsync(s.vol0, s.vol, sizeof(double) * np, cudaMemcpyDeviceToDevice, c->stream));
       c->ops->tl_initial(&c->st, g, c->stream);
-      CKF(cudaMemsetAsync(s.seg, 0, sizeof(int) * seg_words(c), c->stream));
+      CKF(zero_counts(c));
       c->ops->fixed_locate(&c->st, g, 1, c->stream);
       if ((r = sort_pairs(c))) goto fail;
       c->ops->p2g_mass(&c->st, g, 0, 0, c->stream);
@@ -714,7 +722,7 @@ int mpm_step_phase(mpm_ctx* c, int phase) {
     case MPM_PHASE_BEGIN_STEP: o->begin_step(st, g, s); break;
     case MPM_PHASE_GRID_MOMENTUM_INITIAL:
       if (g.tlmpm) {  // TLGridMomentumInitial: momentum with the cells of the initial positions
-        cudaError_t e = cudaMemsetAsync(c->st.seg, 0, sizeof(int) * seg_words(c), s);
+        cudaError_t e = zero_counts(c);
         if (e != cudaSuccess) return cuda_err(c, e, "memset seg");
         o->fixed_locate(st, g, 1, s);
         if ((r = sort_pairs(c))) return r;

@@ -148,6 +148,7 @@ struct DevState {
   int *slot_list, *slot_cnt;
   double* axis;      // node coordinates of the three axes (axis_coord)
   double rdcell[2];  // reciprocal of the cell size as a two-part sum
+  double wave;       // largest wave speed of the materials (UpdateDT), < 0: none counts
   // pairs
   unsigned* val_sorted;  // node-sorted pairs (mpm_pairs.cuh)
   int *seg, *fill, *tiles, *big, *nbig;  // segment ends, places taken, scan tile totals, long segments
@@ -225,16 +226,16 @@ extern const StepOps kOpsNative;   // MPM_FP64_NATIVE
 // the kernel, waits until the predecessor's grid has completed with its writes
 // visible (a no-op in a kernel launched plainly), so order is as without it and
 // only launch latency overlaps: 0.4 us per kernel, 79 -> 74.5 us per step of a
-// 5.8 k-particle scene. No kernel signals its successor earlier: blocks brought
+// 5.8 k-particle scene in the mixed form, 178 -> 162 in FP64. No kernel signals its successor earlier: blocks brought
 // up beside a predecessor that still runs are spread over the SMs it has
 // left, unevenly, and the 94 k-particle beam went from 112 to 131 us per step.
 __device__ __forceinline__ void chain_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args) {
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, unsigned block, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.stream = st;
   cudaLaunchAttribute at[1];

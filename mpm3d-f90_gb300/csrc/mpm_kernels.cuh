@@ -14,6 +14,7 @@
 #pragma once
 
 #include "mpm_physics.cuh"
+#include "mpm_reduce.cuh"
 
 namespace mpm {
 
@@ -25,6 +26,7 @@ __device__ __forceinline__ long long gtid() { return (long long)blockIdx.x * blo
 // ------------------------------------------------------------------ begin
 // MPM3D.f90:72-74
 static __global__ void k_begin_step(DevScalars* sc) {
+  chain_entry();
   sc->istep = sc->istep + 1;
   sc->time = sc->time + sc->dt;
   sc->ie = 0.0;
@@ -277,6 +279,7 @@ __device__ __forceinline__ int gimp_list(const int q[3]) { return (q[0] == 1) + 
 constexpr int kGimpWarps = 4;
 template <class P, bool LISTED>
 __global__ void __launch_bounds__(32 * kGimpWarps) k_gimp_slots(St<P> s, Geometry g, int with_comp) {
+  chain_entry();
   __shared__ double wt[24][32];  // weights (axis, offset), then derivatives
   __shared__ signed char part[3][32];
   __shared__ __align__(4) unsigned char tab[27 * sizeof(GimpCase)];
@@ -360,6 +363,7 @@ __global__ void __launch_bounds__(32 * kGimpWarps) k_gimp_slots(St<P> s, Geometr
 // FindInflNode+NShape_GIMP: k_gimp_slots, in the order listed here)
 template <class P, int SH>
 __global__ void k_locate(St<P> s, Geometry g) {
+  chain_entry();
   using B = typename P::B;
   const long long p = gtid();
   const long long np = g.np;
@@ -595,6 +599,7 @@ __device__ __forceinline__ void pair_walk(const int* walk, const int* seg, const
 // GridMomentumInitial (update_step.f90:288-406), non-SGMP.
 template <class P>
 __global__ void k_p2g_mass(St<P> s, Geometry g, int bc, int vel) {
+  chain_entry();
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
   pair_walk<kWalkFew, 5, 4, 4, 0>(
       s.walk, s.seg, s.val_sorted, np, nn,
@@ -624,6 +629,7 @@ __global__ void k_p2g_mass(St<P> s, Geometry g, int bc, int vel) {
 
 template <class P>
 __global__ void k_node_velocity(St<P> s, Geometry g) {
+  chain_entry();
   const long long n = gtid();
   if (n >= g.nnt) return;
   node_vel(s.mg, s.rm, s.px, s.vg, n, g.nnt, g.cutoff);
@@ -631,6 +637,7 @@ __global__ void k_node_velocity(St<P> s, Geometry g) {
 
 template <class P>
 __global__ void k_apply_bc(St<P> s, Geometry g) {
+  chain_entry();
   const long long n = gtid();
   if (n >= g.nnt) return;
   node_bc(s.fix[n % g.nn], s.px, s.fx, n, g.nnt);
@@ -1114,6 +1121,7 @@ __device__ __forceinline__ void gather_axis(const St<P>& s, const Geometry& g, l
 // ways; beyond, the blocks' waves cost more than that (dam break 31 k 61 -> 74).
 template <class P, int MT, int UV, bool AXES>
 __global__ void __launch_bounds__(AXES ? kAxesBlock : kBlock, AXES || MT == 0 ? 1 : 2) k_stress(St<P> s, Geometry g) {
+  chain_entry();
   using R = typename P::R;
   using B = typename P::B;
   int K;
@@ -1229,6 +1237,7 @@ __global__ void __launch_bounds__(AXES ? kAxesBlock : kBlock, AXES || MT == 0 ? 
 // previous stress update.
 template <class P>
 __global__ void k_depeff_apply(St<P> s, Geometry g) {
+  chain_entry();
   using R = typename P::R;
   using B = typename P::B;
   const long long p = gtid();
@@ -1284,6 +1293,7 @@ __global__ void k_depeff_apply(St<P> s, Geometry g) {
 
 template <class P>
 __global__ void k_depeff_carry(St<P> s, Geometry g) {
+  chain_entry();
   int last = s.setter_scan[g.np - 1];
   if (last >= 0) s.sc->depeff_carry = s.dep[last];
 }
@@ -1293,6 +1303,7 @@ __global__ void k_depeff_carry(St<P> s, Geometry g) {
 // stresses SM - q + SDii, prepared once per particle for the force transfer.
 template <class P>
 __global__ void k_force_prep(St<P> s, Geometry g) {
+  chain_entry();
   using R = typename P::R;
   const long long p = gtid();
   if (p >= g.np) return;
@@ -1339,6 +1350,7 @@ __device__ __forceinline__ void node_integrate(St<P>& s, const Geometry& g, long
 // (update_step.f90:977-982)
 template <class P, bool CONTACT>
 __global__ void k_p2g_force(St<P> s, Geometry g, int integ) {
+  chain_entry();
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
   pair_walk<kWalkMany, CONTACT ? 15 : 14, CONTACT ? 9 : 6, CONTACT ? 6 : 3, 3>(
       s.walk, s.seg, s.val_sorted, np, nn,
@@ -1382,6 +1394,7 @@ __global__ void k_p2g_force(St<P> s, Geometry g, int integ) {
 
 template <class P>
 __global__ void k_integrate(St<P> s, Geometry g) {
+  chain_entry();
   const long long n = gtid();
   if (n >= g.nnt) return;
   const long long nn = g.nnt;
@@ -1403,6 +1416,7 @@ __global__ void k_integrate(St<P> s, Geometry g) {
 // is kept for the total.
 template <class P>
 __global__ void k_contact(St<P> s, Geometry g) {
+  chain_entry();
   const long long n = gtid();
   const long long nn = g.nn, nt = g.nnt;
   if (n >= nn) return;
@@ -1470,6 +1484,7 @@ __global__ void k_contact(St<P> s, Geometry g) {
 // the total contact force (tot_cont_for): one block, fixed summation tree
 template <class P>
 __global__ void k_contact_sum(St<P> s, Geometry g) {
+  chain_entry();
   __shared__ double part[3][kBlock];
   const int t = threadIdx.x;
   const long long nn = g.nn;
@@ -1496,6 +1511,7 @@ __global__ void k_contact_sum(St<P> s, Geometry g) {
 // slope 159 k 147 -> 146.
 template <class P>
 __global__ void k_position(St<P> s, Geometry g) {
+  chain_entry();
   using R = typename P::R;
   int K;
   const long long p = take_particle<P>(s, g, gtid(), K);
@@ -1582,6 +1598,7 @@ __global__ void k_position(St<P> s, Geometry g) {
 // GridMomentumMUSL (update_step.f90:1668-1793), non-SGMP.
 template <class P>
 __global__ void k_p2g_momentum(St<P> s, Geometry g, int vel) {
+  chain_entry();
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
   pair_walk<kWalkFew, 5, 3, 3, 0>(
       s.walk, s.seg, s.val_sorted, np, nn,
@@ -1631,6 +1648,7 @@ __device__ __forceinline__ void for_adjacent_cells(const Geometry& g, long long 
 // GridMomentumInitial, SGMP branch: particles -> cells
 template <class P>
 __global__ void k_sg_cell_mass(St<P> s, Geometry g) {
+  chain_entry();
   const long long np = g.np, nc = g.ncell;
   pair_walk<kWalkFew, 5, 4, 4, 0>(
       s.walk, s.seg, s.val_sorted, np, nc,
@@ -1653,6 +1671,7 @@ __global__ void k_sg_cell_mass(St<P> s, Geometry g) {
 // ... cells -> nodes (mass and momentum, only cells above the cut-off)
 template <class P>
 __global__ void k_sg_node_mass(St<P> s, Geometry g, int bc, int vel) {
+  chain_entry();
   const long long n = gtid();
   const int nn = g.nn;
   bool act = false;
@@ -1683,6 +1702,7 @@ __global__ void k_sg_node_mass(St<P> s, Geometry g, int bc, int vel) {
 // the 8 nodes of each cell (CNShape derivatives at the cell centre)
 template <class P>
 __global__ void k_sg_cell_gradient(St<P> s, Geometry g) {
+  chain_entry();
   const long long c = gtid();
   const int nc = g.ncell;
   if (c >= nc) return;
@@ -1720,6 +1740,7 @@ __global__ void k_sg_cell_gradient(St<P> s, Geometry g) {
 // GridMomentumUpdate, SGMP branch: particles -> cells
 template <class P>
 __global__ void k_sg_cell_force(St<P> s, Geometry g) {
+  chain_entry();
   const long long np = g.np, nc = g.ncell;
   pair_walk<kWalkMany, 11, 9, 9, 0>(
       s.walk, s.seg, s.val_sorted, np, nc,
@@ -1744,6 +1765,7 @@ __global__ void k_sg_cell_force(St<P> s, Geometry g) {
 // ... cells -> nodes (every cell, no cut-off), then optionally integrate
 template <class P>
 __global__ void k_sg_node_force(St<P> s, Geometry g, int integ) {
+  chain_entry();
   const long long n = gtid();
   const int nn = g.nn;
   if (n >= nn) return;
@@ -1774,6 +1796,7 @@ __global__ void k_sg_node_force(St<P> s, Geometry g, int integ) {
 // cells on a fixed or symmetric face)
 template <class P>
 __global__ void k_sg_cell_velocity(St<P> s, Geometry g) {
+  chain_entry();
   const long long c = gtid();
   const int nc = g.ncell;
   if (c >= nc) return;
@@ -1830,6 +1853,7 @@ __global__ void k_sg_cell_velocity(St<P> s, Geometry g) {
 // GridMomentumMUSL, SGMP branch
 template <class P>
 __global__ void k_sg_cell_momentum(St<P> s, Geometry g) {
+  chain_entry();
   const long long np = g.np, nc = g.ncell;
   pair_walk<kWalkFew, 5, 3, 3, 0>(
       s.walk, s.seg, s.val_sorted, np, nc,
@@ -1850,6 +1874,7 @@ __global__ void k_sg_cell_momentum(St<P> s, Geometry g) {
 
 template <class P>
 __global__ void k_sg_node_momentum(St<P> s, Geometry g, int vel) {
+  chain_entry();
   const long long n = gtid();
   const int nn = g.nn;
   if (n >= nn) return;
@@ -1881,6 +1906,7 @@ __global__ void k_sg_node_momentum(St<P> s, Geometry g, int vel) {
 // XN is not set there for non-SGMP shapes and keeps its initial value 0
 template <class P>
 __global__ void k_tl_initial(St<P> s, Geometry g) {
+  chain_entry();
   using B = typename P::B;
   const long long p = gtid();
   if (p >= g.np) return;
@@ -1911,6 +1937,7 @@ __global__ void k_tl_initial(St<P> s, Geometry g) {
 // above the cut-off mass (the mass stays that of GridMassInitial)
 template <class P>
 __global__ void k_tl_sg_node_momentum(St<P> s, Geometry g, int vel) {
+  chain_entry();
   const long long n = gtid();
   const int nn = g.nn;
   if (n >= nn) return;
@@ -1935,6 +1962,7 @@ __global__ void k_tl_sg_node_momentum(St<P> s, Geometry g, int vel) {
 // the TL update never loads (0 in a TL run).
 template <class P>
 __global__ void k_tl_stress(St<P> s, Geometry g) {
+  chain_entry();
   using R = typename P::R;
   using B = typename P::B;
   const long long p = gtid();
@@ -2046,6 +2074,7 @@ __global__ void k_tl_stress(St<P> s, Geometry g) {
 // PK stress on the initial volume, then optionally IntegrateMomentum
 template <class P>
 __global__ void k_tl_p2g_force(St<P> s, Geometry g, int integ) {
+  chain_entry();
   using R = typename P::R;
   const long long n = gtid();
   const long long nn = g.nnt;
@@ -2090,6 +2119,7 @@ __global__ void k_tl_p2g_force(St<P> s, Geometry g, int integ) {
 // ... SGMP: particles -> cells (external force, PK * VOL0)
 template <class P>
 __global__ void k_tl_sg_cell_force(St<P> s, Geometry g) {
+  chain_entry();
   const long long c = gtid();
   const int nc = g.ncell;
   if (c >= nc) return;
@@ -2110,6 +2140,7 @@ __global__ void k_tl_sg_cell_force(St<P> s, Geometry g) {
 // ... cells -> nodes (every cell), then optionally integrate
 template <class P>
 __global__ void k_tl_sg_node_force(St<P> s, Geometry g, int integ) {
+  chain_entry();
   const long long n = gtid();
   const int nn = g.nn;
   if (n >= nn) return;
@@ -2151,6 +2182,7 @@ __global__ void k_tl_sg_node_force(St<P> s, Geometry g, int integ) {
 // XN, SGMP ones at XXN; with_comp: keys in the particle's grid component
 template <class P, int SH>
 __global__ void k_fixed_locate(St<P> s, Geometry g, int with_comp) {
+  chain_entry();
   const long long p = gtid();
   if (p >= g.np) return;
   const long long np = g.np;
@@ -2185,6 +2217,7 @@ __device__ __forceinline__ void smooth_sums(const St<P>& s, const Geometry& g, l
 // particles -> nodes, Gpre / GV_all on the mapped nodes (component 1)
 template <class P>
 __global__ void k_smooth_node(St<P> s, Geometry g) {
+  chain_entry();
   smooth_sums<P>(s, g, g.nnt, [&](long long n, bool in, const double* a) {
     if (!in || n >= g.nn) return;
     const bool mapped = s.seg[n] > (n == 0 ? 0 : s.seg[n - 1]);
@@ -2195,6 +2228,7 @@ __global__ void k_smooth_node(St<P> s, Geometry g) {
 // SGMP: particles -> centre nodes
 template <class P>
 __global__ void k_smooth_cell(St<P> s, Geometry g) {
+  chain_entry();
   smooth_sums<P>(s, g, g.ncell, [&](long long c, bool in, const double* a) {
     if (!in) return;
     s.cgpre[c] = a[0];
@@ -2206,6 +2240,7 @@ __global__ void k_smooth_cell(St<P> s, Geometry g) {
 // mapped, 0/0 where no volume reached it)
 template <class P>
 __global__ void k_smooth_sg_node(St<P> s, Geometry g) {
+  chain_entry();
   const long long n = gtid();
   if (n >= g.nn) return;
   double gp = 0.0, gv = 0.0;
@@ -2219,6 +2254,7 @@ __global__ void k_smooth_sg_node(St<P> s, Geometry g) {
 // SGMP: nodes above the cut-off mass -> centre nodes
 template <class P>
 __global__ void k_smooth_sg_back(St<P> s, Geometry g) {
+  chain_entry();
   const long long c = gtid();
   if (c >= g.ncell) return;
   const int n1 = cell_node1(g, (int)c + 1);
@@ -2233,6 +2269,7 @@ __global__ void k_smooth_sg_back(St<P> s, Geometry g) {
 // (centre) nodes -> particles: Spre
 template <class P>
 __global__ void k_smooth_g2p(St<P> s, Geometry g) {
+  chain_entry();
   const long long p = gtid();
   if (p >= g.np) return;
   const long long np = g.np;
@@ -2254,8 +2291,9 @@ __global__ void k_smooth_g2p(St<P> s, Geometry g) {
 
 // mode bit 0: update the energies and momentum; bit 1: derive the next DT
 template <class P>
-__global__ void k_reduce(St<P> s, Geometry g, int mode) {
-  __shared__ double sh[kRedVals][kBlock];
+__global__ void __launch_bounds__(kBlock) k_reduce(St<P> s, Geometry g, int mode) {
+  chain_entry();
+  __shared__ double sh[kRedVals][kBlock], tot[kRedVals];
   __shared__ bool last;
   const long long np = g.np;
   double acc[kRedVals] = {0, 0, 0, 0, 0, 0};
@@ -2274,17 +2312,10 @@ __global__ void k_reduce(St<P> s, Geometry g, int mode) {
     if (fabs(v2) > a) a = fabs(v2);
     if (acc[5] < a) acc[5] = a;
   }
-  for (int i = 0; i < kRedVals; ++i) sh[i][threadIdx.x] = acc[i];
+  reduce_block<kRedVals, kBlock>(sh, acc, tot);
+  if (threadIdx.x < kRedVals) s.red_part[(long long)threadIdx.x * gridDim.x + blockIdx.x] = tot[threadIdx.x];
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      for (int i = 0; i < 5; ++i) sh[i][threadIdx.x] = sh[i][threadIdx.x] + sh[i][threadIdx.x + w];
-      if (sh[5][threadIdx.x + w] > sh[5][threadIdx.x]) sh[5][threadIdx.x] = sh[5][threadIdx.x + w];
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kRedVals; ++i) s.red_part[(long long)i * gridDim.x + blockIdx.x] = sh[i][0];
     __threadfence();
     unsigned done = atomicAdd(s.red_count, 1u);
     last = (done == gridDim.x - 1);
@@ -2293,24 +2324,16 @@ __global__ void k_reduce(St<P> s, Geometry g, int mode) {
   if (!last) return;
   __threadfence();
   // the last block combines the block partials: thread t takes blocks t,
-  // t + blockDim, ... in order, then the same fixed tree as above
-  double tot[kRedVals] = {0, 0, 0, 0, 0, 0};
+  // t + blockDim, ... in order, then the same fixed order as above
+#pragma unroll
+  for (int i = 0; i < kRedVals; ++i) acc[i] = 0.0;
   for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-    for (int i = 0; i < 5; ++i) tot[i] = tot[i] + s.red_part[(long long)i * gridDim.x + b];
+    for (int i = 0; i < 5; ++i) acc[i] = acc[i] + s.red_part[(long long)i * gridDim.x + b];
     double mv = s.red_part[5LL * gridDim.x + b];
-    if (tot[5] < mv) tot[5] = mv;
+    if (acc[5] < mv) acc[5] = mv;
   }
-  for (int i = 0; i < kRedVals; ++i) sh[i][threadIdx.x] = tot[i];
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      for (int i = 0; i < 5; ++i) sh[i][threadIdx.x] = sh[i][threadIdx.x] + sh[i][threadIdx.x + w];
-      if (sh[5][threadIdx.x + w] > sh[5][threadIdx.x]) sh[5][threadIdx.x] = sh[5][threadIdx.x + w];
-    }
-    __syncthreads();
-  }
+  reduce_block<kRedVals, kBlock>(sh, acc, tot);
   if (threadIdx.x != 0) return;
-  for (int i = 0; i < kRedVals; ++i) tot[i] = sh[i][0];
   DevScalars* sc = s.sc;
   if (mode & 1) {
     sc->ke_prev = sc->ke;
@@ -2322,17 +2345,12 @@ __global__ void k_reduce(St<P> s, Geometry g, int mode) {
   }
   sc->max_vp = tot[5];
   *s.red_count = 0;
+  // UpdateDT: the least DCell / (wave speed + max_vp) over the materials is
+  // that of the largest wave speed
   if (mode & 2) {
     double dt = (double)1e6f;
-    for (int m = 0; m < g.nb_mat; ++m) {
-      const DevMaterial& mt = s.mats[m];
-      if (mt.mat_type == 12) continue;
-      double E = mt.young, nu = mt.poisson, ro = mt.density;
-      double vv = sqrt(E * (1 - nu) / (1 + nu) / (1 - 2 * nu) / ro);
-      if (mt.D > vv) vv = mt.D;
-      if (mt.wavespd > vv) vv = mt.wavespd;
-      vv = vv + tot[5];
-      double t = g.dcell / vv;
+    if (s.wave >= 0.0) {
+      const double t = g.dcell / (s.wave + tot[5]);
       if (t < dt) dt = t;
     }
     sc->dt = dt * g.dtscale;
@@ -2342,6 +2360,7 @@ __global__ void k_reduce(St<P> s, Geometry g, int mode) {
 // dynamicRelaxationDamping (Particle.f90:172-202)
 template <class P>
 __global__ void k_dr_damping(St<P> s, Geometry g) {
+  chain_entry();
   const long long p = gtid();
   const DevScalars* sc = s.sc;
   bool damp = sc->istep != 0 && (sc->ke - sc->ke_prev <= 0.0);
@@ -2353,6 +2372,7 @@ __global__ void k_dr_damping(St<P> s, Geometry g) {
 }
 
 static __global__ void k_dr_finish(DevScalars* sc) {
+  chain_entry();
   if (sc->istep != 0 && (sc->ke - sc->ke_prev <= 0.0)) sc->ke = 0;
 }
 

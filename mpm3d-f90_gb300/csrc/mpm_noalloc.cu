@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "mpm3d_gpu.h"
+#include "mpm_reduce.cuh"
 
 namespace {
 
@@ -40,7 +41,7 @@ void* g_scratch_ptr[kMaxDevices] = {};
 __global__ void k_energy_noalloc(const double* __restrict__ vxp, const double* __restrict__ mass,
                                  const double* __restrict__ ie, long long np, unsigned char* scratch,
                                  double* out) {
-  __shared__ double sh[kVals][kThreads];
+  __shared__ double sh[kVals][kThreads], tot[kVals];
   __shared__ bool last;
   double* part = reinterpret_cast<double*>(scratch);
   unsigned* count = reinterpret_cast<unsigned*>(scratch + kCounterOffset);
@@ -60,17 +61,10 @@ __global__ void k_energy_noalloc(const double* __restrict__ vxp, const double* _
     if (fabs(v2) > a) a = fabs(v2);
     if (acc[5] < a) acc[5] = a;
   }
-  for (int i = 0; i < kVals; ++i) sh[i][threadIdx.x] = acc[i];
+  mpm::reduce_block<kVals, kThreads>(sh, acc, tot);
+  if (threadIdx.x < kVals) part[(long long)threadIdx.x * gridDim.x + blockIdx.x] = tot[threadIdx.x];
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      for (int i = 0; i < 5; ++i) sh[i][threadIdx.x] = sh[i][threadIdx.x] + sh[i][threadIdx.x + w];
-      if (sh[5][threadIdx.x + w] > sh[5][threadIdx.x]) sh[5][threadIdx.x] = sh[5][threadIdx.x + w];
-    }
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kVals; ++i) part[(long long)i * gridDim.x + blockIdx.x] = sh[i][0];
     __threadfence();
     unsigned done = atomicAdd(count, 1u);
     last = (done == gridDim.x - 1);
@@ -78,24 +72,16 @@ __global__ void k_energy_noalloc(const double* __restrict__ vxp, const double* _
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double tot[kVals] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < kVals; ++i) acc[i] = 0.0;
   for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-    for (int i = 0; i < 5; ++i) tot[i] = tot[i] + part[(long long)i * gridDim.x + b];
+    for (int i = 0; i < 5; ++i) acc[i] = acc[i] + part[(long long)i * gridDim.x + b];
     double mv = part[5LL * gridDim.x + b];
-    if (tot[5] < mv) tot[5] = mv;
+    if (acc[5] < mv) acc[5] = mv;
   }
-  for (int i = 0; i < kVals; ++i) sh[i][threadIdx.x] = tot[i];
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      for (int i = 0; i < 5; ++i) sh[i][threadIdx.x] = sh[i][threadIdx.x] + sh[i][threadIdx.x + w];
-      if (sh[5][threadIdx.x + w] > sh[5][threadIdx.x]) sh[5][threadIdx.x] = sh[5][threadIdx.x + w];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  for (int i = 0; i < kVals; ++i) out[i] = sh[i][0];
-  *count = 0;
+  mpm::reduce_block<kVals, kThreads>(sh, acc, tot);
+  if (threadIdx.x < kVals) out[threadIdx.x] = tot[threadIdx.x];
+  if (threadIdx.x == 0) *count = 0;
 }
 
 // Device address of the scratch array for the current device, looked up once

@@ -27,24 +27,24 @@ struct Ops {
 
   static void begin_step(void* st, const Geometry&, cudaStream_t s) {
     prof_begin(K_BEGIN, s);
-    k_begin_step<<<1, 1, 0, s>>>(S(st).sc);
+    launch_chained(k_begin_step, 1, 1, s, S(st).sc);
     prof_end(K_BEGIN, s);
   }
   template <bool LISTED>
   static void gimp_slots(void* st, const Geometry& g, int with_comp, cudaStream_t s) {
-    k_gimp_slots<P, LISTED><<<(unsigned)((g.np + 31) / 32), 32 * kGimpWarps, 0, s>>>(S(st), g, with_comp);
+    launch_chained(k_gimp_slots<P, LISTED>, (unsigned)((g.np + 31) / 32), 32 * kGimpWarps, s, S(st), g, with_comp);
   }
   static void locate(void* st, const Geometry& g, cudaStream_t s) {
     const Shape h(g.np);
     prof_begin(K_LOCATE, s);
     switch (g.shape) {
-      case 0: k_locate<P, 0><<<h.grid, h.block, 0, s>>>(S(st), g); break;
+      case 0: launch_chained(k_locate<P, 0>, h.grid, h.block, s, S(st), g); break;
       case 1:
-        k_locate<P, 1><<<h.grid, h.block, 0, s>>>(S(st), g);
+        launch_chained(k_locate<P, 1>, h.grid, h.block, s, S(st), g);
         gimp_slots<true>(st, g, 1, s);
         break;
-      case 2: k_locate<P, 2><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      default: k_locate<P, 3><<<h.grid, h.block, 0, s>>>(S(st), g);
+      case 2: launch_chained(k_locate<P, 2>, h.grid, h.block, s, S(st), g); break;
+      default: launch_chained(k_locate<P, 3>, h.grid, h.block, s, S(st), g);
     }
     prof_end(K_LOCATE, s);
   }
@@ -52,21 +52,21 @@ struct Ops {
   static void p2g_mass(void* st, const Geometry& g, int bc, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      k_sg_cell_mass<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
-      k_sg_node_mass<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, bc, vel);
+      launch_chained(k_sg_cell_mass<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_chained(k_sg_node_mass<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, bc, vel);
     } else {
-      k_p2g_mass<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g, bc, vel);
+      launch_chained(k_p2g_mass<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g, bc, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
   static void node_velocity(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_NODE_VEL, s);
-    k_node_velocity<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
+    launch_chained(k_node_velocity<P>, Shape(g.nnt).grid, Shape(g.nnt).block, s, S(st), g);
     prof_end(K_NODE_VEL, s);
   }
   static void apply_bc(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_BC, s);
-    k_apply_bc<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
+    launch_chained(k_apply_bc<P>, Shape(g.nnt).grid, Shape(g.nnt).block, s, S(st), g);
     prof_end(K_BC, s);
   }
   // the stress update's instantiation for the deck's one material type; scenes
@@ -77,78 +77,78 @@ struct Ops {
   static void stress_of(void* st, const Geometry& g, cudaStream_t s) {
     const Shape h(g.np);
     if (g.np <= kAxesMost) {
-      k_stress<P, 0, UV, true><<<(unsigned)((g.np + 31) / 32), kAxesBlock, 0, s>>>(S(st), g);
+      launch_chained(k_stress<P, 0, UV, true>, (unsigned)((g.np + 31) / 32), kAxesBlock, s, S(st), g);
       return;
     }
     switch (stress_has(S(st).mat_type) ? S(st).mat_type : 0) {
-      case 1: k_stress<P, 1, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 7: k_stress<P, 7, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 9: k_stress<P, 9, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 10: k_stress<P, 10, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      case 11: k_stress<P, 11, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g); break;
-      default: k_stress<P, 0, UV, false><<<h.grid, h.block, 0, s>>>(S(st), g);
+      case 1: launch_chained(k_stress<P, 1, UV, false>, h.grid, h.block, s, S(st), g); break;
+      case 7: launch_chained(k_stress<P, 7, UV, false>, h.grid, h.block, s, S(st), g); break;
+      case 9: launch_chained(k_stress<P, 9, UV, false>, h.grid, h.block, s, S(st), g); break;
+      case 10: launch_chained(k_stress<P, 10, UV, false>, h.grid, h.block, s, S(st), g); break;
+      case 11: launch_chained(k_stress<P, 11, UV, false>, h.grid, h.block, s, S(st), g); break;
+      default: launch_chained(k_stress<P, 0, UV, false>, h.grid, h.block, s, S(st), g);
     }
   }
   static void stress(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_STRESS, s);
-    if (g.shape == 3) k_sg_cell_gradient<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+    if (g.shape == 3) launch_chained(k_sg_cell_gradient<P>, Shape(g.ncell).grid, Shape(g.ncell).block, s, S(st), g);
     if (g.uvfp) stress_of<1>(st, g, s);
     else stress_of<0>(st, g, s);
     prof_end(K_STRESS, s);
   }
   static void depeff_apply(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_DEPEFF, s);
-    k_depeff_apply<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
-    k_depeff_carry<P><<<1, 1, 0, s>>>(S(st), g);
+    launch_chained(k_depeff_apply<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
+    launch_chained(k_depeff_carry<P>, 1, 1, s, S(st), g);
     prof_end(K_DEPEFF, s);
   }
   static void force_prep(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_FORCE_PREP, s);
-    k_force_prep<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
+    launch_chained(k_force_prep<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
     prof_end(K_FORCE_PREP, s);
   }
   static void p2g_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
-      k_sg_cell_force<P><<<walk_grid(g.ncell), kWalkNodes * kWalkMany, 0, s>>>(S(st), g);
-      k_sg_node_force<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, integ);
+      launch_chained(k_sg_cell_force<P>, walk_grid(g.ncell), kWalkNodes * kWalkMany, s, S(st), g);
+      launch_chained(k_sg_node_force<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, integ);
     } else {
-      if (g.contact) k_p2g_force<P, true><<<walk_grid(g.nnt), kWalkNodes * kWalkMany, 0, s>>>(S(st), g, integ);
-      else k_p2g_force<P, false><<<walk_grid(g.nnt), kWalkNodes * kWalkMany, 0, s>>>(S(st), g, integ);
+      if (g.contact) launch_chained(k_p2g_force<P, true>, walk_grid(g.nnt), kWalkNodes * kWalkMany, s, S(st), g, integ);
+      else launch_chained(k_p2g_force<P, false>, walk_grid(g.nnt), kWalkNodes * kWalkMany, s, S(st), g, integ);
     }
     prof_end(K_P2G_FORCE, s);
   }
   static void integrate(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_INTEGRATE, s);
-    k_integrate<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g);
+    launch_chained(k_integrate<P>, Shape(g.nnt).grid, Shape(g.nnt).block, s, S(st), g);
     prof_end(K_INTEGRATE, s);
   }
   static void position(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_POSITION, s);
-    if (g.shape == 3) k_sg_cell_velocity<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+    if (g.shape == 3) launch_chained(k_sg_cell_velocity<P>, Shape(g.ncell).grid, Shape(g.ncell).block, s, S(st), g);
     const Shape h(g.np);
-    k_position<P><<<dim3(h.grid, 3), h.block, 0, s>>>(S(st), g);
+    launch_chained(k_position<P>, dim3(h.grid, 3), h.block, s, S(st), g);
     prof_end(K_POSITION, s);
   }
   static void p2g_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MOM, s);
     if (g.shape == 3) {
-      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
-      k_sg_node_momentum<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, vel);
+      launch_chained(k_sg_cell_momentum<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_chained(k_sg_node_momentum<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, vel);
     } else {
-      k_p2g_momentum<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g, vel);
+      launch_chained(k_p2g_momentum<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g, vel);
     }
     prof_end(K_P2G_MOM, s);
   }
   static void reduce(void* st, const Geometry& g, int mode, int nblocks, cudaStream_t s) {
     prof_begin(K_REDUCE, s);
-    k_reduce<P><<<nblocks, kBlock, 0, s>>>(S(st), g, mode);
+    launch_chained(k_reduce<P>, nblocks, kBlock, s, S(st), g, mode);
     prof_end(K_REDUCE, s);
   }
   static void dr_damping(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_DR, s);
-    k_dr_damping<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
-    k_dr_finish<<<1, 1, 0, s>>>(S(st).sc);
+    launch_chained(k_dr_damping<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
+    launch_chained(k_dr_finish, 1, 1, s, S(st).sc);
     prof_end(K_DR, s);
   }
 
@@ -156,59 +156,59 @@ struct Ops {
     prof_begin(K_LOCATE, s);
     const Shape h(g.np);
     switch (g.shape) {
-      case 0: k_fixed_locate<P, 0><<<h.grid, h.block, 0, s>>>(S(st), g, with_comp); break;
+      case 0: launch_chained(k_fixed_locate<P, 0>, h.grid, h.block, s, S(st), g, with_comp); break;
       case 1: gimp_slots<false>(st, g, with_comp, s); break;
-      case 2: k_fixed_locate<P, 2><<<h.grid, h.block, 0, s>>>(S(st), g, with_comp); break;
-      default: k_fixed_locate<P, 3><<<h.grid, h.block, 0, s>>>(S(st), g, with_comp);
+      case 2: launch_chained(k_fixed_locate<P, 2>, h.grid, h.block, s, S(st), g, with_comp); break;
+      default: launch_chained(k_fixed_locate<P, 3>, h.grid, h.block, s, S(st), g, with_comp);
     }
     prof_end(K_LOCATE, s);
   }
   static void tl_initial(void* st, const Geometry& g, cudaStream_t s) {
-    k_tl_initial<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
+    launch_chained(k_tl_initial<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
   }
   static void tl_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      k_sg_cell_momentum<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
-      k_tl_sg_node_momentum<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, vel);
+      launch_chained(k_sg_cell_momentum<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_chained(k_tl_sg_node_momentum<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, vel);
     } else {
-      k_p2g_momentum<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g, vel);
+      launch_chained(k_p2g_momentum<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
   static void tl_stress(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_STRESS, s);
-    if (g.shape == 3) k_sg_cell_gradient<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
-    k_tl_stress<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
+    if (g.shape == 3) launch_chained(k_sg_cell_gradient<P>, Shape(g.ncell).grid, Shape(g.ncell).block, s, S(st), g);
+    launch_chained(k_tl_stress<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
     prof_end(K_STRESS, s);
   }
   static void tl_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
-      k_tl_sg_cell_force<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
-      k_tl_sg_node_force<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g, integ);
+      launch_chained(k_tl_sg_cell_force<P>, Shape(g.ncell).grid, Shape(g.ncell).block, s, S(st), g);
+      launch_chained(k_tl_sg_node_force<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, integ);
     } else {
-      k_tl_p2g_force<P><<<Shape(g.nnt).grid, Shape(g.nnt).block, 0, s>>>(S(st), g, integ);
+      launch_chained(k_tl_p2g_force<P>, Shape(g.nnt).grid, Shape(g.nnt).block, s, S(st), g, integ);
     }
     prof_end(K_P2G_FORCE, s);
   }
   static void smooth(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_SMOOTH, s);
     if (g.shape == 3) {
-      k_smooth_cell<P><<<walk_grid(g.ncell), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
-      k_smooth_sg_node<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
-      k_smooth_sg_back<P><<<Shape(g.ncell).grid, Shape(g.ncell).block, 0, s>>>(S(st), g);
+      launch_chained(k_smooth_cell<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_chained(k_smooth_sg_node<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g);
+      launch_chained(k_smooth_sg_back<P>, Shape(g.ncell).grid, Shape(g.ncell).block, s, S(st), g);
     } else {
-      k_smooth_node<P><<<walk_grid(g.nnt), kWalkNodes * kWalkFew, 0, s>>>(S(st), g);
+      launch_chained(k_smooth_node<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g);
     }
-    k_smooth_g2p<P><<<Shape(g.np).grid, Shape(g.np).block, 0, s>>>(S(st), g);
+    launch_chained(k_smooth_g2p<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
     prof_end(K_SMOOTH, s);
   }
 
   static void contact(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_CONTACT, s);
-    k_contact<P><<<Shape(g.nn).grid, Shape(g.nn).block, 0, s>>>(S(st), g);
-    k_contact_sum<P><<<1, kBlock, 0, s>>>(S(st), g);
+    launch_chained(k_contact<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g);
+    launch_chained(k_contact_sum<P>, 1, kBlock, s, S(st), g);
     prof_end(K_CONTACT, s);
   }
 

@@ -20,6 +20,11 @@
 
 namespace mpm {
 
+__global__ void k_zero_words(int* w, long long n) {
+  chain_entry();
+  for (long long i = gtid(); i < n; i += (long long)gridDim.x * blockDim.x) w[i] = 0;
+}
+
 // The order the transfers take the nodes in (pair_walk): by classes of the
 // number of eights of pairs in a segment, longest first, empty segments
 // last, about the grid's order within a class. The order has no bearing on
@@ -55,6 +60,7 @@ constexpr int kWarpPairs = 256;  // longest segment a warp orders
 // count the nodes of each class.
 __global__ void __launch_bounds__(256) k_pair_place(const int* snode, const int* seg, int* fill, unsigned* val,
                                                     long long np, int K, long long nk, int* wcnt, int* nbig) {
+  chain_entry();
   const long long p = gtid();
   const int k = blockIdx.y, lane = threadIdx.x & 31;
   if (p == 0 && k == 0) *nbig = 0;
@@ -122,6 +128,7 @@ __device__ __forceinline__ void warp_order(unsigned* v, int n) {
 // each node's segment in ascending order, one warp per node; segments longer
 // than kWarpPairs are listed for k_pair_long
 __global__ void k_pair_order(const int* seg, long long nk, unsigned* val, int* big, int* nbig) {
+  chain_entry();
   const long long k = gtid() >> 5;
   if (k >= nk) return;
   const int a = k == 0 ? 0 : seg[k - 1], n = seg[k] - a;
@@ -137,6 +144,7 @@ __global__ void k_pair_order(const int* seg, long long nk, unsigned* val, int* b
 // the segments listed in big in ascending order, and the nodes into walk
 __global__ void __launch_bounds__(bm::kSortThreads) k_pair_long(const int* seg, unsigned* val, const int* big,
                                                                 const int* nbig, long long nk, int* wcnt, int* walk) {
+  chain_entry();
   __shared__ unsigned sm[bm::kSmemSeg];
   bm::sort_long(seg, val, big, nbig, sm);
 

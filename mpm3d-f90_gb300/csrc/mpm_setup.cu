@@ -216,8 +216,10 @@ double wave_speed(const std::vector<DevMaterial>& mats) {
   for (const auto& m : mats) {
     if (m.mat_type == 12) continue;
     const double E = m.young, nu = m.poisson, ro = m.density;
-    const double v = std::sqrt(E * (1 - nu) / (1 + nu) / (1 - 2 * nu) / ro);
-    c = std::fmax(c, std::fmax(std::fmax(v, m.D), m.wavespd));  // (a NaN does not count)
+    double v = std::sqrt(E * (1 - nu) / (1 + nu) / (1 - 2 * nu) / ro);
+    if (m.D > v) v = m.D;
+    if (m.wavespd > v) v = m.wavespd;
+    if (v > c) c = v;  // (a material whose speed is a NaN does not count)
   }
   return c;
 }
