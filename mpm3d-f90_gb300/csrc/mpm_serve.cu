@@ -312,9 +312,11 @@ void serve_loop(mpm_server* s) {
             r = mpm_batch_scene_download(s->batch, retire[i], f, buf.data());
             if (r == MPM_OK) t->fields[f].swap(buf);
           }
-        if (r == MPM_OK) r = mpm_batch_remove(s->batch, retire[i]);
         if (r == MPM_OK) done.push_back(t);
       }
+      // (removed together after the last read: a read after a removal would
+      // lay the batch out anew, 1 ms for each of eight scenes that end at once)
+      for (size_t i = 0; i < retire.size() && r == MPM_OK; ++i) r = mpm_batch_remove(s->batch, retire[i]);
     }
     {
       std::lock_guard<std::mutex> lk(s->mu);
