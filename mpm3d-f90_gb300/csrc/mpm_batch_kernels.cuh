@@ -581,6 +581,40 @@ __device__ __forceinline__ int dim_nodes(int shape, float off, int& t0, float w[
   return 2 + (off < 0.25f) + (off > 0.75f);
 }
 
+// The box of a particle's influence nodes for the gathers: index of its first
+// node, strides, and the nodes to visit -- within the particle's count and the
+// grid -- as a mask of three bits per axis, so that the unrolled loops over the
+// 27 nodes test a bit instead of comparing coordinates (stress update of the
+// 1.2 M particle slope 98 -> 85 us, dam break 2 M 153 -> 132; the position
+// update, bound by its loads, 91 -> 90 and 134 -> 129).
+struct NodeBox {
+  long long first;
+  int sy, sz;
+  unsigned m;
+  __device__ __forceinline__ bool x(int k) const { return m >> k & 1u; }
+  __device__ __forceinline__ bool row(int ay, int az) const {
+    const unsigned r = 8u << ay | 64u << az;
+    return (m & r) == r;
+  }
+};
+__device__ __forceinline__ NodeBox node_box(const Scene& sc, const int c[3], const int t0[3], const int nt[3]) {
+  NodeBox q;
+  const int n[3] = {sc.NGx, sc.NGy, sc.NGz};
+  int j[3];
+  q.m = 0u;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    j[a] = c[a] + t0[a];
+    // nodes j .. j + nt - 1 cut to 0 .. n - 1
+    const int lo = max(-j[a], 0), hi = min(nt[a], n[a] - j[a]);
+    q.m |= (((1u << max(hi, 0)) - 1u) & ~((1u << lo) - 1u)) << (3 * a);
+  }
+  q.sy = sc.NGx;
+  q.sz = sc.NGxy;
+  q.first = sc.n0 + ((long long)j[2] * sc.NGy + j[1]) * sc.NGx + j[0];
+  return q;
+}
+
 // The re-sort of the scenes marked by step_tick, in one cooperative launch:
 // counting sort by key (mpm_sort.cuh), then every field permuted into the
 // second particle set and back. A step in which no scene is re-sorted -- most
@@ -1389,21 +1423,18 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
     // sums times the y-z factors: 6 multiply-adds per node instead of the 24
     // of forming de, vort and deFp node by node
     float L[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    const NodeBox box = node_box(sc, c, t0, nt);
 #pragma unroll
     for (int az = 0; az < 3; ++az)
 #pragma unroll
       for (int ay = 0; ay < 3; ++ay) {
-        if (ay >= nt[1] || az >= nt[2]) continue;
-        const int jy = c[1] + t0[1] + ay, jz = c[2] + t0[2] + az;
-        if (jy < 0 || jy >= sc.NGy || jz < 0 || jz >= sc.NGz) continue;
-        const long long row = sc.n0 + ((long long)jz * sc.NGy + jy) * sc.NGx;
+        if (!box.row(ay, az)) continue;
+        const float4* row = b.nvel + box.first + (az * box.sz + ay * box.sy);
         float S[3] = {0, 0, 0}, D[3] = {0, 0, 0};
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
-          if (ax >= nt[0]) continue;
-          const int jx = c[0] + t0[0] + ax;
-          if (jx < 0 || jx >= sc.NGx) continue;
-          const float4 v4 = b.nvel[row + jx];  // zero below the cut-off mass
+          if (!box.x(ax)) continue;
+          const float4 v4 = row[ax];  // zero below the cut-off mass
           S[0] += wd[0][ax] * v4.x;
           S[1] += wd[0][ax] * v4.y;
           S[2] += wd[0][ax] * v4.z;
@@ -1897,23 +1928,21 @@ __device__ __forceinline__ float position_one(BState& b, long long i) {
     int t0[3], nt[3];
     float wd[3][3], dd[3][3];
     for (int a = 0; a < 3; ++a) nt[a] = dim_nodes(sc.shape, off[a], t0[a], wd[a], dd[a]);
-    // node rows along x: bounds and row index once per row, one multiply
-    // per node for its weight (the shape is a tensor product)
+    // node rows along x, one multiply per node for its weight (the shape is a
+    // tensor product)
+    const NodeBox box = node_box(sc, c, t0, nt);
 #pragma unroll
     for (int az = 0; az < 3; ++az)
 #pragma unroll
       for (int ay = 0; ay < 3; ++ay) {
-        if (ay >= nt[1] || az >= nt[2]) continue;
-        const int jy = c[1] + t0[1] + ay, jz = c[2] + t0[2] + az;
-        if (jy < 0 || jy >= sc.NGy || jz < 0 || jz >= sc.NGz) continue;
-        const long long row = sc.n0 + ((long long)jz * sc.NGy + jy) * sc.NGx;
+        if (!box.row(ay, az)) continue;
+        const int o = az * box.sz + ay * box.sy;
+        const float4 *rv = b.nvel + box.first + o, *ra = b.nacc + box.first + o;
         const float wyz = wd[1][ay] * wd[2][az];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
-          if (ax >= nt[0]) continue;
-          const int jx = c[0] + t0[0] + ax;
-          if (jx < 0 || jx >= sc.NGx) continue;
-          const float4 vn = b.nvel[row + jx], an = b.nacc[row + jx];  // zero below the cut-off mass
+          if (!box.x(ax)) continue;
+          const float4 vn = rv[ax], an = ra[ax];  // zero below the cut-off mass
           const float w = wd[0][ax] * wyz;
           v[0] += w * vn.x;
           v[1] += w * vn.y;
