@@ -778,8 +778,9 @@ int commit(mpm_batch* b) {
   shared.mg = al.get<double>(NN);
   shared.px = al.get<double>(3 * NN);
   shared.fx = al.get<double>(3 * NN);
-  shared.nvel = al.get<float4>(NN);
-  shared.nacc = al.get<float4>(NN);
+  shared.nvxy = al.get<float2>(NN);
+  shared.nz = al.get<float2>(NN);
+  shared.naxy = al.get<float2>(NN);
   shared.acc = al.get<unsigned long long>(4 * NN);
   shared.fix = al.get<uint8_t>(NN);
   shared.bd = al.get<uint8_t>(NN);
@@ -843,7 +844,7 @@ int commit(mpm_batch* b) {
     s.xn = shared.xn; s.fs = shared.fs; s.key = shared.key; s.m32 = shared.m32; s.v32 = shared.v32;
     s.perm = shared.perm; s.seg = shared.seg; s.inv = shared.inv;
     s.fill = shared.fill; s.tiles = shared.tiles; s.big = shared.big; s.nbig = shared.nbig; s.mg = shared.mg; s.px = shared.px; s.fx = shared.fx;
-    s.nvel = shared.nvel; s.nacc = shared.nacc; s.acc = shared.acc; s.fix = shared.fix; s.bd = shared.bd; s.node_scene = shared.node_scene;
+    s.nvxy = shared.nvxy; s.nz = shared.nz; s.naxy = shared.naxy; s.acc = shared.acc; s.fix = shared.fix; s.bd = shared.bd; s.node_scene = shared.node_scene;
     s.cacc = shared.cacc; s.cact = shared.cact; s.cgrad = shared.cgrad;
     s.cvel = shared.cvel; s.cacl = shared.cacl; s.cscene = shared.cscene;
     s.setter = shared.setter; s.setter_scan = shared.setter_scan; s.dep = shared.dep; s.jc_aux = shared.jc_aux;
@@ -968,8 +969,9 @@ int commit(mpm_batch* b) {
   BCK(cudaMemsetAsync(shared.mg, 0, sizeof(double) * NN, st));
   BCK(cudaMemsetAsync(shared.px, 0, sizeof(double) * 3 * NN, st));
   BCK(cudaMemsetAsync(shared.fx, 0, sizeof(double) * 3 * NN, st));
-  BCK(cudaMemsetAsync(shared.nvel, 0, sizeof(float4) * NN, st));
-  BCK(cudaMemsetAsync(shared.nacc, 0, sizeof(float4) * NN, st));
+  BCK(cudaMemsetAsync(shared.nvxy, 0, sizeof(float2) * NN, st));
+  BCK(cudaMemsetAsync(shared.nz, 0, sizeof(float2) * NN, st));
+  BCK(cudaMemsetAsync(shared.naxy, 0, sizeof(float2) * NN, st));
   BCK(cudaMemsetAsync(shared.acc, 0, sizeof(unsigned long long) * 4 * NN, st));
   if (NC) {
     BCK(cudaMemsetAsync(shared.cacc, 0, sizeof(unsigned long long) * CQ_N * NC, st));

@@ -118,7 +118,13 @@ struct BState {
   int* task0;  // first particle task (32 sorted particles) of each scene, nscene + 1 entries; SGMP scenes have none
   // grid
   double *mg, *px, *fx;
-  float4 *nvel, *nacc;             // FP32 px / mg and fx / mg for the gathers (zero at or below the cut-off)
+  // FP32 velocity px / mg and acceleration fx / mg for the gathers (zero at or
+  // below the cut-off): (vx, vy), (vz, az), (ax, ay). A warp's load takes the
+  // data path of its 32 lanes' width whatever the addresses share, which bounds
+  // the position update: two float4 per node, eight passes with the unused
+  // components, took 89 us on the 1.2 M particle slope, these six 75 (dam break
+  // 2 M 130 -> 116)
+  float2 *nvxy, *nz, *naxy;
   unsigned long long* acc;         // [NN][4] fixed-point P2G sums, zero between transfers
   uint8_t *fix, *bd;
   uint16_t* node_scene;

@@ -586,7 +586,7 @@ __device__ __forceinline__ int dim_nodes(int shape, float off, int& t0, float w[
 // grid -- as a mask of three bits per axis, so that the unrolled loops over the
 // 27 nodes test a bit instead of comparing coordinates (stress update of the
 // 1.2 M particle slope 98 -> 85 us, dam break 2 M 153 -> 132; the position
-// update, bound by its loads, 91 -> 90 and 134 -> 129).
+// update, bound by its loads then, 91 -> 90 and 134 -> 129).
 struct NodeBox {
   long long first;
   int sy, sz;
@@ -1170,7 +1170,8 @@ __device__ __forceinline__ void node_finish(BState& b, const Scene& sc, long lon
       v.y = (float)b.px[NN + n] / m32;
       v.z = (float)b.px[2 * NN + n] / m32;
     }
-    b.nvel[n] = v;
+    b.nvxy[n] = make_float2(v.x, v.y);
+    b.nz[n].x = v.z;
   }
 }
 
@@ -1314,8 +1315,7 @@ __global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target
           // the node goes idle: clear the rest of its fields once (the idle
           // test of the later transfers skips it from now on)
           for (int a = 0; a < 3; ++a) b.fx[a * NN + n] = 0.0;
-          b.nvel[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-          b.nacc[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+          b.nvxy[n] = b.nz[n] = b.naxy[n] = make_float2(0.f, 0.f);
           // a momentum without mass (the mass contributions quantised to
           // zero, the momentum ones not) keeps the node marked (take_acc)
           if (b.px[n] != 0.0 || b.px[NN + n] != 0.0 || b.px[2 * NN + n] != 0.0) b.mg[n] = -0.0;
@@ -1429,18 +1429,20 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
 #pragma unroll
       for (int ay = 0; ay < 3; ++ay) {
         if (!box.row(ay, az)) continue;
-        const float4* row = b.nvel + box.first + (az * box.sz + ay * box.sy);
+        const int o = az * box.sz + ay * box.sy;
+        const float2 *rv = b.nvxy + box.first + o, *rz = b.nz + box.first + o;
         float S[3] = {0, 0, 0}, D[3] = {0, 0, 0};
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
           if (!box.x(ax)) continue;
-          const float4 v4 = row[ax];  // zero below the cut-off mass
-          S[0] += wd[0][ax] * v4.x;
-          S[1] += wd[0][ax] * v4.y;
-          S[2] += wd[0][ax] * v4.z;
-          D[0] += dd[0][ax] * v4.x;
-          D[1] += dd[0][ax] * v4.y;
-          D[2] += dd[0][ax] * v4.z;
+          const float2 vn = rv[ax];  // zero below the cut-off mass
+          const float vz = rz[ax].x;
+          S[0] += wd[0][ax] * vn.x;
+          S[1] += wd[0][ax] * vn.y;
+          S[2] += wd[0][ax] * vz;
+          D[0] += dd[0][ax] * vn.x;
+          D[1] += dd[0][ax] * vn.y;
+          D[2] += dd[0][ax] * vz;
         }
         const float fx = wd[1][ay] * wd[2][az], fy = dd[1][ay] * wd[2][az], fz = wd[1][ay] * dd[2][az];
         for (int a = 0; a < 3; ++a) {
@@ -1549,11 +1551,13 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
   return force_stage(b, sc, st, i, ps.vol, ps.sm - ps.q, ps.sd);
 }
 
-// (Drucker-Prager runs best at 1536 threads per SM -- 40 registers, some
-// spilled -- faster than at 1024 threads without spills; the other
-// specialised models at 1024)
+// (Drucker-Prager and the null material run better at 1536 threads per SM -- 40
+// registers, some spilled -- than at 1024 with few or none: the 1.2 M particle
+// slope 85 us for 91, the 2 M dam break 124 for 136; the other specialised
+// models at 1024: elastic block 36 k 11.6 us for 12.4, neo-Hookean beam 94 k
+// 17.4 for 21.4)
 template <int MT, int UV>
-__global__ void __launch_bounds__(512, MT == 10 ? 3 : (MT ? 2 : 1))
+__global__ void __launch_bounds__(512, MT == 10 || MT == 9 ? 3 : (MT ? 2 : 1))
     kb_stress(BState b, int usf_pass, int filter, int uvf) {
   chain_entry();
   const long long i = btid();
@@ -1714,7 +1718,8 @@ __device__ __forceinline__ void node_integrate(BState& b, const Scene& sc, long 
     acc.y = (float)b.fx[NN + n] / m32;
     acc.z = (float)b.fx[2 * NN + n] / m32;
   }
-  b.nacc[n] = acc;
+  b.naxy[n] = make_float2(acc.x, acc.y);
+  b.nz[n].y = acc.z;
 }
 
 // (the SGMP form keeps two cells' nine loads in flight at 64 registers)
@@ -1796,7 +1801,8 @@ __global__ void kb_sg_centre_gradient(BState b, int usf_pass) {
   for (int k = 0; k < 8; ++k) {
     long long n = sc.n0 + ((long long)(q[2] + kCorner[k][2]) * sc.NGy + q[1] + kCorner[k][1]) * sc.NGx + q[0] +
                   kCorner[k][0];
-    const float4 v4 = b.nvel[n];  // zero below the cut-off mass
+    const float2 vxy = b.nvxy[n];  // zero below the cut-off mass
+    const float3 v4 = make_float3(vxy.x, vxy.y, b.nz[n].x);
     const float v[3] = {v4.x, v4.y, v4.z};
     const float dx = kSN[0][k] * j4, dy = kSN[1][k] * j4, dz = kSN[2][k] * j4;
     for (int a = 0; a < 3; ++a) {
@@ -1841,7 +1847,8 @@ __global__ void kb_sg_centre_velocity(BState b) {
     if (boundary)
       w = ((float)kSN[0][k] * (float)cxx[0] + 1.f) * ((float)kSN[1][k] * (float)cxx[1] + 1.f) *
           ((float)kSN[2][k] * (float)cxx[2] + 1.f) * 0.125f;
-    const float4 vn = b.nvel[n], an = b.nacc[n];  // zero below the cut-off mass
+    const float2 vxy = b.nvxy[n], axy = b.naxy[n], z = b.nz[n];  // zero below the cut-off mass
+    const float3 vn = make_float3(vxy.x, vxy.y, z.x), an = make_float3(axy.x, axy.y, z.y);
     v[0] += w * vn.x;
     v[1] += w * vn.y;
     v[2] += w * vn.z;
@@ -1937,19 +1944,19 @@ __device__ __forceinline__ float position_one(BState& b, long long i) {
       for (int ay = 0; ay < 3; ++ay) {
         if (!box.row(ay, az)) continue;
         const int o = az * box.sz + ay * box.sy;
-        const float4 *rv = b.nvel + box.first + o, *ra = b.nacc + box.first + o;
+        const float2 *rv = b.nvxy + box.first + o, *rz = b.nz + box.first + o, *ra = b.naxy + box.first + o;
         const float wyz = wd[1][ay] * wd[2][az];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
           if (!box.x(ax)) continue;
-          const float4 vn = rv[ax], an = ra[ax];  // zero below the cut-off mass
+          const float2 vn = rv[ax], z = rz[ax], an = ra[ax];  // zero below the cut-off mass
           const float w = wd[0][ax] * wyz;
           v[0] += w * vn.x;
           v[1] += w * vn.y;
-          v[2] += w * vn.z;
+          v[2] += w * z.x;
           acc[0] += w * an.x;
           acc[1] += w * an.y;
-          acc[2] += w * an.z;
+          acc[2] += w * z.y;
         }
       }
   }
