@@ -144,7 +144,6 @@ __global__ void kb_relocate(BState src, BState dst, const int* map, const uint16
   const long long NP = dst.NP, SP = src.NP;
   for (int a = 0; a < 3; ++a) {
     dst.x[a * NP + i] = src.x[a * SP + j];
-    dst.xx[a * NP + i] = src.xx[a * SP + j];
     dst.v[a * NP + i] = src.v[a * SP + j];
     dst.fxp[a * NP + i] = src.fxp[a * SP + j];
   }
@@ -259,7 +258,6 @@ struct Alloc {
 
 void alloc_particles(Alloc& al, BState& s, long long NP, bool uvfp) {
   s.x = al.get<double>(3 * NP);
-  s.xx = al.get<double>(3 * NP);
   s.v = al.get<double>(3 * NP);
   s.fxp = al.get<double>(3 * NP);
   s.mass = al.get<double>(NP);
@@ -284,7 +282,7 @@ void alloc_particles(Alloc& al, BState& s, long long NP, bool uvfp) {
 }
 
 long long scene_bytes(long long np, long long nn, long long ncell, bool sgmp, bool uvfp, bool jc) {
-  long long per_p = 2 * (16 * 8 + 17 * 4 + (uvfp ? 72 : 0) + 1 + 2 + 2 + 4);  // two particle buffer sets
+  long long per_p = 2 * (13 * 8 + 17 * 4 + (uvfp ? 72 : 0) + 1 + 2 + 2 + 4);  // two particle buffer sets
   per_p += 4 * 3 + 4 * 9 + 4 * 6 + 4 * 9 + 4 * 4;                          // derived + force staging + FP32 m, v
   per_p += 4 * 3;                                                         // sort key, permutation, inverse
   if (jc) per_p += 4 * 2 + 8 * 6 + 1;
@@ -329,7 +327,6 @@ int upload_scene_particles(mpm_batch* b, HostScene* h, BState& s) {
   const double *x = h->in_x(), *v = h->in_v(), *fxp = h->in_fxp();
   for (int a = 0; a < 3; ++a) {
     BCK(upd(s.x + a * NP + p0, x + a * np, np));
-    BCK(cudaMemcpyAsync(s.xx + a * NP + p0, s.x + a * NP + p0, sizeof(double) * np, cudaMemcpyDeviceToDevice, st));
     BCK(upd(s.v + a * NP + p0, v + a * np, np));
     BCK(upd(s.fxp + a * NP + p0, fxp + a * np, np));
   }
@@ -1448,9 +1445,6 @@ int mpm_batch_scene_restore(mpm_batch* b, int id, const unsigned char* in, size_
       BCK(cudaMemcpy(static_cast<char*>(f.p) + ((size_t)a * NP + p0) * f.elem, in + at, n, cudaMemcpyHostToDevice));
       at += n;
     }
-  // positions and their copy agree at the end of every step
-  for (int a = 0; a < 3; ++a)
-    BCK(cudaMemcpy(s.xx + a * NP + p0, s.x + a * NP + p0, sizeof(double) * np, cudaMemcpyDeviceToDevice));
   // (images of USF scenes written before the momentum bound was carried from
   // step to step have none)
   const bool bounds = st.qmax[Q_MOM_MUSL] == 0u;

@@ -6,7 +6,7 @@
 //   is re-sorted (stable sort, then a permutation of every field) on its first
 //   step and whenever its mass transfer meets too many particles out of order
 //   (step_tick) -- component-major over the total particle count NP:
-//     FP64: x[3], xx[3], v[3], fxp[3], mass, ie
+//     FP64: x[3], v[3], fxp[3], mass, ie (XX of the reference is x between steps)
 //     FP32: vol, evol (V / V0 - 1), sig_y, sm, seqv, sd[6], fp[9], epeff, celsius,
 //     dmg, lt, cp, q
 //     per step (written by the mass transfer): cell (scene-local cell, -1
@@ -93,7 +93,7 @@ struct BState {
   int nscene;
   int any_uvfp, any_sgmp, any_jc;
   // particles (A = the working set, B = the re-sort's permutation target)
-  double *x, *xx, *v, *fxp, *mass, *ie;
+  double *x, *v, *fxp, *mass, *ie;
   float *vol, *evol, *sig_y, *sm, *seqv, *sd, *fp, *epeff, *celsius, *dmg, *lt, *cp, *q;
   uint8_t* failure;
   uint16_t *body, *scene;

@@ -1552,8 +1552,6 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
   b.celsius[i] = ps.celsius;
   b.failure[i] = ps.failure ? 1 : 0;
   if (!isfinite(ps.sm) || !isfinite(ps.ie)) atomicOr(&b.sst[s].status, (unsigned)ST_NONFINITE);
-  if (!sc.usf)
-    for (int a = 0; a < 3; ++a) b.x[a * NP + i] = b.xx[a * NP + i];
   // GridMomentumUpdate follows a USF stress update directly: stage its
   // force input from the registers (the stress state is final unless a
   // Johnson-Cook tail still runs)
@@ -1977,13 +1975,13 @@ __device__ __forceinline__ float position_one(BState& b, long long i) {
   float pv[3];
   for (int a = 0; a < 3; ++a) {
     const double xx = x0[a] + f64_of(v[a]) * dt;
-    b.xx[a * NP + i] = xx;
+    // (XX and, at the end of the step, Xp: nothing in between reads positions)
+    b.x[a * NP + i] = xx;
     const double vv = v0[a];
     const double vn = st.istep == 1 ? vv + f64_of(acc[a]) * dt * 0.5 : vv + f64_of(acc[a]) * dt;
     b.v[a * NP + i] = vn;
     pv[a] = f32_rn(vn);
     b.v32[a * NP + i] = pv[a];  // for the momentum transfers of this step (MUSL) and the next
-    if (sc.usf) b.x[a * NP + i] = xx;
   }
   // bound of those transfers' contributions
   const float m = b.m32[i];
