@@ -204,6 +204,7 @@ struct mpm_batch {
   int pblock = 256, nblock = 256;
   int scatter_blocks = 9728;  // scatter grid cap (64 blocks per SM; warps stride over the occupied cells)
   int sort_blocks = 152;      // grid cap of the re-sort (co-resident blocks, at most three per SM)
+  int sort_polls = 0;         // polls of the re-sort's waits (0: by the particles, barrier_polls)
   int sms = 152;              // multiprocessors of the device
   int loop_min_steps = 0;     // steps a device loop takes before it honours an interrupt
   long long ntask = 0;        // particle tasks of the linear / GIMP / B-spline scenes (32 particles each)
@@ -366,7 +367,8 @@ int enqueue_resort(mpm_batch* b) {
   prof_begin(K_SORT, b->stream);
   const long long want = gridn(std::max(b->A.NP, b->A.NK), kSortThreads);
   const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(want, b->sort_blocks));
-  void* args[] = {&b->A, &b->B};
+  int polls = b->sort_polls ? b->sort_polls : barrier_polls(b->A.NP);
+  void* args[] = {&b->A, &b->B, &polls};
   BCK(cudaLaunchCooperativeKernel((const void*)kb_resort, dim3(grid), dim3(kSortThreads), args, 0, b->stream));
   prof_end(K_SORT, b->stream);
   return MPM_OK;
@@ -1533,6 +1535,11 @@ int mpm_batch_set_option(mpm_batch* b, int option, int value) {
       if (value < 0) return berr(b, MPM_ERR_ARG, "loop minimum steps %d < 0", value);
       b->loop_min_steps = value;
       return MPM_OK;
+    case MPM_BATCH_SORT_POLLS:
+      if (value < 0) return berr(b, MPM_ERR_ARG, "re-sort polls %d < 0", value);
+      if (b->sort_polls != value) drop_graph(b);
+      b->sort_polls = value;
+      return MPM_OK;
     default: return berr(b, MPM_ERR_ARG, "unknown batch option %d", option);
   }
 }
@@ -1544,6 +1551,7 @@ int mpm_batch_get_option(const mpm_batch* b, int option) {
     case MPM_BATCH_NODE_BLOCK: return b->nblock;
     case MPM_BATCH_SCATTER_BLOCKS: return b->scatter_blocks / b->sms;
     case MPM_BATCH_LOOP_MIN_STEPS: return b->loop_min_steps;
+    case MPM_BATCH_SORT_POLLS: return b->sort_polls;
     default: return -1;
   }
 }

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(bm::kSortThreads) k_pair_long(const int* seg, 
                                                                 const int* nbig, long long nk, int* wcnt, int* walk) {
   chain_entry();
   __shared__ unsigned sm[bm::kSmemSeg];
-  bm::sort_long(seg, val, big, nbig, sm);
+  bm::sort_long(seg, val, big, nbig, sm, [](int, unsigned* v, int n) { bm::block_bitonic(v, n); });
 
   constexpr int NW = bm::kSortThreads / 32;
   static_assert(kWalkClasses == 32, "a lane per class");

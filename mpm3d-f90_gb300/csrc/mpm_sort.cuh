@@ -178,11 +178,16 @@ struct IntScan {
 // ------------------------------------------------------------ grid barrier
 // Barrier over the blocks of one cooperative launch. bar[0] counts arrivals
 // (zero when the launch starts, never reset inside it), so round r is complete
-// at r * gridDim.x arrivals; bar[1] is set when a wait runs out, after which
-// every block leaves its launch at its next barrier. Returns false then.
-constexpr int kBarrierSpins = 1 << 22;  // about a second of polling
+// at r * gridDim.x arrivals; bar[1] is set when a wait runs out of polls, after
+// which every block leaves its launch at its next barrier. Returns false then.
+// The work between two barriers is linear in the particles and keys (the
+// longest segment included, order_segment), so the limit is too: a fixed part,
+// far above any phase of a small scene, and one poll (0.7 us) for every 64
+// particles, above 10 ns for each of them.
+constexpr int kBarrierPolls = 1 << 22;
+inline int barrier_polls(long long np) { return np / 64 < INT_MAX - kBarrierPolls ? kBarrierPolls + (int)(np / 64) : INT_MAX; }
 
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round) {
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round, int polls) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -191,7 +196,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round) {
     const unsigned want = round * gridDim.x;
     volatile unsigned* v = bar;
     int spins = 0;
-    while (v[0] < want && v[1] == 0u && ++spins < kBarrierSpins) __nanosleep(100);
+    while (v[0] < want && v[1] == 0u && ++spins < polls) __nanosleep(100);
     if (v[0] < want) atomicExch(&bar[1], 1u);
     ok = v[1] == 0u;
     __threadfence();
@@ -353,10 +358,11 @@ __device__ __forceinline__ void block_bitonic(T* d, int n) {
 }
 
 // the long segments: one block per segment (grid-stride over the list), in
-// shared memory (sm, kSmemSeg values) up to kSmemSeg values, in place in
-// global memory beyond
-template <class T>
-__device__ __forceinline__ void sort_long(const int* seg, T* perm, const int* big, const int* nbig, T* sm) {
+// shared memory (sm, kSmemSeg values) up to kSmemSeg values; beyond, by
+// longer(k, p, n)
+template <class T, class Longer>
+__device__ __forceinline__ void sort_long(const int* seg, T* perm, const int* big, const int* nbig, T* sm,
+                                          Longer longer) {
   const int nb = *nbig;
   for (int b = blockIdx.x; b < nb; b += gridDim.x) {
     const int k = big[b];
@@ -368,9 +374,72 @@ __device__ __forceinline__ void sort_long(const int* seg, T* perm, const int* bi
       block_bitonic(sm, n);
       for (int j = threadIdx.x; j < n; j += blockDim.x) p[j] = sm[j];
     } else {
-      block_bitonic(p, n);
+      longer(k, p, n);
     }
     __syncthreads();
+  }
+}
+
+// Ascending order of the n > kSmemSeg particles p of key k by one block: the
+// particles between the first and the last of them that have the key, in
+// order. A scene's particles outside its grid all share one key, so n reaches
+// the scene's size; a bitonic network in global memory over 1.0, 4.1 and 8.0 M
+// particles took 91, 443 and 951 ms, this the whole step 0.7, 2.3 and 4.4 ms
+// (27 M: over 5 s and 17 ms). Where the key's particles are strewn over more
+// than kScanRatio times their number (the order of a deck; a sorted scene has
+// them close together) the network is shorter.
+constexpr int kScanRatio = 64;
+
+__device__ __forceinline__ void order_segment(const unsigned* key, unsigned k, int* p, int n) {
+  constexpr int NW = kSortThreads / 32, Q = 16;
+  __shared__ int range[2], cnt[2][NW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 2) range[threadIdx.x] = p[0];
+  __syncthreads();
+  int lo = p[0], hi = p[0];
+  for (int j = threadIdx.x; j < n; j += kSortThreads) {
+    lo = min(lo, p[j]);
+    hi = max(hi, p[j]);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) {
+    atomicMin(&range[0], lo);
+    atomicMax(&range[1], hi);
+  }
+  __syncthreads();
+  lo = range[0];
+  hi = range[1];
+  if ((long long)hi - lo >= (long long)kScanRatio * n) {
+    block_bitonic(p, n);
+    return;
+  }
+  // tiles of Q rows of 32 particles per warp; the rows' votes give the places
+  int done = 0;
+  for (long long i0 = lo, t = 0; i0 <= hi; i0 += kSortThreads * Q, ++t) {
+    const long long w0 = i0 + warp * (32 * Q) + lane;
+    unsigned row[Q];
+    int mine = 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) row[q] = w0 + 32 * q <= hi ? key[w0 + 32 * q] : kNoKey;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      row[q] = __ballot_sync(0xffffffffu, row[q] == k);
+      mine += __popc(row[q]);
+    }
+    if (lane == 0) cnt[t & 1][warp] = mine;
+    __syncthreads();  // (one a tile: this half of cnt is written again after the next one)
+    int at = done;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (w < warp) at += cnt[t & 1][w];
+      done += cnt[t & 1][w];
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (row[q] >> lane & 1u) p[at + __popc(row[q] & ((1u << lane) - 1u))] = (int)(w0 + 32 * q);
+      at += __popc(row[q]);
+    }
   }
 }
 
