@@ -197,7 +197,11 @@ int64_t mpm_scene_device_bytes(const mpm_deck* deck);
 int64_t mpm_batch_device_bytes(const mpm_batch* b);
 int mpm_batch_scene_count(const mpm_batch* b);
 /* nsteps steps of every resident scene (a scene stops at its step count);
- * use_graph replays a CUDA graph captured once per batch composition. */
+ * use_graph replays a CUDA graph captured once per batch composition.
+ * Re-sorting the particles has blocks of a kernel wait for one another; should
+ * such a wait ever run out (MPM_BATCH_SORT_POLLS), the resident scenes' states
+ * are lost: every later call that steps or reads them, and mpm_batch_commit,
+ * returns MPM_ERR_TIMEOUT until all of them are removed. */
 int mpm_batch_run(mpm_batch* b, int nsteps, int use_graph);
 /* Device-resident run loop (no counterpart in the reference, whose time
  * loop is one scene on the host, MPM3D.f90:66-160): one launch of a CUDA

@@ -214,6 +214,10 @@ struct mpm_batch {
   LoopCtl* ctl = nullptr;
   volatile int* loop_flag_h = nullptr;
   int* loop_flag_d = nullptr;
+  // set by a re-sort whose wait ran out, which leaves the resident scenes'
+  // particles half moved (page-locked, mapped; beside the request flag)
+  volatile int* stall_h = nullptr;
+  int* stall_d = nullptr;
   cudaGraphExec_t loop_graph = nullptr;
   Profiler prof;
   // particle value gather (curve output)
@@ -368,7 +372,7 @@ int enqueue_resort(mpm_batch* b) {
   const long long want = gridn(std::max(b->A.NP, b->A.NK), kSortThreads);
   const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(want, b->sort_blocks));
   int polls = b->sort_polls ? b->sort_polls : barrier_polls(b->A.NP);
-  void* args[] = {&b->A, &b->B, &polls};
+  void* args[] = {&b->A, &b->B, &polls, &b->stall_d};
   BCK(cudaLaunchCooperativeKernel((const void*)kb_resort, dim3(grid), dim3(kSortThreads), args, 0, b->stream));
   prof_end(K_SORT, b->stream);
   return MPM_OK;
@@ -679,8 +683,27 @@ struct BProfScope {
   ~BProfScope() { prof_set_current(prev); }
 };
 
+// MPM_ERR_TIMEOUT once a re-sort has given up (up to date after a wait for the
+// stream): the states of the resident scenes are lost, and every call that
+// steps or reads them says so until all of them are removed
+int stalled(mpm_batch* b) {
+  return *b->stall_h ? berr(b, MPM_ERR_TIMEOUT, "a re-sort's wait ran out: the resident scenes' states are lost") : MPM_OK;
+}
+
+// the work enqueued so far done, and done to the end
+int settle(mpm_batch* b) {
+  BCK(cudaStreamSynchronize(b->stream));
+  return stalled(b);
+}
+
 int commit(mpm_batch* b) {
   cudaStream_t st = b->stream;
+  bool resident = false;
+  for (HostScene* h : b->order) resident = resident || h->resident;
+  BCK(cudaStreamSynchronize(st));
+  if (resident)
+    if (int r = stalled(b)) return r;
+  *b->stall_h = 0;
   if (b->order.empty()) {
     drop_graph(b);
     if (b->arena) cudaFree(b->arena);
@@ -1017,8 +1040,7 @@ int commit(mpm_batch* b) {
 }
 
 int ensure_committed(mpm_batch* b) {
-  if (b->dirty) return commit(b);
-  return MPM_OK;
+  return b->dirty ? commit(b) : stalled(b);
 }
 
 HostScene* find(mpm_batch* b, int id) {
@@ -1054,7 +1076,7 @@ int mpm_batch_create(int device, mpm_batch** out) {
       cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaMalloc((void**)&b->ctl, sizeof(LoopCtl)) != cudaSuccess ||
       cudaMemset(b->ctl, 0, sizeof(LoopCtl)) != cudaSuccess ||
-      cudaHostAlloc((void**)&b->loop_flag_h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
+      cudaHostAlloc((void**)&b->loop_flag_h, 2 * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
       cudaHostGetDevicePointer((void**)&b->loop_flag_d, (void*)b->loop_flag_h, 0) != cudaSuccess) {
     if (b->ctl) cudaFree(b->ctl);
     if (b->loop_flag_h) cudaFreeHost((void*)b->loop_flag_h);
@@ -1066,6 +1088,9 @@ int mpm_batch_create(int device, mpm_batch** out) {
     delete b;
     return MPM_ERR_CUDA;
   }
+  b->stall_h = b->loop_flag_h + 1;
+  b->stall_d = b->loop_flag_d + 1;
+  *b->stall_h = 0;
   *out = b;
   return MPM_OK;
 }
@@ -1134,7 +1159,6 @@ int mpm_batch_remove(mpm_batch* b, int id) {
 int mpm_batch_commit(mpm_batch* b) {
   if (!b) return MPM_ERR_ARG;
   cudaSetDevice(b->device);
-  BCK(cudaStreamSynchronize(b->stream));
   return commit(b);
 }
 
@@ -1202,7 +1226,7 @@ int mpm_batch_run_loop(mpm_batch* b, int max_steps, int* steps) {
   BCK(cudaStreamSynchronize(b->stream));
   *b->loop_flag_h = 0;  // an interrupt is consumed by the loop it ended (or the next one)
   *steps = 1 + 2 * c.iters;
-  return MPM_OK;
+  return stalled(b);
 }
 
 int mpm_batch_interrupt(mpm_batch* b) {
@@ -1213,12 +1237,10 @@ int mpm_batch_interrupt(mpm_batch* b) {
 
 int mpm_batch_sync(mpm_batch* b) {
   if (!b) return MPM_ERR_ARG;
-  BCK(cudaStreamSynchronize(b->stream));
+  if (int r = settle(b)) return r;
   if (b->A.nscene == 0) return MPM_OK;
   std::vector<SceneState> s((size_t)b->A.nscene);
   BCK(cudaMemcpy(s.data(), b->A.sst, sizeof(SceneState) * s.size(), cudaMemcpyDeviceToHost));
-  for (auto& x : s)
-    if (x.status & ST_STALLED) return berr(b, MPM_ERR_TIMEOUT, "a re-sort's grid barrier ran out of time");
   for (auto& x : s)
     if (x.status & ST_NONFINITE) return berr(b, MPM_ERR_NONFINITE, "non-finite particle state");
   return MPM_OK;
@@ -1242,7 +1264,7 @@ int mpm_batch_time_steps(mpm_batch* b, int nsteps, int use_graph, double* ms) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (b->prof.on) prof_harvest(&b->prof, b->stream);
-  return r;
+  return r ? r : stalled(b);
 }
 
 int mpm_batch_scene_scalars(mpm_batch* b, int id, double* o) {
@@ -1251,9 +1273,9 @@ int mpm_batch_scene_scalars(mpm_batch* b, int id, double* o) {
   if (!h) return berr(b, MPM_ERR_ARG, "no scene %d", id);
   memset(o, 0, sizeof(double) * MPM_NSCALARS);
   SceneState s = h->st;
-  if (h->resident && !b->dirty) {
-    BCK(cudaStreamSynchronize(b->stream));
-    BCK(cudaMemcpy(&s, b->A.sst + h->index, sizeof s, cudaMemcpyDeviceToHost));
+  if (h->resident) {
+    if (int r = settle(b)) return r;
+    if (!b->dirty) BCK(cudaMemcpy(&s, b->A.sst + h->index, sizeof s, cudaMemcpyDeviceToHost));
   }
   o[0] = s.istep; o[1] = s.time; o[2] = s.dt; o[3] = s.ke; o[4] = s.ie;
   o[5] = s.mom[0]; o[6] = s.mom[1]; o[7] = s.mom[2]; o[8] = s.ke_prev;
@@ -1313,7 +1335,7 @@ int mpm_batch_scene_download(mpm_batch* b, int id, int field, double* out) {
   if (r) return r;
   HostScene* h = find(b, id);
   if (!h) return berr(b, MPM_ERR_ARG, "no scene %d", id);
-  BCK(cudaStreamSynchronize(b->stream));
+  if ((r = settle(b))) return r;
   const BState& s = b->A;
   const long long NP = s.NP, np = h->np, p0 = h->p0;
   const int nc = mpm_field_components(field);
@@ -1405,7 +1427,7 @@ int mpm_batch_scene_snapshot(mpm_batch* b, int id, std::vector<unsigned char>& o
   if (r) return r;
   HostScene* h = find(b, id);
   if (!h) return berr(b, MPM_ERR_ARG, "no scene %d", id);
-  BCK(cudaStreamSynchronize(b->stream));
+  if ((r = settle(b))) return r;
   const BState& s = b->A;
   const long long NP = s.NP, np = h->np, p0 = h->p0;
   SceneState st;
@@ -1431,7 +1453,7 @@ int mpm_batch_scene_restore(mpm_batch* b, int id, const unsigned char* in, size_
   if (r) return r;
   HostScene* h = find(b, id);
   if (!h) return berr(b, MPM_ERR_ARG, "no scene %d", id);
-  BCK(cudaStreamSynchronize(b->stream));
+  if ((r = settle(b))) return r;
   const BState& s = b->A;
   const long long NP = s.NP, np = h->np, p0 = h->p0;
   const std::vector<RestartField> fields = restart_fields(s, h->su.g.uvfp != 0);
@@ -1505,6 +1527,7 @@ int mpm_batch_scene_gather_wait(mpm_batch* b, double* out) {
   if (!b || !out) return MPM_ERR_ARG;
   if (!b->g_done) return berr(b, MPM_ERR_STATE, "no gather in flight");
   BCK(cudaEventSynchronize(b->g_done));
+  if (int r = stalled(b)) return r;
   memcpy(out, b->g_out_h, sizeof(double) * (size_t)b->g_n);
   return MPM_OK;
 }
@@ -1672,11 +1695,10 @@ int batch_progress(mpm_batch* b, std::vector<BatchProgress>& out) {
   if (r) return r;
   if (b->order.empty()) return MPM_OK;
   std::vector<SceneState> s((size_t)b->A.nscene);
-  BCK(cudaStreamSynchronize(b->stream));
+  if ((r = settle(b))) return r;
   BCK(cudaMemcpy(s.data(), b->A.sst, sizeof(SceneState) * s.size(), cudaMemcpyDeviceToHost));
   for (HostScene* h : b->order) {
     const SceneState& t = s[h->index];
-    if (t.status & ST_STALLED) return berr(b, MPM_ERR_TIMEOUT, "a re-sort's grid barrier ran out of time");
     out.push_back(BatchProgress{h->id, t.istep, h->steps, h->np, t.status});
   }
   return MPM_OK;

@@ -632,7 +632,7 @@ __device__ __forceinline__ NodeBox node_box(const Scene& sc, const int c[3], con
 // 10 us for an IF node around the phases as kernels of their own and 16 to 34
 // us for those kernels returning one by one (5.8 k to 1.2 M particles). The
 // barriers between the phases cost a re-sort about what launches would.
-__global__ void __launch_bounds__(kSortThreads, 3) kb_resort(BState a, BState o, int polls) {
+__global__ void __launch_bounds__(kSortThreads, 3) kb_resort(BState a, BState o, int polls, int* stall) {
   chain_entry();
   if (!*a.any_resort) return;
   __shared__ int sm[kSmemSeg];  // (the scan's tile, then the long segments)
@@ -641,23 +641,23 @@ __global__ void __launch_bounds__(kSortThreads, 3) kb_resort(BState a, BState o,
   unsigned round = 0;
   for (long long k = g0; k < a.NK; k += gs) a.seg[k] = 0;
   if (g0 == 0) *a.nbig = 0;
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_keys(a);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_tile_totals(a.seg, a.NK, a.tiles, thr, wsum);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_tile_prefix(a.NK, a.tiles, thr, wsum);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_tile_scan(a.seg, a.fill, a.NK, a.tiles, sm, thr, wsum);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_place(a.key, a.seg, a.fill, a.perm, a.NP);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_segments(a.seg, a.NK, a.perm, a.big, a.nbig);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_long(a.seg, a.perm, a.big, a.nbig, sm, [&](int k, int* p, int n) { order_segment(a.key, (unsigned)k, p, n); });
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   for (long long i = g0; i < a.NP; i += gs) permute_one(a, o, i);
-  if (!grid_barrier(a.gbar, ++round, polls)) return;
+  if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   for (long long i = g0; i < a.NP; i += gs) permute_back(o, a, i);
 }
 
@@ -2079,7 +2079,6 @@ __device__ __forceinline__ void reduce_scene_finish(BState& b, int s, int mode, 
   reduce_block<6, 256>(sh, acc, tot);
   if (threadIdx.x != 0) return;
   SceneState& st = b.sst[s];
-  if (b.gbar[1]) st.status |= (unsigned)ST_STALLED;  // a re-sort gave up
   if (mode & 1) {
     st.ke_prev = st.ke;
     st.ke = tot[0];

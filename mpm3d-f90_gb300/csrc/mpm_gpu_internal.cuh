@@ -44,8 +44,7 @@ enum StatusBits : unsigned {
   ST_NONFINITE = 1u << 0,
   ST_OUT_OF_GRID = 1u << 1,
   ST_NEGATIVE_VOLUME = 1u << 2,
-  ST_BAD_EOS = 1u << 3,
-  ST_STALLED = 1u << 4  // a bounded wait inside a kernel ran out (batched engine's re-sort)
+  ST_BAD_EOS = 1u << 3
 };
 
 struct DevMaterial {

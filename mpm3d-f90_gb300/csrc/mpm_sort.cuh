@@ -179,7 +179,8 @@ struct IntScan {
 // Barrier over the blocks of one cooperative launch. bar[0] counts arrivals
 // (zero when the launch starts, never reset inside it), so round r is complete
 // at r * gridDim.x arrivals; bar[1] is set when a wait runs out of polls, after
-// which every block leaves its launch at its next barrier. Returns false then.
+// which every block leaves its launch at its next barrier. Returns false then,
+// and the host finds *stall (its own memory, mapped) set.
 // The work between two barriers is linear in the particles and keys (the
 // longest segment included, order_segment), so the limit is too: a fixed part,
 // far above any phase of a small scene, and one poll (0.7 us) for every 64
@@ -187,7 +188,7 @@ struct IntScan {
 constexpr int kBarrierPolls = 1 << 22;
 inline int barrier_polls(long long np) { return np / 64 < INT_MAX - kBarrierPolls ? kBarrierPolls + (int)(np / 64) : INT_MAX; }
 
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round, int polls) {
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round, int polls, volatile int* stall) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -197,7 +198,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned round, int 
     volatile unsigned* v = bar;
     int spins = 0;
     while (v[0] < want && v[1] == 0u && ++spins < polls) __nanosleep(100);
-    if (v[0] < want) atomicExch(&bar[1], 1u);
+    if (v[0] < want) {
+      atomicExch(&bar[1], 1u);
+      *stall = 1;
+    }
     ok = v[1] == 0u;
     __threadfence();
   }
