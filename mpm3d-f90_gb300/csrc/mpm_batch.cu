@@ -1462,18 +1462,21 @@ int mpm_batch_scene_restore(mpm_batch* b, int id, const unsigned char* in, size_
   if (bytes != need) return berr(b, MPM_ERR_STATE, "restart image of %zu bytes, the scene needs %zu", bytes, need);
   SceneState st;
   memcpy(&st, in, sizeof st);
+  // (on the batch's stream: a plain copy of pageable memory may return before
+  // it has arrived, and the kernel below would not wait for it)
   size_t at = sizeof st;
   for (const RestartField& f : fields)
     for (int a = 0; a < f.nc; ++a) {
       const size_t n = (size_t)np * f.elem;
-      BCK(cudaMemcpy(static_cast<char*>(f.p) + ((size_t)a * NP + p0) * f.elem, in + at, n, cudaMemcpyHostToDevice));
+      BCK(cudaMemcpyAsync(static_cast<char*>(f.p) + ((size_t)a * NP + p0) * f.elem, in + at, n, cudaMemcpyHostToDevice,
+                          b->stream));
       at += n;
     }
   // (images of USF scenes written before the momentum bound was carried from
   // step to step have none)
   const bool bounds = st.qmax[Q_MOM_MUSL] == 0u;
   if (bounds) st.active = 1;
-  BCK(cudaMemcpy(s.sst + h->index, &st, sizeof st, cudaMemcpyHostToDevice));
+  BCK(cudaMemcpyAsync(s.sst + h->index, &st, sizeof st, cudaMemcpyHostToDevice, b->stream));
   kb_init_f32<<<gridn(NP, 256), 256, 0, b->stream>>>(s, h->index, bounds ? 1 : 0);
   BCK(cudaGetLastError());
   BCK(cudaStreamSynchronize(b->stream));
