@@ -707,8 +707,9 @@ __device__ __forceinline__ long long sg_corner_cell(const Scene& sc, int dx, int
 //      and its (y, z) factors per channel;
 //   2. lane = (y, z) row of the box and channel: the walk along the task's
 //      particles in storage order (FP32 sums of x factor times (y, z) factor for
-//      the row's three nodes). The sums of a node are quantised and added to its
-//      64-bit accumulator with one integer atomic when the walk leaves the node:
+//      the row's three nodes). A segment's sums are quantised at its end, and a
+//      node's added to its 64-bit accumulator with one integer atomic when the
+//      walk leaves the node:
 //      a segment whose box lies one node further along x -- the usual next key
 //      -- leaves one node of the row, any other box all three.
 // Bound by instruction issue and the shared-memory / L1 data pipe (76 and 60 % of
@@ -720,8 +721,8 @@ __device__ __forceinline__ long long sg_corner_cell(const Scene& sc, int dx, int
 // the force's as pairs for paired multiply-adds (two per instruction), and
 // flushes under half as often. A node's accumulators are adjacent
 // (acc[node][4], one 32-byte sector), which a row's lanes hit together. Force
-// 93 -> 79, mass 84 -> 78 us (1.2 M particles, GIMP); 309 -> 250, 282 -> 250,
-// MUSL 229 -> 181 us (4.1 M); 120 -> 109, 107 -> 105, 87 -> 77 us (2 M, B-spline).
+// 93 -> 80, mass 84 -> 81 us (1.2 M particles, GIMP); 309 -> 256, 282 -> 260,
+// MUSL 229 -> 189 us (4.1 M); 120 -> 113, 107 -> 107, 87 -> 81 us (2 M, B-spline).
 // The task boundaries are fixed by the scene's own sorted order (32 t from
 // the scene's first particle), so a scene's sums are the same alone or in a
 // batch. Phase 2's walk and its segment ends are the same for every lane
@@ -886,22 +887,25 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
   const float* fr = ws + yz * PITCH + (MODE == 2 ? 2 * ch : ch);
   const float* mr = ws + (MODE == 0 ? PS::MAT + yz * PS::STRIDE : 0);
   // segment by segment: the segment ends come from a warp vote, so the walk
-  // and its flushes are the same for every lane. acc[a] is the lane's channel
-  // at node a of its row's window; a segment whose box lies one node further
-  // along x slides the window (its first node is flushed, the other two go
-  // on), any other box flushes it
+  // and its flushes are the same for every lane. A segment's FP32 sums end with
+  // it, quantised: q[a] is the lane's channel at node a of its row's window; a
+  // segment whose box lies one node further along x slides the window (its
+  // first node is flushed, the other two go on), any other box flushes it.
+  // (Sums carried on in FP32 over the window's keys were rounded at the size of
+  // their total: RMS error of the node forces after 21 steps 4.4e-7 for 3.4e-7
+  // on a slope, 5.8e-6 for 3.4e-7 on an SGMP beam, whose internal forces cancel;
+  // they took 78 us for the mass and force transfers of the 1.2 M particle slope,
+  // this 81 and 80.)
   unsigned long long* an = nullptr;  // the window's first node, and its x
   int wb = -2, wx = 0;
   bool row_in = false;
-  float acc[3] = {0.f, 0.f, 0.f}, mass = 0.f;  // (mode 0: mass = node ch of the window)
+  long long q[3] = {0, 0, 0}, qm = 0;  // (mode 0: qm = the mass of node ch of the window)
   auto flush = [&](int a) {
-    const long long q = quant(acc[a], MODE == 0 ? sB : sA);
-    if (q && row_in && wx + a >= 0 && wx + a < sc.NGx)
-      atomicAdd(an + 4 * a + (MODE == 0 ? 1 + ch : ch), (unsigned long long)q);
+    if (q[a] && row_in && wx + a >= 0 && wx + a < sc.NGx)
+      atomicAdd(an + 4 * a + (MODE == 0 ? 1 + ch : ch), (unsigned long long)q[a]);
   };
   auto flush_mass = [&](bool mine) {
-    const long long q = quant(mass, sA);
-    if (q && mine && row_in && wx + ch >= 0 && wx + ch < sc.NGx) atomicAdd(an + 4 * ch, (unsigned long long)q);
+    if (qm && mine && row_in && wx + ch >= 0 && wx + ch < sc.NGx) atomicAdd(an + 4 * ch, (unsigned long long)qm);
   };
   unsigned rem = lasts;
   int j = 0;
@@ -913,12 +917,12 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
       flush(0);
       if (MODE == 0) {
         flush_mass(ch == 0);
-        mass = __shfl_down_sync(0xffffffffu, mass, 1);
-        if (ch == nt - 1) mass = 0.f;
+        qm = __shfl_down_sync(0xffffffffu, qm, 1);
+        if (ch == nt - 1) qm = 0;
       }
-      acc[0] = acc[1];
-      acc[1] = nt == 3 ? acc[2] : 0.f;
-      acc[2] = 0.f;
+      q[0] = q[1];
+      q[1] = nt == 3 ? q[2] : 0;
+      q[2] = 0;
       an += 4;
     } else {
       if (an) {
@@ -931,12 +935,14 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
         const int jy = __shfl_sync(0xffffffffu, c[1], e) + tlo + sy, jz = __shfl_sync(0xffffffffu, c[2], e) + tlo + sz;
         row_in = row_in && jy >= 0 && jy < sc.NGy && jz >= 0 && jz < sc.NGz;
       }
-      acc[0] = acc[1] = acc[2] = mass = 0.f;
+      q[0] = q[1] = q[2] = qm = 0;
       an = b.acc + 4 * (sc.n0 + nb + soff);
     }
     wb = nb;
     wx = jx;
+    float acc[3] = {0.f, 0.f, 0.f};
     if (MODE != 2) {
+      float mass = 0.f;
 #pragma unroll 4
       for (; j <= e; ++j) {
         const float4 x = *reinterpret_cast<const float4*>(xr + j * XF);
@@ -946,8 +952,9 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
         if (nt == 3) acc[2] += x.z * f;
         if (MODE == 0) mass += xr[j * XF + ch] * mr[j];
       }
+      if (MODE == 0) qm += quant(mass, sA);
     } else {
-      float2 s[3] = {{acc[0], 0.f}, {acc[1], 0.f}, {acc[2], 0.f}};
+      float2 s[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 4
       for (; j <= e; ++j) {
         const float4 x = *reinterpret_cast<const float4*>(xr + j * XF);
@@ -959,6 +966,8 @@ __device__ __forceinline__ int part_scatter_task(BState& b, const Scene& sc, lon
 #pragma unroll
       for (int a = 0; a < 3; ++a) acc[a] = s[a].x + s[a].y;
     }
+#pragma unroll
+    for (int a = 0; a < nt; ++a) q[a] += quant(acc[a], MODE == 0 ? sB : sA);
   }
 #pragma unroll
   for (int a = 0; a < nt; ++a) flush(a);
@@ -1044,19 +1053,17 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
   constexpr int NA = MODE == 2 ? 3 : 1;  // accumulators per lane
   const int koff = (k & 1) + (k >> 1 & 1) * sc.NCx + (k >> 2 & 1) * sc.NCxy;
   const int ncell = sc.NCxy * sc.NCz;
-  float acc[NA];
+  long long q[NA];  // the lane's sums over the window's segments, quantised segment by segment
 #pragma unroll
-  for (int a = 0; a < NA; ++a) acc[a] = 0.f;
+  for (int a = 0; a < NA; ++a) q[a] = 0;
   int wc = -2;  // first corner of the window
   auto flush = [&](bool mine) {
     const int cid = wc + koff;  // (corners past the last cell are dropped)
     if (!mine || !active || cid >= ncell) return;
     unsigned long long* ca = b.cacc + (CH0 + g) * b.NC + sc.c0 + cid;
 #pragma unroll
-    for (int a = 0; a < NA; ++a) {
-      const long long q = quant(acc[a], MODE == 0 && g != 0 ? sB : sA);
-      if (q) atomicAdd(ca + 3 * a * b.NC, (unsigned long long)q);
-    }
+    for (int a = 0; a < NA; ++a)
+      if (q[a]) atomicAdd(ca + 3 * a * b.NC, (unsigned long long)q[a]);
     // every corner of a dual cell with particles takes part in the step,
     // whether or not a sum reached it (the auxiliary weights near a fixed
     // face differ from these)
@@ -1072,15 +1079,18 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
       flush(left);
 #pragma unroll
       for (int a = 0; a < NA; ++a) {
-        const float r = __shfl_down_sync(0xffffffffu, acc[a], NPER);
-        acc[a] = left ? r : 0.f;
+        const long long r = __shfl_down_sync(0xffffffffu, q[a], NPER);
+        q[a] = left ? r : 0;
       }
     } else {
       if (wc >= 0) flush(true);
 #pragma unroll
-      for (int a = 0; a < NA; ++a) acc[a] = 0.f;
+      for (int a = 0; a < NA; ++a) q[a] = 0;
     }
     wc = cj;
+    float acc[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) acc[a] = 0.f;
 #pragma unroll 4
     for (; j <= e; ++j) {
       const float w = wr[j];
@@ -1093,6 +1103,8 @@ __device__ __forceinline__ int sg_part_task(BState& b, const Scene& sc, long lon
         acc[0] += w * vr[j];
       }
     }
+#pragma unroll
+    for (int a = 0; a < NA; ++a) q[a] += quant(acc[a], MODE == 0 && g != 0 ? sB : sA);
   }
   flush(true);
   __syncwarp();
