@@ -1579,9 +1579,10 @@ __device__ __forceinline__ float stress_one(BState& b, long long i, int usf_pass
 // registers, some spilled -- than at 1024 with few or none: the 1.2 M particle
 // slope 85 us for 91, the 2 M dam break 124 for 136; the other specialised
 // models at 1024: elastic block 36 k 11.6 us for 12.4, neo-Hookean beam 94 k
-// 17.4 for 21.4)
+// 17.4 for 21.4. The null material with the deformation gradient spills too
+// much at 40: dam break 208 us for 159, 27 k particles 15.2 for 13.3)
 template <int MT, int UV>
-__global__ void __launch_bounds__(512, MT == 10 || MT == 9 ? 3 : (MT ? 2 : 1))
+__global__ void __launch_bounds__(512, MT == 10 || (MT == 9 && !UV) ? 3 : (MT ? 2 : 1))
     kb_stress(BState b, int usf_pass, int filter, int uvf) {
   chain_entry();
   const long long i = btid();
