@@ -310,14 +310,15 @@ int sort_pairs(mpm_ctx* c) {
   const long long np = c->g.np;
   prof_begin(K_SORT, st);
   scan_tiles(PairScan{s.seg, s.fill, s.wcnt, c->nkeys}, s.tiles, st);
-  const dim3 rows((unsigned)((np + 255) / 256), (unsigned)c->g.K + 1);
-  launch_chained(k_pair_place, rows, 256, st, s.snode, s.seg, s.fill, s.val_sorted, np, c->g.K, (long long)c->nkeys,
+  const long long nk = c->nkeys, row = (np + 255) / 256;
+  const unsigned tiles = (unsigned)((nk + bm::kSortThreads - 1) / bm::kSortThreads);
+  launch_chained(k_pair_place, (unsigned)(row * c->g.K + std::min(tiles, 608u)), 256, st, s.snode, s.seg, s.fill, s.val_sorted, np, c->g.K, nk,
                  s.wcnt, s.nbig);
-  launch_chained(k_pair_order, (unsigned)(((long long)c->nkeys * 32 + 127) / 128), 128, st, s.seg, (long long)c->nkeys,
-                 s.val_sorted, s.big, s.nbig);
-  const unsigned tiles = (unsigned)((c->nkeys + bm::kSortThreads - 1) / bm::kSortThreads);
+  const int share = order_share(nk);
+  launch_chained(k_pair_order, (unsigned)((nk + 4 * share - 1) / (4 * share)), 128, st, s.seg, nk, s.val_sorted, s.big,
+                 s.nbig, share);
   launch_chained(k_pair_long, std::min(std::max(tiles, 76u), 608u), bm::kSortThreads, st, s.seg, s.val_sorted, s.big,
-                 s.nbig, (long long)c->nkeys, s.wcnt, s.walk);
+                 s.nbig, nk, s.wcnt, s.walk);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_err(c, e, "pair sort");
   prof_end(K_SORT, st);

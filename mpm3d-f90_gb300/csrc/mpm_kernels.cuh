@@ -499,18 +499,28 @@ __device__ __forceinline__ void count_active(bool active, unsigned long long* ou
 // us, slope 159 k 426 -> 246 -> 165, Taylor bar 17 k 102 -> 46 -> 28, Cook
 // 5.8 k 72 -> 26 -> 22.
 //
+// The groups without pairs, at the end of the order, are left to the blocks
+// after the last one with some, a thread per node: a grid is often mostly
+// empty, and launch_walk bounds the blocks by the pairs. (With a block per group
+// of empty nodes, and a warp per node in k_pair_order, a step of 1000 particles
+// in a grid of 100^3 cells took 690 us with linear shapes, 717 with GIMP, 1056
+// with SGMP; now 117, 159, 550. 27 k particles in 1.5 M nodes: 739, 850, 1365;
+// now 222, 390, 965.)
+//
 // NV addends per pair, NC channels: channel c adds two of them, 2 c and
 // 2 c + 1, for the TWO first channels and one, c + TWO, after those.
 // load(p, idx, raw) fetches the NR values a pair's addends are formed of, for
 // the particle and the index in the shape cache, form(raw, v) forms them;
-// fin(n, in, acc) gets a node's sums (in: there is a node).
+// fin(n, in, acc) gets a node's sums (in: there is a node), called by a whole
+// warp.
 constexpr int kWalkNodes = 8;
 constexpr int kWalkFew = 16;   // PAIRS of the transfers with few products a pair
 constexpr int kWalkMany = 8;   // ... with many
+constexpr int kWalkClasses = 32;   // of segment lengths (walk_class); the last one: no pairs
 
 template <int PAIRS, int NR, int NV, int NC, int TWO, class Load, class Form, class Fin>
-__device__ __forceinline__ void pair_walk(const int* walk, const int* seg, const unsigned* val, long long np,
-                                          long long nn, Load load, Form form, Fin fin) {
+__device__ __forceinline__ void pair_walk(const int* walk, const int* wcnt, const int* seg, const unsigned* val,
+                                          long long np, long long nn, Load load, Form form, Fin fin) {
   static_assert(NV == NC + TWO, "addends");
   // (row pitch: the nodes and pairs of a half-warp fall on distinct banks)
   constexpr int PITCH = kWalkNodes + (PAIRS > 8 ? 1 : 2);
@@ -519,8 +529,13 @@ __device__ __forceinline__ void pair_walk(const int* walk, const int* seg, const
   __shared__ int s_beg[kWalkNodes], s_end[kWalkNodes];
   __shared__ int s_rounds;
   const int t = threadIdx.x;
-  int node = -1;  // of the thread (the first kWalkNodes)
-  if (t < 32) {
+  const int groups = (int)((nn - wcnt[kWalkClasses - 1] + kWalkNodes - 1) / kWalkNodes);  // with pairs
+  const bool idle = (int)blockIdx.x >= groups;
+  int node = -1;  // of the thread (a block with pairs: of the first kWalkNodes)
+  if (idle) {  // one node a thread (launch_walk), sums of zero
+    const long long w = (long long)groups * kWalkNodes + (long long)(blockIdx.x - groups) * (kWalkNodes * PAIRS) + t;
+    if (w < nn) node = walk[w];
+  } else if (t < 32) {
     const long long w = (long long)blockIdx.x * kWalkNodes + t;
     int a = 0, e = 0;
     if (t < kWalkNodes && w < nn) {
@@ -535,64 +550,67 @@ __device__ __forceinline__ void pair_walk(const int* walk, const int* seg, const
     const int longest = __reduce_max_sync(0xffffffffu, e - a);
     if (t == 0) s_rounds = (longest + PAIRS - 1) / PAIRS;
   }
-  __syncthreads();
-  const int rounds = s_rounds;
-  const int g = t / PAIRS, q = t % PAIRS;
-  int j = s_beg[g] + q;                  // the thread's pairs: j, j + PAIRS, ...
-  const int je = s_end[g];
-  const int sn = t % kWalkNodes, sc = t / kWalkNodes;  // the node and first channel the thread sums
-  const int len = s_end[sn] - s_beg[sn];
-  double acc[PER];
+  double a[NC];
 #pragma unroll
-  for (int e = 0; e < PER; ++e) acc[e] = 0.0;
-  double raw[NR];
-  auto fetch = [&] {
-    if (j < je) {
-      const unsigned pv = val[j];
-      const long long p = (long long)(pv >> 5);
-      load(p, (long long)(pv & 31u) * np + p, raw);
-    }
-  };
-  fetch();
-  for (int r = 0; r < rounds; ++r) {
-    double(*b)[PAIRS][PITCH] = buf[r & 1];
-    if (j < je) {
-      double v[NV];
-      form(raw, v);
-#pragma unroll
-      for (int k = 0; k < NV; ++k) b[k][q][g] = v[k];
-    }
-    j += PAIRS;
-    fetch();
-    // (one barrier a round: this half of buf is written again after the next
-    // one, which the summing warps reach when they are done with it)
+  for (int c = 0; c < NC; ++c) a[c] = 0.0;
+  if (!idle) {
     __syncthreads();
-    const int cnt = min(len - r * PAIRS, PAIRS);
+    const int rounds = s_rounds;
+    const int g = t / PAIRS, q = t % PAIRS;
+    int j = s_beg[g] + q;                  // the thread's pairs: j, j + PAIRS, ...
+    const int je = s_end[g];
+    const int sn = t % kWalkNodes, sc = t / kWalkNodes;  // the node and first channel the thread sums
+    const int len = s_end[sn] - s_beg[sn];
+    double acc[PER];
 #pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      const int c = sc + e * PAIRS;
-      if (c < TWO) {
+    for (int e = 0; e < PER; ++e) acc[e] = 0.0;
+    double raw[NR];
+    auto fetch = [&] {
+      if (j < je) {
+        const unsigned pv = val[j];
+        const long long p = (long long)(pv >> 5);
+        load(p, (long long)(pv & 31u) * np + p, raw);
+      }
+    };
+    fetch();
+    for (int r = 0; r < rounds; ++r) {
+      double(*b)[PAIRS][PITCH] = buf[r & 1];
+      if (j < je) {
+        double v[NV];
+        form(raw, v);
 #pragma unroll
-        for (int k = 0; k < PAIRS; ++k)
-          if (k < cnt) acc[e] = acc[e] + b[2 * c][k][sn] + b[2 * c + 1][k][sn];
-      } else if (c < NC) {
+        for (int k = 0; k < NV; ++k) b[k][q][g] = v[k];
+      }
+      j += PAIRS;
+      fetch();
+      // (one barrier a round: this half of buf is written again after the next
+      // one, which the summing warps reach when they are done with it)
+      __syncthreads();
+      const int cnt = min(len - r * PAIRS, PAIRS);
 #pragma unroll
-        for (int k = 0; k < PAIRS; ++k)
-          if (k < cnt) acc[e] = acc[e] + b[c + TWO][k][sn];
+      for (int e = 0; e < PER; ++e) {
+        const int c = sc + e * PAIRS;
+        if (c < TWO) {
+#pragma unroll
+          for (int k = 0; k < PAIRS; ++k)
+            if (k < cnt) acc[e] = acc[e] + b[2 * c][k][sn] + b[2 * c + 1][k][sn];
+        } else if (c < NC) {
+#pragma unroll
+          for (int k = 0; k < PAIRS; ++k)
+            if (k < cnt) acc[e] = acc[e] + b[c + TWO][k][sn];
+        }
       }
     }
-  }
-  __syncthreads();
+    __syncthreads();
 #pragma unroll
-  for (int e = 0; e < PER; ++e)
-    if (sc + e * PAIRS < NC) buf[0][sc + e * PAIRS][0][sn] = acc[e];
-  __syncthreads();
-  if (t < 32) {
-    double a[NC];
+    for (int e = 0; e < PER; ++e)
+      if (sc + e * PAIRS < NC) buf[0][sc + e * PAIRS][0][sn] = acc[e];
+    __syncthreads();
+    if (t >= 32) return;
 #pragma unroll
     for (int c = 0; c < NC; ++c) a[c] = buf[0][c][0][sn];
-    fin(node, node >= 0, a);
   }
+  fin(node, node >= 0, a);
 }
 
 // --------------------------------------------------- P2G: mass, momentum
@@ -602,7 +620,7 @@ __global__ void k_p2g_mass(St<P> s, Geometry g, int bc, int vel) {
   chain_entry();
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
   pair_walk<kWalkFew, 5, 4, 4, 0>(
-      s.walk, s.seg, s.val_sorted, np, nn,
+      s.walk, s.wcnt, s.seg, s.val_sorted, np, nn,
       [&](long long p, long long idx, double* r) {
         r[0] = (double)s.shp[idx];
         r[1] = s.mass[p];
@@ -1353,7 +1371,7 @@ __global__ void k_p2g_force(St<P> s, Geometry g, int integ) {
   chain_entry();
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
   pair_walk<kWalkMany, CONTACT ? 15 : 14, CONTACT ? 9 : 6, CONTACT ? 6 : 3, 3>(
-      s.walk, s.seg, s.val_sorted, np, nn,
+      s.walk, s.wcnt, s.seg, s.val_sorted, np, nn,
       [&](long long p, long long idx, double* r) {
         r[0] = s.shp[idx];
         r[1] = s.dndx[idx];
@@ -1601,7 +1619,7 @@ __global__ void k_p2g_momentum(St<P> s, Geometry g, int vel) {
   chain_entry();
   const long long nn = g.nnt, np = g.np;  // nn: every grid component
   pair_walk<kWalkFew, 5, 3, 3, 0>(
-      s.walk, s.seg, s.val_sorted, np, nn,
+      s.walk, s.wcnt, s.seg, s.val_sorted, np, nn,
       [&](long long p, long long idx, double* r) {
         r[0] = (double)s.shp[idx];
         r[1] = s.mass[p];
@@ -1651,7 +1669,7 @@ __global__ void k_sg_cell_mass(St<P> s, Geometry g) {
   chain_entry();
   const long long np = g.np, nc = g.ncell;
   pair_walk<kWalkFew, 5, 4, 4, 0>(
-      s.walk, s.seg, s.val_sorted, np, nc,
+      s.walk, s.wcnt, s.seg, s.val_sorted, np, nc,
       [&](long long p, long long idx, double* r) {
         r[0] = (double)s.shp[idx];
         r[1] = s.mass[p];
@@ -1743,7 +1761,7 @@ __global__ void k_sg_cell_force(St<P> s, Geometry g) {
   chain_entry();
   const long long np = g.np, nc = g.ncell;
   pair_walk<kWalkMany, 11, 9, 9, 0>(
-      s.walk, s.seg, s.val_sorted, np, nc,
+      s.walk, s.wcnt, s.seg, s.val_sorted, np, nc,
       [&](long long p, long long idx, double* r) {
         r[0] = s.shp[idx];
         r[1] = s.vol[p];
@@ -1856,7 +1874,7 @@ __global__ void k_sg_cell_momentum(St<P> s, Geometry g) {
   chain_entry();
   const long long np = g.np, nc = g.ncell;
   pair_walk<kWalkFew, 5, 3, 3, 0>(
-      s.walk, s.seg, s.val_sorted, np, nc,
+      s.walk, s.wcnt, s.seg, s.val_sorted, np, nc,
       [&](long long p, long long idx, double* r) {
         r[0] = (double)s.shp[idx];
         r[1] = s.mass[p];
@@ -2201,7 +2219,7 @@ __global__ void k_fixed_locate(St<P> s, Geometry g, int with_comp) {
 template <class P, class Fin>
 __device__ __forceinline__ void smooth_sums(const St<P>& s, const Geometry& g, long long nn, Fin fin) {
   pair_walk<kWalkFew, 3, 2, 2, 0>(
-      s.walk, s.seg, s.val_sorted, g.np, nn,
+      s.walk, s.wcnt, s.seg, s.val_sorted, g.np, nn,
       [&](long long p, long long idx, double* r) {
         r[0] = (double)s.shp[idx];
         r[1] = (double)s.sm[p];

@@ -18,8 +18,15 @@ struct Shape {
     grid = (unsigned)((n + block - 1) / block);
   }
 };
-// blocks of a pair_walk kernel over n nodes or cells
-inline unsigned walk_grid(long long n) { return (unsigned)((n + kWalkNodes - 1) / kWalkNodes); }
+// a pair_walk kernel over n nodes or cells: a block per group of nodes, no more
+// than there can be groups with pairs and blocks of nodes without
+template <int PAIRS, class... P, class... A>
+inline void launch_walk(void (*kernel)(P...), long long n, const Geometry& g, cudaStream_t st, A... args) {
+  constexpr int T = kWalkNodes * PAIRS;
+  const long long all = (n + kWalkNodes - 1) / kWalkNodes;
+  const long long some = (g.np * g.K + kWalkNodes - 1) / kWalkNodes + (n + T - 1) / T;
+  launch_chained(kernel, (unsigned)(all < some ? all : some), T, st, args...);
+}
 
 template <class P>
 struct Ops {
@@ -52,10 +59,10 @@ struct Ops {
   static void p2g_mass(void* st, const Geometry& g, int bc, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      launch_chained(k_sg_cell_mass<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_walk<kWalkFew>(k_sg_cell_mass<P>, g.ncell, g, s, S(st), g);
       launch_chained(k_sg_node_mass<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, bc, vel);
     } else {
-      launch_chained(k_p2g_mass<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g, bc, vel);
+      launch_walk<kWalkFew>(k_p2g_mass<P>, g.nnt, g, s, S(st), g, bc, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
@@ -110,11 +117,11 @@ struct Ops {
   static void p2g_force(void* st, const Geometry& g, int integ, cudaStream_t s) {
     prof_begin(K_P2G_FORCE, s);
     if (g.shape == 3) {
-      launch_chained(k_sg_cell_force<P>, walk_grid(g.ncell), kWalkNodes * kWalkMany, s, S(st), g);
+      launch_walk<kWalkMany>(k_sg_cell_force<P>, g.ncell, g, s, S(st), g);
       launch_chained(k_sg_node_force<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, integ);
     } else {
-      if (g.contact) launch_chained(k_p2g_force<P, true>, walk_grid(g.nnt), kWalkNodes * kWalkMany, s, S(st), g, integ);
-      else launch_chained(k_p2g_force<P, false>, walk_grid(g.nnt), kWalkNodes * kWalkMany, s, S(st), g, integ);
+      if (g.contact) launch_walk<kWalkMany>(k_p2g_force<P, true>, g.nnt, g, s, S(st), g, integ);
+      else launch_walk<kWalkMany>(k_p2g_force<P, false>, g.nnt, g, s, S(st), g, integ);
     }
     prof_end(K_P2G_FORCE, s);
   }
@@ -133,10 +140,10 @@ struct Ops {
   static void p2g_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MOM, s);
     if (g.shape == 3) {
-      launch_chained(k_sg_cell_momentum<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_walk<kWalkFew>(k_sg_cell_momentum<P>, g.ncell, g, s, S(st), g);
       launch_chained(k_sg_node_momentum<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, vel);
     } else {
-      launch_chained(k_p2g_momentum<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g, vel);
+      launch_walk<kWalkFew>(k_p2g_momentum<P>, g.nnt, g, s, S(st), g, vel);
     }
     prof_end(K_P2G_MOM, s);
   }
@@ -169,10 +176,10 @@ struct Ops {
   static void tl_momentum(void* st, const Geometry& g, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
-      launch_chained(k_sg_cell_momentum<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_walk<kWalkFew>(k_sg_cell_momentum<P>, g.ncell, g, s, S(st), g);
       launch_chained(k_tl_sg_node_momentum<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g, vel);
     } else {
-      launch_chained(k_p2g_momentum<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g, vel);
+      launch_walk<kWalkFew>(k_p2g_momentum<P>, g.nnt, g, s, S(st), g, vel);
     }
     prof_end(K_P2G_MASS, s);
   }
@@ -195,11 +202,11 @@ struct Ops {
   static void smooth(void* st, const Geometry& g, cudaStream_t s) {
     prof_begin(K_SMOOTH, s);
     if (g.shape == 3) {
-      launch_chained(k_smooth_cell<P>, walk_grid(g.ncell), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_walk<kWalkFew>(k_smooth_cell<P>, g.ncell, g, s, S(st), g);
       launch_chained(k_smooth_sg_node<P>, Shape(g.nn).grid, Shape(g.nn).block, s, S(st), g);
       launch_chained(k_smooth_sg_back<P>, Shape(g.ncell).grid, Shape(g.ncell).block, s, S(st), g);
     } else {
-      launch_chained(k_smooth_node<P>, walk_grid(g.nnt), kWalkNodes * kWalkFew, s, S(st), g);
+      launch_walk<kWalkFew>(k_smooth_node<P>, g.nnt, g, s, S(st), g);
     }
     launch_chained(k_smooth_g2p<P>, Shape(g.np).grid, Shape(g.np).block, s, S(st), g);
     prof_end(K_SMOOTH, s);

@@ -29,7 +29,6 @@ __global__ void k_zero_words(int* w, long long n) {
 // number of eights of pairs in a segment, longest first, empty segments
 // last, about the grid's order within a class. The order has no bearing on
 // results.
-constexpr int kWalkClasses = 32;
 __device__ __forceinline__ int walk_class(int n) {
   return kWalkClasses - 1 - min((n + 7) / 8, kWalkClasses - 1);
 }
@@ -54,21 +53,22 @@ struct PairScan {
 
 constexpr int kWarpPairs = 256;  // longest segment a warp orders
 
-// a place in its node's segment for each pair (thread = particle, blockIdx.y =
-// slot: every pair's atomic in flight at once). Neighbouring particles often
-// share a slot's node: one atomic per node and warp. The blocks of one more row
-// count the nodes of each class.
+// a place in its node's segment for each pair (thread = particle; rows of blocks,
+// one per slot: every pair's atomic in flight at once). Neighbouring particles
+// often share a slot's node: one atomic per node and warp. The blocks after the
+// last row, by the number of nodes, count the nodes of each class.
 __global__ void __launch_bounds__(256) k_pair_place(const int* snode, const int* seg, int* fill, unsigned* val,
                                                     long long np, int K, long long nk, int* wcnt, int* nbig) {
   chain_entry();
-  const long long p = gtid();
-  const int k = blockIdx.y, lane = threadIdx.x & 31;
+  const int row = (int)((np + 255) / 256), lane = threadIdx.x & 31;
+  const int k = min((int)blockIdx.x / row, K), at = blockIdx.x - k * row;  // (slot K: the counting blocks)
+  const long long p = (long long)at * 256 + threadIdx.x;
   if (p == 0 && k == 0) *nbig = 0;
   if (k == K) {
     __shared__ int hist[kWalkClasses];
     if (threadIdx.x < kWalkClasses) hist[threadIdx.x] = 0;
     __syncthreads();
-    for (long long n0 = (long long)blockIdx.x * 256; n0 < nk; n0 += (long long)gridDim.x * 256) {
+    for (long long n0 = p - threadIdx.x; n0 < nk; n0 += (long long)(gridDim.x - K * row) * 256) {
       const long long n = n0 + threadIdx.x;
       const int c = n < nk ? walk_class(seg[n] - (n == 0 ? 0 : seg[n - 1])) : -1;
       const unsigned grp = __match_any_sync(0xffffffffu, c);
@@ -125,20 +125,34 @@ __device__ __forceinline__ void warp_order(unsigned* v, int n) {
     if (r * 32 + lane < n) v[r * 32 + lane] = x[r];
 }
 
-// each node's segment in ascending order, one warp per node; segments longer
-// than kWarpPairs are listed for k_pair_long
-__global__ void k_pair_order(const int* seg, long long nk, unsigned* val, int* big, int* nbig) {
+// each node's segment in ascending order, a warp taking share (1 .. 32) nodes,
+// of which it looks at all together; segments longer than kWarpPairs are listed
+// for k_pair_long. share keeps the warps of a large grid, most of whose nodes
+// have nothing to order, to about kOrderWarps.
+constexpr long long kOrderWarps = 65536;
+inline int order_share(long long nk) {
+  int s = 1;
+  while (s < 32 && nk > s * kOrderWarps) s *= 2;
+  return s;
+}
+__global__ void k_pair_order(const int* seg, long long nk, unsigned* val, int* big, int* nbig, int share) {
   chain_entry();
-  const long long k = gtid() >> 5;
-  if (k >= nk) return;
-  const int a = k == 0 ? 0 : seg[k - 1], n = seg[k] - a;
-  unsigned* v = val + a;
-  if (n <= 1) return;
-  if (n <= 32) warp_order<1>(v, n);
-  else if (n <= 64) warp_order<2>(v, n);
-  else if (n <= 128) warp_order<4>(v, n);
-  else if (n <= kWarpPairs) warp_order<8>(v, n);
-  else if ((threadIdx.x & 31) == 0) big[atomicAdd(nbig, 1)] = (int)k;
+  const int lane = threadIdx.x & 31;
+  const long long k0 = (gtid() >> 5) * share, kl = k0 + lane;
+  const bool own = lane < share && kl < nk;
+  const int al = own && kl > 0 ? seg[kl - 1] : 0, nl = own ? seg[kl] - al : 0;
+  unsigned rest = __ballot_sync(0xffffffffu, nl > 1);
+  while (rest) {
+    const int l = __ffs(rest) - 1;
+    rest &= rest - 1;
+    const int a = __shfl_sync(0xffffffffu, al, l), n = __shfl_sync(0xffffffffu, nl, l);
+    unsigned* v = val + a;
+    if (n <= 32) warp_order<1>(v, n);
+    else if (n <= 64) warp_order<2>(v, n);
+    else if (n <= 128) warp_order<4>(v, n);
+    else if (n <= kWarpPairs) warp_order<8>(v, n);
+    else if (lane == 0) big[atomicAdd(nbig, 1)] = (int)(k0 + l);
+  }
 }
 
 // the segments listed in big in ascending order, and the nodes into walk
