@@ -213,8 +213,6 @@ def kernel_bytes(kernel: str, np_: int, nn_active: float, usf: bool = True) -> f
     if kernel == "g2p_position":
         # read x, v; write x, v; node velocity and acceleration read once
         return np_ * 96 + nn_active * 24
-    if kernel == "permute":
-        return np_ * 2 * (6 * 8 + 6 * 8 + 16 * 4 + 1 + 2 + 2 + 4)
     return np_ * 100.0
 
 

@@ -187,7 +187,6 @@ struct StepOps {
   size_t bulk_size, real_size;
   void (*begin_step)(void* st, const Geometry& g, cudaStream_t s);
   void (*locate)(void* st, const Geometry& g, cudaStream_t s);
-  void (*node_offsets)(void* st, const Geometry& g, long long npairs, cudaStream_t s);
   // P2G of mass + momentum; bc: apply the fixed-DOF zeroing; vel: write vg
   void (*p2g_mass)(void* st, const Geometry& g, int bc, int vel, cudaStream_t s);
   void (*node_velocity)(void* st, const Geometry& g, cudaStream_t s);
@@ -250,8 +249,8 @@ void prof_begin(int kernel_id, cudaStream_t s);
 void prof_end(int kernel_id, cudaStream_t s);
 
 enum KernelId {
-  K_BEGIN = 0, K_LOCATE, K_SORT, K_SEG, K_P2G_MASS, K_NODE_VEL, K_BC, K_STRESS, K_DEPEFF,
-  K_FORCE_PREP, K_P2G_FORCE, K_INTEGRATE, K_POSITION, K_P2G_MOM, K_REDUCE, K_DR, K_PERMUTE,
+  K_BEGIN = 0, K_LOCATE, K_SORT, K_P2G_MASS, K_NODE_VEL, K_BC, K_STRESS, K_DEPEFF,
+  K_FORCE_PREP, K_P2G_FORCE, K_INTEGRATE, K_POSITION, K_P2G_MOM, K_REDUCE, K_DR,
   K_SCATTER_MASS, K_SCATTER_FORCE, K_SCATTER_MOM, K_SG_CLEAR, K_SG_GRADIENT, K_SG_VELOCITY, K_SMOOTH,
   K_CONTACT, K_COUNT
 };

@@ -55,7 +55,6 @@ struct Ops {
     }
     prof_end(K_LOCATE, s);
   }
-  static void node_offsets(void*, const Geometry&, long long, cudaStream_t) {}
   static void p2g_mass(void* st, const Geometry& g, int bc, int vel, cudaStream_t s) {
     prof_begin(K_P2G_MASS, s);
     if (g.shape == 3) {
@@ -226,7 +225,6 @@ struct Ops {
     o.real_size = sizeof(typename P::R);
     o.begin_step = begin_step;
     o.locate = locate;
-    o.node_offsets = node_offsets;
     o.p2g_mass = p2g_mass;
     o.node_velocity = node_velocity;
     o.apply_bc = apply_bc;
