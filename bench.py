@@ -188,15 +188,16 @@ def dominant_kernel(stats: list, steps: int) -> dict:
 def kernel_bytes(kernel: str, np_: int, nn_active: float, usf: bool = True) -> float:
     """Algorithmic bytes of one launch of a kernel of the mixed (batched) step:
     the particle and node fields it must touch, each read once and written
-    once, at their stored widths (FP64 position, velocity, mass, energy, grid;
-    FP32 stress state). Sort keys, permutation and per-step scratch are
+    once, at the widths it reads and writes (FP64 position, velocity, energy,
+    grid; FP32 stress state, cell offsets, and the FP32 copies of mass and
+    velocity where it takes those). Sort keys, permutation and indices are
     implementation overhead and are not counted."""
     if kernel == "p2g_mass_scatter":
-        # read x, mass, v; add node mass + momentum
-        return np_ * (24 + 8 + 24) + nn_active * 32
+        # read x, mass, v (FP32 copies); write cell and offsets; add node mass + momentum
+        return np_ * (24 + 4 + 12 + 16) + nn_active * 32
     if kernel == "p2g_force_scatter":
-        # read x, sigma * vol (6), external force (3); add node force
-        return np_ * (24 + 36) + nn_active * 24
+        # read cell and offsets, sigma * vol (6), external force (3); add node force
+        return np_ * (16 + 36) + nn_active * 24
     if kernel == "p2g_mass":
         # node finalize: node mass + momentum written (+ velocity under USF)
         return nn_active * (32 + (12 if usf else 0))
@@ -204,15 +205,16 @@ def kernel_bytes(kernel: str, np_: int, nn_active: float, usf: bool = True) -> f
         # node finalize: read mass + momentum, write force, momentum, velocity, acceleration
         return nn_active * (32 + 24 + 24 + 24)
     if kernel == "stress_update":
-        # read x, vol, SM, SD, q, ie, cp, epeff, sig_y; write vol, SM, SD, q,
-        # ie, seqv, epeff; node velocity read once; under USF the kernel also
-        # stages the force input (read mass, point loads; write sigma * vol
-        # and the external force)
-        staged = np_ * (8 + 24 + 36) if usf else 0
-        return np_ * (24 + 4 * 13 + 8) + np_ * (4 * 11 + 8) + nn_active * 12 + staged
+        # read cell and offsets, vol, volumetric strain, SM, SD, q, epeff,
+        # mass, ie; write vol, volumetric strain, SM, SD, q, ie, seqv, epeff;
+        # node velocity read once; under USF the kernel also stages the force
+        # input (sigma * vol and the external force; no point loads here)
+        staged = np_ * 36 if usf else 0
+        return np_ * (16 + 4 * 12 + 8) + np_ * (4 * 12 + 8) + nn_active * 12 + staged
     if kernel == "g2p_position":
-        # read x, v; write x, v; node velocity and acceleration read once
-        return np_ * 96 + nn_active * 24
+        # read cell and offsets, x, v, mass; write x, v and the FP32 v; node
+        # velocity and acceleration read once
+        return np_ * (16 + 96 + 4 + 12) + nn_active * 24
     return np_ * 100.0
 
 
@@ -438,7 +440,7 @@ def run_ours(args) -> dict:
     peaks = measured_peaks()
     dom = dominant_kernel(mixed["kernels"], args.steps)
     nn_active = mixed["scalars"]["active_nodes"]
-    kb = kernel_bytes(dom["kernel"], npart, nn_active)
+    kb = kernel_bytes(dom["kernel"], npart, nn_active, bool(deck.flags["USF"]))
     achieved = kb / (dom["avg_ms"] / 1e3) / 1e9
     line = {
         "metric": "particle-steps/s (mixed precision vs plain FP64 GPU, stated error)",

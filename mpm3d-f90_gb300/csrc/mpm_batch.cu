@@ -344,7 +344,7 @@ int upload_scene_particles(mpm_batch* b, HostScene* h, BState& s) {
 }
 
 // sort keys of a scene: one per cell (linear, B-spline), per node (GIMP: a
-// particle is binned with its nearest node, see kb_keys) or per dual cell
+// particle is binned with its nearest node, see gimp_key) or per dual cell
 // (SGMP, ncell of them), plus the bucket of the particles outside the grid
 long long scene_keys(const Geometry& g) { return (g.shape == 1 ? (long long)g.nn : (long long)g.ncell) + 1; }
 

@@ -12,23 +12,23 @@
 //     per step (written by the mass transfer): cell (scene-local cell, -1
 //     outside), off[3] (offset in the cell, in cells), SGMP dual cell, nearest
 //     node, xxn[3], xn[3]; body, scene, orig (scene-local input index)
-//   grid nodes concatenated: FP64 mg, px[3], fx[3]; FP32 float4 velocity and
-//     acceleration (for the particle gathers); fix, bd, node scene
+//   grid nodes concatenated: FP64 mg, px[3], fx[3]; FP32 velocity and
+//     acceleration in three float2 (for the gathers); fix, bd, node scene
 //   SGMP centre nodes (one per cell) concatenated: 64-bit fixed-point
 //     accumulators cacc[13] (mass, momentum[3], external force[3], internal
 //     force[6]); FP32 velocity gradient, velocity, acceleration
 //   sort keys: scene s owns keys [k0, k0 + nk), the last one collects the
-//     particles outside its grid; seg[k] = end of key k's particle range
-//     (kept for SGMP scenes). Linear / B-spline: one key per cell; GIMP:
+//     particles outside its grid; seg[k] = end of key k's range among the
+//     particles being re-sorted (cleared and used by a re-sort alone). Linear / B-spline: one key per cell; GIMP:
 //     one key per node (the particle's nearest node); SGMP: one key per dual
 //     cell.
 //   P2G accumulators: acc[NN][4] 64-bit fixed point (see the scatter kernels).
 //
-// Transfers particle -> grid are scatters of FP32 per-cell partial sums
-// (one warp per occupied cell, or dual cell for SGMP), summed exactly in
-// 64-bit fixed point into the nodes (SGMP: the centre nodes, whose integer
-// sums the node kernels add up exactly). They are deterministic and give a
-// scene the same results alone or in a batch.
+// Transfers particle -> grid are scatters of FP32 sums over the particles of a
+// key (a warp per 32 particles), added up exactly in 64-bit fixed point in the
+// nodes (SGMP: the centre nodes, whose integer sums the node kernels add up
+// exactly). They are deterministic and give a scene the same results alone or
+// in a batch.
 // Transfers grid -> particle are particle-centric with shape functions
 // evaluated on the fly in FP32.
 #pragma once
@@ -80,7 +80,7 @@ struct SceneState {
 
 // State of the device-resident run loop (mpm_batch_run_loop).
 struct LoopCtl {
-  int finished;   // scenes that took their last step (counted by kb_begin, never reset)
+  int finished;   // scenes that took their last step (counted by step_tick, never reset)
   int fin0;       // finished when the loop began
   int iters;      // loop iterations taken (two steps each)
   int max_iters;  // iteration budget

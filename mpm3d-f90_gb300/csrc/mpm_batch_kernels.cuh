@@ -155,7 +155,7 @@ __device__ __forceinline__ void f32_split(double x, float& hi, float& lo) {
 // cell of a position (InWhichCell, Grid.f90:123-155) and the offset in it, in
 // cells (FP32); false off the grid. Every transfer and gather takes a
 // particle's cell and shape-function offsets from this one routine (through
-// the per-step data the permutation writes).
+// the per-step data the mass transfer writes).
 __device__ __forceinline__ bool cell_of(const Scene& sc, const double x[3], int cc[3], float off[3]) {
   bool in = true;
   for (int a = 0; a < 3; ++a) {
@@ -497,8 +497,8 @@ __device__ __forceinline__ void permute_back(const BState& src, BState& dst, lon
 // 2^E, and contributions are scaled by 2^(61 - E), so no sum can reach 2^62.
 // The rounding of a contribution to the fixed-point grid (np * B * 2^-61)
 // is far below its FP32 rounding.
-// The bounds are taken by the kernels that run before each transfer
-// (permutation, force staging, position update).
+// The bounds are taken by the kernels that run before each transfer (layout or
+// restore for the first step, force staging, position update).
 
 // Max of non-negative values v[k] over the block into sst[s].qmax[slot[k]],
 // per scene s (s < 0: no value). Every thread of the block must call it.

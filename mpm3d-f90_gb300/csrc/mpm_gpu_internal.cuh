@@ -143,7 +143,7 @@ struct DevState {
   int* snode;
   R *shp, *dndx, *dndy, *dndz;
   // particles by their number of cpGIMP slots (k_gimp_slots): four lists [4][Np]
-  // and their lengths (behind seg); null for the other shapes and TLMPM
+  // and their lengths (behind seg); null for the other shapes
   int *slot_list, *slot_cnt;
   double* axis;      // node coordinates of the three axes (axis_coord)
   double rdcell[2];  // reciprocal of the cell size as a two-part sum

@@ -8,8 +8,8 @@
 //     reference order (particle index, then slot): the contributions are
 //     formed in parallel and added in that order (pair_walk), so every node
 //     sum is the reference's sequential sum;
-//   * node -> particle transfers run one thread per particle over its slots
-//     in the reference slot order;
+//   * node -> particle transfers run over a particle's slots in the reference
+//     slot order, a thread per particle or per particle and axis;
 //   * reductions use a fixed block tree and a fixed final order.
 #pragma once
 

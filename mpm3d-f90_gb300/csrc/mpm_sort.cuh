@@ -2,10 +2,11 @@
 // key, and the tile scans it uses. It runs on the scenes whose order has
 // become stale (step_tick); the others have no key (kNoKey) and no count.
 //
-// The particles arrive in the last sort's key order with a few per cent moved
+// (On a scene's first step the particles are in the deck's order.) Later on
+// they arrive in the last sort's key order with a few per cent moved
 // to a neighbouring key, so a key's particles are nearly contiguous already
 // and a key holds a handful of particles (about 8 at 8 particles per cell).
-// The sort is a counting sort: per-key counts (taken by kb_keys),
+// The sort is a counting sort: per-key counts (taken by sort_keys),
 // an inclusive scan of the counts into segment ends, placement of every
 // particle into its key's segment through a per-key fill counter (one
 // atomic per key and warp), then the order inside each segment restored to
