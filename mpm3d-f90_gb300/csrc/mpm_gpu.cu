@@ -1017,12 +1017,13 @@ int mpm_upload(mpm_ctx* c, int field, const double* in) {
   if (!p) return set_err(c, MPM_ERR_ARG, "field %d is not kept by this context", field);
   CK(cudaStreamSynchronize(c->stream));
   if (elem == 8) {
-    CK(cudaMemcpy(p, in, (size_t)n * 8, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(p, in, (size_t)n * 8, cudaMemcpyHostToDevice, c->stream));
   } else {
     std::vector<float> tmp((size_t)n);
     for (long long i = 0; i < n; ++i) tmp[i] = (float)in[i];
-    CK(cudaMemcpy(p, tmp.data(), (size_t)n * 4, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(p, tmp.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
   }
+  CK(cudaStreamSynchronize(c->stream));
   if (c->graph_exec) {
     cudaGraphExecDestroy(c->graph_exec);
     c->graph_exec = nullptr;
@@ -1264,12 +1265,16 @@ int mpm_snapshot_load(mpm_ctx* c, const char* path) {
       r = set_err(c, MPM_ERR_IO, "truncated snapshot");
       break;
     }
-    cudaError_t e = cudaMemcpy(p, buf.data(), buf.size(), cudaMemcpyHostToDevice);
+    // (on the context's stream: behind the steps still running and before the
+    // next ones)
+    cudaError_t e = cudaMemcpyAsync(p, buf.data(), buf.size(), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) r = cuda_err(c, e, "snapshot upload");
   }
   fclose(f);
   if (r) return r;
-  CK(cudaMemcpy(c->st.sc, &sc, sizeof sc, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->st.sc, &sc, sizeof sc, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   return MPM_OK;
 }
 
