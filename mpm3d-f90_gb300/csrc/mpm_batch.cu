@@ -207,6 +207,7 @@ struct mpm_batch {
   int sort_polls = 0;         // polls of the re-sort's waits (0: by the particles, barrier_polls)
   int sms = 152;              // multiprocessors of the device
   int loop_min_steps = 0;     // steps a device loop takes before it honours an interrupt
+  long long n_sgmp = 0;       // first node of the SGMP scenes, which come last
   long long ntask = 0;        // particle tasks of the linear / GIMP / B-spline scenes (32 particles each)
   // device-resident run loop (mpm_batch_run_loop): its state, the host's
   // request flag (page-locked, mapped into the device's address space) and
@@ -419,8 +420,11 @@ int enqueue_back(mpm_batch* b) {
   const int pb = b->pblock, nb = b->nblock;
   prof_begin(K_P2G_MASS, st);
   // (the last block of the first one starts the step)
-  if (b->any_nonsgmp) launch_chained(kb_p2g_mass<false>, gridn(s.NN, nb) + 1, nb, st, s, 1, 1, b->d_target, 1);
-  if (b->any_sgmp) launch_chained(kb_p2g_mass<true>, gridn(s.NN, nb) + 1, nb, st, s, 1, 1, b->d_target, !b->any_nonsgmp);
+  // (the nodes of the SGMP scenes come after the others')
+  const long long ns = b->n_sgmp;
+  if (b->any_nonsgmp) launch_chained(kb_p2g_mass<false>, gridn(ns, nb) + 1, nb, st, s, 0, ns, 1, 1, b->d_target, 1);
+  if (b->any_sgmp)
+    launch_chained(kb_p2g_mass<true>, gridn(s.NN - ns, nb) + 1, nb, st, s, ns, s.NN, 1, 1, b->d_target, !b->any_nonsgmp);
   prof_end(K_P2G_MASS, st);
   int r = enqueue_resort(b);
   if (r) return r;
@@ -471,8 +475,8 @@ int enqueue_back(mpm_batch* b) {
   enqueue_scatter(b, 2);
   prof_end(K_SCATTER_FORCE, st);
   prof_begin(K_P2G_FORCE, st);
-  if (b->any_nonsgmp) launch_chained(kb_p2g_force<false>, gridn(s.NN, nb), nb, st, s);
-  if (b->any_sgmp) launch_chained(kb_p2g_force<true>, gridn(s.NN, nb), nb, st, s);
+  if (b->any_nonsgmp) launch_chained(kb_p2g_force<false>, gridn(ns, nb), nb, st, s, 0, ns);
+  if (b->any_sgmp) launch_chained(kb_p2g_force<true>, gridn(s.NN - ns, nb), nb, st, s, ns, s.NN);
   prof_end(K_P2G_FORCE, st);
   if (b->any_sgmp) {
     prof_begin(K_SG_VELOCITY, st);
@@ -487,8 +491,8 @@ int enqueue_back(mpm_batch* b) {
     enqueue_scatter(b, 1);
     prof_end(K_SCATTER_MOM, st);
     prof_begin(K_P2G_MOM, st);
-    if (b->any_nonsgmp) launch_chained(kb_p2g_momentum<false>, gridn(s.NN, nb), nb, st, s);
-    if (b->any_sgmp) launch_chained(kb_p2g_momentum<true>, gridn(s.NN, nb), nb, st, s);
+    if (b->any_nonsgmp) launch_chained(kb_p2g_momentum<false>, gridn(ns, nb), nb, st, s, 0, ns);
+    if (b->any_sgmp) launch_chained(kb_p2g_momentum<true>, gridn(s.NN - ns, nb), nb, st, s, ns, s.NN);
     prof_end(K_P2G_MOM, st);
   }
   if (b->any_later && (r = stress(0))) return r;
@@ -723,7 +727,12 @@ int commit(mpm_batch* b) {
     for (HostScene* h : b->order)
       if (h->resident) h->st = old[h->index];
   }
-  // new layout
+  // new layout, the SGMP scenes last: the node kernels of either family run over
+  // its own nodes (over all of them in batches of both, every node of the other
+  // family cost a look at its scene: 4000 scenes of 512 particles 1807 us a step
+  // for 1675)
+  std::stable_partition(b->order.begin(), b->order.end(), [](const HostScene* h) { return h->su.g.shape != 3; });
+  b->n_sgmp = 0;
   long long NP = 0, NN = 0, NK = 0, NC = 0, NR = 0;
   int nmat = 0, nbody = 0;
   std::vector<int> old_index;
@@ -751,6 +760,7 @@ int commit(mpm_batch* b) {
     h->body0 = nbody;
     NP += h->np;
     NN += h->nn;
+    if (g.shape != 3) b->n_sgmp = NN;
     NK += scene_keys(h->su.g);
     if (g.shape == 3) NC += h->ncell;
     NR += h->nr;

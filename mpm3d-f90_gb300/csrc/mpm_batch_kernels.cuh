@@ -1210,33 +1210,33 @@ constexpr float kDisorder = 1.f;
 
 __device__ __forceinline__ void step_tick(BState& b, const int* target) {
   __shared__ long long thr[512], wsum[32];
-  long long carry = 0;
   int any = 0;
+  for (int s = threadIdx.x; s < b.nscene; s += blockDim.x) {
+    SceneState& t = b.sst[s];
+    int rs = 0;
+    b.ract[s] = t.active;
+    if (t.active) {
+      t.istep = t.istep + 1;
+      if (t.istep == target[s]) atomicAdd(&b.ctl->finished, 1);  // the scene's last step
+      t.time = t.time + t.dt;
+      t.ftime = (float)t.time;
+      rs = t.istep == 1 || (float)b.disorder[s] > kDisorder * (float)((b.scenes[s].np + 31) / 32);
+    }
+    b.resort[s] = rs;
+    any |= rs;
+  }
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) *b.any_resort = any;
+  // (the scan of a batch of 4000 scenes takes 50 us: only where some are re-sorted)
+  if (!any) return;
+  long long carry = 0;
   for (int s0 = 0; s0 < b.nscene; s0 += blockDim.x) {
     const int s = s0 + threadIdx.x;
-    long long np = 0;
-    int rs = 0;
-    if (s < b.nscene) {
-      SceneState& t = b.sst[s];
-      b.ract[s] = t.active;
-      if (t.active) {
-        t.istep = t.istep + 1;
-        if (t.istep == target[s]) atomicAdd(&b.ctl->finished, 1);  // the scene's last step
-        t.time = t.time + t.dt;
-        t.ftime = (float)t.time;
-        const long long n = b.scenes[s].np;
-        rs = t.istep == 1 || (float)b.disorder[s] > kDisorder * (float)((n + 31) / 32);
-        if (rs) np = n;
-      }
-      b.resort[s] = rs;
-    }
-    const long long before = block_scan<long long, ScanSum>(np, thr, wsum);
-    const long long total = thr[blockDim.x - 1];
+    const bool rs = s < b.nscene && b.resort[s];
+    const long long before = block_scan<long long, ScanSum>(rs ? b.scenes[s].np : 0, thr, wsum);
     if (rs) b.shift[s] = b.scenes[s].p0 - (carry + before);
-    carry += total;
-    any = __syncthreads_or(any || rs);
+    carry += thr[blockDim.x - 1];
   }
-  if (threadIdx.x == 0) *b.any_resort = any;
 }
 
 // the cells next to grid node j that take part in the step (bit dx + 2 dy + 4 dz
@@ -1257,21 +1257,21 @@ __device__ __forceinline__ unsigned sg_active_cells(const BState& b, const Scene
 }
 
 // SG: the nodes of the SGMP scenes (an instantiation of its own: the 8 cells' loads
-// in flight take registers that the others would pay for); tick: the last
-// block starts the step
+// in flight take registers that the others would pay for); the nodes n0 .. n1 - 1
+// are all of that family; tick: the last block starts the step
 template <bool SG>
-__global__ void kb_p2g_mass(BState b, int bc_usf, int vel_usf, const int* target, int tick) {
+__global__ void kb_p2g_mass(BState b, long long n0, long long n1, int bc_usf, int vel_usf, const int* target, int tick) {
   chain_entry();
   if (tick && blockIdx.x == gridDim.x - 1) {  // the last block starts the step instead of finishing nodes
     step_tick(b, target);
     return;
   }
-  long long n = btid();
+  const long long n = n0 + btid();
   bool act = false;
   int s = -1;
-  if (n < b.NN) {
+  if (n < n1) {
     s = scene_of(b, b.node_scene, n);
-    if (scene_live(b, s) && (b.scenes[s].shape == 3) == SG) {
+    if (scene_live(b, s)) {
       const Scene& sc = b.scenes[s];
       const long long NN = b.NN;
       double M = 0, P0 = 0, P1 = 0, P2 = 0;
@@ -1749,14 +1749,13 @@ __device__ __forceinline__ void node_integrate(BState& b, const Scene& sc, int s
 
 // (the SGMP form keeps two cells' nine loads in flight at 64 registers)
 template <bool SG>
-__global__ void __launch_bounds__(512, SG ? 2 : 1) kb_p2g_force(BState b) {
+__global__ void __launch_bounds__(512, SG ? 2 : 1) kb_p2g_force(BState b, long long n0, long long n1) {
   chain_entry();
-  long long n = btid();
-  if (n >= b.NN) return;
+  const long long n = n0 + btid();
+  if (n >= n1) return;
   const int s = SG ? (int)b.node_scene[n] : scene_of(b, b.node_scene, n);
   if (!scene_live(b, s)) return;
   const Scene& sc = b.scenes[s];
-  if ((sc.shape == 3) != SG) return;
   double F[3] = {0, 0, 0};
   if (SG) {
     int j[3];
@@ -2018,14 +2017,14 @@ __global__ void __launch_bounds__(512, 3) kb_position(BState b) {
 
 // GridMomentumMUSL: momentum re-map with the new particle velocities
 template <bool SG>
-__global__ void kb_p2g_momentum(BState b) {
+__global__ void kb_p2g_momentum(BState b, long long n0, long long n1) {
   chain_entry();
-  long long n = btid();
-  if (n >= b.NN) return;
+  const long long n = n0 + btid();
+  if (n >= n1) return;
   const int s = scene_of(b, b.node_scene, n);
   if (!scene_live(b, s)) return;
   const Scene& sc = b.scenes[s];
-  if (!sc.musl || (sc.shape == 3) != SG) return;
+  if (!sc.musl) return;
   const long long NN = b.NN;
   double P0 = 0, P1 = 0, P2 = 0;
   if (SG) {
