@@ -835,10 +835,10 @@ int commit(mpm_batch* b) {
   shared.scenes = al.get<Scene>((long long)b->order.size());
   shared.task0 = al.get<int>((long long)b->order.size() + 1);
   shared.disorder = al.get<int>((long long)b->order.size());
-  shared.resort = al.get<int>((long long)b->order.size());
+  shared.resort = al.get<int>(kResortScenes + 2 * (long long)b->order.size() + 1);
   shared.shift = al.get<int>((long long)b->order.size());
   shared.ract = al.get<int>((long long)b->order.size());
-  shared.any_resort = al.get<int>(1);
+  shared.kshift = al.get<int>((long long)b->order.size());
   shared.gbar = al.get<unsigned>(2);
   shared.sst = al.get<SceneState>((long long)b->order.size());
   shared.mats = al.get<DevMaterial>(nmat);
@@ -882,7 +882,7 @@ int commit(mpm_batch* b) {
     s.setter = shared.setter; s.setter_scan = shared.setter_scan; s.dep = shared.dep; s.jc_aux = shared.jc_aux;
     s.deferred = shared.deferred; s.red_part = shared.red_part; s.rscene = shared.rscene; s.scenes = shared.scenes;
     s.task0 = shared.task0; s.disorder = shared.disorder; s.resort = shared.resort; s.shift = shared.shift;
-    s.ract = shared.ract; s.any_resort = shared.any_resort; s.gbar = shared.gbar;
+    s.ract = shared.ract; s.kshift = shared.kshift; s.gbar = shared.gbar;
     s.sst = shared.sst; s.mats = shared.mats; s.fmats = shared.fmats; s.bodies = shared.bodies;
   };
   share(A);
@@ -995,7 +995,7 @@ int commit(mpm_batch* b) {
   BCK(cudaMemcpyAsync(shared.rscene, rscene.data(), 2 * NR, cudaMemcpyHostToDevice, st));
   BCK(cudaMemcpyAsync(d_target, target.data(), sizeof(int) * target.size(), cudaMemcpyHostToDevice, st));
   BCK(cudaMemcpyAsync(shared.sst, sst.data(), sizeof(SceneState) * sst.size(), cudaMemcpyHostToDevice, st));
-  BCK(cudaMemsetAsync(shared.any_resort, 0, sizeof(int), st));
+  BCK(cudaMemsetAsync(shared.resort, 0, sizeof(int) * kResortScenes, st));
   BCK(cudaMemsetAsync(shared.gbar, 0, 2 * sizeof(unsigned), st));
   BCK(cudaMemcpyAsync(shared.ract, ract.data(), sizeof(int) * ract.size(), cudaMemcpyHostToDevice, st));
   BCK(cudaMemsetAsync(shared.mg, 0, sizeof(double) * NN, st));

@@ -88,6 +88,8 @@ struct LoopCtl {
   int pad_;
 };
 
+constexpr int kResortScenes = 2;  // (BState::resort)
+
 struct BState {
   long long NP, NN, NK, NC, NR;
   int nscene;
@@ -108,11 +110,14 @@ struct BState {
   unsigned* key;
   int *perm, *seg;
   int *fill, *tiles, *big, *nbig;  // per-key slots taken, scan tile totals, long segments
-  // re-sort control, per scene: particles out of order (counted by the mass
-  // transfer), re-sorted this step, number of a re-sorted scene's particle i =
-  // i - shift; ract: the scene takes the step whose reduction runs next
+  // re-sort control: particles out of order per scene (counted by the mass
+  // transfer); the scenes re-sorted this step (step_tick): their number, the
+  // number of their keys, from kResortScenes on their indices (room for
+  // nscene) and behind these each one's first chunk of the sort's blocks, and the
+  // chunks of all; number of such a scene's particle i = i - shift; ract: the scene
+  // takes the step whose reduction runs next
   int *disorder, *resort, *shift, *ract;
-  int* any_resort;  // some scene is re-sorted this step
+  int* kshift;  // number of a re-sorted scene's key k = k - kshift
   unsigned* gbar;   // grid barrier of the re-sort: arrivals, a wait that ran out (stays set)
   LoopCtl* ctl;  // run-loop state (one per batch, outside the layout arena)
   int* task0;  // first particle task (32 sorted particles) of each scene, nscene + 1 entries; SGMP scenes have none

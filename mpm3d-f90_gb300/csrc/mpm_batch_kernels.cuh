@@ -331,49 +331,68 @@ __device__ __forceinline__ int gimp_key(const Scene& sc, int c[3], const float o
 }
 
 // ------------------------------------------------------------------ keys
-// Sort keys and per-key counts of the scenes that are re-sorted this step
-// (BState::resort), from the step's derived data; the scene's last key
-// collects the particles outside the grid. Scenes that keep their order get
-// no key and no count.
+// f(s, i, in) for every particle i of the scenes s that are re-sorted this step
+// (BState::resort), in chunks of a block's threads; in: the thread has a
+// particle. Every thread of the grid calls it. A block takes a run of chunks: one
+// search for its first scene (a search for every chunk: the sort of 4000 scenes of
+// 512 particles 340 us for 273).
+template <class F>
+__device__ __forceinline__ void for_resorted(const BState& b, F f) {
+  const int *scene = b.resort + kResortScenes, *first = scene + b.nscene;
+  const int n = b.resort[0], chunks = first[n];
+  const int per = (chunks + gridDim.x - 1) / gridDim.x;
+  const int t0 = min((long long)blockIdx.x * per, (long long)chunks), t1 = min(t0 + per, chunks);
+  if (t0 >= t1) return;
+  int lo = 0, hi = n - 1;  // the last scene whose first chunk is at or before t0
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (first[mid] <= t0) lo = mid;
+    else hi = mid - 1;
+  }
+  for (int t = t0; t < t1; ++t) {
+    while (first[lo + 1] <= t) ++lo;
+    const int s = scene[lo];
+    const long long l = (long long)(t - first[lo]) * kSortThreads + threadIdx.x;
+    f(s, b.scenes[s].p0 + l, l < b.scenes[s].np);
+  }
+}
+
+// Sort keys and per-key counts of the scenes that are re-sorted this step, from
+// the step's derived data; the scene's last key collects the particles outside
+// the grid. The sort numbers those scenes' keys and particles without gaps: a
+// scene's key k is number k0 + k - kshift[s], its particle i number i - shift[s].
 __device__ __forceinline__ void sort_keys(BState& b) {
   const long long NP = b.NP;
-  for (long long b0 = (long long)blockIdx.x * kSortThreads; b0 < NP; b0 += (long long)gridDim.x * kSortThreads) {
-    const long long i = b0 + threadIdx.x;
+  for_resorted(b, [&](int s, long long i, bool in) {
     unsigned key = kNoKey;
-    if (i < NP) {
-      const int s = b.scene[i];
-      if (b.resort[s]) {
-        const Scene& sc = b.scenes[s];
-        int k = sc.shape == 3 ? b.dual[i] : b.cell[i];
-        if (sc.shape == 1 && k >= 0) {
-          int c[3];
-          c[2] = div_by(k, sc.mNCxy);
-          const int rem = k - c[2] * sc.NCxy;
-          c[1] = div_by(rem, sc.mNCx);
-          c[0] = rem - c[1] * sc.NCx;
-          const float off[3] = {b.off[i], b.off[NP + i], b.off[2 * NP + i]};
-          k = gimp_key(sc, c, off);
-        }
-        key = (unsigned)(sc.k0 + (k >= 0 ? k : sc.nk - 1));
+    if (in) {
+      const Scene& sc = b.scenes[s];
+      int k = sc.shape == 3 ? b.dual[i] : b.cell[i];
+      if (sc.shape == 1 && k >= 0) {
+        int c[3];
+        c[2] = div_by(k, sc.mNCxy);
+        const int rem = k - c[2] * sc.NCxy;
+        c[1] = div_by(rem, sc.mNCx);
+        c[0] = rem - c[1] * sc.NCx;
+        const float off[3] = {b.off[i], b.off[NP + i], b.off[2 * NP + i]};
+        k = gimp_key(sc, c, off);
       }
+      key = (unsigned)(sc.k0 - b.kshift[s] + (k >= 0 ? k : sc.nk - 1));
       b.key[i] = key;
     }
     // per-key counts: neighbours mostly share a key -- one atomic per key and
     // warp
     const unsigned grp = __match_any_sync(0xffffffffu, key);
     if (key != kNoKey && (threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&b.seg[key], __popc(grp));
-  }
+  });
 }
 
 // ---------------------------------------------------- permutation + derived
 // dst[i] = src[perm[i]] for every persistent particle field of the scenes
 // being re-sorted, then the step's derived data of the particle at its new
 // place; permute_back returns the fields to the set every other kernel
-// uses. The sort numbers the re-sorted scenes' particles without gaps, a
-// scene's particle i being number i - shift[scene].
-__device__ __forceinline__ void permute_one(const BState& src, BState& dst, long long i) {
-  const int s = src.scene[i];  // (a scene's particles stay in its range)
-  if (!src.resort[s]) return;
+// uses.
+__device__ __forceinline__ void permute_one(const BState& src, BState& dst, int s, long long i) {
   // every value is loaded before the first store: the stores could alias the
   // loads as far as the compiler knows, so interleaving them would serialise
   // one memory round trip per field
@@ -435,10 +454,8 @@ __device__ __forceinline__ void permute_one(const BState& src, BState& dst, long
 
 // the re-sorted scenes' fields from the permutation's target set back to the
 // working set (a straight copy)
-__device__ __forceinline__ void permute_back(const BState& src, BState& dst, long long i) {
+__device__ __forceinline__ void permute_back(const BState& src, BState& dst, int s, long long i) {
   const long long NP = src.NP;
-  const int s = dst.scene[i];
-  if (!src.resort[s]) return;
   const Scene& sc = src.scenes[s];
   double x[3], v[3], f[3] = {0.0, 0.0, 0.0};
   for (int a = 0; a < 3; ++a) {
@@ -627,38 +644,46 @@ __device__ __forceinline__ NodeBox node_box(const Scene& sc, const int c[3], con
 
 // The re-sort of the scenes marked by step_tick, in one cooperative launch:
 // counting sort by key (mpm_sort.cuh), then every field permuted into the
-// second particle set and back. A step in which no scene is re-sorted -- most
+// second particle set and back; over the marked scenes' particles and keys alone
+// (over the whole batch, 500 scenes of 512 particles that fly on their own, of
+// which some are re-sorted in every step, took 334 us a step linear, 362 GIMP, 520
+// SGMP; now 308, 336, 487). A step in which no scene is re-sorted -- most
 // of them -- pays one launch that returns at once: 1.6 us of the step, against
 // 10 us for an IF node around the phases as kernels of their own and 16 to 34
 // us for those kernels returning one by one (5.8 k to 1.2 M particles). The
 // barriers between the phases cost a re-sort about what launches would.
 __global__ void __launch_bounds__(kSortThreads, 3) kb_resort(BState a, BState o, int polls, int* stall) {
   chain_entry();
-  if (!*a.any_resort) return;
+  if (!a.resort[0]) return;
+  const long long nk = a.resort[1];  // keys of the scenes to sort
   __shared__ int sm[kSmemSeg];  // (the scan's tile, then the long segments)
   __shared__ int thr[kSortThreads], wsum[32];
   const long long g0 = (long long)blockIdx.x * kSortThreads + threadIdx.x, gs = (long long)gridDim.x * kSortThreads;
   unsigned round = 0;
-  for (long long k = g0; k < a.NK; k += gs) a.seg[k] = 0;
+  for (long long k = g0; k < nk; k += gs) a.seg[k] = 0;
   if (g0 == 0) *a.nbig = 0;
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_keys(a);
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  sort_tile_totals(a.seg, a.NK, a.tiles, thr, wsum);
+  sort_tile_totals(a.seg, nk, a.tiles, thr, wsum);
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  sort_tile_prefix(a.NK, a.tiles, thr, wsum);
+  sort_tile_prefix(nk, a.tiles, thr, wsum);
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  sort_tile_scan(a.seg, a.fill, a.NK, a.tiles, sm, thr, wsum);
+  sort_tile_scan(a.seg, a.fill, nk, a.tiles, sm, thr, wsum);
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  sort_place(a.key, a.seg, a.fill, a.perm, a.NP);
+  for_resorted(a, [&](int, long long i, bool in) { sort_place(in ? a.key[i] : kNoKey, i, a.seg, a.fill, a.perm); });
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  sort_segments(a.seg, a.NK, a.perm, a.big, a.nbig);
+  sort_segments(a.seg, nk, a.perm, a.big, a.nbig);
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
   sort_long(a.seg, a.perm, a.big, a.nbig, sm, [&](int k, int* p, int n) { order_segment(a.key, (unsigned)k, p, n); });
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  for (long long i = g0; i < a.NP; i += gs) permute_one(a, o, i);
+  for_resorted(a, [&](int s, long long i, bool in) {
+    if (in) permute_one(a, o, s, i);
+  });
   if (!grid_barrier(a.gbar, ++round, polls, stall)) return;
-  for (long long i = g0; i < a.NP; i += gs) permute_back(o, a, i);
+  for_resorted(a, [&](int s, long long i, bool in) {
+    if (in) permute_back(o, a, s, i);
+  });
 }
 
 // FP32 mass and velocity of the particles of a scene (-1: of every scene),
@@ -1204,38 +1229,106 @@ __device__ __forceinline__ void node_finish(BState& b, const Scene& sc, long lon
 // flush of a node box per transfer), so the order is renewed once that costs
 // about as much as a sort does; results depend on the order only through FP32
 // partial sums, and the decision only on the scene's own particles and order.
-// Also numbers the re-sorted scenes' particles for the sort (shift). One
-// block.
+// Also lists the scenes to re-sort and numbers their particles and keys for the
+// sort (BState::resort, shift, kshift). One block.
 constexpr float kDisorder = 1.f;
 
 __device__ __forceinline__ void step_tick(BState& b, const int* target) {
   __shared__ long long thr[512], wsum[32];
+  constexpr int U = 2;  // scenes of a thread whose loads are in flight together
+  int *scene = b.resort + kResortScenes, *first = scene + b.nscene;
   int any = 0;
-  for (int s = threadIdx.x; s < b.nscene; s += blockDim.x) {
-    SceneState& t = b.sst[s];
-    int rs = 0;
-    b.ract[s] = t.active;
-    if (t.active) {
-      t.istep = t.istep + 1;
-      if (t.istep == target[s]) atomicAdd(&b.ctl->finished, 1);  // the scene's last step
-      t.time = t.time + t.dt;
-      t.ftime = (float)t.time;
-      rs = t.istep == 1 || (float)b.disorder[s] > kDisorder * (float)((b.scenes[s].np + 31) / 32);
+  for (int s0 = threadIdx.x; s0 < b.nscene; s0 += U * blockDim.x) {
+    SceneState t[U];
+    int last[U], dis[U];
+    long long np[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u * blockDim.x;
+      if (s >= b.nscene) continue;
+      t[u].active = b.sst[s].active;
+      t[u].istep = b.sst[s].istep;
+      t[u].time = b.sst[s].time;
+      t[u].dt = b.sst[s].dt;
+      last[u] = target[s];
+      dis[u] = b.disorder[s];
+      np[u] = b.scenes[s].np;
     }
-    b.resort[s] = rs;
-    any |= rs;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int s = s0 + u * blockDim.x;
+      if (s >= b.nscene) continue;
+      int rs = 0;
+      b.ract[s] = t[u].active;
+      if (t[u].active) {
+        SceneState& st = b.sst[s];
+        const int istep = t[u].istep + 1;
+        const double time = t[u].time + t[u].dt;
+        st.istep = istep;
+        st.time = time;
+        st.ftime = (float)time;
+        if (istep == last[u]) atomicAdd(&b.ctl->finished, 1);  // the scene's last step
+        rs = istep == 1 || (float)dis[u] > kDisorder * (float)((np[u] + 31) / 32);
+      }
+      b.shift[s] = rs;  // (read below by the thread of the scene's strip)
+      any |= rs;
+    }
   }
   any = __syncthreads_or(any);
-  if (threadIdx.x == 0) *b.any_resort = any;
-  // (the scan of a batch of 4000 scenes takes 50 us: only where some are re-sorted)
-  if (!any) return;
-  long long carry = 0;
-  for (int s0 = 0; s0 < b.nscene; s0 += blockDim.x) {
-    const int s = s0 + threadIdx.x;
-    const bool rs = s < b.nscene && b.resort[s];
-    const long long before = block_scan<long long, ScanSum>(rs ? b.scenes[s].np : 0, thr, wsum);
-    if (rs) b.shift[s] = b.scenes[s].p0 - (carry + before);
-    carry += thr[blockDim.x - 1];
+  if (!any) {
+    if (threadIdx.x == 0) b.resort[0] = 0;
+    return;
+  }
+  // a strip of scenes per thread: how many of them are marked and their chunks,
+  // particles and keys, two sums to a 64-bit value
+  const int strip = (b.nscene + blockDim.x - 1) / blockDim.x;
+  const int s0 = min((int)threadIdx.x * strip, b.nscene), s1 = min(s0 + strip, b.nscene);
+  auto sizes = [&](int s, long long& nc, long long& pk) {
+    const Scene& sc = b.scenes[s];
+    nc = (1LL << 32) + (sc.np + kSortThreads - 1) / kSortThreads;
+    pk = (sc.np << 32) + sc.nk;
+  };
+  long long nc = 0, pk = 0;
+  for (int s = s0; s < s1; ++s)
+    if (b.shift[s]) {
+      long long c, p;
+      sizes(s, c, p);
+      nc += c;
+      pk += p;
+    }
+  nc = block_scan<long long, ScanSum>(nc, thr, wsum);
+  const long long tnc = thr[blockDim.x - 1];
+  __syncthreads();
+  pk = block_scan<long long, ScanSum>(pk, thr, wsum);
+  const long long tpk = thr[blockDim.x - 1];
+  for (int s = s0; s < s1; s += U) {
+    long long c[U], p[U], p0[U], k0[U];
+    int rs[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      rs[u] = s + u < s1 ? b.shift[s + u] : 0;
+      if (!rs[u]) continue;
+      sizes(s + u, c[u], p[u]);
+      p0[u] = b.scenes[s + u].p0;
+      k0[u] = b.scenes[s + u].k0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (!rs[u]) continue;
+      const int at = (int)(nc >> 32);
+      scene[at] = s + u;
+      first[at] = (int)(nc & 0xffffffff);
+      b.shift[s + u] = (int)(p0[u] - (pk >> 32));
+      b.kshift[s + u] = (int)(k0[u] - (pk & 0xffffffff));
+      nc += c[u];
+      pk += p[u];
+    }
+  }
+  if (threadIdx.x == 0) {
+    const int n = (int)(tnc >> 32);
+    b.resort[0] = n;
+    b.resort[1] = (int)(tpk & 0xffffffff);
+    first[n] = (int)(tnc & 0xffffffff);
   }
 }
 

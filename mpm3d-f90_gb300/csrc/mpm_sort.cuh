@@ -1,6 +1,7 @@
 // mpm_sort.cuh -- the batched engine's counting sort of particles by sort
 // key, and the tile scans it uses. It runs on the scenes whose order has
-// become stale (step_tick); the others have no key (kNoKey) and no count.
+// become stale (step_tick), whose keys and particles are numbered without gaps;
+// the others take no part.
 //
 // (On a scene's first step the particles are in the deck's order.) Later on
 // they arrive in the last sort's key order with a few per cent moved
@@ -275,21 +276,17 @@ __device__ __forceinline__ void sort_tile_scan(int* seg, int* fill, long long nk
   }
 }
 
-// perm[seg start + slot] = i for every particle i with a key, the slot taken
-// from the key's fill counter (one atomic per key and warp; lanes of a warp
-// with the same key take consecutive slots in lane order)
-__device__ __forceinline__ void sort_place(const unsigned* key, const int* seg, int* fill, int* perm, long long n) {
+// perm[seg start + slot] = i for a warp's particles i with key k (kNoKey: none),
+// the slot taken from the key's fill counter (one atomic per key and warp; lanes
+// of a warp with the same key take consecutive slots in lane order)
+__device__ __forceinline__ void sort_place(unsigned k, long long i, const int* seg, int* fill, int* perm) {
   const int lane = threadIdx.x & 31;
-  for (long long b0 = (long long)blockIdx.x * kSortThreads; b0 < n; b0 += (long long)gridDim.x * kSortThreads) {
-    const long long i = b0 + threadIdx.x;
-    const unsigned k = i < n ? key[i] : kNoKey;
-    const unsigned grp = __match_any_sync(0xffffffffu, k);
-    const int leader = __ffs(grp) - 1, rank = __popc(grp & ((1u << lane) - 1u));
-    int base = 0;
-    if (lane == leader && k != kNoKey) base = atomicAdd(&fill[k], __popc(grp));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (k != kNoKey) perm[(k == 0 ? 0 : seg[k - 1]) + base + rank] = (int)i;
-  }
+  const unsigned grp = __match_any_sync(0xffffffffu, k);
+  const int leader = __ffs(grp) - 1, rank = __popc(grp & ((1u << lane) - 1u));
+  int base = 0;
+  if (lane == leader && k != kNoKey) base = atomicAdd(&fill[k], __popc(grp));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (k != kNoKey) perm[(k == 0 ? 0 : seg[k - 1]) + base + rank] = (int)i;
 }
 
 // Ascending order of perm inside each key's segment: segments of up to
