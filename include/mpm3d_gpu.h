@@ -235,8 +235,8 @@ enum mpm_batch_option {
   MPM_BATCH_NODE_BLOCK = 2,
   MPM_BATCH_SCATTER_BLOCKS = 3, /* grid cap of the particle -> grid transfers, blocks per SM (1..64) */
   MPM_BATCH_LOOP_MIN_STEPS = 4, /* steps a device loop takes before it honours mpm_batch_interrupt (0) */
-  MPM_BATCH_SORT_POLLS = 5      /* polls (about 0.7 us each) after which a wait inside the re-sort gives up
-                                   (0: a few seconds, more for more particles) */
+  MPM_BATCH_SORT_POLLS = 5      /* polls (about 0.4 us each) after which a wait inside the re-sort gives up
+                                   (0: 1.6 s, more for more particles) */
 };
 int mpm_batch_set_option(mpm_batch* b, int option, int value);
 int mpm_batch_get_option(const mpm_batch* b, int option);

@@ -184,9 +184,10 @@ struct IntScan {
 // which every block leaves its launch at its next barrier. Returns false then,
 // and the host finds *stall (its own memory, mapped) set.
 // The work between two barriers is linear in the particles and keys (the
-// longest segment included, order_segment), so the limit is too: a fixed part,
-// far above any phase of a small scene, and one poll (0.7 us) for every 64
-// particles, above 10 ns for each of them.
+// longest segment included, order_segment), so the limit is too: a fixed part of
+// 1.6 s (a poll takes 0.38 us), far above any phase of a small scene, and one poll
+// for every 64 particles, 6 ns for each of them (order_segment takes 2 at most,
+// where its network sorts a 64th of a scene).
 constexpr int kBarrierPolls = 1 << 22;
 inline int barrier_polls(long long np) { return np / 64 < INT_MAX - kBarrierPolls ? kBarrierPolls + (int)(np / 64) : INT_MAX; }
 

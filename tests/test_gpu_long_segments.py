@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 FIELDS = ["Xp", "VXp", "SM", "ie"]
 STEPS = 2
-# about 14 ms: the other phases of these sorts take under 1 ms, a bitonic
+# about 8 ms: the other phases of these sorts take under 1 ms, a bitonic
 # network over the long key in global memory 17 ms (216 k particles) to 94 ms (1 M)
 POLLS = 20000
 
